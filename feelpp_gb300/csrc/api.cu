@@ -396,8 +396,7 @@ int fgpu_space_destroy(fgpu_space* V) {
     cudaFree(V->d_inc);
     for (auto& fs : V->face_sets) cudaFree(fs.d_faces);
     cudaFree(V->d_pos);
-    cudaFree(V->d_gptr);
-    cudaFree(V->d_gidx);
+    gather_plan_free(V);
     stream_plan_free(V->stream_plan);
     delete V;
     return FGPU_OK;

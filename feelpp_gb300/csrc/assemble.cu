@@ -74,17 +74,26 @@ DevTables* get_dev_tables(int order, int qdeg, std::string& err) {
                 T7tl[(size_t)k * ntri + t] = T7l[((size_t)k * n + i) * n + j];
             }
         }
-    std::vector<float> Sth((size_t)9 * ntri), Stl((size_t)9 * ntri);
-    for (int i = 0, t = 0; i < n; ++i)
-        for (int j = i; j < n; ++j, ++t)
-            for (int ab = 0; ab < 9; ++ab) {
-                const double v = R.S[((size_t)ab * n + i) * n + j];
-                Sth[(size_t)ab * ntri + t] = (float)v;
-                Stl[(size_t)ab * ntri + t] = (float)(v - (double)(float)v);
-            }
+    // the two-phase element buffer's order
+    const std::vector<uint16_t> pairs = entry_order(4, order, n);
+    std::vector<float> T7bh((size_t)7 * ntri), T7bl((size_t)7 * ntri), Sbh((size_t)9 * ntri), Sbl((size_t)9 * ntri);
+    for (int t = 0; t < ntri; ++t) {
+        const size_t ij = (size_t)(pairs[t] >> 8) * n + (pairs[t] & 255);
+        for (int k = 0; k < 7; ++k) {
+            T7bh[(size_t)k * ntri + t] = T7h[(size_t)k * n * n + ij];
+            T7bl[(size_t)k * ntri + t] = T7l[(size_t)k * n * n + ij];
+        }
+        for (int ab = 0; ab < 9; ++ab) {
+            const double v = R.S[(size_t)ab * n * n + ij];
+            Sbh[(size_t)ab * ntri + t] = (float)v;
+            Sbl[(size_t)ab * ntri + t] = (float)(v - (double)(float)v);
+        }
+    }
     cudaError_t e = cudaSuccess;
-    if (e == cudaSuccess) e = upload(Sth, &D->d_Sth);
-    if (e == cudaSuccess) e = upload(Stl, &D->d_Stl);
+    if (e == cudaSuccess) e = upload(T7bh, &D->d_T7bh);
+    if (e == cudaSuccess) e = upload(T7bl, &D->d_T7bl);
+    if (e == cudaSuccess) e = upload(Sbh, &D->d_Sbh);
+    if (e == cudaSuccess) e = upload(Sbl, &D->d_Sbl);
     if (e == cudaSuccess) e = upload(T7th, &D->d_T7th);
     if (e == cudaSuccess) e = upload(T7tl, &D->d_T7tl);
     if (e == cudaSuccess) e = upload(tri, &D->d_tri);
@@ -1357,63 +1366,6 @@ __global__ void __launch_bounds__(256) batch_element_kernel(int nprob, const Bat
     }
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(256) batch_gather_map_kernel(int nprob, const BatchProblem* __restrict__ probs,
-                                                               const int64_t* __restrict__ nz_off, int64_t total, int accumulate) {
-    int p = -1;
-    int64_t pz0 = 0, pz1 = 0;
-    for (int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; g < total; g += (int64_t)gridDim.x * blockDim.x) {
-        if (g < pz0 || g >= pz1) {
-            p = batch_find(nz_off, nprob, g);
-            pz0 = nz_off[p];
-            pz1 = nz_off[p + 1];
-        }
-        const BatchProblem& P = probs[p];
-        const int64_t k = g - pz0;
-        const uint32_t p0 = __ldg(P.gptr + k), p1 = __ldg(P.gptr + k + 1);
-        if (MODE == kModeDF64) {
-            // the single-matrix gather's compensated sum (same bits)
-            const float2* kb = reinterpret_cast<const float2*>(P.kbuf);
-            float sh = 0.0f, sl = 0.0f;
-            for (uint32_t q = p0; q < p1; q += 4) {
-                uint32_t ix[4];
-                float2 v[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) ix[u] = q + u < p1 ? __ldg(P.gidx + q + u) : 0u;
-#pragma unroll
-                for (int u = 0; u < 4; ++u) v[u] = q + u < p1 ? __ldg(kb + (ix[u] & 0x7FFFFFFFu)) : make_float2(0.0f, 0.0f);
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    if (q + u < p1) {
-                        const df t = two_sum(sh, v[u].x);
-                        sh = t.hi;
-                        sl = f_add(sl, f_add(t.lo, v[u].y));
-                    }
-            }
-            df s = two_sum(sh, sl);
-            double* out = reinterpret_cast<double*>(P.val) + k;
-            if (accumulate) s = df_add(d2df(*out), s);
-            *out = df2d(s);
-        } else {
-            const float* kb = reinterpret_cast<const float*>(P.kbuf);
-            float s = 0.0f;
-            for (uint32_t q = p0; q < p1; q += 4) {
-                uint32_t ix[4];
-                float v[4];
-#pragma unroll
-                for (int u = 0; u < 4; ++u) ix[u] = q + u < p1 ? __ldg(P.gidx + q + u) : 0u;
-#pragma unroll
-                for (int u = 0; u < 4; ++u) v[u] = q + u < p1 ? __ldg(kb + (ix[u] & 0x7FFFFFFFu)) : 0.0f;
-#pragma unroll
-                for (int u = 0; u < 4; ++u)
-                    if (q + u < p1) s = (q + u == p0) ? v[u] : f_add(s, v[u]);
-            }
-            float* out = reinterpret_cast<float*>(P.val) + k;
-            *out = accumulate ? f_add(*out, s) : s;
-        }
-    }
-}
-
 static std::map<int, std::pair<float*, float*>> g_btri;
 static int batch_tri_tables(fgpu_ctx* ctx, float** h, float** l) {
     std::lock_guard<std::mutex> lock(g_btab_mutex);
@@ -1427,8 +1379,8 @@ static int batch_tri_tables(fgpu_ctx* ctx, float** h, float** l) {
         DevTables* t = get_dev_tables(order, 2 * order, err);
         if (!t) { ctx->err = err; return FGPU_ERR_INVALID; }
         const size_t nb = (size_t)7 * (t->n * (t->n + 1) / 2) * sizeof(float);
-        FGPU_CUDA_CHECK(ctx, cudaMemcpy(dh + batch_tri_off(order), t->d_T7th, nb, cudaMemcpyDeviceToDevice));
-        FGPU_CUDA_CHECK(ctx, cudaMemcpy(dl + batch_tri_off(order), t->d_T7tl, nb, cudaMemcpyDeviceToDevice));
+        FGPU_CUDA_CHECK(ctx, cudaMemcpy(dh + batch_tri_off(order), t->d_T7bh, nb, cudaMemcpyDeviceToDevice));
+        FGPU_CUDA_CHECK(ctx, cudaMemcpy(dl + batch_tri_off(order), t->d_T7bl, nb, cudaMemcpyDeviceToDevice));
     }
     g_btri[ctx->device] = {dh, dl};
     *h = dh;
@@ -1437,7 +1389,7 @@ static int batch_tri_tables(fgpu_ctx* ctx, float** h, float** l) {
 }
 
 int launch_batch_two_phase(fgpu_ctx* ctx, int nprob, const BatchProblem* d_probs, const int64_t* d_grp_off,
-                           int64_t total_groups, const int64_t* d_nz_off, int64_t total_nnz, int f32, int threads,
+                           int64_t total_groups, const int64_t* d_slice_off, int64_t total_slices, int f32, int threads,
                            int accumulate) {
     float *Th = nullptr, *Tl = nullptr;
     int rc = batch_tri_tables(ctx, &Th, &Tl);
@@ -1457,14 +1409,7 @@ int launch_batch_two_phase(fgpu_ctx* ctx, int nprob, const BatchProblem* d_probs
         prof_end(ctx, ev);
         FGPU_CUDA_CHECK(ctx, cudaGetLastError());
     }
-    const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((total_nnz + threads - 1) / threads, (int64_t)sms * (2048 / threads) * 4));
-    PendingEvent ev;
-    prof_begin(ctx, "batch_gather", ev);
-    if (f32) batch_gather_map_kernel<kModeF32><<<(int)blocks, threads, 0, ctx->stream>>>(nprob, d_probs, d_nz_off, total_nnz, accumulate);
-    else batch_gather_map_kernel<kModeDF64><<<(int)blocks, threads, 0, ctx->stream>>>(nprob, d_probs, d_nz_off, total_nnz, accumulate);
-    prof_end(ctx, ev);
-    FGPU_CUDA_CHECK(ctx, cudaGetLastError());
-    return FGPU_OK;
+    return launch_batch_gather_slices(ctx, nprob, d_probs, d_slice_off, total_slices, f32, threads, accumulate);
 }
 
 int launch_batch_gather(fgpu_ctx* ctx, int nprob, const BatchProblem* d_probs, const int64_t* d_row_off, int64_t total_rows,
@@ -1500,13 +1445,11 @@ int launch_batch_gather(fgpu_ctx* ctx, int nprob, const BatchProblem* d_probs, c
 //   exactly symmetric), into a device buffer; each warp forms the coefficient
 //   records of 32 elements (one per lane, in shared memory), then their
 //   matrices with lanes over entries, contiguous writes.
-//   Phase 2 (gather_map_kernel): one thread per CSR entry sums its
-//   contributions in element order through a gather map built once per space
-//   (gptr: nnz + 1 offsets, gidx: buffer index of each contribution), which is
-//   the order in which the reference's element loop adds element blocks into
-//   the matrix (bilinearformcontext.hpp:784-847 -> MatSetValues ADD_VALUES).
-//   No float atomics; the gather is a streaming pass over gptr, gidx and the
-//   CSR values.
+//   Phase 2 (gather.cu): one lane per pair of dofs sums its contributions in
+//   element order through a gather map built once per space, which is the
+//   order in which the reference's element loop adds element blocks into the
+//   matrix (bilinearformcontext.hpp:784-847 -> MatSetValues ADD_VALUES).
+//   No float atomics.
 // ---------------------------------------------------------------------------
 template <int MODE, int N>
 __global__ void __launch_bounds__(256) element_tri_kernel(int64_t nt, GeoIn geo, const float* __restrict__ Thg,
@@ -1539,310 +1482,11 @@ __global__ void __launch_bounds__(256) element_tri_kernel(int64_t nt, GeoIn geo,
     }
 }
 
-// One thread per CSR entry, its contributions in batches of B (the index and
-// value loads of a batch are issued together; the sum stays in element
-// order, so B, like the launch shape, does not change the result; the tuner
-// picks it). Measured against three alternatives at P2 48^3 (this: 0.32 ms):
-// entries sorted by contribution count within 256-entry windows (0.50 ms: the
-// permuted writes lose their coalescing); a warp-flat load of the 32 entries'
-// contributions staged in shared memory (0.39 ms: fewer loads in flight per
-// warp); a split into entries with at most 2 contributions (one unrolled step,
-// 0.21 ms, 70 % of DRAM peak) and the others taken from a list sorted by count
-// (0.30 ms: the sorted list scatters the reads of the element buffer, 1.75 GB
-// of DRAM reads for 5.4 M entries). At P2 64^3 two entries per thread (k and
-// k + stride, loads issued together) took 0.90 ms against 0.655 ms. A symmetric
-// map (entries j >= i only, each thread also storing its value at the transpose's
-// position) halves the map and the buffer reads on paper but took 0.785 ms
-// against 0.64 ms: at 48^3 its DRAM reads stayed at 888 MB (the transposes'
-// second reads of the buffer hit L2 here), with more warp instructions (half the
-// lanes idle) and scattered stores. One batch of 6 per entry with the entries of
-// more than 6 contributions (the vertex-row diagonals, 0.5 % of the entries) left
-// to a second kernel over their list: timed by the tuner against B = 2, 4, 8 and
-// never picked at P2 or P3 64^3 (the warps' longest entries are not what bounds
-// the kernel). L2 eviction hints (map and values evict-first, element buffer
-// evict-last) raised the DRAM reads at P2 48^3 from 900 to 1010 MB and the time
-// from 0.275 to 0.295 ms. The grid matters for the reads: with more blocks than
-// fit at once, each wave of resident blocks strides over the whole matrix and an
-// entry and its transpose are read in different waves (900 MB); one entry per
-// thread sweeps the entries in order and reads exactly the design bytes (660 MB)
-// but took 0.30 ms: the kernel is bound by issue and by the latency of its three
-// dependent loads, not by DRAM.
-template <int MODE, int B = 4>
-__global__ void __launch_bounds__(256) gather_map_kernel(int64_t nnz, const uint32_t* __restrict__ gptr,
-                                                         const uint32_t* __restrict__ gidx, const void* __restrict__ kbuf,
-                                                         void* __restrict__ valv, int accumulate, double* __restrict__ hout) {
-    // hout (binary64 results only): a mapped page-locked host buffer that receives a copy of each value
-    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < nnz; k += (int64_t)gridDim.x * blockDim.x) {
-        const uint32_t p0 = __ldg(gptr + k), p1 = __ldg(gptr + k + 1);
-        if (MODE == kModeDF64) {
-            // compensated sum in element order: the high parts through TwoSum, their rounding errors and
-            // the low parts in one binary32 accumulator, normalised once (error ~ (count) u^2 |sum|)
-            const float2* kb = reinterpret_cast<const float2*>(kbuf);
-            float sh = 0.0f, sl = 0.0f;
-            for (uint32_t p = p0; p < p1; p += B) {
-                uint32_t ix[B];
-                float2 v[B];
-#pragma unroll
-                for (int u = 0; u < B; ++u) ix[u] = p + u < p1 ? __ldg(gidx + p + u) : 0u;
-#pragma unroll
-                for (int u = 0; u < B; ++u) v[u] = p + u < p1 ? __ldg(kb + (ix[u] & 0x7FFFFFFFu)) : make_float2(0.0f, 0.0f);
-#pragma unroll
-                for (int u = 0; u < B; ++u)
-                    if (p + u < p1) {
-                        const df t = two_sum(sh, v[u].x);
-                        sh = t.hi;
-                        sl = f_add(sl, f_add(t.lo, v[u].y));
-                    }
-            }
-            df s = two_sum(sh, sl);
-            double* out = reinterpret_cast<double*>(valv) + k;
-            if (accumulate) s = df_add(d2df(*out), s);
-            const double r = df2d(s);
-            *out = r;
-            if (hout) hout[k] = r;
-        } else {
-            const float* kb = reinterpret_cast<const float*>(kbuf);
-            float s = 0.0f;
-            for (uint32_t p = p0; p < p1; p += B) {
-                uint32_t ix[B];
-                float v[B];
-#pragma unroll
-                for (int u = 0; u < B; ++u) ix[u] = p + u < p1 ? __ldg(gidx + p + u) : 0u;
-#pragma unroll
-                for (int u = 0; u < B; ++u) v[u] = p + u < p1 ? __ldg(kb + (ix[u] & 0x7FFFFFFFu)) : 0.0f;
-#pragma unroll
-                for (int u = 0; u < B; ++u)
-                    if (p + u < p1) s = (p + u == p0) ? v[u] : f_add(s, v[u]);
-            }
-            float* out = reinterpret_cast<float*>(valv) + k;
-            *out = accumulate ? f_add(*out, s) : s;
-        }
-    }
-}
-
-// The same gather software-pipelined over a thread's grid-stride entries. One entry costs three
-// dependent loads (its gptr range, then its gidx indices, then the element-buffer values), so the
-// plain kernel keeps one round trip of DRAM latency per load level in flight per thread. Here
-// iteration i issues the element-buffer loads of entry k (indices already in registers), the gidx
-// loads of entry k + S and the gptr loads of entry k + 2S together, then sums entry k: one latency
-// per entry instead of three. Entries with more than B contributions load their further batches
-// in place. The sum of every entry is the same sequence of operations as in gather_map_kernel, so
-// the values are the same bits. Measured at 64^3 (tuned shapes): binary32 P3 1.87 against 2.12 ms,
-// P2 0.43 against 0.46 ms; df64 P2 0.66 against 0.64 ms (more registers, and the three entries in
-// flight widen the window of element-buffer lines: 880 against 803 MB of DRAM reads at 48^3). The
-// tuner times both.
-template <int MODE, int B = 4>
-__global__ void __launch_bounds__(256) gather_map_pipe_kernel(int64_t nnz, const uint32_t* __restrict__ gptr,
-                                                              const uint32_t* __restrict__ gidx, const void* __restrict__ kbuf,
-                                                              void* __restrict__ valv, int accumulate, double* __restrict__ hout) {
-    const int64_t S = (int64_t)gridDim.x * blockDim.x;
-    int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (k >= nnz) return;
-    uint32_t a0 = __ldg(gptr + k), a1 = __ldg(gptr + k + 1);          // entry k
-    int64_t kn = k + S;
-    uint32_t b0 = 0, b1 = 0;                                            // entry k + S
-    if (kn < nnz) {
-        b0 = __ldg(gptr + kn);
-        b1 = __ldg(gptr + kn + 1);
-    }
-    uint32_t ix[B];
-#pragma unroll
-    for (int u = 0; u < B; ++u) ix[u] = a0 + u < a1 ? __ldg(gidx + a0 + u) : 0u;
-    for (;;) {
-        // loads of three entries in flight together
-        uint32_t nx[B];
-        uint32_t c0 = 0, c1 = 0;
-        const int64_t knn = kn + S;
-        if (MODE == kModeDF64) {
-            const float2* kb = reinterpret_cast<const float2*>(kbuf);
-            float2 v[B];
-#pragma unroll
-            for (int u = 0; u < B; ++u) v[u] = a0 + u < a1 ? __ldg(kb + (ix[u] & 0x7FFFFFFFu)) : make_float2(0.0f, 0.0f);
-#pragma unroll
-            for (int u = 0; u < B; ++u) nx[u] = b0 + u < b1 ? __ldg(gidx + b0 + u) : 0u;
-            if (knn < nnz) {
-                c0 = __ldg(gptr + knn);
-                c1 = __ldg(gptr + knn + 1);
-            }
-            float sh = 0.0f, sl = 0.0f;
-#pragma unroll
-            for (int u = 0; u < B; ++u)
-                if (a0 + u < a1) {
-                    const df t = two_sum(sh, v[u].x);
-                    sh = t.hi;
-                    sl = f_add(sl, f_add(t.lo, v[u].y));
-                }
-            for (uint32_t p = a0 + B; p < a1; p += B) {
-                uint32_t jx[B];
-                float2 w[B];
-#pragma unroll
-                for (int u = 0; u < B; ++u) jx[u] = p + u < a1 ? __ldg(gidx + p + u) : 0u;
-#pragma unroll
-                for (int u = 0; u < B; ++u) w[u] = p + u < a1 ? __ldg(kb + (jx[u] & 0x7FFFFFFFu)) : make_float2(0.0f, 0.0f);
-#pragma unroll
-                for (int u = 0; u < B; ++u)
-                    if (p + u < a1) {
-                        const df t = two_sum(sh, w[u].x);
-                        sh = t.hi;
-                        sl = f_add(sl, f_add(t.lo, w[u].y));
-                    }
-            }
-            df sum = two_sum(sh, sl);
-            double* out = reinterpret_cast<double*>(valv) + k;
-            if (accumulate) sum = df_add(d2df(*out), sum);
-            const double r = df2d(sum);
-            *out = r;
-            if (hout) hout[k] = r;
-        } else {
-            const float* kb = reinterpret_cast<const float*>(kbuf);
-            float v[B];
-#pragma unroll
-            for (int u = 0; u < B; ++u) v[u] = a0 + u < a1 ? __ldg(kb + (ix[u] & 0x7FFFFFFFu)) : 0.0f;
-#pragma unroll
-            for (int u = 0; u < B; ++u) nx[u] = b0 + u < b1 ? __ldg(gidx + b0 + u) : 0u;
-            if (knn < nnz) {
-                c0 = __ldg(gptr + knn);
-                c1 = __ldg(gptr + knn + 1);
-            }
-            float sum = 0.0f;
-#pragma unroll
-            for (int u = 0; u < B; ++u)
-                if (a0 + u < a1) sum = (u == 0) ? v[u] : f_add(sum, v[u]);
-            for (uint32_t p = a0 + B; p < a1; p += B) {
-                uint32_t jx[B];
-                float w[B];
-#pragma unroll
-                for (int u = 0; u < B; ++u) jx[u] = p + u < a1 ? __ldg(gidx + p + u) : 0u;
-#pragma unroll
-                for (int u = 0; u < B; ++u) w[u] = p + u < a1 ? __ldg(kb + (jx[u] & 0x7FFFFFFFu)) : 0.0f;
-#pragma unroll
-                for (int u = 0; u < B; ++u)
-                    if (p + u < a1) sum = f_add(sum, w[u]);
-            }
-            float* out = reinterpret_cast<float*>(valv) + k;
-            *out = accumulate ? f_add(*out, sum) : sum;
-        }
-        if (kn >= nnz) break;
-        k = kn;
-        kn = knn;
-        a0 = b0;
-        a1 = b1;
-        b0 = c0;
-        b1 = c1;
-#pragma unroll
-        for (int u = 0; u < B; ++u) ix[u] = nx[u];
-    }
-}
-
-// ---- gather map construction (once per space) ----
-// contributions per CSR entry (integer atomics: the counts do not depend on order)
-__global__ void map_count_kernel(int64_t nt, int n, const int32_t* __restrict__ l2n, const int64_t* __restrict__ ia,
-                                 const uint8_t* __restrict__ pos, uint32_t* __restrict__ cnt) {
-    const int64_t total = nt * n * n;
-    for (int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; t < total; t += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t e = t / (n * n);
-        const int i = (int)((t - e * n * n) / n);
-        atomicAdd(cnt + ia[l2n[e * n + i]] + pos[t], 1u);
-    }
-}
-
-// fill: one warp per row, incident elements in element order, lanes over the
-// element row's columns (distinct entries), a per-entry cursor in shared memory
-__global__ void __launch_bounds__(256) map_fill_kernel(int64_t nrows, int n, int ntri, const int64_t* __restrict__ ia,
-                                                       const int64_t* __restrict__ inc_ptr, const int32_t* __restrict__ inc,
-                                                       const uint8_t* __restrict__ pos, const uint16_t* __restrict__ trig,
-                                                       const uint32_t* __restrict__ gptr, uint32_t* __restrict__ gidx,
-                                                       int* __restrict__ status) {
-    __shared__ uint32_t cur[8][256];
-    __shared__ uint16_t tri[32 * 32];   // n <= 32 (checked by the launcher)
-    for (int k = threadIdx.x; k < n * n; k += blockDim.x) tri[k] = trig[k];
-    __syncthreads();
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    for (int64_t r = (int64_t)blockIdx.x * 8 + warp; r < nrows; r += (int64_t)gridDim.x * 8) {
-        const int64_t start = ia[r];
-        const int len = (int)(ia[r + 1] - start);
-        if (len > 256) {
-            if (lane == 0) atomicOr(status, kStatusRowOverflow);
-            continue;
-        }
-        for (int k = lane; k < len; k += 32) cur[warp][k] = gptr[start + k];
-        __syncwarp();
-        for (int64_t t = inc_ptr[r]; t < inc_ptr[r + 1]; ++t) {
-            const int32_t code = inc[t];
-            const int64_t e = code >> 5;
-            const int li = code & 31;
-            if (lane < n) {
-                const int p = pos[(e * n + li) * n + lane];
-                const uint32_t slot = cur[warp][p];
-                cur[warp][p] = slot + 1;
-                // bit 31: the contribution is K_e(li, lj) with li > lj, stored as (lj, li)
-                gidx[slot] = (uint32_t)(e * ntri + tri[li * n + lane]) | (li > lane ? 0x80000000u : 0u);
-            }
-            __syncwarp();
-        }
-    }
-}
-
-int launch_build_gather_map(fgpu_ctx* ctx, fgpu_space* V) {
-    if (V->d_gptr) return FGPU_OK;
-    const DevPattern& P = *V->pattern;
-    const int n = V->n;
-    const int64_t nt = V->mesh->nt, nnz = P.nnz;
-    const int64_t contrib = nt * n * n;
-    if (contrib >= (int64_t)UINT32_MAX || nt * (int64_t)(n * (n + 1) / 2) >= ((int64_t)1 << 31)) {
-        ctx->err = "gather map: more than 2^32 contributions or 2^31 buffered entries";
-        return FGPU_ERR_INVALID;
-    }
-    if (!V->d_pos) { ctx->err = "gather map: no position table"; return FGPU_ERR_INVALID; }
-    if (n > 32) { ctx->err = "gather map: more than 32 local dofs"; return FGPU_ERR_INVALID; }
-    // upper-triangle index of (min(i,j), max(i,j)) in the element buffer's row-major (i <= j) order
-    std::vector<uint16_t> htri((size_t)n * n);
-    for (int i = 0; i < n; ++i)
-        for (int j = 0; j < n; ++j) {
-            const int a = std::min(i, j), b = std::max(i, j);
-            htri[(size_t)i * n + j] = (uint16_t)(a * n - a * (a - 1) / 2 + (b - a));
-        }
-    uint16_t* d_tri = nullptr;
-    uint32_t *cnt = nullptr, *gptr = nullptr, *gidx = nullptr;
-    cudaError_t e = cudaMalloc(&d_tri, htri.size() * sizeof(uint16_t));
-    if (e == cudaSuccess) e = cudaMemcpyAsync(d_tri, htri.data(), htri.size() * sizeof(uint16_t), cudaMemcpyHostToDevice, ctx->stream);
-    if (e == cudaSuccess) e = cudaMalloc(&cnt, nnz * sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&gptr, (nnz + 1) * sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&gidx, contrib * sizeof(uint32_t));
-    if (e != cudaSuccess) {
-        cudaGetLastError();
-        cudaFree(d_tri); cudaFree(cnt); cudaFree(gptr); cudaFree(gidx);
-        ctx->err = "gather map: allocation failed";
-        return FGPU_ERR_ALLOC;
-    }
-    int sms = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
-    cudaMemsetAsync(cnt, 0, nnz * sizeof(uint32_t), ctx->stream);
-    map_count_kernel<<<sms * 16, 256, 0, ctx->stream>>>(nt, n, V->d_l2n, P.d_ia, V->d_pos, cnt);
-    uint64_t total = 0;
-    int rcs = scan_u32(ctx, cnt, gptr, nnz, &total);
-    if (rcs) { cudaFree(d_tri); cudaFree(cnt); cudaFree(gptr); cudaFree(gidx); return rcs; }
-    map_fill_kernel<<<sms * 8, 256, 0, ctx->stream>>>(P.nrows, n, n * (n + 1) / 2, P.d_ia, V->d_inc_ptr, V->d_inc, V->d_pos,
-                                                      d_tri, gptr, gidx, ctx->d_status);
-    ctx->launches += 2;
-    e = cudaGetLastError();
-    cudaStreamSynchronize(ctx->stream);
-    cudaFree(cnt);
-    cudaFree(d_tri);
-    if (e != cudaSuccess) {
-        cudaFree(gptr); cudaFree(gidx);
-        ctx->err = std::string("gather map: ") + cudaGetErrorString(e);
-        return FGPU_ERR_CUDA;
-    }
-    V->d_gptr = gptr;
-    V->d_gidx = gidx;
-    return FGPU_OK;
-}
-
 // Launch shape of the two-phase kernels: threads per block and blocks per SM of the element kernel
-// and of the gather, and the gather's contributions per load batch. None changes the values.
+// and of the gather (64: one warp per slice), the gather's contributions per load batch and whether
+// its next indices are loaded ahead. None changes the values.
 struct TwoPhaseShape {
-    int el_threads = 256, el_bpsm = 16, g_threads = 256, g_bpsm = 32, g_batch = 4, g_pipe = 0;
+    int el_threads = 256, el_bpsm = 16, g_threads = 256, g_bpsm = 64, g_batch = 4, g_pipe = 0;
 };
 
 template <int MODE, int N>
@@ -1851,28 +1495,12 @@ static void launch_element_tri(fgpu_ctx* ctx, fgpu_matrix* A, const DevTables* t
     const int64_t nt = A->space->mesh->nt;
     const int64_t warps = (nt + 31) / 32, wpb = sh.el_threads / 32;       // 32 elements per warp
     const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((warps + wpb - 1) / wpb, (int64_t)sms * sh.el_bpsm));
-    element_tri_kernel<MODE, N><<<(int)blocks, sh.el_threads, 0, ctx->stream>>>(nt, *geo, tab->d_T7th, tab->d_T7tl, A->d_kbuf,
+    element_tri_kernel<MODE, N><<<(int)blocks, sh.el_threads, 0, ctx->stream>>>(nt, *geo, tab->d_T7bh, tab->d_T7bl, A->d_kbuf,
                                                                              ctx->d_status);
 }
 
-template <int MODE>
-static void launch_gather_map(fgpu_ctx* ctx, fgpu_matrix* A, int sms, const TwoPhaseShape& sh, int accumulate, double* hout) {
-    const fgpu_space* V = A->space;
-    const int64_t nnz = A->pattern->nnz;
-    const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((nnz + sh.g_threads - 1) / sh.g_threads, (int64_t)sms * sh.g_bpsm));
-    if (sh.g_pipe) {
-        switch (sh.g_batch) {
-            case 2: gather_map_pipe_kernel<MODE, 2><<<(int)blocks, sh.g_threads, 0, ctx->stream>>>(nnz, V->d_gptr, V->d_gidx, A->d_kbuf, A->d_val, accumulate, hout); break;
-            case 8: gather_map_pipe_kernel<MODE, 8><<<(int)blocks, sh.g_threads, 0, ctx->stream>>>(nnz, V->d_gptr, V->d_gidx, A->d_kbuf, A->d_val, accumulate, hout); break;
-            default: gather_map_pipe_kernel<MODE, 4><<<(int)blocks, sh.g_threads, 0, ctx->stream>>>(nnz, V->d_gptr, V->d_gidx, A->d_kbuf, A->d_val, accumulate, hout); break;
-        }
-        return;
-    }
-    switch (sh.g_batch) {
-        case 2: gather_map_kernel<MODE, 2><<<(int)blocks, sh.g_threads, 0, ctx->stream>>>(nnz, V->d_gptr, V->d_gidx, A->d_kbuf, A->d_val, accumulate, hout); break;
-        case 8: gather_map_kernel<MODE, 8><<<(int)blocks, sh.g_threads, 0, ctx->stream>>>(nnz, V->d_gptr, V->d_gidx, A->d_kbuf, A->d_val, accumulate, hout); break;
-        default: gather_map_kernel<MODE, 4><<<(int)blocks, sh.g_threads, 0, ctx->stream>>>(nnz, V->d_gptr, V->d_gidx, A->d_kbuf, A->d_val, accumulate, hout); break;
-    }
+static void launch_gather_map(fgpu_ctx* ctx, fgpu_matrix* A, const TwoPhaseShape& sh, int accumulate) {
+    launch_gather_slices(ctx, A, sh.g_threads, sh.g_bpsm >= 64 ? 0 : sh.g_bpsm, sh.g_batch, sh.g_pipe, accumulate);
 }
 
 // median of 5 timed launches (after one warm-up) of fn on the context's stream, in ms
@@ -1912,25 +1540,24 @@ static int tune_two_phase(fgpu_ctx* ctx, fgpu_matrix* A, const DevTables* tab, c
         }
     best_ms = 1e30f;
     for (int th : {128, 256})
-        for (int bp : {8, 16, 32, 64})
+        for (int bp : {8 * (256 / th), 64})        // a sweep by the resident blocks, or one warp per slice
             for (int b : {2, 4, 8}) {
                 s.g_threads = th;
                 s.g_bpsm = bp;
                 s.g_batch = b;
-                const float ms = median_ms(ctx, [&] { launch_gather_map<MODE>(ctx, A, sms, s, 0, nullptr); });
+                const float ms = median_ms(ctx, [&] { launch_gather_map(ctx, A, s, 0); });
                 if (ms < best_ms) { best_ms = ms; best.g_threads = th; best.g_bpsm = bp; best.g_batch = b; }
             }
-    // the software-pipelined gather, its grid at most the resident blocks (a sweep over the entries)
+    // indices loaded ahead: shorter chains, for matrices that do not fill the device
+    s.g_pipe = 1;
     for (int th : {128, 256})
-        for (int bp : {2, 4, 6, 8})
-            for (int b : {2, 4}) {
-                s.g_threads = th;
-                s.g_bpsm = bp * (256 / th);
-                s.g_batch = b;
-                s.g_pipe = 1;
-                const float ms = median_ms(ctx, [&] { launch_gather_map<MODE>(ctx, A, sms, s, 0, nullptr); });
-                if (ms < best_ms) { best_ms = ms; best.g_threads = th; best.g_bpsm = s.g_bpsm; best.g_batch = b; best.g_pipe = 1; }
-            }
+        for (int b : {4, 8}) {
+            s.g_threads = th;
+            s.g_bpsm = 8 * (256 / th);
+            s.g_batch = b;
+            const float ms = median_ms(ctx, [&] { launch_gather_map(ctx, A, s, 0); });
+            if (ms < best_ms) { best_ms = ms; best.g_threads = th; best.g_bpsm = s.g_bpsm; best.g_batch = b; best.g_pipe = 1; }
+        }
     FGPU_CUDA_CHECK(ctx, cudaGetLastError());
     return FGPU_OK;
 }
@@ -1948,7 +1575,7 @@ static int run_two_phase(fgpu_ctx* ctx, fgpu_matrix* A, const DevTables* tab, co
         if (rc) return rc;
         rec = reinterpret_cast<const float4*>(A->d_coef);
     }
-    if (!V->d_gptr) {
+    if (!gather_plan_ready(V)) {
         if (ctx->capturing) { ctx->err = "two-phase assembly: assemble once before capturing (gather map)"; return FGPU_ERR_INVALID; }
         int rc = launch_build_gather_map(ctx, V);
         if (rc) return rc;
@@ -1981,7 +1608,7 @@ static int run_two_phase(fgpu_ctx* ctx, fgpu_matrix* A, const DevTables* tab, co
         prof_begin(ctx, "assemble_elements", ev);
         if (tc) {
             // the df64 element matrices on the tensor cores (bf16 slices, exact level sums)
-            const int rc = launch_element_tri_tc(ctx, V->order, nt, rec, tab->d_T7th, tab->d_T7tl, A->d_kbuf);
+            const int rc = launch_element_tri_tc(ctx, V->order, nt, rec, tab->d_T7bh, tab->d_T7bl, A->d_kbuf);
             if (rc) return rc;
         } else {
             launch_element_tri<MODE, N>(ctx, A, tab, geo, sms, shape);
@@ -1992,7 +1619,7 @@ static int run_two_phase(fgpu_ctx* ctx, fgpu_matrix* A, const DevTables* tab, co
     if (host) return launch_gather_phase_to_host(ctx, A, host, 4);
     PendingEvent ev;
     prof_begin(ctx, "assemble_gather", ev);
-    launch_gather_map<MODE>(ctx, A, sms, shape, accumulate, nullptr);
+    launch_gather_map(ctx, A, shape, accumulate);
     prof_end(ctx, ev);
     FGPU_CUDA_CHECK(ctx, cudaGetLastError());
     return FGPU_OK;
@@ -2002,7 +1629,7 @@ static int run_two_phase(fgpu_ctx* ctx, fgpu_matrix* A, const DevTables* tab, co
 // element buffer of at least `need` bytes, then phase 2 for the matrix's precision.
 int ensure_two_phase(fgpu_ctx* ctx, fgpu_matrix* A, size_t need) {
     fgpu_space* V = A->space;
-    if (!V->d_gptr) {
+    if (!gather_plan_ready(V)) {
         if (ctx->capturing) { ctx->err = "two-phase assembly: assemble once before capturing (gather map)"; return FGPU_ERR_INVALID; }
         int rc = launch_build_gather_map(ctx, V);
         if (rc) return rc;
@@ -2015,86 +1642,6 @@ int ensure_two_phase(fgpu_ctx* ctx, fgpu_matrix* A, size_t need) {
         if (cudaMalloc(&A->d_kbuf, need) != cudaSuccess) { cudaGetLastError(); ctx->err = "two-phase assembly: element buffer allocation failed"; return FGPU_ERR_ALLOC; }
         A->kbuf_bytes = need;
     }
-    return FGPU_OK;
-}
-
-int launch_gather_phase(fgpu_ctx* ctx, fgpu_matrix* A, int accumulate) {
-    fgpu_space* V = A->space;
-    int sms = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
-    const int64_t nnz = A->pattern->nnz;
-    const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((nnz + 255) / 256, (int64_t)sms * 32));
-    PendingEvent ev;
-    prof_begin(ctx, "assemble_gather", ev);
-    if (A->precision == FGPU_F32)
-        gather_map_kernel<kModeF32><<<(int)blocks, 256, 0, ctx->stream>>>(nnz, V->d_gptr, V->d_gidx, A->d_kbuf, A->d_val, accumulate, nullptr);
-    else
-        gather_map_kernel<kModeDF64><<<(int)blocks, 256, 0, ctx->stream>>>(nnz, V->d_gptr, V->d_gidx, A->d_kbuf, A->d_val, accumulate, nullptr);
-    prof_end(ctx, ev);
-    FGPU_CUDA_CHECK(ctx, cudaGetLastError());
-    return FGPU_OK;
-}
-
-// Phase 2 in nchunks ranges of CSR entries, each range copied to host memory (pinned for overlap) on
-// its own copy stream as soon as its gather ends: the copies of earlier ranges overlap the gathers of
-// later ones. FP64 matrices.
-int launch_gather_phase_to_host(fgpu_ctx* ctx, fgpu_matrix* A, double* host, int nchunks) {
-    fgpu_space* V = A->space;
-    int sms = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
-    const int64_t nnz = A->pattern->nnz;
-    nchunks = std::max(1, std::min(nchunks, 4));
-    if (!ctx->copy_streams[0]) {
-        for (int i = 0; i < 4; ++i) FGPU_CUDA_CHECK(ctx, cudaStreamCreateWithFlags(&ctx->copy_streams[i], cudaStreamNonBlocking));
-        for (int i = 0; i < 5; ++i) FGPU_CUDA_CHECK(ctx, cudaEventCreateWithFlags(&ctx->copy_events[i], cudaEventDisableTiming));
-    }
-    // direct stores: the gather writes every value to device memory and to the mapped host buffer.
-    // (Element kernel and gather in eight ranges each, a range of entries gathered on a side stream
-    // once the element ranges it reads were done, measured slower: 16.4 against 19.2 Gnnz/s end to
-    // end at P2 64^3; so was a variant with the elements ordered by the first of four row chunks that
-    // reads them: 16.8-16.9 against 19.7 Gnnz/s, with a gather grid of 4 or 32 blocks per SM.)
-    double* hdev = nullptr;
-    if (ctx->host_transfer != FGPU_HOST_TRANSFER_COPY) {
-        cudaPointerAttributes pa{};
-        if (cudaPointerGetAttributes(&pa, host) == cudaSuccess && pa.type == cudaMemoryTypeHost && pa.devicePointer)
-            hdev = static_cast<double*>(pa.devicePointer);
-        else
-            cudaGetLastError();
-        if (!hdev && ctx->host_transfer == FGPU_HOST_TRANSFER_DIRECT) {
-            ctx->err = "direct host transfer: the host buffer is not page-locked and mapped";
-            return FGPU_ERR_INVALID;
-        }
-    }
-    if (hdev) {
-        const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((nnz + 255) / 256, (int64_t)sms * 32));
-        PendingEvent ev;
-        prof_begin(ctx, "assemble_gather", ev);
-        gather_map_kernel<kModeDF64><<<(int)blocks, 256, 0, ctx->stream>>>(nnz, V->d_gptr, V->d_gidx, A->d_kbuf, A->d_val, 0, hdev);
-        prof_end(ctx, ev);
-        ctx->launches++;
-        FGPU_CUDA_CHECK(ctx, cudaGetLastError());
-        FGPU_CUDA_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
-        return FGPU_OK;
-    }
-    const int64_t chunk = ((nnz + nchunks - 1) / nchunks + 255) & ~(int64_t)255;
-    PendingEvent ev;
-    prof_begin(ctx, "assemble_gather", ev);
-    for (int c = 0; c < nchunks; ++c) {
-        const int64_t k0 = (int64_t)c * chunk;
-        if (k0 >= nnz) break;
-        const int64_t k1 = std::min(nnz, k0 + chunk);
-        const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((k1 - k0 + 255) / 256, (int64_t)sms * 32));
-        gather_map_kernel<kModeDF64><<<(int)blocks, 256, 0, ctx->stream>>>(k1 - k0, V->d_gptr + k0, V->d_gidx, A->d_kbuf,
-                                                                         (double*)A->d_val + k0, 0, nullptr);
-        ctx->launches++;
-        FGPU_CUDA_CHECK(ctx, cudaGetLastError());
-        FGPU_CUDA_CHECK(ctx, cudaEventRecord(ctx->copy_events[c], ctx->stream));
-        FGPU_CUDA_CHECK(ctx, cudaStreamWaitEvent(ctx->copy_streams[c], ctx->copy_events[c], 0));
-        FGPU_CUDA_CHECK(ctx, cudaMemcpyAsync(host + k0, (const double*)A->d_val + k0, (k1 - k0) * sizeof(double),
-                                             cudaMemcpyDeviceToHost, ctx->copy_streams[c]));
-    }
-    prof_end(ctx, ev);
-    for (int c = 0; c < nchunks; ++c) FGPU_CUDA_CHECK(ctx, cudaStreamSynchronize(ctx->copy_streams[c]));
     return FGPU_OK;
 }
 
@@ -2142,10 +1689,10 @@ int launch_assemble_two_phase(fgpu_ctx* ctx, fgpu_matrix* A, const DevTables* ta
 //   lambda J Y_cd + mu J Y_dc + delta_cd mu J tr(Y).
 // Records: 24 floats per element: hi parts of (B_00..B_22, lambda J, mu J, 0), then lo parts.
 // Phase 1 stores the blocks of the pairs i <= j (n(n+1)/2 x 9 values per element);
-// phase 2, one warp per scalar pattern row, lanes over its entries, sums the 9
-// entries of each node pair over the contributions of the gather map in element
-// order (a contribution with li > lj reads its block transposed) and writes them
-// into the expanded CSR (row 3m+c, columns 3n'+d).
+// phase 2 (gather.cu), one lane per node pair, sums the 9 entries over the
+// contributions of the gather map in element order (a contribution with li > lj
+// reads its block transposed) and writes them and their transpose into the
+// expanded CSR (row 3m+c, columns 3n'+d).
 // ---------------------------------------------------------------------------
 __global__ void geometry_el_df_kernel(int64_t nt, const double* __restrict__ xyz, const int32_t* __restrict__ tets, double lam,
                                       double mu, float4* __restrict__ rec, int* __restrict__ status) {
@@ -2302,67 +1849,12 @@ __global__ void __launch_bounds__(128) element_el_kernel(int64_t nt, const float
     }
 }
 
-template <int MODE>
-__global__ void __launch_bounds__(256) gather_el_kernel(int64_t nrows, const int64_t* __restrict__ sia, const uint32_t* __restrict__ gptr,
-                                                        const uint32_t* __restrict__ gidx, const void* __restrict__ kbuf,
-                                                        void* __restrict__ valv, int accumulate) {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
-    for (int64_t m = (int64_t)blockIdx.x * (blockDim.x >> 5) + warp; m < nrows; m += nw) {
-        const int64_t s0 = sia[m];
-        const int len = (int)(sia[m + 1] - s0);
-        for (int pos = lane; pos < len; pos += 32) {
-            const int64_t ks = s0 + pos;
-            const uint32_t p0 = __ldg(gptr + ks), p1 = __ldg(gptr + ks + 1);
-            // (a compensated sum per component, as in gather_map_kernel, took 4.71 against 4.25 ms for the
-            // P2 48^3 elasticity assembly: the nine components' two accumulators)
-            df acc[9];
-            float accf[9];
-#pragma unroll
-            for (int k = 0; k < 9; ++k) { acc[k] = df{0.0f, 0.0f}; accf[k] = 0.0f; }
-            for (uint32_t p = p0; p < p1; ++p) {
-                const uint32_t g = __ldg(gidx + p);
-                const bool tr = (g & 0x80000000u) != 0;
-                const int64_t base = (int64_t)(g & 0x7FFFFFFFu) * 9;
-#pragma unroll
-                for (int c = 0; c < 3; ++c)
-#pragma unroll
-                    for (int d = 0; d < 3; ++d) {
-                        const int k = tr ? d * 3 + c : c * 3 + d;
-                        if (MODE == kModeDF64) {
-                            const float2 v = __ldg(reinterpret_cast<const float2*>(kbuf) + base + k);
-                            acc[c * 3 + d] = p == p0 ? df{v.x, v.y} : df_add(acc[c * 3 + d], df{v.x, v.y});
-                        } else {
-                            const float v = __ldg(reinterpret_cast<const float*>(kbuf) + base + k);
-                            accf[c * 3 + d] = p == p0 ? v : f_add(accf[c * 3 + d], v);
-                        }
-                    }
-            }
-#pragma unroll
-            for (int c = 0; c < 3; ++c)
-#pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                    const int64_t o = 9 * s0 + (int64_t)c * 3 * len + 3 * pos + d;
-                    if (MODE == kModeDF64) {
-                        double* out = reinterpret_cast<double*>(valv) + o;
-                        df a = acc[c * 3 + d];
-                        if (accumulate) a = df_add(d2df(*out), a);
-                        *out = df2d(a);
-                    } else {
-                        float* out = reinterpret_cast<float*>(valv) + o;
-                        *out = accumulate ? f_add(*out, accf[c * 3 + d]) : accf[c * 3 + d];
-                    }
-                }
-        }
-    }
-}
-
 template <int MODE, int N>
 static int run_el_two_phase(fgpu_ctx* ctx, fgpu_matrix* A, const DevTables* tab, const float4* rec, int accumulate) {
     fgpu_space* V = A->space;
     const int64_t nt = V->mesh->nt;
     constexpr int NTRI = N * (N + 1) / 2;
-    if (!V->d_gptr) {
+    if (!gather_plan_ready(V)) {
         if (ctx->capturing) { ctx->err = "two-phase assembly: assemble once before capturing (gather map)"; return FGPU_ERR_INVALID; }
         int rc = launch_build_gather_map(ctx, V);
         if (rc) return rc;
@@ -2382,18 +1874,11 @@ static int run_el_two_phase(fgpu_ctx* ctx, fgpu_matrix* A, const DevTables* tab,
         const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((nt + 3) / 4, (int64_t)sms * 16));
         PendingEvent ev;
         prof_begin(ctx, "assemble_elements", ev);
-        element_el_kernel<MODE, N><<<(int)blocks, 128, 0, ctx->stream>>>(nt, rec, tab->d_Sth, tab->d_Stl, A->d_kbuf);
+        element_el_kernel<MODE, N><<<(int)blocks, 128, 0, ctx->stream>>>(nt, rec, tab->d_Sbh, tab->d_Sbl, A->d_kbuf);
         prof_end(ctx, ev);
         FGPU_CUDA_CHECK(ctx, cudaGetLastError());
     }
-    const DevPattern& P = *A->pattern;
-    const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((P.nrows + 7) / 8, (int64_t)sms * 16));
-    PendingEvent ev;
-    prof_begin(ctx, "assemble_gather_elasticity", ev);
-    gather_el_kernel<MODE><<<(int)blocks, 256, 0, ctx->stream>>>(P.nrows, P.d_ia, V->d_gptr, V->d_gidx, A->d_kbuf, A->d_val, accumulate);
-    prof_end(ctx, ev);
-    FGPU_CUDA_CHECK(ctx, cudaGetLastError());
-    return FGPU_OK;
+    return launch_gather_elasticity(ctx, A, accumulate);
 }
 
 int launch_assemble_elasticity_two_phase(fgpu_ctx* ctx, fgpu_matrix* A, const DevTables* tab, const float4* rec, int accumulate) {

@@ -28,13 +28,13 @@ struct fgpu_batch {
     int nprob = 0;
     int f32 = 0;
     int acc_floats = 0;              // per-warp staging floats (max over problems of EPB * maxrow * width)
-    int64_t total_rows = 0, total_elems = 0, total_nnz = 0, total_groups = 0;
+    int64_t total_rows = 0, total_elems = 0, total_slices = 0, total_groups = 0;
     bool two_phase = false;          // element buffers + gather maps (else the fused row-owner gather)
     BatchProblem* d_probs = nullptr;
     int64_t* d_row_off = nullptr;
     int64_t* d_elem_off = nullptr;
     int64_t* d_grp_off = nullptr;    // groups of 32 elements per problem (two-phase element kernel)
-    int64_t* d_nz_off = nullptr;
+    int64_t* d_slice_off = nullptr;  // gather slices per problem (two-phase)
     unsigned long long* d_counter = nullptr;
     BatchLaunch launch;
     bool tuned = false;
@@ -70,7 +70,7 @@ int batch_finish(fgpu_ctx* ctx) {
 int run_gather(fgpu_batch* b, const BatchLaunch& cfg, int accumulate) {
     fgpu_ctx* ctx = b->ctx;
     if (b->two_phase)
-        return launch_batch_two_phase(ctx, b->nprob, b->d_probs, b->d_grp_off, b->total_groups, b->d_nz_off, b->total_nnz, b->f32,
+        return launch_batch_two_phase(ctx, b->nprob, b->d_probs, b->d_grp_off, b->total_groups, b->d_slice_off, b->total_slices, b->f32,
                                       cfg.threads, accumulate);
     return launch_batch_gather(ctx, b->nprob, b->d_probs, b->d_row_off, b->total_rows, b->f32, b->acc_floats, b->d_counter, cfg,
                                accumulate);
@@ -165,7 +165,7 @@ int fgpu_batch_create(fgpu_ctx* ctx, int nprob, fgpu_matrix* const* mats, const 
             Am->coef_cap = V->mesh->nt * 8;
         }
         BatchProblem& P = probs[k];
-        std::memset(&P, 0, sizeof(P));
+        P = BatchProblem{};
         P.order = V->order;
         P.n = V->n;
         P.maxrow = A->pattern->max_row;
@@ -199,20 +199,20 @@ int fgpu_batch_create(fgpu_ctx* ctx, int nprob, fgpu_matrix* const* mats, const 
             const int n = V->n;
             const size_t kb = (size_t)V->mesh->nt * (n * (n + 1) / 2) * (f32 ? 4 : 8);
             if (A->kbuf_bytes < kb) need += kb;
-            if (!V->d_gptr) need += ((size_t)V->mesh->nt * n * n + (size_t)A->pattern->nnz * 2 + 1) * sizeof(uint32_t);
+            if (!gather_plan_ready(V)) need += gather_plan_bytes(V->mesh->nt, n, A->pattern->nnz);
             if ((int64_t)V->mesh->nt * n * n >= (int64_t)UINT32_MAX) two_phase = false;
         }
         size_t free_b = 0, total_b = 0;
         if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) { cudaGetLastError(); two_phase = false; }
         if (need + need / 10 >= free_b) two_phase = false;
     }
-    std::vector<int64_t> nz_off(nprob + 1, 0);
+    std::vector<int64_t> slice_off(nprob + 1, 0);
     for (int k = 0; k < nprob && two_phase; ++k) {
         fgpu_matrix* A = mats[k];
         fgpu_space* V = A->space;
         const int n = V->n;
         const size_t kb = (size_t)V->mesh->nt * (n * (n + 1) / 2) * (f32 ? 4 : 8);
-        if (!V->d_gptr && launch_build_gather_map(ctx, V) != FGPU_OK) { two_phase = false; break; }
+        if (!gather_plan_ready(V) && launch_build_gather_map(ctx, V) != FGPU_OK) { two_phase = false; break; }
         if (A->kbuf_bytes < kb) {
             cudaFree(A->d_kbuf);
             A->d_kbuf = nullptr;
@@ -220,18 +220,16 @@ int fgpu_batch_create(fgpu_ctx* ctx, int nprob, fgpu_matrix* const* mats, const 
             if (cudaMalloc(&A->d_kbuf, kb) != cudaSuccess) { cudaGetLastError(); two_phase = false; break; }
             A->kbuf_bytes = kb;
         }
-        probs[k].nz0 = nz_off[k];
         probs[k].nnz = A->pattern->nnz;
-        probs[k].gptr = V->d_gptr;
-        probs[k].gidx = V->d_gidx;
+        probs[k].plan = V->plan;
         probs[k].kbuf = A->d_kbuf;
-        nz_off[k + 1] = nz_off[k] + A->pattern->nnz;
+        slice_off[k + 1] = slice_off[k] + V->plan.nslices;
     }
     ctx->err.clear();
     fgpu_batch* b = new (std::nothrow) fgpu_batch();
     if (!b) return FGPU_ERR_ALLOC;
     b->two_phase = two_phase;
-    b->total_nnz = two_phase ? nz_off[nprob] : 0;
+    b->total_slices = two_phase ? slice_off[nprob] : 0;
     b->ctx = ctx;
     b->nprob = nprob;
     b->f32 = f32;
@@ -245,8 +243,8 @@ int fgpu_batch_create(fgpu_ctx* ctx, int nprob, fgpu_matrix* const* mats, const 
     if (e == cudaSuccess) e = cudaMalloc(&b->d_elem_off, (nprob + 1) * sizeof(int64_t));
     if (e == cudaSuccess) e = cudaMalloc(&b->d_grp_off, (nprob + 1) * sizeof(int64_t));
     if (e == cudaSuccess) e = cudaMalloc(&b->d_counter, sizeof(unsigned long long));
-    if (e == cudaSuccess) e = cudaMalloc(&b->d_nz_off, (nprob + 1) * sizeof(int64_t));
-    if (e == cudaSuccess) e = cudaMemcpy(b->d_nz_off, nz_off.data(), (nprob + 1) * sizeof(int64_t), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMalloc(&b->d_slice_off, (nprob + 1) * sizeof(int64_t));
+    if (e == cudaSuccess) e = cudaMemcpy(b->d_slice_off, slice_off.data(), (nprob + 1) * sizeof(int64_t), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(b->d_probs, probs.data(), nprob * sizeof(BatchProblem), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(b->d_row_off, row_off.data(), (nprob + 1) * sizeof(int64_t), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(b->d_elem_off, elem_off.data(), (nprob + 1) * sizeof(int64_t), cudaMemcpyHostToDevice);
@@ -286,7 +284,7 @@ int fgpu_batch_set_algo(fgpu_batch* b, int algo) {
     if (algo == FGPU_ALGO_GATHER) {
         b->two_phase = false;
     } else if (algo == FGPU_ALGO_TWO_PHASE || algo == FGPU_ALGO_AUTO) {
-        if (b->total_nnz == 0) return batch_err(b->ctx, FGPU_ERR_INVALID, "batch: no two-phase buffers (device memory)");
+        if (b->total_slices == 0) return batch_err(b->ctx, FGPU_ERR_INVALID, "batch: no two-phase buffers (device memory)");
         b->two_phase = true;
     } else {
         return batch_err(b->ctx, FGPU_ERR_INVALID, "batch: algorithm must be GATHER, TWO_PHASE or AUTO");
@@ -310,7 +308,7 @@ int fgpu_batch_destroy(fgpu_batch* b) {
     cudaFree(b->d_elem_off);
     cudaFree(b->d_grp_off);
     cudaFree(b->d_counter);
-    cudaFree(b->d_nz_off);
+    cudaFree(b->d_slice_off);
     delete b;
     return FGPU_OK;
 }

@@ -14,6 +14,13 @@
 namespace fgpu {
 
 struct StreamPlan;                   // schedule of the streamed assembly (stream_asm.cu)
+struct GatherPlan {                  // two-phase gather map of a space, in slices of 32 sums (gather.cu)
+    int64_t nslices = 0;
+    uint32_t* pos0 = nullptr;        // slices x 32: CSR position of the sum (row <= column), 0xFFFFFFFF: none
+    uint32_t* pos1 = nullptr;        // position of the transpose, 0xFFFFFFFF on the diagonal
+    uint32_t* soff = nullptr;        // slices + 1: first row of a slice in sidx
+    uint32_t* sidx = nullptr;        // rows of 32 element-buffer indices, one row per step of a slice
+};
 void stream_plan_free(StreamPlan* p);
 
 // ---------------------------------------------------------------------------
@@ -294,8 +301,7 @@ struct fgpu_space {
     int bnd_xmax_on = 0;
     double bnd_xmax = 0;
     uint64_t bnd_coords = 0;
-    uint32_t* d_gptr = nullptr;      // two-phase gather map: nnz + 1 offsets into d_gidx
-    uint32_t* d_gidx = nullptr;      // T n n element-buffer indices, per CSR entry in element order
+    fgpu::GatherPlan plan;           // two-phase gather map (built on first use)
     fgpu::StreamPlan* stream_plan = nullptr;   // streamed assembly: task order and waits (built on first use)
 };
 
@@ -362,8 +368,10 @@ struct DevTables {                     // device copies of the reference tables
     float* d_T7th = nullptr;           // the same split in upper-triangle order: 7 x n(n+1)/2
     float* d_T7tl = nullptr;
     uint16_t* d_tri = nullptr;         // n x n: (i, j) -> upper-triangle index of (min, max)
-    float* d_Sth = nullptr;            // elasticity tensors S_ab(i, j), i <= j, df64 split: 9 x n(n+1)/2
-    float* d_Stl = nullptr;
+    float* d_T7bh = nullptr;           // the split in the two-phase element buffer's order (entry_order)
+    float* d_T7bl = nullptr;
+    float* d_Sbh = nullptr;            // elasticity tensors S_ab in that order, df64 split: 9 x n(n+1)/2
+    float* d_Sbl = nullptr;
     double* d_phi = nullptr;           // Q n
     double* d_dphi = nullptr;          // Q n 3
     double* d_qx = nullptr;            // Q 3
@@ -400,6 +408,12 @@ int launch_assemble_streamed(fgpu_ctx* ctx, fgpu_matrix* A, const DevTables* tab
 int launch_geometry_el_df(fgpu_ctx* ctx, const fgpu_mesh* mesh, double lam, double mu, float4* d_rec);
 int launch_assemble_elasticity_two_phase(fgpu_ctx* ctx, fgpu_matrix* A, const DevTables* tab, const float4* rec, int accumulate);
 int launch_build_gather_map(fgpu_ctx* ctx, fgpu_space* V);
+bool gather_plan_ready(const fgpu_space* V);
+void gather_plan_free(fgpu_space* V);
+size_t gather_plan_bytes(int64_t nt, int n, int64_t nnz);
+void launch_gather_slices(fgpu_ctx* ctx, const fgpu_matrix* A, int threads, int bpsm, int batch, int pipe, int accumulate);
+int launch_gather_elasticity(fgpu_ctx* ctx, const fgpu_matrix* A, int accumulate);
+std::vector<uint16_t> entry_order(int cell_vertices, int order, int n);
 int mf_apply_f32_gated(fgpu_ctx* ctx, fgpu_operator* op, const float* x, float* y, const int* stop);
 int64_t operator_nnodes(const fgpu_operator* op);
 int operator_precision(const fgpu_operator* op);
@@ -447,9 +461,8 @@ struct BatchProblem {
     float4* rec;                     // coefficient records (the matrix's d_coef)
     void* val;                       // matrix values
     // two-phase batches
-    int64_t nz0, nnz;                // global CSR entry range
-    const uint32_t* gptr;            // the space's gather map
-    const uint32_t* gidx;
+    int64_t nnz;                     // CSR entries
+    GatherPlan plan;                 // the space's gather map
     void* kbuf;                      // the matrix's element buffer
 };
 struct BatchLaunch {                 // launch configuration picked by the batch tuner
@@ -459,8 +472,10 @@ struct BatchLaunch {                 // launch configuration picked by the batch
 int launch_batch_geometry(fgpu_ctx* ctx, int nprob, const BatchProblem* d_probs, const int64_t* d_elem_off,
                           int64_t total_elems);
 int launch_batch_two_phase(fgpu_ctx* ctx, int nprob, const BatchProblem* d_probs, const int64_t* d_grp_off,
-                           int64_t total_groups, const int64_t* d_nz_off, int64_t total_nnz, int f32, int threads,
+                           int64_t total_groups, const int64_t* d_slice_off, int64_t total_slices, int f32, int threads,
                            int accumulate);
+int launch_batch_gather_slices(fgpu_ctx* ctx, int nprob, const BatchProblem* d_probs, const int64_t* d_slice_off, int64_t total_slices,
+                               int f32, int threads, int accumulate);
 int launch_batch_gather(fgpu_ctx* ctx, int nprob, const BatchProblem* d_probs, const int64_t* d_row_off,
                         int64_t total_rows, int f32, int acc_floats, unsigned long long* d_counter,
                         const BatchLaunch& cfg, int accumulate);

@@ -1,0 +1,693 @@
+// Phase 2 of the two-phase assembly: every CSR entry is the sum, in element order, of its
+// contributions in the element buffer (bilinearformcontext.hpp:784-847 -> MatSetValues
+// ADD_VALUES adds element blocks in that order).
+//
+// The element matrices are symmetric and the buffer holds their upper triangles, so an entry (i, j)
+// and its transpose are one sum: it is formed once and stored at both positions. The map of the sums
+// is kept in slices (GatherPlan, built once per space):
+//  * a sum (a pair of dofs i <= j) belongs to the bin of the first element that contributes to it
+//    (a bin is a run of elements with about a thousand sums);
+//  * inside a bin the sums are sorted by their number of contributions (descending), then by the
+//    buffer index of the first one, and taken 32 at a time as slices: the lanes of a warp run the
+//    same number of steps;
+//  * the buffer keeps an element's entries grouped by the vertex, edge, face or cell that their two
+//    dofs span (entry_order): the sums of one group have the same contributing elements, so
+//    neighbouring lanes read neighbouring buffer entries at every step;
+//  * a slice stores its indices step by step, 32 lanes side by side (soff: its first row of 32,
+//    padding 0xFFFFFFFF): a step is one coalesced load of indices and one gather of values.
+//
+// What bounds it: sectors between L2 and the SMs, and DRAM. At P2 48^3 (25.8 M entries, 66 M
+// contributions; ncu) 26 M load and 19 M store sectors, 568 MB read and 183 MB written, 0.159 ms with
+// DRAM, L2 and L1 each at about 60 %. Before, one thread per entry walked the entry's own index list:
+// 269 M warp instructions (the lanes of a warp have 1 to 24 contributions) against 112 M, 896 MB read,
+// 0.275 ms. Sizes measured, gather phase before -> after: P2 64^3 0.640 -> 0.380 ms, P3 41x37x40
+// 0.661 -> 0.465 ms, binary32 P2 47x50x49 0.192 -> 0.122 ms. Tried on the way: slices over all entries
+// (no symmetry) with the sums staged in shared memory and stored in CSR order, 0.244 ms at P2 48^3
+// (62 M load sectors: 8-byte values in scattered 32-byte sectors).
+#include <algorithm>
+#include <string>
+#include <type_traits>
+#include <vector>
+
+#include "df64.h"
+#include "fgpu_core.h"
+#include "scan.cuh"
+#include "asm_device.cuh"
+
+namespace fgpu {
+
+namespace {
+
+constexpr uint32_t kNoIndex = 0xFFFFFFFFu;
+
+// Sum of the lane's contributions in steps r0 .. r1 - 1 of its slice, B steps' loads together; PIPE: the
+// next batch's indices travel with this batch's values. df64: compensated sum in element order, the high
+// parts through TwoSum, their rounding errors and the low parts in one binary32 accumulator, normalised
+// once by the caller (error ~ (count) u^2 |sum|). binary32: a plain sum.
+template <int MODE, int B, bool PIPE>
+__device__ __forceinline__ float2 slice_sum(uint32_t r0, uint32_t r1, int lane, const uint32_t* __restrict__ sidx,
+                                            const void* __restrict__ kbuf) {
+    typedef typename std::conditional<MODE == kModeDF64, float2, float>::type V;
+    const V* kb = reinterpret_cast<const V*>(kbuf);
+    float sh = 0.0f, sl = 0.0f;
+    uint32_t ix[B];
+    if (PIPE) {
+#pragma unroll
+        for (int u = 0; u < B; ++u) ix[u] = r0 + u < r1 ? __ldg(sidx + (size_t)(r0 + u) * 32 + lane) : kNoIndex;
+    }
+    for (uint32_t r = r0; r < r1; r += B) {
+        V v[B];
+        if (!PIPE) {
+#pragma unroll
+            for (int u = 0; u < B; ++u) ix[u] = r + u < r1 ? __ldg(sidx + (size_t)(r + u) * 32 + lane) : kNoIndex;
+        }
+#pragma unroll
+        for (int u = 0; u < B; ++u) v[u] = ix[u] != kNoIndex ? __ldg(kb + ix[u]) : V{};
+        if (PIPE && r + B < r1) {
+#pragma unroll
+            for (int u = 0; u < B; ++u) ix[u] = r + B + u < r1 ? __ldg(sidx + (size_t)(r + B + u) * 32 + lane) : kNoIndex;
+        }
+#pragma unroll
+        for (int u = 0; u < B; ++u)
+            if (r + u < r1) {
+                if constexpr (MODE == kModeDF64) {
+                    const df t = two_sum(sh, v[u].x);
+                    sh = t.hi;
+                    sl = f_add(sl, f_add(t.lo, v[u].y));
+                } else {
+                    sh = r + u == r0 ? v[u] : f_add(sh, v[u]);
+                }
+            }
+    }
+    return make_float2(sh, sl);
+}
+
+template <int MODE>
+__device__ __forceinline__ void store_sum(float2 v, void* __restrict__ valv, uint32_t k0, uint32_t k1, int accumulate) {
+    if (MODE == kModeDF64) {
+        double* val = reinterpret_cast<double*>(valv);
+        const df s = two_sum(v.x, v.y);
+        if (accumulate) {
+            val[k0] = df2d(df_add(d2df(val[k0]), s));
+            if (k1 != kNoIndex) val[k1] = df2d(df_add(d2df(val[k1]), s));
+        } else {
+            const double r = df2d(s);
+            val[k0] = r;
+            if (k1 != kNoIndex) val[k1] = r;
+        }
+    } else {
+        float* val = reinterpret_cast<float*>(valv);
+        val[k0] = accumulate ? f_add(val[k0], v.x) : v.x;
+        if (k1 != kNoIndex) val[k1] = accumulate ? f_add(val[k1], v.x) : v.x;
+    }
+}
+
+// one slice per warp
+template <int MODE, int B, bool PIPE>
+__device__ __forceinline__ void gather_slice(const GatherPlan& G, int64_t s, const void* __restrict__ kbuf, void* __restrict__ valv,
+                                             int accumulate) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t r0 = __ldg(G.soff + s), r1 = __ldg(G.soff + s + 1);
+    const uint32_t k0 = __ldg(G.pos0 + s * 32 + lane), k1 = __ldg(G.pos1 + s * 32 + lane);
+    const float2 v = slice_sum<MODE, B, PIPE>(r0, r1, lane, G.sidx, kbuf);
+    if (k0 != kNoIndex) store_sum<MODE>(v, valv, k0, k1, accumulate);
+}
+
+template <int MODE, int B, bool PIPE>
+__global__ void __launch_bounds__(256) gather_slices_kernel(GatherPlan G, const void* __restrict__ kbuf, void* __restrict__ valv,
+                                                            int accumulate) {
+    const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
+    for (int64_t s = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); s < G.nslices; s += nw)
+        gather_slice<MODE, B, PIPE>(G, s, kbuf, valv, accumulate);
+}
+
+// the slices of all problems of a batch (slice_off: prefix sums of their slice counts)
+template <int MODE>
+__global__ void __launch_bounds__(256) batch_gather_slices_kernel(int nprob, const BatchProblem* __restrict__ probs,
+                                                                  const int64_t* __restrict__ slice_off, int64_t total, int accumulate) {
+    const int64_t s = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (s >= total) return;
+    int lo = 0, hi = nprob - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (__ldg(slice_off + mid) <= s) lo = mid;
+        else hi = mid - 1;
+    }
+    const BatchProblem& P = probs[lo];
+    gather_slice<MODE, 4, false>(P.plan, s - slice_off[lo], P.kbuf, P.val, accumulate);
+}
+
+// Vector elasticity: one lane per pair of nodes i <= j, its 3x3 block (row 3i+c, columns 3j+d) summed
+// over the contributions in element order (bit 31 of an index: stored as (j, i), read transposed) and
+// stored with its transpose at (j, i). sia, ja: the scalar pattern.
+template <int MODE>
+__global__ void __launch_bounds__(128) gather_elasticity_slices_kernel(GatherPlan G, const int64_t* __restrict__ sia,
+                                                                       const int32_t* __restrict__ ja, const void* __restrict__ kbuf,
+                                                                       void* __restrict__ valv, int accumulate) {
+    typedef typename std::conditional<MODE == kModeDF64, float2, float>::type V;
+    const int lane = threadIdx.x & 31;
+    const int64_t s = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (s >= G.nslices) return;
+    const uint32_t r0 = __ldg(G.soff + s), r1 = __ldg(G.soff + s + 1);
+    const uint32_t k0 = __ldg(G.pos0 + s * 32 + lane), k1 = __ldg(G.pos1 + s * 32 + lane);
+    df acc[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) acc[k] = df{0.0f, 0.0f};
+    for (uint32_t r = r0; r < r1; ++r) {
+        const uint32_t g = __ldg(G.sidx + (size_t)r * 32 + lane);
+        if (g == kNoIndex) continue;
+        const bool tr = (g & 0x80000000u) != 0;
+        const V* b = reinterpret_cast<const V*>(kbuf) + (size_t)(g & 0x7FFFFFFFu) * 9;
+        V v[9];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) v[k] = __ldg(b + k);
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                const V w = tr ? v[d * 3 + c] : v[c * 3 + d];
+                df& a = acc[c * 3 + d];
+                if constexpr (MODE == kModeDF64) a = r == r0 ? df{w.x, w.y} : df_add(a, df{w.x, w.y});
+                else a.hi = r == r0 ? w : f_add(a.hi, w);
+            }
+    }
+    if (k0 == kNoIndex) return;
+    for (int side = 0; side < 2; ++side) {
+        const uint32_t k = side ? k1 : k0;
+        if (k == kNoIndex) break;
+        const int32_t row = k1 == kNoIndex ? __ldg(ja + k0) : __ldg(ja + (side ? k0 : k1));
+        const int64_t s0 = sia[row];
+        const int64_t len = sia[row + 1] - s0;
+        const int64_t o = 9 * s0 + 3 * ((int64_t)k - s0);
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                df a = side ? acc[d * 3 + c] : acc[c * 3 + d];
+                if constexpr (MODE == kModeDF64) {
+                    double* out = reinterpret_cast<double*>(valv) + o + c * 3 * len + d;
+                    if (accumulate) a = df_add(d2df(*out), a);
+                    *out = df2d(a);
+                } else {
+                    float* out = reinterpret_cast<float*>(valv) + o + c * 3 * len + d;
+                    *out = accumulate ? f_add(*out, a.hi) : a.hi;
+                }
+            }
+    }
+}
+
+// the values of the matrix to a mapped page-locked host buffer
+__global__ void __launch_bounds__(256) values_to_host_kernel(int64_t nnz, const double* __restrict__ val, double* __restrict__ hout) {
+    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < nnz; k += (int64_t)gridDim.x * blockDim.x) hout[k] = val[k];
+}
+
+// ---- the plan (once per space) ----
+
+// The space's tables that the plan is built from; tri: pair (a, b) of local dofs -> buffer entry.
+struct PlanIn {
+    int64_t nrows;
+    uint32_t n, ntri;
+    int bin_shift, mark;                  // a bin is 2^bin_shift elements
+    const int64_t* ia;
+    const int64_t* inc_ptr;
+    const int32_t* inc;
+    const int32_t* l2n;
+    const uint8_t* pos;
+    const uint16_t* tri;
+};
+
+// One warp per row r, its incident elements in element order, 32 / n of them at a time with one lane
+// per element dof; the dofs j >= r are the row's sums. first[idx], idx a buffer entry: the sum whose
+// first contribution it is (0: none).
+// FILL 0: first[idx] = the sum's number of contributions (counted in any order; the first by minimum).
+// FILL 1: first[idx] holds 1 + the sum's place in its bin; the sum's CSR positions and the buffer
+// indices of its steps, in element order.
+// mark: bit 31 of an index whose element entry is stored as (j, i).
+template <int FILL, int U>
+__global__ void __launch_bounds__(256, 6) plan_walk_kernel(PlanIn in, uint16_t* __restrict__ first, const uint32_t* __restrict__ slice0,
+                                                        const uint32_t* __restrict__ soff, uint32_t* __restrict__ pos0,
+                                                        uint32_t* __restrict__ pos1, uint32_t* __restrict__ sidx,
+                                                        int* __restrict__ status) {
+    __shared__ uint32_t at[8][256];     // 0: first buffer entry; 1: place of the sum's next step
+    __shared__ uint32_t cnt[FILL ? 1 : 8][256];
+    __shared__ uint16_t tri[32 * 32];   // n <= 32 (checked by the launcher)
+    const uint32_t n = in.n;
+    for (uint32_t k = threadIdx.x; k < n * n; k += blockDim.x) tri[k] = in.tri[k];
+    __syncthreads();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int epw = 32 / (int)n, grp = lane / (int)n, lj = lane - grp * (int)n;
+    // (32-bit indices: fewer than 2^32 contributions, checked by the launcher)
+    for (uint32_t r = blockIdx.x * 8 + warp; r < (uint32_t)in.nrows; r += gridDim.x * 8) {
+        const int64_t start = in.ia[r];
+        const int len = (int)(in.ia[r + 1] - start);
+        if (len > 256) {
+            if (lane == 0) atomicOr(status, kStatusRowOverflow);
+            continue;
+        }
+        if (!FILL)
+            for (int k = lane; k < len; k += 32) {
+                at[warp][k] = kNoIndex;
+                cnt[FILL ? 0 : warp][k] = 0;
+            }
+        __syncwarp();
+        // U = 2 steps' loads together: the chain of a step is up to five dependent loads, its work a few
+        // instructions (P2 64^3 fill 1.36 ms, 1.47 a step at a time; U = 4 at P3 1.54 against 1.29; rows
+        // pipelined over iterations 2.7 ms: fewer warps per SM)
+        const uint32_t t1 = (uint32_t)in.inc_ptr[r + 1];
+        for (uint32_t t = (uint32_t)in.inc_ptr[r]; t < t1; t += U * epw) {
+            uint32_t code[U], idx[U], w0[U];
+            int32_t j[U];
+            int p[U];
+            bool on[U];
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                on[u] = grp < epw && t + u * epw + grp < t1;
+                code[u] = on[u] ? (uint32_t)in.inc[t + u * epw + grp] : 0u;
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                const uint32_t e = code[u] >> 5, li = code[u] & 31u;
+                j[u] = on[u] ? in.l2n[e * n + lj] : -1;
+                p[u] = on[u] ? in.pos[(e * n + li) * n + lj] : 0;
+                idx[u] = e * in.ntri + (on[u] ? tri[li * n + lj] : 0u);
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                on[u] = on[u] && (uint32_t)j[u] >= r;
+                w0[u] = FILL && on[u] ? first[idx[u]] : 0u;
+            }
+            if (FILL) {
+#pragma unroll
+                for (int u = 0; u < U; ++u)
+                    if (w0[u]) {                   // the sum's first contribution: its positions and its place
+                        const uint32_t e = code[u] >> 5, li = code[u] & 31u;
+                        const uint32_t slot = slice0[e >> in.bin_shift] * 32 + w0[u] - 1;
+                        at[warp][p[u]] = soff[slot >> 5] * 32 + (slot & 31);
+                        pos0[slot] = (uint32_t)start + p[u];
+                        if ((uint32_t)j[u] != r) pos1[slot] = (uint32_t)in.ia[j[u]] + in.pos[(e * n + lj) * n + li];
+                    }
+                __syncwarp();
+            }
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                if (!FILL) {
+                    if (on[u]) {
+                        atomicAdd(&cnt[FILL ? 0 : warp][p[u]], 1u);
+                        atomicMin(&at[warp][p[u]], idx[u]);
+                    }
+                } else {
+                    // places in element order: the step's elements one after another (their dofs are distinct)
+                    uint32_t w = 0;
+                    for (int g = 0; g < epw; ++g) {
+                        if (on[u] && g == grp) {
+                            w = at[warp][p[u]];
+                            at[warp][p[u]] = w + 32;
+                        }
+                        __syncwarp();
+                    }
+                    if (on[u]) sidx[w] = idx[u] | (in.mark && (code[u] & 31u) > (uint32_t)lj ? 0x80000000u : 0u);
+                }
+            }
+            __syncwarp();
+        }
+        if (!FILL)
+            for (int k = lane; k < len; k += 32) {
+                const uint32_t c = cnt[FILL ? 0 : warp][k];
+                if (c) first[at[warp][k]] = (uint16_t)min(c, 0xFFFFu);
+            }
+        __syncwarp();
+    }
+}
+
+// sums of each bin (one warp per bin, eight counts per load; a bin starts at a multiple of `per`)
+__global__ void __launch_bounds__(256) bin_count_kernel(int64_t nbins, int64_t total, int per, const uint16_t* __restrict__ first,
+                                                        uint32_t* __restrict__ cnt) {
+    const int64_t bin = (int64_t)blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (bin >= nbins) return;
+    const int lane = threadIdx.x & 31;
+    const int64_t b = bin * per, e = b + per < total ? b + per : total;
+    const int64_t b8 = (b + 7) & ~(int64_t)7, e8 = e & ~(int64_t)7;
+    uint32_t c = 0;
+    if (b8 < e8) {
+        for (int64_t k = b8 + 8 * lane; k < e8; k += 256) {
+            const uint4 v = *reinterpret_cast<const uint4*>(first + k);
+            const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int u = 0; u < 4; ++u) c += ((w[u] & 0xFFFFu) != 0) + ((w[u] >> 16) != 0);
+        }
+        if (b + lane < b8) c += first[b + lane] != 0;
+        if (e8 + lane < e) c += first[e8 + lane] != 0;
+    } else {
+        for (int64_t k = b + lane; k < e; k += 32) c += first[k] != 0;
+    }
+    for (int o = 16; o > 0; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+    if (lane == 0) cnt[bin] = c;
+}
+
+// one block: the first slice of every bin, and the number of slices
+__global__ void __launch_bounds__(1024) bin_scan_kernel(int64_t nbins, const uint32_t* __restrict__ cnt, uint32_t* __restrict__ slice0,
+                                                        unsigned long long* __restrict__ total) {
+    __shared__ unsigned long long part[1024];
+    unsigned long long run = 0;
+    for (int64_t b0 = 0; b0 < nbins; b0 += 4096) {          // four consecutive bins per thread
+        const int64_t k0 = b0 + 4 * threadIdx.x;
+        uint32_t c[4];
+        unsigned long long t = 0;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            c[u] = k0 + u < nbins ? (cnt[k0 + u] + 31) / 32 : 0u;
+            t += c[u];
+        }
+        part[threadIdx.x] = t;
+        __syncthreads();
+        for (int o = 1; o < 1024; o <<= 1) {
+            const unsigned long long v = threadIdx.x >= (unsigned)o ? part[threadIdx.x - o] : 0ull;
+            __syncthreads();
+            part[threadIdx.x] += v;
+            __syncthreads();
+        }
+        unsigned long long x = run + part[threadIdx.x] - t;
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+            if (k0 + u < nbins) {
+                slice0[k0 + u] = (uint32_t)x;
+                x += c[u];
+            }
+        run += part[1023];
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) *total = run;
+}
+
+// One block per bin: the places of its sums by a stable counting sort (contributions descending, then
+// buffer entry), written over the counts as place + 1, and each slice's number of steps (zero before).
+__global__ void __launch_bounds__(256) bin_rank_kernel(int64_t total, int per, uint16_t* __restrict__ first, const uint32_t* __restrict__ slice0,
+                                                       uint32_t* __restrict__ steps) {
+    __shared__ uint32_t off[256];       // by class min(contributions, 255): next place
+    __shared__ uint16_t wcnt[8][256];   // the class's sums in each warp's part of a batch
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int64_t base = (int64_t)blockIdx.x * per;
+    const int cnt = (int)(total - base < per ? total - base : per);
+    off[tid] = 0;
+    for (int k = tid; k < 8 * 256; k += 256) (&wcnt[0][0])[k] = 0;
+    __syncthreads();
+    for (int k = tid; k < cnt; k += 256) {
+        const uint32_t c = first[base + k];
+        if (c) atomicAdd(&off[min(c, 255u)], 1u);
+    }
+    __syncthreads();
+    // exclusive sums from the largest class down
+    __shared__ uint32_t part[256];
+    const uint32_t own = off[255 - tid];
+    part[tid] = own;
+    __syncthreads();
+    for (int o = 1; o < 256; o <<= 1) {
+        const uint32_t v = tid >= o ? part[tid - o] : 0u;
+        __syncthreads();
+        part[tid] += v;
+        __syncthreads();
+    }
+    off[255 - tid] = part[tid] - own;
+    __syncthreads();
+    for (int b0 = 0; b0 < cnt; b0 += 256) {
+        const int k = b0 + tid;
+        const uint32_t c = k < cnt ? first[base + k] : 0u, cls = min(c, 255u);
+        const unsigned same = __match_any_sync(0xffffffffu, cls);
+        const bool leader = c && lane == __ffs(same) - 1;
+        if (leader) wcnt[warp][cls] = (uint16_t)__popc(same);
+        __syncthreads();
+        if (c) {
+            uint32_t place = off[cls] + __popc(same & ((1u << lane) - 1u));
+            for (int w = 0; w < warp; ++w) place += wcnt[w][cls];
+            first[base + k] = (uint16_t)(place + 1);
+            if ((place & 31) == 0 || cls == 255u) atomicMax(steps + slice0[blockIdx.x] + (place >> 5), c);
+        }
+        __syncthreads();
+        if (leader) {
+            atomicAdd(&off[cls], (uint32_t)__popc(same));
+            wcnt[warp][cls] = 0;
+        }
+        __syncthreads();
+    }
+}
+
+template <int FILL>
+void launch_walk(fgpu_ctx* ctx, int blocks, const PlanIn& in, uint16_t* first, const uint32_t* slice0, const uint32_t* soff,
+                 uint32_t* pos0, uint32_t* pos1, uint32_t* sidx) {
+    plan_walk_kernel<FILL, 2><<<blocks, 256, 0, ctx->stream>>>(in, first, slice0, soff, pos0, pos1, sidx, ctx->d_status);
+}
+
+int sm_count(const fgpu_ctx* ctx) {
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+    return std::max(sms, 1);
+}
+
+template <int MODE, bool PIPE>
+void launch_slices(fgpu_ctx* ctx, const fgpu_matrix* A, int threads, int bpsm, int batch, int accumulate) {
+    const GatherPlan& G = A->space->plan;
+    const int64_t need = (G.nslices + threads / 32 - 1) / (threads / 32);
+    const int blocks = (int)std::max<int64_t>(1, bpsm > 0 ? std::min<int64_t>(need, (int64_t)sm_count(ctx) * bpsm) : need);
+    switch (batch) {
+        case 2: gather_slices_kernel<MODE, 2, PIPE><<<blocks, threads, 0, ctx->stream>>>(G, A->d_kbuf, A->d_val, accumulate); break;
+        case 8: gather_slices_kernel<MODE, 8, PIPE><<<blocks, threads, 0, ctx->stream>>>(G, A->d_kbuf, A->d_val, accumulate); break;
+        default: gather_slices_kernel<MODE, 4, PIPE><<<blocks, threads, 0, ctx->stream>>>(G, A->d_kbuf, A->d_val, accumulate); break;
+    }
+}
+
+// the vertices of the cell that a local dof's entity spans, as a bit mask
+uint32_t span_mask(int cell_vertices, int order, int dof) {
+    if (dof < cell_vertices) return 1u << dof;
+    dof -= cell_vertices;
+    uint32_t m = 0;
+    if (cell_vertices == 8) {
+        if (dof < 12) return (1u << kHexEdgeVerts[dof][0]) | (1u << kHexEdgeVerts[dof][1]);
+        if (dof < 18) {
+            for (int k = 0; k < 4; ++k) m |= 1u << kHexFaceVerts[dof - 12][k];
+            return m;
+        }
+        return 0xFFu;
+    }
+    const int per_edge = order - 1;
+    if (dof < 6 * per_edge) return (1u << kEdgeVerts[dof / per_edge][0]) | (1u << kEdgeVerts[dof / per_edge][1]);
+    for (int k = 0; k < 3; ++k) m |= 1u << kFaceVerts[dof - 6 * per_edge][k];
+    return m;
+}
+
+}  // namespace
+
+// Order of an element's upper-triangle entries in the two-phase element buffer: grouped by the smallest
+// vertex set, edge, face or cell that holds both dofs, small ones first, row-major inside a group.
+// order[t]: the pair a * 256 + b (a <= b) of buffer entry t.
+std::vector<uint16_t> entry_order(int cell_vertices, int order, int n) {
+    std::vector<uint32_t> holders;                 // candidate vertex sets, by size
+    for (int v = 0; v < cell_vertices; ++v) holders.push_back(1u << v);
+    if (cell_vertices == 8) {
+        for (auto& e : kHexEdgeVerts) holders.push_back((1u << e[0]) | (1u << e[1]));
+        for (auto& f : kHexFaceVerts) holders.push_back((1u << f[0]) | (1u << f[1]) | (1u << f[2]) | (1u << f[3]));
+    } else {
+        for (auto& e : kEdgeVerts) holders.push_back((1u << e[0]) | (1u << e[1]));
+        for (auto& f : kFaceVerts) holders.push_back((1u << f[0]) | (1u << f[1]) | (1u << f[2]));
+    }
+    holders.push_back((1u << cell_vertices) - 1u);
+    std::vector<std::vector<uint16_t>> groups(holders.size());
+    for (int a = 0; a < n; ++a)
+        for (int b = a; b < n; ++b) {
+            const uint32_t m = span_mask(cell_vertices, order, a) | span_mask(cell_vertices, order, b);
+            size_t g = 0;
+            while ((holders[g] & m) != m) ++g;
+            groups[g].push_back((uint16_t)(a * 256 + b));
+        }
+    std::vector<uint16_t> out;
+    for (auto& g : groups) out.insert(out.end(), g.begin(), g.end());
+    return out;
+}
+
+void gather_plan_free(fgpu_space* V) {
+    cudaFree(V->plan.pos0);
+    cudaFree(V->plan.sidx);
+    V->plan = GatherPlan{};
+}
+
+bool gather_plan_ready(const fgpu_space* V) { return V->plan.sidx != nullptr; }
+
+// Device memory of the map while it is built, in bytes (nt elements, n local dofs).
+size_t gather_plan_bytes(int64_t nt, int n, int64_t nnz) { return (size_t)nt * n * (n + 1) / 2 * 7 + (size_t)nnz * 6 + (size_t)nt * 300; }
+
+int launch_build_gather_map(fgpu_ctx* ctx, fgpu_space* V) {
+    if (gather_plan_ready(V)) return FGPU_OK;
+    const DevPattern& P = *V->pattern;
+    const int n = V->n, ntri = n * (n + 1) / 2;
+    const int64_t nt = V->mesh->nt, nnz = P.nnz, entries = nt * ntri;
+    if (nt * (int64_t)n * n >= (int64_t)UINT32_MAX || entries >= ((int64_t)1 << 31)) {
+        ctx->err = "gather map: more than 2^32 contributions or 2^31 buffered entries";
+        return FGPU_ERR_INVALID;
+    }
+    if (!V->d_pos) { ctx->err = "gather map: no position table"; return FGPU_ERR_INVALID; }
+    if (n > 32) { ctx->err = "gather map: more than 32 local dofs"; return FGPU_ERR_INVALID; }
+    const std::vector<uint16_t> ab = entry_order(V->mesh->cv, V->order, n);
+    std::vector<uint16_t> tri((size_t)n * n);
+    for (int t = 0; t < ntri; ++t) tri[(ab[t] >> 8) * n + (ab[t] & 255)] = tri[(ab[t] & 255) * n + (ab[t] >> 8)] = (uint16_t)t;
+    // elements per bin: about a thousand sums on average, fewer than 2^16 buffer entries
+    int shift = 0;
+    while ((2 << shift) * ntri < 65536 && nnz / 2 * (2 << shift) <= 1400 * nt) ++shift;
+    const int per_bin = 1 << shift;
+    const int64_t nbins = (nt + per_bin - 1) / per_bin;
+    const int64_t max_slices = (nnz + P.nrows) / 64 + nbins + 1;     // a sum per pair i <= j, one partial slice per bin
+    const int sms = sm_count(ctx);
+    // scratch in one block: totals, scan sums, bins, steps, the first contributions, the pair table
+    const size_t s_tot = 16, s_sum = (scan_chunks(max_slices) + 1) * 8, s_bin = (size_t)nbins * 8, s_step = (size_t)max_slices * 4,
+                 s_first = ((size_t)entries * 2 + 15) & ~(size_t)15;
+    char* scratch = nullptr;
+    GatherPlan G{};
+    cudaError_t e = cudaMalloc(&scratch, s_tot + s_sum + s_bin + s_step + 16 + s_first + tri.size() * 2);
+    unsigned long long* d_total = reinterpret_cast<unsigned long long*>(scratch);
+    unsigned long long* sums = d_total + 2;
+    uint32_t *cnt = reinterpret_cast<uint32_t*>(scratch + s_tot + s_sum), *slice0 = cnt + nbins, *steps = slice0 + nbins;
+    uint16_t* first = reinterpret_cast<uint16_t*>(scratch + ((s_tot + s_sum + s_bin + s_step + 15) & ~(size_t)15));
+    uint16_t* d_tri = reinterpret_cast<uint16_t*>(reinterpret_cast<char*>(first) + s_first);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(d_tri, tri.data(), tri.size() * sizeof(uint16_t), cudaMemcpyHostToDevice, ctx->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(first, 0, (size_t)entries * sizeof(uint16_t), ctx->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(steps, 0, s_step, ctx->stream);
+    const PlanIn in{P.nrows, (uint32_t)n, (uint32_t)ntri, shift, V->ncomp > 1, P.d_ia, V->d_inc_ptr, V->d_inc, V->d_l2n, V->d_pos, d_tri};
+    const int walkers = (int)std::max<int64_t>(1, std::min<int64_t>((P.nrows + 7) / 8, (int64_t)sms * 64));
+    if (e == cudaSuccess) {
+        launch_walk<0>(ctx, walkers, in, first, nullptr, nullptr, nullptr, nullptr, nullptr);
+        bin_count_kernel<<<(int)((nbins + 7) / 8), 256, 0, ctx->stream>>>(nbins, entries, per_bin * ntri, first, cnt);
+        bin_scan_kernel<<<1, 1024, 0, ctx->stream>>>(nbins, cnt, slice0, d_total);
+        bin_rank_kernel<<<(int)nbins, 256, 0, ctx->stream>>>(entries, per_bin * ntri, first, slice0, steps);
+        ctx->launches += 4;
+        e = cudaGetLastError();
+    }
+    const size_t slots = (size_t)max_slices * 32;
+    if (e == cudaSuccess) e = cudaMalloc(&G.pos0, (2 * slots + max_slices + 1) * sizeof(uint32_t));
+    G.pos1 = G.pos0 + slots;
+    G.soff = G.pos1 + slots;
+    if (e == cudaSuccess) e = cudaMemsetAsync(G.pos0, 0xFF, 2 * slots * sizeof(uint32_t), ctx->stream);
+    if (e == cudaSuccess) {
+        scan_u32_launch(ctx, steps, G.soff, max_slices, sums);
+        e = cudaGetLastError();
+    }
+    unsigned long long nslices = 0, rows = 0;
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&nslices, d_total, sizeof(nslices), cudaMemcpyDeviceToHost, ctx->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&rows, sums + scan_chunks(max_slices), sizeof(rows), cudaMemcpyDeviceToHost, ctx->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    G.nslices = (int64_t)nslices;
+    const size_t words = std::max<size_t>(1, (size_t)rows * 32);
+    int rc = FGPU_OK;
+    if (e == cudaSuccess && words > 0xFFFFFFFFull) {
+        ctx->err = "gather map: more than 2^32 padded contributions";
+        rc = FGPU_ERR_INVALID;
+    }
+    if (e == cudaSuccess && rc == FGPU_OK) e = cudaMalloc(&G.sidx, words * sizeof(uint32_t));
+    if (e == cudaSuccess && rc == FGPU_OK) e = cudaMemsetAsync(G.sidx, 0xFF, words * sizeof(uint32_t), ctx->stream);
+    if (e == cudaSuccess && rc == FGPU_OK) {
+        launch_walk<1>(ctx, walkers, in, first, slice0, G.soff, G.pos0, G.pos1, G.sidx);
+        ctx->launches++;
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    cudaFree(scratch);
+    if (e != cudaSuccess || rc != FGPU_OK) {
+        cudaFree(G.pos0); cudaFree(G.sidx);
+        if (rc) return rc;
+        cudaGetLastError();
+        ctx->err = std::string("gather map: ") + cudaGetErrorString(e);
+        return e == cudaErrorMemoryAllocation ? FGPU_ERR_ALLOC : FGPU_ERR_CUDA;
+    }
+    V->plan = G;
+    return FGPU_OK;
+}
+
+void launch_gather_slices(fgpu_ctx* ctx, const fgpu_matrix* A, int threads, int bpsm, int batch, int pipe, int accumulate) {
+    if (A->precision == FGPU_F32) {
+        if (pipe) launch_slices<kModeF32, true>(ctx, A, threads, bpsm, batch, accumulate);
+        else launch_slices<kModeF32, false>(ctx, A, threads, bpsm, batch, accumulate);
+    } else {
+        if (pipe) launch_slices<kModeDF64, true>(ctx, A, threads, bpsm, batch, accumulate);
+        else launch_slices<kModeDF64, false>(ctx, A, threads, bpsm, batch, accumulate);
+    }
+}
+
+int launch_gather_phase(fgpu_ctx* ctx, fgpu_matrix* A, int accumulate) {
+    PendingEvent ev;
+    prof_begin(ctx, "assemble_gather", ev);
+    launch_gather_slices(ctx, A, 256, 0, 4, 0, accumulate);
+    prof_end(ctx, ev);
+    FGPU_CUDA_CHECK(ctx, cudaGetLastError());
+    return FGPU_OK;
+}
+
+int launch_gather_elasticity(fgpu_ctx* ctx, const fgpu_matrix* A, int accumulate) {
+    const GatherPlan& G = A->space->plan;
+    const DevPattern& P = *A->pattern;
+    const int blocks = (int)std::max<int64_t>(1, (G.nslices + 3) / 4);
+    PendingEvent ev;
+    prof_begin(ctx, "assemble_gather_elasticity", ev);
+    if (A->precision == FGPU_F32)
+        gather_elasticity_slices_kernel<kModeF32><<<blocks, 128, 0, ctx->stream>>>(G, P.d_ia, P.d_ja, A->d_kbuf, A->d_val, accumulate);
+    else
+        gather_elasticity_slices_kernel<kModeDF64><<<blocks, 128, 0, ctx->stream>>>(G, P.d_ia, P.d_ja, A->d_kbuf, A->d_val, accumulate);
+    prof_end(ctx, ev);
+    FGPU_CUDA_CHECK(ctx, cudaGetLastError());
+    return FGPU_OK;
+}
+
+// Phase 2, then the values to the host: by kernel stores where the buffer is page-locked and mapped
+// (CSR order, at the host link's rate), else in nchunks ranges on as many copy streams. FP64 matrices.
+int launch_gather_phase_to_host(fgpu_ctx* ctx, fgpu_matrix* A, double* host, int nchunks) {
+    const int64_t nnz = A->pattern->nnz;
+    nchunks = std::max(1, std::min(nchunks, 4));
+    if (!ctx->copy_streams[0]) {
+        for (int i = 0; i < 4; ++i) FGPU_CUDA_CHECK(ctx, cudaStreamCreateWithFlags(&ctx->copy_streams[i], cudaStreamNonBlocking));
+        for (int i = 0; i < 5; ++i) FGPU_CUDA_CHECK(ctx, cudaEventCreateWithFlags(&ctx->copy_events[i], cudaEventDisableTiming));
+    }
+    double* hdev = nullptr;
+    if (ctx->host_transfer != FGPU_HOST_TRANSFER_COPY) {
+        cudaPointerAttributes pa{};
+        if (cudaPointerGetAttributes(&pa, host) == cudaSuccess && pa.type == cudaMemoryTypeHost && pa.devicePointer)
+            hdev = static_cast<double*>(pa.devicePointer);
+        else
+            cudaGetLastError();
+        if (!hdev && ctx->host_transfer == FGPU_HOST_TRANSFER_DIRECT) {
+            ctx->err = "direct host transfer: the host buffer is not page-locked and mapped";
+            return FGPU_ERR_INVALID;
+        }
+    }
+    int rc = launch_gather_phase(ctx, A, 0);
+    if (rc) return rc;
+    if (hdev) {
+        const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((nnz + 255) / 256, (int64_t)sm_count(ctx) * 32));
+        values_to_host_kernel<<<(int)blocks, 256, 0, ctx->stream>>>(nnz, (const double*)A->d_val, hdev);
+        ctx->launches++;
+        FGPU_CUDA_CHECK(ctx, cudaGetLastError());
+        FGPU_CUDA_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
+        return FGPU_OK;
+    }
+    const int64_t chunk = ((nnz + nchunks - 1) / nchunks + 255) & ~(int64_t)255;
+    FGPU_CUDA_CHECK(ctx, cudaEventRecord(ctx->copy_events[0], ctx->stream));
+    for (int c = 0; c < nchunks; ++c) {
+        const int64_t k0 = (int64_t)c * chunk;
+        if (k0 >= nnz) break;
+        const int64_t k1 = std::min(nnz, k0 + chunk);
+        FGPU_CUDA_CHECK(ctx, cudaStreamWaitEvent(ctx->copy_streams[c], ctx->copy_events[0], 0));
+        FGPU_CUDA_CHECK(ctx, cudaMemcpyAsync(host + k0, (const double*)A->d_val + k0, (k1 - k0) * sizeof(double),
+                                             cudaMemcpyDeviceToHost, ctx->copy_streams[c]));
+    }
+    for (int c = 0; c < nchunks; ++c) FGPU_CUDA_CHECK(ctx, cudaStreamSynchronize(ctx->copy_streams[c]));
+    return FGPU_OK;
+}
+
+int launch_batch_gather_slices(fgpu_ctx* ctx, int nprob, const BatchProblem* d_probs, const int64_t* d_slice_off, int64_t total_slices,
+                               int f32, int threads, int accumulate) {
+    const int blocks = (int)std::max<int64_t>(1, (total_slices + threads / 32 - 1) / (threads / 32));
+    PendingEvent ev;
+    prof_begin(ctx, "batch_gather", ev);
+    if (f32) batch_gather_slices_kernel<kModeF32><<<blocks, threads, 0, ctx->stream>>>(nprob, d_probs, d_slice_off, total_slices, accumulate);
+    else batch_gather_slices_kernel<kModeDF64><<<blocks, threads, 0, ctx->stream>>>(nprob, d_probs, d_slice_off, total_slices, accumulate);
+    prof_end(ctx, ev);
+    FGPU_CUDA_CHECK(ctx, cudaGetLastError());
+    return FGPU_OK;
+}
+
+}  // namespace fgpu

@@ -58,7 +58,7 @@ struct HoTables {
     float* d_gdl = nullptr;    //                               (lo)
     float* d_qwh = nullptr;    // Q: weights as double-float (hi)
     float* d_qwl = nullptr;    //                            (lo)
-    uint8_t* d_ti = nullptr;   // ntri: row of each upper-triangle entry
+    uint8_t* d_ti = nullptr;   // ntri: row of each upper-triangle entry (entry_order)
     uint8_t* d_tj = nullptr;   // ntri: column
     float* d_tcB = nullptr;    // tensor-core B operand: per chunk of points, per accumulator, tf32 hi / lo
     std::vector<double> dphi, phi;   // Q n 3, Q n (host copies for building d_tcB)
@@ -109,11 +109,10 @@ HoTables* get_ho_tables(fgpu_ctx* ctx, int order, int qdeg, bool hex = false) {
         qwl[k] = (float)(R.qw[k] - (double)qwh[k]);
     }
     std::vector<uint8_t> ti, tj;
-    for (int i = 0; i < R.n; ++i)
-        for (int j = i; j < R.n; ++j) {
-            ti.push_back((uint8_t)i);
-            tj.push_back((uint8_t)j);
-        }
+    for (uint16_t p : entry_order(hex ? 8 : 4, order, R.n)) {
+        ti.push_back((uint8_t)(p >> 8));
+        tj.push_back((uint8_t)(p & 255));
+    }
     cudaError_t e = up(&T->d_dh, dh);
     if (e == cudaSuccess) e = up(&T->d_dl, dl);
     if (e == cudaSuccess) e = up(&T->d_ph, ph);
@@ -664,11 +663,10 @@ static int ho_tc_tables(fgpu_ctx* ctx, HoTables* T) {
     const int Q = T->Q, nch = (Q + kHoTcQC - 1) / kHoTcQC;
     std::vector<float> B((size_t)nch * (D::BSTAGE / 4), 0.0f);
     std::vector<int> ti, tj;
-    for (int i = 0; i < N; ++i)
-        for (int j = i; j < N; ++j) {
-            ti.push_back(i);
-            tj.push_back(j);
-        }
+    for (uint16_t p : entry_order(GN == 8 ? 8 : 4, N == 4 || N == 8 ? 1 : N == 20 ? 3 : 2, N)) {
+        ti.push_back(p >> 8);
+        tj.push_back(p & 255);
+    }
     auto tf32_hi_host = [](float x) {
         uint32_t u;
         std::memcpy(&u, &x, 4);

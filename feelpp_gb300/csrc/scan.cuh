@@ -73,20 +73,27 @@ static __global__ void scan_chunks_kernel(int64_t n, const uint32_t* __restrict_
     if (c == gridDim.x - 1 && lane == 0) out[n] = (uint32_t)sums[gridDim.x];
 }
 
-// out[0..n]: exclusive prefix sums of in[0..n), out[n] = total (written to *total
-// too, after a stream sync). The total must fit in 32 bits.
+// out[0..n]: exclusive prefix sums of in[0..n), out[n] = total modulo 2^32; the total itself is left in
+// sums[scan_chunks(n)] (sums: scan_chunks(n) + 1 words of scratch). Launches only.
+static inline int64_t scan_chunks(int64_t n) { return std::max<int64_t>(1, (n + kScanChunk - 1) / kScanChunk); }
+static inline void scan_u32_launch(fgpu_ctx* ctx, const uint32_t* in, uint32_t* out, int64_t n, unsigned long long* sums) {
+    const int64_t nchunks = scan_chunks(n);
+    scan_chunk_sums_kernel<<<(int)nchunks, 256, 0, ctx->stream>>>(n, in, sums);
+    scan_sums_kernel<<<1, 1024, 0, ctx->stream>>>(nchunks, sums);
+    scan_chunks_kernel<<<(int)nchunks, 32, 0, ctx->stream>>>(n, in, sums, out);
+    ctx->launches += 3;
+}
+
+// the same with its own scratch; the total must fit in 32 bits (written to *total after a stream sync)
 static int scan_u32(fgpu_ctx* ctx, const uint32_t* in, uint32_t* out, int64_t n, uint64_t* total) {
-    const int64_t nchunks = std::max<int64_t>(1, (n + kScanChunk - 1) / kScanChunk);
+    const int64_t nchunks = scan_chunks(n);
     unsigned long long* sums = nullptr;
     if (cudaMalloc(&sums, (nchunks + 1) * sizeof(unsigned long long)) != cudaSuccess) {
         cudaGetLastError();
         ctx->err = "scan: allocation failed";
         return FGPU_ERR_ALLOC;
     }
-    scan_chunk_sums_kernel<<<(int)nchunks, 256, 0, ctx->stream>>>(n, in, sums);
-    scan_sums_kernel<<<1, 1024, 0, ctx->stream>>>(nchunks, sums);
-    scan_chunks_kernel<<<(int)nchunks, 32, 0, ctx->stream>>>(n, in, sums, out);
-    ctx->launches += 3;
+    scan_u32_launch(ctx, in, out, n, sums);
     unsigned long long t = 0;
     cudaMemcpyAsync(&t, sums + nchunks, sizeof(t), cudaMemcpyDeviceToHost, ctx->stream);
     const cudaError_t e = cudaStreamSynchronize(ctx->stream);
