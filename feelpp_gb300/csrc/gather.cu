@@ -30,6 +30,7 @@
 #include <vector>
 
 #include "df64.h"
+#include "entries.h"
 #include "fgpu_core.h"
 #include "scan.cuh"
 #include "asm_device.cuh"
@@ -122,7 +123,7 @@ __global__ void __launch_bounds__(256) gather_slices_kernel(GatherPlan G, const 
 }
 
 // the slices of all problems of a batch (slice_off: prefix sums of their slice counts)
-template <int MODE>
+template <int MODE, bool PIPE>
 __global__ void __launch_bounds__(256) batch_gather_slices_kernel(int nprob, const BatchProblem* __restrict__ probs,
                                                                   const int64_t* __restrict__ slice_off, int64_t total, int accumulate) {
     const int64_t s = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -134,13 +135,13 @@ __global__ void __launch_bounds__(256) batch_gather_slices_kernel(int nprob, con
         else hi = mid - 1;
     }
     const BatchProblem& P = probs[lo];
-    gather_slice<MODE, 4, false>(P.plan, s - slice_off[lo], P.kbuf, P.val, accumulate);
+    gather_slice<MODE, PIPE ? 8 : 4, PIPE>(P.plan, s - slice_off[lo], P.kbuf, P.val, accumulate);
 }
 
 // Vector elasticity: one lane per pair of nodes i <= j, its 3x3 block (row 3i+c, columns 3j+d) summed
 // over the contributions in element order (bit 31 of an index: stored as (j, i), read transposed) and
 // stored with its transpose at (j, i). sia, ja: the scalar pattern.
-template <int MODE>
+template <int MODE, int B>
 __global__ void __launch_bounds__(128) gather_elasticity_slices_kernel(GatherPlan G, const int64_t* __restrict__ sia,
                                                                        const int32_t* __restrict__ ja, const void* __restrict__ kbuf,
                                                                        void* __restrict__ valv, int accumulate) {
@@ -150,50 +151,67 @@ __global__ void __launch_bounds__(128) gather_elasticity_slices_kernel(GatherPla
     if (s >= G.nslices) return;
     const uint32_t r0 = __ldg(G.soff + s), r1 = __ldg(G.soff + s + 1);
     const uint32_t k0 = __ldg(G.pos0 + s * 32 + lane), k1 = __ldg(G.pos1 + s * 32 + lane);
+    // B contributions' blocks in flight, the next indices with them
     df acc[9];
 #pragma unroll
     for (int k = 0; k < 9; ++k) acc[k] = df{0.0f, 0.0f};
-    for (uint32_t r = r0; r < r1; ++r) {
-        const uint32_t g = __ldg(G.sidx + (size_t)r * 32 + lane);
-        if (g == kNoIndex) continue;
-        const bool tr = (g & 0x80000000u) != 0;
-        const V* b = reinterpret_cast<const V*>(kbuf) + (size_t)(g & 0x7FFFFFFFu) * 9;
-        V v[9];
+    uint32_t ix[B];
 #pragma unroll
-        for (int k = 0; k < 9; ++k) v[k] = __ldg(b + k);
+    for (int u = 0; u < B; ++u) ix[u] = r0 + u < r1 ? __ldg(G.sidx + (size_t)(r0 + u) * 32 + lane) : kNoIndex;
+    for (uint32_t r = r0; r < r1; r += B) {
+        V v[B][9];
+        uint32_t cur[B];
 #pragma unroll
-        for (int c = 0; c < 3; ++c)
+        for (int u = 0; u < B; ++u) {
+            cur[u] = ix[u];
+            const V* b = reinterpret_cast<const V*>(kbuf) + (size_t)(cur[u] & 0x7FFFFFFFu) * 9;
 #pragma unroll
-            for (int d = 0; d < 3; ++d) {
-                const V w = tr ? v[d * 3 + c] : v[c * 3 + d];
-                df& a = acc[c * 3 + d];
-                if constexpr (MODE == kModeDF64) a = r == r0 ? df{w.x, w.y} : df_add(a, df{w.x, w.y});
-                else a.hi = r == r0 ? w : f_add(a.hi, w);
-            }
+            for (int k = 0; k < 9; ++k) v[u][k] = cur[u] != kNoIndex ? __ldg(b + k) : V{};
+        }
+#pragma unroll
+        for (int u = 0; u < B; ++u) ix[u] = r + B + u < r1 ? __ldg(G.sidx + (size_t)(r + B + u) * 32 + lane) : kNoIndex;
+#pragma unroll
+        for (int u = 0; u < B; ++u) {
+            if (cur[u] == kNoIndex) continue;
+            const bool tr = (cur[u] & 0x80000000u) != 0;
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    const V w = tr ? v[u][d * 3 + c] : v[u][c * 3 + d];
+                    df& a = acc[c * 3 + d];
+                    if constexpr (MODE == kModeDF64) a = r + u == r0 ? df{w.x, w.y} : df_add(a, df{w.x, w.y});
+                    else a.hi = r + u == r0 ? w : f_add(a.hi, w);
+                }
+        }
     }
     if (k0 == kNoIndex) return;
-    for (int side = 0; side < 2; ++side) {
-        const uint32_t k = side ? k1 : k0;
-        if (k == kNoIndex) break;
-        const int32_t row = k1 == kNoIndex ? __ldg(ja + k0) : __ldg(ja + (side ? k0 : k1));
+    typedef typename std::conditional<MODE == kModeDF64, double, float>::type T;
+    T* const val = reinterpret_cast<T*>(valv);
+    T x[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) {
+        if constexpr (MODE == kModeDF64) x[k] = df2d(acc[k]);
+        else x[k] = acc[k].hi;
+    }
+    auto put = [&](uint32_t k, int32_t row, bool tr) {
         const int64_t s0 = sia[row];
         const int64_t len = sia[row + 1] - s0;
-        const int64_t o = 9 * s0 + 3 * ((int64_t)k - s0);
+        T* const out = val + 9 * s0 + 3 * ((int64_t)k - s0);
 #pragma unroll
         for (int c = 0; c < 3; ++c)
 #pragma unroll
             for (int d = 0; d < 3; ++d) {
-                df a = side ? acc[d * 3 + c] : acc[c * 3 + d];
-                if constexpr (MODE == kModeDF64) {
-                    double* out = reinterpret_cast<double*>(valv) + o + c * 3 * len + d;
-                    if (accumulate) a = df_add(d2df(*out), a);
-                    *out = df2d(a);
-                } else {
-                    float* out = reinterpret_cast<float*>(valv) + o + c * 3 * len + d;
-                    *out = accumulate ? f_add(*out, a.hi) : a.hi;
-                }
+                T* const o = out + c * 3 * len + d;
+                const int q = tr ? d * 3 + c : c * 3 + d;
+                if (!accumulate) *o = x[q];
+                else if constexpr (MODE == kModeDF64) *o = df2d(df_add(d2df(*o), acc[q]));
+                else *o = f_add(*o, x[q]);
             }
-    }
+    };
+    const int32_t j = __ldg(ja + k0), i = k1 == kNoIndex ? j : __ldg(ja + k1);
+    put(k0, i, false);
+    if (k1 != kNoIndex) put(k1, j, true);
 }
 
 // the values of the matrix to a mapped page-locked host buffer
@@ -431,16 +449,21 @@ __global__ void __launch_bounds__(256) bin_rank_kernel(int64_t total, int per, u
     }
 }
 
-template <int FILL>
-void launch_walk(fgpu_ctx* ctx, int blocks, const PlanIn& in, uint16_t* first, const uint32_t* slice0, const uint32_t* soff,
-                 uint32_t* pos0, uint32_t* pos1, uint32_t* sidx) {
-    plan_walk_kernel<FILL, 2><<<blocks, 256, 0, ctx->stream>>>(in, first, slice0, soff, pos0, pos1, sidx, ctx->d_status);
-}
-
 int sm_count(const fgpu_ctx* ctx) {
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
     return std::max(sms, 1);
+}
+
+// All slices resident at once (64 warps per SM): the kernel lasts as long as its longest chain of loads,
+// which the pipelined sum shortens (P1 10x9x11: 3.8 against 6.2 us); where warps queue, the plain sum's
+// fewer instructions win (P2 64^3: 0.380 against 0.400 ms).
+bool one_wave(const fgpu_ctx* ctx, int64_t nslices) { return nslices <= 64 * (int64_t)sm_count(ctx); }
+
+template <int FILL>
+void launch_walk(fgpu_ctx* ctx, int blocks, const PlanIn& in, uint16_t* first, const uint32_t* slice0, const uint32_t* soff,
+                 uint32_t* pos0, uint32_t* pos1, uint32_t* sidx) {
+    plan_walk_kernel<FILL, 2><<<blocks, 256, 0, ctx->stream>>>(in, first, slice0, soff, pos0, pos1, sidx, ctx->d_status);
 }
 
 template <int MODE, bool PIPE>
@@ -455,51 +478,13 @@ void launch_slices(fgpu_ctx* ctx, const fgpu_matrix* A, int threads, int bpsm, i
     }
 }
 
-// the vertices of the cell that a local dof's entity spans, as a bit mask
-uint32_t span_mask(int cell_vertices, int order, int dof) {
-    if (dof < cell_vertices) return 1u << dof;
-    dof -= cell_vertices;
-    uint32_t m = 0;
-    if (cell_vertices == 8) {
-        if (dof < 12) return (1u << kHexEdgeVerts[dof][0]) | (1u << kHexEdgeVerts[dof][1]);
-        if (dof < 18) {
-            for (int k = 0; k < 4; ++k) m |= 1u << kHexFaceVerts[dof - 12][k];
-            return m;
-        }
-        return 0xFFu;
-    }
-    const int per_edge = order - 1;
-    if (dof < 6 * per_edge) return (1u << kEdgeVerts[dof / per_edge][0]) | (1u << kEdgeVerts[dof / per_edge][1]);
-    for (int k = 0; k < 3; ++k) m |= 1u << kFaceVerts[dof - 6 * per_edge][k];
-    return m;
-}
-
 }  // namespace
 
-// Order of an element's upper-triangle entries in the two-phase element buffer: grouped by the smallest
-// vertex set, edge, face or cell that holds both dofs, small ones first, row-major inside a group.
-// order[t]: the pair a * 256 + b (a <= b) of buffer entry t.
+// the order as pairs a * 256 + b (a <= b)
 std::vector<uint16_t> entry_order(int cell_vertices, int order, int n) {
-    std::vector<uint32_t> holders;                 // candidate vertex sets, by size
-    for (int v = 0; v < cell_vertices; ++v) holders.push_back(1u << v);
-    if (cell_vertices == 8) {
-        for (auto& e : kHexEdgeVerts) holders.push_back((1u << e[0]) | (1u << e[1]));
-        for (auto& f : kHexFaceVerts) holders.push_back((1u << f[0]) | (1u << f[1]) | (1u << f[2]) | (1u << f[3]));
-    } else {
-        for (auto& e : kEdgeVerts) holders.push_back((1u << e[0]) | (1u << e[1]));
-        for (auto& f : kFaceVerts) holders.push_back((1u << f[0]) | (1u << f[1]) | (1u << f[2]));
-    }
-    holders.push_back((1u << cell_vertices) - 1u);
-    std::vector<std::vector<uint16_t>> groups(holders.size());
-    for (int a = 0; a < n; ++a)
-        for (int b = a; b < n; ++b) {
-            const uint32_t m = span_mask(cell_vertices, order, a) | span_mask(cell_vertices, order, b);
-            size_t g = 0;
-            while ((holders[g] & m) != m) ++g;
-            groups[g].push_back((uint16_t)(a * 256 + b));
-        }
+    const EntryOrder E = make_entry_order(cell_vertices, order, n);
     std::vector<uint16_t> out;
-    for (auto& g : groups) out.insert(out.end(), g.begin(), g.end());
+    for (int t = 0; t < E.ntri; ++t) out.push_back((uint16_t)(E.a[t] * 256 + E.b[t]));
     return out;
 }
 
@@ -612,7 +597,8 @@ void launch_gather_slices(fgpu_ctx* ctx, const fgpu_matrix* A, int threads, int 
 int launch_gather_phase(fgpu_ctx* ctx, fgpu_matrix* A, int accumulate) {
     PendingEvent ev;
     prof_begin(ctx, "assemble_gather", ev);
-    launch_gather_slices(ctx, A, 256, 0, 4, 0, accumulate);
+    if (one_wave(ctx, A->space->plan.nslices)) launch_gather_slices(ctx, A, 256, 0, 8, 1, accumulate);
+    else launch_gather_slices(ctx, A, 256, 0, 4, 0, accumulate);
     prof_end(ctx, ev);
     FGPU_CUDA_CHECK(ctx, cudaGetLastError());
     return FGPU_OK;
@@ -624,10 +610,15 @@ int launch_gather_elasticity(fgpu_ctx* ctx, const fgpu_matrix* A, int accumulate
     const int blocks = (int)std::max<int64_t>(1, (G.nslices + 3) / 4);
     PendingEvent ev;
     prof_begin(ctx, "assemble_gather_elasticity", ev);
-    if (A->precision == FGPU_F32)
-        gather_elasticity_slices_kernel<kModeF32><<<blocks, 128, 0, ctx->stream>>>(G, P.d_ia, P.d_ja, A->d_kbuf, A->d_val, accumulate);
-    else
-        gather_elasticity_slices_kernel<kModeDF64><<<blocks, 128, 0, ctx->stream>>>(G, P.d_ia, P.d_ja, A->d_kbuf, A->d_val, accumulate);
+    // two blocks in flight per lane (P2 36x28x30: 0.378 ms, 0.635 one at a time); six where every slice is
+    // resident and the longest chain, a vertex's 24 blocks, is what counts (P1 8^3: 48 against 56 us a pass)
+#define EL_GATHER(MODE, B) gather_elasticity_slices_kernel<MODE, B><<<blocks, 128, 0, ctx->stream>>>(G, P.d_ia, P.d_ja, A->d_kbuf, A->d_val, accumulate)
+    if (one_wave(ctx, G.nslices)) {
+        if (A->precision == FGPU_F32) EL_GATHER(kModeF32, 6); else EL_GATHER(kModeDF64, 6);
+    } else {
+        if (A->precision == FGPU_F32) EL_GATHER(kModeF32, 2); else EL_GATHER(kModeDF64, 2);
+    }
+#undef EL_GATHER
     prof_end(ctx, ev);
     FGPU_CUDA_CHECK(ctx, cudaGetLastError());
     return FGPU_OK;
@@ -683,8 +674,13 @@ int launch_batch_gather_slices(fgpu_ctx* ctx, int nprob, const BatchProblem* d_p
     const int blocks = (int)std::max<int64_t>(1, (total_slices + threads / 32 - 1) / (threads / 32));
     PendingEvent ev;
     prof_begin(ctx, "batch_gather", ev);
-    if (f32) batch_gather_slices_kernel<kModeF32><<<blocks, threads, 0, ctx->stream>>>(nprob, d_probs, d_slice_off, total_slices, accumulate);
-    else batch_gather_slices_kernel<kModeDF64><<<blocks, threads, 0, ctx->stream>>>(nprob, d_probs, d_slice_off, total_slices, accumulate);
+#define BATCH_GATHER(MODE, PIPE) batch_gather_slices_kernel<MODE, PIPE><<<blocks, threads, 0, ctx->stream>>>(nprob, d_probs, d_slice_off, total_slices, accumulate)
+    if (one_wave(ctx, total_slices)) {
+        if (f32) BATCH_GATHER(kModeF32, true); else BATCH_GATHER(kModeDF64, true);
+    } else {
+        if (f32) BATCH_GATHER(kModeF32, false); else BATCH_GATHER(kModeDF64, false);
+    }
+#undef BATCH_GATHER
     prof_end(ctx, ev);
     FGPU_CUDA_CHECK(ctx, cudaGetLastError());
     return FGPU_OK;
