@@ -18,17 +18,46 @@ enum GatherMode { kModeF32 = 0, kModeDF64 = 1 };
 // K's entries are formed in FP64 (9 subtractions of vertex coordinates), the rest
 // in df64 (geomap.hpp:1971-1991, 2310-2350). ksc: an extra factor of kappa
 // (a time-dependent coefficient read from device memory).
-__device__ __forceinline__ void geometry_df_record(int64_t e, const double* __restrict__ xyz, const int32_t* __restrict__ tets,
-                                                   const double* __restrict__ kappa, df kc, df mc, df ksc,
+struct GeoElem {                     // what the record of one element is formed from
+    double x[4][3];
+    double kappa;
+};
+__device__ __forceinline__ GeoElem geometry_load(int64_t e, const double* __restrict__ xyz, const int32_t* __restrict__ tets,
+                                                 const double* __restrict__ kappa) {
+    const int4 t = *reinterpret_cast<const int4*>(tets + 4 * e);
+    const int32_t v[4] = {t.x, t.y, t.z, t.w};
+    GeoElem g;
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+        for (int r = 0; r < 3; ++r) g.x[a][r] = xyz[3 * (int64_t)v[a] + r];
+    g.kappa = kappa ? kappa[e] : 0.0;
+    return g;
+}
+// s + e += a b (high product by TwoSum into s, its error and the cross terms into e)
+__device__ __forceinline__ void df_dot_term(df a, df b, float& s, float& e) {
+    const float p = f_mul(a.hi, b.hi);
+    e = f_fma(a.hi, b.lo, e);
+    e = f_fma(a.lo, b.hi, e);
+    e = f_add(e, f_fma(a.hi, b.hi, -p));
+    const df t = two_sum(s, p);
+    s = t.hi;
+    e = f_add(e, t.lo);
+}
+__device__ __forceinline__ df df_dot3(df a0, df b0, df a1, df b1, df a2, df b2) {
+    float s = f_mul(a0.hi, b0.hi);
+    float e = f_fma(a0.hi, b0.lo, f_fma(a0.lo, b0.hi, f_fma(a0.hi, b0.hi, -s)));
+    df_dot_term(a1, b1, s, e);
+    df_dot_term(a2, b2, s, e);
+    return two_sum(s, e);
+}
+__device__ __forceinline__ void geometry_df_record(const GeoElem& g, const double* __restrict__ kappa, df kc, df mc, df ksc,
                                                    float4* __restrict__ o, int* __restrict__ status) {
-    int4 t = *reinterpret_cast<const int4*>(tets + 4 * e);
-    const double* X0 = xyz + 3 * (int64_t)t.x;
-    const double* Xv[3] = {xyz + 3 * (int64_t)t.y, xyz + 3 * (int64_t)t.z, xyz + 3 * (int64_t)t.w};
     df K[9];
 #pragma unroll
     for (int c = 0; c < 3; ++c)
 #pragma unroll
-        for (int r = 0; r < 3; ++r) K[r * 3 + c] = df_scale(d2df(Xv[c][r] - X0[r]), 0.5f);
+        for (int r = 0; r < 3; ++r) K[r * 3 + c] = df_scale(d2df(g.x[c + 1][r] - g.x[0][r]), 0.5f);
     df C[9];
     C[0] = df_sub(df_mul(K[4], K[8]), df_mul(K[5], K[7]));
     C[1] = df_sub(df_mul(K[5], K[6]), df_mul(K[3], K[8]));
@@ -39,24 +68,26 @@ __device__ __forceinline__ void geometry_df_record(int64_t e, const double* __re
     C[6] = df_sub(df_mul(K[1], K[5]), df_mul(K[2], K[4]));
     C[7] = df_sub(df_mul(K[2], K[3]), df_mul(K[0], K[5]));
     C[8] = df_sub(df_mul(K[0], K[4]), df_mul(K[1], K[3]));
-    df det = df_add(df_add(df_mul(K[0], C[0]), df_mul(K[1], C[1])), df_mul(K[2], C[2]));
-    df J = det.hi < 0.0f ? df_neg(det) : det;
+    const df det = df_dot3(K[0], C[0], K[1], C[1], K[2], C[2]);
+    const df J = det.hi < 0.0f ? df_neg(det) : det;
     if (!(J.hi > 0.0f) || !isfinite(J.hi)) atomicOr(status, kStatusBadElement);
-    df inv = df_recip(J);
-    df s = df_mul(df_mul(kappa ? d2df(kappa[e]) : kc, ksc), inv);
+    const df s = df_mul(df_mul(kappa ? d2df(g.kappa) : kc, ksc), df_recip(J));
     const int pa[6] = {0, 1, 2, 0, 0, 1}, pb[6] = {0, 1, 2, 1, 2, 2};
     df c[8];
 #pragma unroll
-    for (int k = 0; k < 6; ++k) {
-        df g = df_add(df_add(df_mul(C[pa[k]], C[pb[k]]), df_mul(C[3 + pa[k]], C[3 + pb[k]])), df_mul(C[6 + pa[k]], C[6 + pb[k]]));
-        c[k] = df_mul(s, g);
-    }
+    for (int k = 0; k < 6; ++k)
+        c[k] = df_mul(s, df_dot3(C[pa[k]], C[pb[k]], C[3 + pa[k]], C[3 + pb[k]], C[6 + pa[k]], C[6 + pb[k]]));
     c[6] = df_mul(mc, J);
     c[7] = J;
     o[0] = make_float4(c[0].hi, c[1].hi, c[2].hi, c[3].hi);
     o[1] = make_float4(c[4].hi, c[5].hi, c[6].hi, c[7].hi);
     o[2] = make_float4(c[0].lo, c[1].lo, c[2].lo, c[3].lo);
     o[3] = make_float4(c[4].lo, c[5].lo, c[6].lo, c[7].lo);
+}
+__device__ __forceinline__ void geometry_df_record(int64_t e, const double* __restrict__ xyz, const int32_t* __restrict__ tets,
+                                                   const double* __restrict__ kappa, df kc, df mc, df ksc,
+                                                   float4* __restrict__ o, int* __restrict__ status) {
+    geometry_df_record(geometry_load(e, xyz, tets, kappa), kappa, kc, mc, ksc, o, status);
 }
 
 // Element-matrix entry K_e(i, j) = sum_k c_k T_k(i, j) (the 7 reference tensors

@@ -7,16 +7,14 @@
 // (vertices, then the edge nodes in e2p order). Element matrices by quadrature:
 //   K_e(i, j) = sum_q dphi_i(q)^T G_q dphi_j(q) + m_q phi_i(q) phi_j(q),
 //   G_q = w_q |det K_q| kappa B_q^T B_q,  m_q = w_q |det K_q| mass,
-// where dphi are reference gradients. One warp per element: the lanes first
-// take one quadrature point each and form G_q, m_q (the map, its cofactors,
-// determinant and inverse) in double-float on the FP32 pipes (binary64 runs at
-// 1/71 of the binary32 rate here; binary32 for FP32 matrices), stored in shared
-// memory; then for every
-// q the lanes form W_q = G_q dphi_j(q) for one local dof each, and each lane
-// adds dphi_i . W_j + m_q phi_i phi_j into the upper-triangle entries it owns
-// (double-float on the FP32 pipes for FP64 matrices, binary32 for FP32). The
-// element matrices go to the two-phase element buffer and the gather map sums
-// them per CSR entry in element order, as for affine elements.
+// where dphi are reference gradients, in double-float on the FP32 pipes for FP64 matrices (binary64 runs
+// at 1/71 of the binary32 rate here). P1 and P2 tetrahedra: one lane per element (ho_lane_kernel). P3
+// tetrahedra and hexahedra (and binary32 without the tensor cores): one warp per element
+// (ho_element_kernel): the lanes first take one quadrature point each and form G_q, m_q in shared memory;
+// then for every q they form W_q = G_q dphi_j(q) for one local dof each, and each lane adds
+// dphi_i . W_j + m_q phi_i phi_j into the upper-triangle entries it owns. The element matrices go to the
+// two-phase element buffer and the gather sums them per CSR entry in element order, as for affine
+// elements.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -24,9 +22,12 @@
 #include <mutex>
 #include <string>
 #include <tuple>
+#include <type_traits>
 #include <vector>
 
 #include "df64.h"
+#include "closed.cuh"
+#include "entries.h"
 #include "fgpu_core.h"
 #include "tc_ptx.cuh"
 
@@ -60,6 +61,7 @@ struct HoTables {
     float* d_qwl = nullptr;    //                            (lo)
     uint8_t* d_ti = nullptr;   // ntri: row of each upper-triangle entry (entry_order)
     uint8_t* d_tj = nullptr;   // ntri: column
+    float2* d_lane = nullptr;  // per point: tables of ho_lane_kernel (P1, P2 tetrahedra)
     float* d_tcB = nullptr;    // tensor-core B operand: per chunk of points, per accumulator, tf32 hi / lo
     std::vector<double> dphi, phi;   // Q n 3, Q n (host copies for building d_tcB)
 };
@@ -72,6 +74,42 @@ cudaError_t up(T** dst, const std::vector<T>& v) {
     cudaError_t e = cudaMalloc(dst, std::max<size_t>(v.size(), 1) * sizeof(T));
     if (e == cudaSuccess && !v.empty()) e = cudaMemcpy(*dst, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice);
     return e;
+}
+
+// ---- tables of ho_lane_kernel, per quadrature point (double-float pairs) ----
+// 2 lambda_1..3, the weight; P2: the products of barycentric derivatives that pairs of basis functions
+// meet, (4 l_a - 1)(4 l_b - 1), a <= b; (4 l_a - 1) 4 l_c; 16 l_c l_d, c <= d; then phi_i phi_j in
+// entry_order.
+constexpr int kLaneVE = 4 + 10, kLaneEE = kLaneVE + 16, kLaneM2 = kLaneEE + 10, kLaneM1 = 4;
+constexpr int lane_stride(int n) { return n == 10 ? kLaneM2 + 56 : kLaneM1 + 10; }   // even: 16-byte rows
+
+std::vector<float2> lane_tables(int order, const RefTables& R) {
+    const int n = R.n, S = lane_stride(n);
+    std::vector<float2> out((size_t)R.Q * S, make_float2(0.0f, 0.0f));
+    const EntryOrder E = make_entry_order(4, order, n);
+    for (int q = 0; q < R.Q; ++q) {
+        double l[4] = {1.0, 0.0, 0.0, 0.0};
+        for (int k = 0; k < 3; ++k) {
+            l[k + 1] = 0.5 * (1.0 + R.qx[3 * q + k]);
+            l[0] -= l[k + 1];
+        }
+        float2* o = &out[(size_t)q * S];
+        auto put = [&](int k, double v) {
+            o[k].x = (float)v;
+            o[k].y = (float)(v - (double)o[k].x);
+        };
+        for (int k = 0; k < 3; ++k) put(k, 2.0 * l[k + 1]);
+        put(3, R.qw[q]);
+        if (n == 10)
+            for (int a = 0; a < 4; ++a)
+                for (int b = 0; b < 4; ++b) {
+                    if (a <= b) put(4 + sym4(a, b), (4.0 * l[a] - 1.0) * (4.0 * l[b] - 1.0));
+                    if (a <= b) put(kLaneEE + sym4(a, b), 16.0 * l[a] * l[b]);
+                    put(kLaneVE + 4 * a + b, (4.0 * l[a] - 1.0) * 4.0 * l[b]);
+                }
+        for (int t = 0; t < E.ntri; ++t) put((n == 10 ? kLaneM2 : kLaneM1) + t, R.phi[q * n + E.a[t]] * R.phi[q * n + E.b[t]]);
+    }
+    return out;
 }
 
 // hex: Q1/Q2 hexahedra (geometry Q1), else P-order tetrahedra with P2 geometry
@@ -127,6 +165,7 @@ HoTables* get_ho_tables(fgpu_ctx* ctx, int order, int qdeg, bool hex = false) {
     if (e == cudaSuccess) e = up(&T->d_qwl, qwl);
     if (e == cudaSuccess) e = up(&T->d_ti, ti);
     if (e == cudaSuccess) e = up(&T->d_tj, tj);
+    if (e == cudaSuccess && !hex && order <= 2) e = up(&T->d_lane, lane_tables(order, R));
     if (e != cudaSuccess) {
         cudaGetLastError();
         ctx->err = std::string("curved-element tables: ") + cudaGetErrorString(e);
@@ -161,19 +200,174 @@ __device__ __forceinline__ double ho_map(const double* X /* GN x 3 */, const dou
 }
 
 __device__ __forceinline__ df ldf(const float* h, const float* l, int k) { return df{h[k], l[k]}; }
-// s + e += a b: the exact product of the high parts (FMA) split into its rounded value, added to s by
-// TwoSum, and its error; the cross terms a.hi b.lo + a.lo b.hi and the TwoSum error go to e
-__device__ __forceinline__ void ho_dot_term(df a, df b, float& s, float& e) {
-    const float p = f_mul(a.hi, b.hi);
-    e = f_fma(a.hi, b.lo, e);
-    e = f_fma(a.lo, b.hi, e);
-    e = f_add(e, f_fma(a.hi, b.hi, -p));
-    const df t = two_sum(s, p);
-    s = t.hi;
-    e = f_add(e, t.lo);
-}
 __device__ __forceinline__ df dfun(float2 v) { return df{v.x, v.y}; }
 __device__ __forceinline__ float2 dfpack(df v) { return make_float2(v.hi, v.lo); }
+
+// the table entry of the product of derivative k of function i with derivative m of function j
+constexpr int bary_product(int i, int k, int j, int m) {
+    if (i < 4 && j < 4) return 4 + sym4(i, j);
+    if (i < 4) return kLaneVE + 4 * i + bary_factor(j, m);
+    if (j < 4) return kLaneVE + 4 * j + bary_factor(i, k);
+    return kLaneEE + sym4(bary_factor(i, k), bary_factor(j, m));
+}
+
+// P1 and P2 on curved tetrahedra in double-float, one lane per element: every step of the geometry and of
+// the entries runs on full warps and nothing is exchanged between lanes (with a warp per element, 24 of 32
+// lanes took a point, 10 of 32 a row of W = G dphi and 55 of 64 slots an entry: 11 023 warp instructions
+// per P2 element against 2 830; P2 32^3, 24 points: 2.01 ms -> 0.70 ms, issue-bound: ncu 65 % issue active
+// with 8 warps per SM; three blocks per SM at 168 registers spill, 0.97 ms).
+//  * The map is quadratic, so its derivatives are linear in the barycentric coordinates:
+//    dx/dxi_c = A_c + sum_d 2 lambda_d h_cd with A_c = 2 d_0c - d_c / 2, h_cc = d_c - 2 d_0c and
+//    h_cd = d_cd - d_0c - d_0d (d_x: node x minus vertex 0; formed once per element in binary64): 27
+//    values per element in shared memory and 27 products per point, not 90, and no cancellation between
+//    absolute coordinates.
+//  * With g_ab = kappa w / |det K| c_a . c_b / 4 for the four barycentric gradients (c_a the cofactor
+//    columns, c_0 = -(c_1 + c_2 + c_3)), a vertex function has one derivative and an edge function two, so
+//    the 55 stiffness entries take 129 products per point (3 x 3 reference gradients: 220, and 90 for W).
+//  * An entry is a compensated dot product over the points (df_dot_term): 110 registers of accumulators,
+//    so eight warps per SM, whose independent chains keep the pipes busy. The four warps of a block take
+//    every fourth point of the same 32 elements and add their sums in warp order at the end: a block per
+//    SM slot lasts a quarter as long as a warp per 32 elements would and the last wave costs little
+//    (P2 32^3: 5.05 waves took the time of 6).
+template <int N>
+__global__ void __launch_bounds__(128, 2) ho_lane_kernel(int64_t nt, const double* __restrict__ xyz, const int32_t* __restrict__ tets,
+                                                         const double* __restrict__ ho, int Q, const float2* __restrict__ tabg,
+                                                         const double* __restrict__ d_kappa, double kappa, double mass,
+                                                         const double* __restrict__ kscale, float2* __restrict__ kbuf,
+                                                         int* __restrict__ status) {
+    constexpr int S = lane_stride(N), NTRI = N * (N + 1) / 2, M0 = N == 10 ? kLaneM2 : kLaneM1;
+    extern __shared__ __align__(16) float2 smem[];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float2* tab = smem;                            // Q x S
+    float2* geo = smem + Q * S + lane;             // 27 values per element, 32 apart: A_c[r], h_cd[r]
+    for (int k = threadIdx.x; k < Q * S; k += 128) tab[k] = tabg[k];
+    const int64_t e0 = (int64_t)blockIdx.x * 32;
+    const bool live = e0 + lane < nt;
+    const int64_t e = live ? e0 + lane : nt - 1;   // lanes past the end repeat the last element and store nothing
+    if (warp < 3) {                                // coordinate r = warp
+        const int r = warp;
+        const int4 t = *reinterpret_cast<const int4*>(tets + 4 * e);
+        const int32_t v[4] = {t.x, t.y, t.z, t.w};
+        const double x0 = xyz[3 * (int64_t)v[0] + r];
+        double d[4][4];                            // d[a][b]: edge node (a, b), d[a][a]: vertex a
+#pragma unroll
+        for (int a = 1; a < 4; ++a) d[a][a] = xyz[3 * (int64_t)v[a] + r] - x0;
+        unrolled<0, 6>([&](auto I) {
+            constexpr int a = kTetE[decltype(I)::value][0], b = kTetE[decltype(I)::value][1];
+            d[a][b] = d[b][a] = ho[18 * e + 3 * decltype(I)::value + r] - x0;
+        });
+#pragma unroll
+        for (int c = 1; c < 4; ++c) geo[(3 * (c - 1) + r) * 32] = dfpack(d2df(fma(2.0, d[0][c], -0.5 * d[c][c])));
+        int k = 0;
+#pragma unroll
+        for (int c = 1; c < 4; ++c)
+#pragma unroll
+            for (int f = c; f < 4; ++f, ++k)
+                geo[(9 + 3 * k + r) * 32] = dfpack(d2df(c == f ? fma(-2.0, d[0][c], d[c][c]) : d[c][f] - (d[0][c] + d[0][f])));
+    }
+    __syncthreads();
+    const df kap = df_mul(d2df(d_kappa ? d_kappa[e] : kappa), d2df(kscale ? *kscale : 1.0));
+    const df quarter = df_scale(kap, 0.25f), massd = d2df(mass);
+    float s[NTRI], er[NTRI];
+#pragma unroll
+    for (int t = 0; t < NTRI; ++t) s[t] = er[t] = 0.0f;
+    bool bad = false;
+#pragma unroll 1
+    for (int q = warp; q < Q; q += 4) {
+        const float2* P = tab + q * S;
+        df g[10], m;
+        {
+            df K[9];                               // K[3 r + c]
+            const df l0 = dfun(P[0]), l1 = dfun(P[1]), l2 = dfun(P[2]);
+#pragma unroll
+            for (int r = 0; r < 3; ++r)
+#pragma unroll
+                for (int c = 0; c < 3; ++c) {
+                    const df a = dfun(geo[(3 * c + r) * 32]);
+                    float ks = a.hi, ke = a.lo;
+                    // h_c0 h_c1 h_c2 among 00 01 02 11 12 22
+                    const int i0 = c, i1 = c == 0 ? 1 : c + 2, i2 = c == 0 ? 2 : c == 1 ? 4 : 5;
+                    df_dot_term(dfun(geo[(9 + 3 * i0 + r) * 32]), l0, ks, ke);
+                    df_dot_term(dfun(geo[(9 + 3 * i1 + r) * 32]), l1, ks, ke);
+                    df_dot_term(dfun(geo[(9 + 3 * i2 + r) * 32]), l2, ks, ke);
+                    K[3 * r + c] = quick_two_sum(ks, ke);
+                }
+            df C[9];
+            C[0] = df_sub(df_mul(K[4], K[8]), df_mul(K[5], K[7]));
+            C[1] = df_sub(df_mul(K[5], K[6]), df_mul(K[3], K[8]));
+            C[2] = df_sub(df_mul(K[3], K[7]), df_mul(K[4], K[6]));
+            C[3] = df_sub(df_mul(K[2], K[7]), df_mul(K[1], K[8]));
+            C[4] = df_sub(df_mul(K[0], K[8]), df_mul(K[2], K[6]));
+            C[5] = df_sub(df_mul(K[1], K[6]), df_mul(K[0], K[7]));
+            C[6] = df_sub(df_mul(K[1], K[5]), df_mul(K[2], K[4]));
+            C[7] = df_sub(df_mul(K[2], K[3]), df_mul(K[0], K[5]));
+            C[8] = df_sub(df_mul(K[0], K[4]), df_mul(K[1], K[3]));
+            const df det = df_add(df_add(df_mul(K[0], C[0]), df_mul(K[1], C[1])), df_mul(K[2], C[2]));
+            const df J = det.hi < 0.0f ? df_neg(det) : det;
+            bad = bad || !(J.hi > 0.0f) || !isfinite(J.hi);
+            const df w = dfun(P[3]);
+            const df sc = df_mul(df_mul(w, quarter), df_recip(J));
+            m = df_mul(df_mul(w, J), massd);
+#pragma unroll
+            for (int a = 1; a < 4; ++a)
+#pragma unroll
+                for (int b = a; b < 4; ++b) {
+                    float ps = 0.0f, pe = 0.0f;
+#pragma unroll
+                    for (int r = 0; r < 3; ++r) df_dot_term(C[3 * r + a - 1], C[3 * r + b - 1], ps, pe);
+                    g[sym4(a, b)] = df_mul(sc, quick_two_sum(ps, pe));
+                }
+#pragma unroll
+            for (int a = 1; a < 4; ++a) g[sym4(0, a)] = df_neg(df_add(df_add(g[sym4(1, a)], g[sym4(2, a)]), g[sym4(3, a)]));
+            g[0] = df_neg(df_add(df_add(g[sym4(0, 1)], g[sym4(0, 2)]), g[sym4(0, 3)]));
+        }
+        unrolled<0, NTRI>([&](auto T) {
+            constexpr int t = decltype(T)::value;
+            constexpr EntryOrder O = make_entry_order(4, N == 10 ? 2 : 1, N);
+            constexpr int i = O.a[t], j = O.b[t];
+            if constexpr (N == 10) {
+                unrolled<0, bary_comps(i) * bary_comps(j)>([&](auto U) {
+                    constexpr int k = decltype(U)::value / bary_comps(j), l = decltype(U)::value % bary_comps(j);
+                    if constexpr (i == j && k > l) return;               // (k, l) and (l, k) of one function are equal
+                    constexpr int pi = bary_product(i, k, j, l), gi = sym4(bary_comp(i, k), bary_comp(j, l));
+                    const df p = dfun(P[pi]);
+                    df_dot_term(g[gi], i == j && k < l ? df_scale(p, 2.0f) : p, s[t], er[t]);
+                });
+            } else {
+                constexpr int gi = sym4(i, j);
+                const df x = two_sum(s[t], g[gi].hi);
+                s[t] = x.hi;
+                er[t] = f_add(er[t], f_add(x.lo, g[gi].lo));
+            }
+            df_dot_term(m, dfun(P[M0 + t]), s[t], er[t]);
+        });
+    }
+    if (bad && live) atomicOr(status, kStatusBadElement);
+    // the four warps' sums, in warp order (over the tables and the geometry)
+    __syncthreads();
+#pragma unroll
+    for (int t = 0; t < NTRI; ++t) smem[(warp * NTRI + t) * 33 + lane] = dfpack(quick_two_sum(s[t], er[t]));
+    __syncthreads();
+    const int cnt = (int)(nt - e0 < 32 ? nt - e0 : 32) * NTRI;
+    for (int k = threadIdx.x; k < cnt; k += 128) {
+        const int el = k / NTRI, t = k - el * NTRI;
+        df v = dfun(smem[t * 33 + el]);
+#pragma unroll
+        for (int w = 1; w < 4; ++w) v = df_add(v, dfun(smem[(w * NTRI + t) * 33 + el]));
+        kbuf[e0 * NTRI + k] = dfpack(v);
+    }
+}
+
+template <int N>
+int launch_ho_lane(fgpu_ctx* ctx, fgpu_matrix* A, const HoTables* T, const double* d_kappa, const fgpu_form_desc* f) {
+    const fgpu_mesh* M = A->space->mesh;
+    auto kern = ho_lane_kernel<N>;
+    const int smem = std::max(T->Q * lane_stride(N) + 27 * 32, 4 * 33 * (N * (N + 1) / 2)) * (int)sizeof(float2);
+    FGPU_CUDA_CHECK(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    kern<<<(int)((M->nt + 31) / 32), 128, smem, ctx->stream>>>(M->nt, M->d_xyz, M->d_tets, M->d_ho, T->Q, T->d_lane, d_kappa, f->kappa,
+                                                                f->mass, f->kappa_scale, (float2*)A->d_kbuf, ctx->d_status);
+    return FGPU_OK;
+}
 
 // LPG lanes per element (32: one element per warp; 8: four elements per warp, for at most 8 points)
 template <int MODE, int N, int GN, int LPG = 32>
@@ -334,10 +528,10 @@ __global__ void __launch_bounds__(128) ho_element_kernel(int64_t nt, const doubl
                 const int i = ti[t], j = tj[t];
                 const int bi = (q * N + i) * 3;
                 if (MODE == kHoDF64) {
-                    ho_dot_term(ldf(Dh, Dl, bi), dfun(WsG[j]), acs[u], ace[u]);
-                    ho_dot_term(ldf(Dh, Dl, bi + 1), dfun(WsG[N + j]), acs[u], ace[u]);
-                    ho_dot_term(ldf(Dh, Dl, bi + 2), dfun(WsG[2 * N + j]), acs[u], ace[u]);
-                    ho_dot_term(dfun(G[6]), df_mul(ldf(Ph, Pl, q * N + i), ldf(Ph, Pl, q * N + j)), acs[u], ace[u]);
+                    df_dot_term(ldf(Dh, Dl, bi), dfun(WsG[j]), acs[u], ace[u]);
+                    df_dot_term(ldf(Dh, Dl, bi + 1), dfun(WsG[N + j]), acs[u], ace[u]);
+                    df_dot_term(ldf(Dh, Dl, bi + 2), dfun(WsG[2 * N + j]), acs[u], ace[u]);
+                    df_dot_term(dfun(G[6]), df_mul(ldf(Ph, Pl, q * N + i), ldf(Ph, Pl, q * N + j)), acs[u], ace[u]);
                 } else {
                     float v = Dh[bi] * WsG[j].x;
                     v = fmaf(Dh[bi + 1], WsG[N + j].x, v);
@@ -868,12 +1062,13 @@ int launch_assemble_ho(fgpu_ctx* ctx, fgpu_matrix* A, const fgpu_form_desc* f, c
         if (rc) return rc;
     } else {
         switch (V->n) {
-            case 4: if (f32) HO_LAUNCH(kHoF32, 4); else HO_LAUNCH(kHoDF64, 4); break;
-            case 10: if (f32) HO_LAUNCH(kHoF32, 10); else HO_LAUNCH(kHoDF64, 10); break;
+            case 4: if (f32) HO_LAUNCH(kHoF32, 4); else rc = launch_ho_lane<4>(ctx, A, T, d_kappa, f); break;
+            case 10: if (f32) HO_LAUNCH(kHoF32, 10); else rc = launch_ho_lane<10>(ctx, A, T, d_kappa, f); break;
             default: if (f32) HO_LAUNCH(kHoF32, 20); else HO_LAUNCH(kHoDF64, 20); break;
         }
     }
 #undef HO_LAUNCH
+    if (rc) return rc;
     prof_end(ctx, ev);
     ctx->launches++;
     FGPU_CUDA_CHECK(ctx, cudaGetLastError());
