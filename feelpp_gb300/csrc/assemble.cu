@@ -30,6 +30,7 @@
 #include "fgpu_core.h"
 #include "scan.cuh"
 #include "asm_device.cuh"
+#include "closed.cuh"
 
 namespace fgpu {
 
@@ -44,6 +45,35 @@ static cudaError_t upload(const std::vector<T>& h, T** d) {
     cudaError_t e = cudaMalloc((void**)d, h.size() * sizeof(T));
     if (e != cudaSuccess) return e;
     return cudaMemcpy(*d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice);
+}
+
+// Whether the rule's reference tensors are the exact integrals that closed.cuh sums (P1 and P2, a rule of
+// degree 2p or more): every tensor against the closed form, to the rounding of the 15-digit rules.
+static bool closed_form_holds(const RefTables& R) {
+    const int n = R.n;
+    if (n != 4 && n != 10) return false;
+    double top = 0.0, off = 0.0;
+    for (int k = 0; k < 7; ++k) {
+        // h_ab (P1) or h_ab / 5 (P2) of the unit coefficient k, as closed_entries forms it
+        const int pa[6] = {1, 2, 3, 1, 1, 2}, pb[6] = {1, 2, 3, 2, 3, 3};
+        double h[4][4] = {};
+        if (k < 6) h[pa[k]][pb[k]] = h[pb[k]][pa[k]] = n == 10 ? 1.0 / 15.0 : 1.0 / 3.0;
+        for (int a = 1; a < 4; ++a) h[0][a] = h[a][0] = -(h[1][a] + h[2][a] + h[3][a]);
+        h[0][0] = -(h[0][1] + h[0][2] + h[0][3]);
+        for (int i = 0; i < n; ++i)
+            for (int j = 0; j < n; ++j) {
+                double v = 0.0;
+                if (k == 6) v = n == 10 ? p2_mass_coef(i, j) / 315.0 : (i == j ? 2.0 : 1.0) / 15.0;
+                else if (n == 4) v = h[i][j];
+                else
+                    for (int q = 0; q < bary_comps(i); ++q)
+                        for (int m = 0; m < bary_comps(j); ++m) v += p2_stiff_coef(i, q, j, m) * h[bary_comp(i, q)][bary_comp(j, m)];
+                const double t = R.T7[((size_t)k * n + i) * n + j];
+                top = std::max(top, std::fabs(t));
+                off = std::max(off, std::fabs(t - v));
+            }
+    }
+    return off <= 1e-14 * top * n;
 }
 
 DevTables* get_dev_tables(int order, int qdeg, std::string& err) {
@@ -89,6 +119,7 @@ DevTables* get_dev_tables(int order, int qdeg, std::string& err) {
             Sbl[(size_t)ab * ntri + t] = (float)(v - (double)(float)v);
         }
     }
+    D->closed = closed_form_holds(R);
     cudaError_t e = cudaSuccess;
     if (e == cudaSuccess) e = upload(T7bh, &D->d_T7bh);
     if (e == cudaSuccess) e = upload(T7bl, &D->d_T7bl);
@@ -1315,19 +1346,45 @@ __device__ __forceinline__ void tri_group_entries(void* __restrict__ kbuf, int64
 // ---- two-phase batches: the element kernel and the gather-map kernel of the
 // single-problem path over all problems (same per-entry arithmetic and order,
 // so each matrix gets the bits FGPU_ALGO_TWO_PHASE gives it alone) ----
-// upper-triangle tables of orders 1..3 in one block: 7 n(n+1)/2 each
-__host__ __device__ constexpr int batch_tri_off(int order) { return order == 1 ? 0 : order == 2 ? 7 * 10 : 7 * 10 + 7 * 55; }
-constexpr int kBatchTriFloats = 7 * 10 + 7 * 55 + 7 * 210;
+// the P1 and P2 problems of a batch (grp_off counts their groups only): the single-problem kernel's groups
+template <int MODE>
+__global__ void __launch_bounds__(128) batch_element_closed_kernel(int nprob, const BatchProblem* __restrict__ probs,
+                                                                   const int64_t* __restrict__ grp_off, int64_t total_groups,
+                                                                   int* __restrict__ status) {
+    extern __shared__ __align__(128) unsigned char stages[];
+    unsigned char* stage = stages + (threadIdx.x >> 5) * closed_stage_bytes<MODE, 10>();
+    const int64_t nw = (int64_t)gridDim.x * 4;
+    int p = -1;
+    int64_t pg0 = 0, pg1 = 0;
+    for (int64_t g = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5); g < total_groups; g += nw) {
+        if (g < pg0 || g >= pg1) {
+            p = batch_find(grp_off, nprob, g);
+            pg0 = grp_off[p];
+            pg1 = grp_off[p + 1];
+        }
+        const BatchProblem& P = probs[p];
+        const int64_t e0 = (g - pg0) * 32;
+        const int cnt = (int)(P.nt - e0 < 32 ? P.nt - e0 : 32);
+        const df kc = d2df(P.kappa_c), mc = d2df(P.mass), one = df{1.0f, 0.0f};
+        const int lane = threadIdx.x & 31;
+        const GeoElem in = geometry_load(e0 + (lane < cnt ? lane : cnt - 1), P.xyz, P.tets, P.kappa);
+        if (P.order == 1) closed_group<MODE, 4>(e0, cnt, in, P.kappa, kc, closed_mass<4>(mc), closed_stiff<4>(one), stage, P.kbuf, status);
+        else closed_group<MODE, 10>(e0, cnt, in, P.kappa, kc, closed_mass<10>(mc), closed_stiff<10>(one), stage, P.kbuf, status);
+    }
+    closed_stores_done();
+}
 
+// the P3 problems
 template <int MODE>
 __global__ void __launch_bounds__(256) batch_element_kernel(int nprob, const BatchProblem* __restrict__ probs,
                                                             const int64_t* __restrict__ grp_off, int64_t total_groups,
                                                             const float* __restrict__ Thg, const float* __restrict__ Tlg,
                                                             int* __restrict__ status) {
-    __shared__ float Th[kBatchTriFloats];
-    __shared__ float Tl[MODE == kModeDF64 ? kBatchTriFloats : 1];
+    constexpr int NT = 7 * 210;
+    __shared__ float Th[NT];
+    __shared__ float Tl[MODE == kModeDF64 ? NT : 1];
     __shared__ float4 srec[8 * 32 * 4];                  // per warp: the records of 32 elements
-    for (int k = threadIdx.x; k < kBatchTriFloats; k += blockDim.x) {
+    for (int k = threadIdx.x; k < NT; k += blockDim.x) {
         Th[k] = Thg[k];
         if (MODE == kModeDF64) Tl[k] = Tlg[k];
     }
@@ -1351,64 +1408,46 @@ __global__ void __launch_bounds__(256) batch_element_kernel(int nprob, const Bat
             geometry_df_record(e0 + lane, P.xyz, P.tets, P.kappa, d2df(P.kappa_c), d2df(P.mass), df{1.0f, 0.0f}, wrec + 4 * lane,
                                status);
         __syncwarp();
-        float th0[7], tl0[7], th1[7], tl1[7];
-        const int to = batch_tri_off(P.order);
-        if (P.order == 1) {
-            tri_lane_tables<MODE, 4>(Th + to, Tl + to, lane, th0, tl0, th1, tl1);
-            tri_group_entries<MODE, 4>(P.kbuf, e0, cnt, wrec, Th + to, Tl + to, lane, th0, tl0, th1, tl1);
-        } else if (P.order == 2) {
-            tri_lane_tables<MODE, 10>(Th + to, Tl + to, lane, th0, tl0, th1, tl1);
-            tri_group_entries<MODE, 10>(P.kbuf, e0, cnt, wrec, Th + to, Tl + to, lane, th0, tl0, th1, tl1);
-        } else {
-            tri_group_entries<MODE, 20>(P.kbuf, e0, cnt, wrec, Th + to, Tl + to, lane, th0, tl0, th1, tl1);
-        }
+        tri_group_entries<MODE, 20>(P.kbuf, e0, cnt, wrec, Th, Tl, lane, nullptr, nullptr, nullptr, nullptr);
         __syncwarp();
     }
 }
 
-static std::map<int, std::pair<float*, float*>> g_btri;
-static int batch_tri_tables(fgpu_ctx* ctx, float** h, float** l) {
-    std::lock_guard<std::mutex> lock(g_btab_mutex);
-    auto it = g_btri.find(ctx->device);
-    if (it != g_btri.end()) { *h = it->second.first; *l = it->second.second; return FGPU_OK; }
-    float *dh = nullptr, *dl = nullptr;
-    FGPU_CUDA_CHECK(ctx, cudaMalloc(&dh, kBatchTriFloats * sizeof(float)));
-    FGPU_CUDA_CHECK(ctx, cudaMalloc(&dl, kBatchTriFloats * sizeof(float)));
-    for (int order = 1; order <= 3; ++order) {
-        std::string err;
-        DevTables* t = get_dev_tables(order, 2 * order, err);
-        if (!t) { ctx->err = err; return FGPU_ERR_INVALID; }
-        const size_t nb = (size_t)7 * (t->n * (t->n + 1) / 2) * sizeof(float);
-        FGPU_CUDA_CHECK(ctx, cudaMemcpy(dh + batch_tri_off(order), t->d_T7bh, nb, cudaMemcpyDeviceToDevice));
-        FGPU_CUDA_CHECK(ctx, cudaMemcpy(dl + batch_tri_off(order), t->d_T7bl, nb, cudaMemcpyDeviceToDevice));
-    }
-    g_btri[ctx->device] = {dh, dl};
-    *h = dh;
-    *l = dl;
-    return FGPU_OK;
-}
-
-int launch_batch_two_phase(fgpu_ctx* ctx, int nprob, const BatchProblem* d_probs, const int64_t* d_grp_off,
-                           int64_t total_groups, const int64_t* d_slice_off, int64_t total_slices, int f32, int threads,
-                           int accumulate) {
-    float *Th = nullptr, *Tl = nullptr;
-    int rc = batch_tri_tables(ctx, &Th, &Tl);
-    if (rc) return rc;
+int launch_batch_two_phase(fgpu_ctx* ctx, int nprob, const BatchProblem* d_probs, const int64_t* d_closed_off, int64_t closed_groups,
+                           const int64_t* d_p3_off, int64_t p3_groups, const int64_t* d_slice_off, int64_t total_slices, int f32,
+                           int threads, int accumulate) {
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
-    {
-        const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((total_groups + 7) / 8, (int64_t)sms * 16));
-        PendingEvent ev;
-        prof_begin(ctx, "batch_elements", ev);
-        if (f32)
-            batch_element_kernel<kModeF32><<<(int)blocks, 256, 0, ctx->stream>>>(nprob, d_probs, d_grp_off, total_groups, Th, Tl,
-                                                                                 ctx->d_status);
-        else
-            batch_element_kernel<kModeDF64><<<(int)blocks, 256, 0, ctx->stream>>>(nprob, d_probs, d_grp_off, total_groups, Th, Tl,
-                                                                                  ctx->d_status);
-        prof_end(ctx, ev);
+    PendingEvent ev;
+    prof_begin(ctx, "batch_elements", ev);
+    if (closed_groups > 0) {
+        const int blocks = (int)std::min<int64_t>((closed_groups + 3) / 4, (int64_t)sms * 16);
+        if (f32) {
+            constexpr int smem = 4 * closed_stage_bytes<kModeF32, 10>();
+            FGPU_CUDA_CHECK(ctx, cudaFuncSetAttribute(batch_element_closed_kernel<kModeF32>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+            batch_element_closed_kernel<kModeF32><<<blocks, 128, smem, ctx->stream>>>(nprob, d_probs, d_closed_off, closed_groups, ctx->d_status);
+        } else {
+            constexpr int smem = 4 * closed_stage_bytes<kModeDF64, 10>();
+            FGPU_CUDA_CHECK(ctx, cudaFuncSetAttribute(batch_element_closed_kernel<kModeDF64>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+            batch_element_closed_kernel<kModeDF64><<<blocks, 128, smem, ctx->stream>>>(nprob, d_probs, d_closed_off, closed_groups, ctx->d_status);
+        }
         FGPU_CUDA_CHECK(ctx, cudaGetLastError());
     }
+    if (p3_groups > 0) {
+        std::string err;
+        const DevTables* t = get_dev_tables(3, 6, err);
+        if (!t) { ctx->err = err; return FGPU_ERR_INVALID; }
+        const int blocks = (int)std::min<int64_t>((p3_groups + 7) / 8, (int64_t)sms * 16);
+        if (f32)
+            batch_element_kernel<kModeF32><<<blocks, 256, 0, ctx->stream>>>(nprob, d_probs, d_p3_off, p3_groups, t->d_T7bh, t->d_T7bl,
+                                                                           ctx->d_status);
+        else
+            batch_element_kernel<kModeDF64><<<blocks, 256, 0, ctx->stream>>>(nprob, d_probs, d_p3_off, p3_groups, t->d_T7bh, t->d_T7bl,
+                                                                            ctx->d_status);
+        if (closed_groups > 0) ctx->launches++;
+        FGPU_CUDA_CHECK(ctx, cudaGetLastError());
+    }
+    prof_end(ctx, ev);
     return launch_batch_gather_slices(ctx, nprob, d_probs, d_slice_off, total_slices, f32, threads, accumulate);
 }
 
@@ -1482,6 +1521,33 @@ __global__ void __launch_bounds__(256) element_tri_kernel(int64_t nt, GeoIn geo,
     }
 }
 
+// Phase 1 where closed.cuh applies: one lane per element, the 32 elements of a warp staged in shared memory
+// and stored to the buffer as one contiguous piece by a bulk copy (a piece is a multiple of 16 bytes from a
+// 16-byte boundary; the last, partial one by plain stores). The next group's coordinates are loaded under
+// this group's arithmetic. P2 64^3 (692 MB written): 0.193 ms, 0.330 with the seven-term sums of
+// element_tri_kernel; binary32 P2 47x50x49 (152 MB): 0.048, 0.055 before. Issue-bound still (ncu at P2
+// 48^3: 61 % issue active with the 14 warps per SM that the staging leaves, DRAM 37 %): of about 2 850
+// instructions per warp of elements the geometry takes 900 and the entries 1 300.
+template <int MODE, int N>
+__global__ void __launch_bounds__(256) element_closed_kernel(int64_t nt, GeoIn geo, void* __restrict__ kbuf, int* __restrict__ status) {
+    extern __shared__ __align__(128) unsigned char stages[];
+    unsigned char* stage = stages + (threadIdx.x >> 5) * closed_stage_bytes<MODE, N>();
+    const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
+    const df kc = d2df(geo.kc), mc = closed_mass<N>(d2df(geo.mc));
+    const df ksc = closed_stiff<N>(geo.kscale ? d2df(*geo.kscale) : df{1.0f, 0.0f});
+    const int lane = threadIdx.x & 31;
+    int64_t e0 = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 32;
+    // (lanes past the end load the last element and store nothing)
+    GeoElem in = geometry_load(e0 + lane < nt ? e0 + lane : nt - 1, geo.xyz, geo.tets, geo.kappa);
+    for (; e0 < nt; e0 += nw * 32) {
+        const GeoElem cur = in;
+        const int64_t next = e0 + nw * 32;
+        if (next < nt) in = geometry_load(next + lane < nt ? next + lane : nt - 1, geo.xyz, geo.tets, geo.kappa);
+        closed_group<MODE, N>(e0, (int)(nt - e0 < 32 ? nt - e0 : 32), cur, geo.kappa, kc, mc, ksc, stage, kbuf, status);
+    }
+    closed_stores_done();
+}
+
 // Launch shape of the two-phase kernels: threads per block and blocks per SM of the element kernel
 // and of the gather (64: one warp per slice), the gather's contributions per load batch and whether
 // its next indices are loaded ahead. None changes the values.
@@ -1495,6 +1561,14 @@ static void launch_element_tri(fgpu_ctx* ctx, fgpu_matrix* A, const DevTables* t
     const int64_t nt = A->space->mesh->nt;
     const int64_t warps = (nt + 31) / 32, wpb = sh.el_threads / 32;       // 32 elements per warp
     const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((warps + wpb - 1) / wpb, (int64_t)sms * sh.el_bpsm));
+    if constexpr (N <= 10) {
+        if (tab->closed) {
+            const int smem = (int)wpb * closed_stage_bytes<MODE, N>();
+            cudaFuncSetAttribute(element_closed_kernel<MODE, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+            element_closed_kernel<MODE, N><<<(int)blocks, sh.el_threads, smem, ctx->stream>>>(nt, *geo, A->d_kbuf, ctx->d_status);
+            return;
+        }
+    }
     element_tri_kernel<MODE, N><<<(int)blocks, sh.el_threads, 0, ctx->stream>>>(nt, *geo, tab->d_T7bh, tab->d_T7bl, A->d_kbuf,
                                                                              ctx->d_status);
 }

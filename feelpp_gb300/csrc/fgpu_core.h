@@ -368,6 +368,7 @@ struct DevTables {                     // device copies of the reference tables
     float* d_T7th = nullptr;           // the same split in upper-triangle order: 7 x n(n+1)/2
     float* d_T7tl = nullptr;
     uint16_t* d_tri = nullptr;         // n x n: (i, j) -> upper-triangle index of (min, max)
+    bool closed = false;               // closed.cuh's closed form equals these tensors
     float* d_T7bh = nullptr;           // the split in the two-phase element buffer's order (entry_order)
     float* d_T7bl = nullptr;
     float* d_Sbh = nullptr;            // elasticity tensors S_ab in that order, df64 split: 9 x n(n+1)/2
@@ -471,9 +472,9 @@ struct BatchLaunch {                 // launch configuration picked by the batch
 };
 int launch_batch_geometry(fgpu_ctx* ctx, int nprob, const BatchProblem* d_probs, const int64_t* d_elem_off,
                           int64_t total_elems);
-int launch_batch_two_phase(fgpu_ctx* ctx, int nprob, const BatchProblem* d_probs, const int64_t* d_grp_off,
-                           int64_t total_groups, const int64_t* d_slice_off, int64_t total_slices, int f32, int threads,
-                           int accumulate);
+int launch_batch_two_phase(fgpu_ctx* ctx, int nprob, const BatchProblem* d_probs, const int64_t* d_closed_off, int64_t closed_groups,
+                           const int64_t* d_p3_off, int64_t p3_groups, const int64_t* d_slice_off, int64_t total_slices, int f32,
+                           int threads, int accumulate);
 int launch_batch_gather_slices(fgpu_ctx* ctx, int nprob, const BatchProblem* d_probs, const int64_t* d_slice_off, int64_t total_slices,
                                int f32, int threads, int accumulate);
 int launch_batch_gather(fgpu_ctx* ctx, int nprob, const BatchProblem* d_probs, const int64_t* d_row_off,

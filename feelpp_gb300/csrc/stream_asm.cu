@@ -32,6 +32,7 @@
 #include <vector>
 
 #include "asm_device.cuh"
+#include "closed.cuh"
 #include "df64.h"
 #include "fgpu_core.h"
 
@@ -90,6 +91,7 @@ struct StreamArgs {
     void* val;
     double* hout;                         // mapped page-locked host copy of the values (FP64) or null
     int accumulate;
+    bool closed;                          // element matrices in closed form (closed.cuh)
     const int32_t* ticket;                // >= 0: element task k; < 0: gather task -(s + 1)
     const int32_t* e_need_g;              // per element task: gather watermark to wait for
     const int32_t* g_need_e;              // per gather task: element watermark to wait for
@@ -228,8 +230,14 @@ __global__ void __launch_bounds__(kThreads, 3) stream_assemble_kernel(StreamArgs
     float* acc = accb + (size_t)warp * RPW * a.maxrow * ACCW;
     for (int k = lane; k < RPW * a.maxrow * ACCW; k += 32) acc[k] = MODE == kModeDF64 ? 0.0f : -0.0f;
     const uint64_t keep = evict_last_policy();
-    const df kc = d2df(a.kappa_c), mc = d2df(a.mass);
-    const df ksc = a.kscale ? d2df(*a.kscale) : df{1.0f, 0.0f};
+    const df kc = d2df(a.kappa_c);
+    df mc = d2df(a.mass), ksc = a.kscale ? d2df(*a.kscale) : df{1.0f, 0.0f};
+    if constexpr (N <= 10) {
+        if (a.closed) {
+            mc = closed_mass<N>(mc);
+            ksc = closed_stiff<N>(ksc);
+        }
+    }
     uint32_t* abort = a.ctl + 3;
     uint32_t* e_done = a.ctl + 4;
     uint32_t* g_done = e_done + a.ne;
@@ -261,6 +269,17 @@ __global__ void __launch_bounds__(kThreads, 3) stream_assemble_kernel(StreamArgs
             const int esub = lane / NTRI < EPW ? lane / NTRI : EPW;
             const int t0 = EPW > 1 ? lane - esub * NTRI : lane;
             const int64_t slot0 = e0 & a.ring_mask;
+            if constexpr (N <= 10) {
+                if (a.closed && tid < cnt) {
+                    // the two-phase kernel's closed form (same bits), one lane per element
+                    closed_entries<MODE, N>(reinterpret_cast<const float4*>(rec + 16 * tid), [&](auto I, VT v) {
+                        constexpr EntryOrder O = make_entry_order(4, N == 10 ? 2 : 1, N);
+                        constexpr int i = O.a[decltype(I)::value], j = O.b[decltype(I)::value], tt = i * N - i * (i - 1) / 2 + j - i;
+                        st_keep(reinterpret_cast<VT*>(a.ring) + (slot0 + tid) * NTRI + tt, v, keep);
+                    });
+                }
+            }
+            if (!a.closed)
             for (int le = warp * EPW + esub; esub < EPW && le < cnt; le += kWarps * EPW) {
                 float ch[7], cl[7];
                 const float* r = rec + 16 * le;
@@ -606,6 +625,7 @@ static int run_streamed(fgpu_ctx* ctx, fgpu_matrix* A, const DevTables* tab, con
     args.Th = tab->d_T7th;                  // binary32 matrices use the high parts (fl32 of the tensors)
     args.Tl = tab->d_T7tl;
     args.tri = tab->d_tri;
+    args.closed = tab->closed;
     args.ring = A->d_kbuf;
     args.ring_mask = plan.ring - 1;
     args.val = A->d_val;
