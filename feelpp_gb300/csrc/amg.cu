@@ -426,7 +426,7 @@ int amg_vcycle_f32(fgpu_amg* M, const float* r, const int* stop, const float** x
     fgpu_amg::Level& V = M->L[0];
     cudaStream_t st = M->ctx->stream;
     if (!M->xacc) {
-        if (cudaMalloc(&M->xacc, V.n * sizeof(float)) != cudaSuccess || cudaMalloc(&M->tres, V.n * sizeof(float)) != cudaSuccess) {
+        if (pool_malloc(st, &M->xacc, V.n * sizeof(float)) != cudaSuccess || pool_malloc(st, &M->tres, V.n * sizeof(float)) != cudaSuccess) {
             cudaGetLastError();
             return nl;                // no room: one cycle
         }
@@ -474,10 +474,10 @@ template PcHook<PolF32> amg_pc_hook<PolF32>(fgpu_amg*);
 namespace {
 
 void free_level(fgpu_amg::Level& V) {
-    cudaFree(V.dinv);
-    cudaFree(V.s_ptr); cudaFree(V.s_len); cudaFree(V.s_perm); cudaFree(V.s_col); cudaFree(V.s_val);
-    cudaFree(V.p_ia); cudaFree(V.p_ja); cudaFree(V.p_a); cudaFree(V.r_ia); cudaFree(V.r_ja); cudaFree(V.r_a);
-    cudaFree(V.x); cudaFree(V.b); cudaFree(V.w); cudaFree(V.d0); cudaFree(V.d1); cudaFree(V.e);
+    pool_free(V.dinv);
+    pool_free(V.s_ptr); pool_free(V.s_len); pool_free(V.s_perm); pool_free(V.s_col); pool_free(V.s_val);
+    pool_free(V.p_ia); pool_free(V.p_ja); pool_free(V.p_a); pool_free(V.r_ia); pool_free(V.r_ja); pool_free(V.r_a);
+    pool_free(V.x); pool_free(V.b); pool_free(V.w); pool_free(V.d0); pool_free(V.d1); pool_free(V.e);
     V = fgpu_amg::Level();
 }
 
@@ -498,16 +498,18 @@ void cheb_coefs(fgpu_amg::Level& V, int K) {
     }
 }
 
+// (in stream order: the block may have been freed by work still queued on the stream)
 template <typename T>
-cudaError_t upload(T** dst, const T* src, size_t n) {
-    cudaError_t e = cudaMalloc(dst, std::max<size_t>(n, 1) * sizeof(T));
-    if (e == cudaSuccess && n) e = cudaMemcpy(*dst, src, n * sizeof(T), cudaMemcpyHostToDevice);
+cudaError_t upload(cudaStream_t stream, T** dst, const T* src, size_t n) {
+    cudaError_t e = pool_malloc(stream, dst, std::max<size_t>(n, 1) * sizeof(T));
+    if (e == cudaSuccess && n) e = cudaMemcpyAsync(*dst, src, n * sizeof(T), cudaMemcpyHostToDevice, stream);
+    if (e == cudaSuccess && n) e = cudaStreamSynchronize(stream);
     return e;
 }
 
 // SELL-C-sigma of a host CSR: rows sorted by length (descending, ties by row) inside windows
 // of 256 rows, slices of 32 rows padded to their longest row (padding: column = the row, value 0)
-cudaError_t upload_sell(fgpu_amg::Level& V, const HostCsr& A) {
+cudaError_t upload_sell(cudaStream_t stream, fgpu_amg::Level& V, const HostCsr& A) {
     constexpr int kC = 32, kSigma = 256;
     const int64_t n = A.nrows;
     V.nslices = (n + kC - 1) / kC;
@@ -541,11 +543,11 @@ cudaError_t upload_sell(fgpu_amg::Level& V, const HostCsr& A) {
             val[base + k * kC] = real ? (float)A.a[p] : 0.0f;
         }
     }
-    cudaError_t e = upload(&V.s_ptr, ptr.data(), ptr.size());
-    if (e == cudaSuccess) e = upload(&V.s_len, len.data(), len.size());
-    if (e == cudaSuccess) e = upload(&V.s_perm, perm.data(), perm.size());
-    if (e == cudaSuccess) e = upload(&V.s_col, col.data(), col.size());
-    if (e == cudaSuccess) e = upload(&V.s_val, val.data(), val.size());
+    cudaError_t e = upload(stream, &V.s_ptr, ptr.data(), ptr.size());
+    if (e == cudaSuccess) e = upload(stream, &V.s_len, len.data(), len.size());
+    if (e == cudaSuccess) e = upload(stream, &V.s_perm, perm.data(), perm.size());
+    if (e == cudaSuccess) e = upload(stream, &V.s_col, col.data(), col.size());
+    if (e == cudaSuccess) e = upload(stream, &V.s_val, val.data(), val.size());
     return e;
 }
 
@@ -580,8 +582,8 @@ int upload_level0_device(fgpu_ctx* ctx, const fgpu_matrix* A, fgpu_amg::Level& V
     V.s_len = L->d_slice_len; L->d_slice_len = nullptr;
     V.s_perm = L->d_perm; L->d_perm = nullptr;
     V.s_col = L->d_col; L->d_col = nullptr;
-    FGPU_CUDA_CHECK(ctx, cudaMalloc(&V.s_val, std::max<int64_t>(L->nstored, 1) * sizeof(float)));
-    FGPU_CUDA_CHECK(ctx, cudaMalloc(&V.dinv, std::max<int64_t>(V.n, 1) * sizeof(float)));
+    FGPU_CUDA_CHECK(ctx, pool_malloc(ctx->stream, &V.s_val, std::max<int64_t>(L->nstored, 1) * sizeof(float)));
+    FGPU_CUDA_CHECK(ctx, pool_malloc(ctx->stream, &V.dinv, std::max<int64_t>(V.n, 1) * sizeof(float)));
     const int g = (int)std::max<int64_t>(1, std::min<int64_t>((L->nstored + 255) / 256, 152 * 32));
     amg_sell_values_kernel<<<g, 256, 0, ctx->stream>>>(L->nstored, L->d_src, (const double*)A->d_val, V.s_val);
     const int gd = (int)std::max<int64_t>(1, std::min<int64_t>((V.n + 255) / 256, 152 * 16));
@@ -592,10 +594,10 @@ int upload_level0_device(fgpu_ctx* ctx, const fgpu_matrix* A, fgpu_amg::Level& V
     return FGPU_OK;
 }
 
-cudaError_t upload_f32(float** dst, const std::vector<double>& v) {
+cudaError_t upload_f32(cudaStream_t stream, float** dst, const std::vector<double>& v) {
     std::vector<float> f(v.size());
     for (size_t i = 0; i < v.size(); ++i) f[i] = (float)v[i];
-    return upload(dst, f.data(), f.size());
+    return upload(stream, dst, f.data(), f.size());
 }
 
 }  // namespace
@@ -608,7 +610,7 @@ static __global__ void amg_f32_kernel(int64_t n, const double* __restrict__ a, f
 // prolongator / restriction of a device-built level: the CSR index arrays are taken over, the values
 // rounded to binary32 (the host path's (float)a)
 static int take_transfer(fgpu_ctx* ctx, AmgDevCsr& D, int64_t** ia, int32_t** ja, float** a) {
-    FGPU_CUDA_CHECK(ctx, cudaMalloc(a, std::max<int64_t>(D.nnz, 1) * sizeof(float)));
+    FGPU_CUDA_CHECK(ctx, pool_malloc(ctx->stream, a, std::max<int64_t>(D.nnz, 1) * sizeof(float)));
     const int g = (int)std::max<int64_t>(1, std::min<int64_t>((D.nnz + 255) / 256, 152 * 16));
     amg_f32_kernel<<<g, 256, 0, ctx->stream>>>(D.nnz, D.a, *a);
     ctx->launches++;
@@ -683,8 +685,8 @@ int amg_setup(fgpu_ctx* ctx, const fgpu_matrix* A, const fgpu_amg_cfg* cfg, fgpu
             for (int64_t i = 0; i < V.n; ++i)
                 for (int64_t p = HA.ia[i]; p < HA.ia[i + 1]; ++p)
                     if (HA.ja[p] == i) dinv[i] = 1.0 / HA.a[p];
-            FGPU_CUDA_CHECK(ctx, upload_f32(&V.dinv, dinv));
-            FGPU_CUDA_CHECK(ctx, upload_sell(V, HA));
+            FGPU_CUDA_CHECK(ctx, upload_f32(ctx->stream, &V.dinv, dinv));
+            FGPU_CUDA_CHECK(ctx, upload_sell(ctx->stream, V, HA));
         }
         if (!coarsest && dev) {
             AmgDevLevel& dl = D.levels[l];
@@ -700,17 +702,17 @@ int amg_setup(fgpu_ctx* ctx, const fgpu_matrix* A, const fgpu_amg_cfg* cfg, fgpu
             V.r_nnz = (int64_t)hl->R.ja.size();
             V.pG = lanes_for(hl->P.nrows, V.p_nnz);
             V.rG = lanes_for(hl->R.nrows, V.r_nnz);
-            FGPU_CUDA_CHECK(ctx, upload(&V.p_ia, hl->P.ia.data(), hl->P.ia.size()));
-            FGPU_CUDA_CHECK(ctx, upload(&V.p_ja, hl->P.ja.data(), hl->P.ja.size()));
-            FGPU_CUDA_CHECK(ctx, upload_f32(&V.p_a, hl->P.a));
-            FGPU_CUDA_CHECK(ctx, upload(&V.r_ia, hl->R.ia.data(), hl->R.ia.size()));
-            FGPU_CUDA_CHECK(ctx, upload(&V.r_ja, hl->R.ja.data(), hl->R.ja.size()));
-            FGPU_CUDA_CHECK(ctx, upload_f32(&V.r_a, hl->R.a));
+            FGPU_CUDA_CHECK(ctx, upload(ctx->stream, &V.p_ia, hl->P.ia.data(), hl->P.ia.size()));
+            FGPU_CUDA_CHECK(ctx, upload(ctx->stream, &V.p_ja, hl->P.ja.data(), hl->P.ja.size()));
+            FGPU_CUDA_CHECK(ctx, upload_f32(ctx->stream, &V.p_a, hl->P.a));
+            FGPU_CUDA_CHECK(ctx, upload(ctx->stream, &V.r_ia, hl->R.ia.data(), hl->R.ia.size()));
+            FGPU_CUDA_CHECK(ctx, upload(ctx->stream, &V.r_ja, hl->R.ja.data(), hl->R.ja.size()));
+            FGPU_CUDA_CHECK(ctx, upload_f32(ctx->stream, &V.r_a, hl->R.a));
         }
         float** vecs[6] = {&V.x, &V.b, &V.w, &V.d0, &V.d1, &V.e};
-        for (float** v : vecs) FGPU_CUDA_CHECK(ctx, cudaMalloc(v, std::max<int64_t>(V.n, 1) * sizeof(float)));
+        for (float** v : vecs) FGPU_CUDA_CHECK(ctx, pool_malloc(ctx->stream, v, std::max<int64_t>(V.n, 1) * sizeof(float)));
         if (coarsest && !H.coarse_inv.empty()) {
-            FGPU_CUDA_CHECK(ctx, upload_f32(&M->coarse_inv, H.coarse_inv));
+            FGPU_CUDA_CHECK(ctx, upload_f32(ctx->stream, &M->coarse_inv, H.coarse_inv));
             nl += l == 0 ? 2 : 1;
         } else if (coarsest) {
             nl += M->coarse_degree;               // start + coarse_degree - 1 steps
@@ -753,7 +755,7 @@ extern "C" int fgpu_amg_create(fgpu_ctx* ctx, const fgpu_matrix* A, const fgpu_a
     rc = amg_setup(ctx, A, &M->cfg, M);
     if (rc) {
         for (auto& V : M->L) free_level(V);
-        cudaFree(M->coarse_inv);
+        pool_free(M->coarse_inv);
         delete M;
         return rc;
     }
@@ -766,7 +768,7 @@ extern "C" int fgpu_amg_update(fgpu_amg* M) {
     fgpu_ctx* ctx = M->ctx;
     if (ctx->capturing) { ctx->err = "gamg: set-up is not capturable"; return FGPU_ERR_INVALID; }
     for (auto& V : M->L) free_level(V);
-    cudaFree(M->coarse_inv);
+    pool_free(M->coarse_inv);
     M->coarse_inv = nullptr;
     return amg_setup(ctx, M->A, &M->cfg, M);
 }
@@ -796,9 +798,9 @@ extern "C" int fgpu_amg_setup_info(const fgpu_amg* M, int* device_levels, double
 extern "C" int fgpu_amg_destroy(fgpu_amg* M) {
     if (!M) return FGPU_OK;
     for (auto& V : M->L) free_level(V);
-    cudaFree(M->coarse_inv);
-    cudaFree(M->xacc);
-    cudaFree(M->tres);
+    pool_free(M->coarse_inv);
+    pool_free(M->xacc);
+    pool_free(M->tres);
     delete M;
     return FGPU_OK;
 }

@@ -47,7 +47,7 @@ AmgDevCsr& AmgDevCsr::operator=(AmgDevCsr&& o) noexcept {
     return *this;
 }
 AmgDevCsr::~AmgDevCsr() {
-    if (own) { cudaFree(ia); cudaFree(ja); cudaFree(a); }
+    if (own) { pool_free(ia); pool_free(ja); pool_free(a); }
 }
 
 namespace {
@@ -67,16 +67,17 @@ int grid_rows(int64_t n, int per_block, int cap = 152 * 16) {
     return (int)std::max<int64_t>(1, std::min<int64_t>((n + per_block - 1) / per_block, cap));
 }
 
-struct Work {                                // device scratch freed at scope exit
+struct Work {                                // device scratch returned to the pool at scope exit
+    cudaStream_t stream;
     std::vector<void*> ptrs;
-    Work() = default;
+    explicit Work(fgpu_ctx* ctx) : stream(ctx->stream) {}
     Work(const Work&) = delete;
     Work& operator=(const Work&) = delete;
-    ~Work() { for (void* p : ptrs) cudaFree(p); }
+    ~Work() { for (void* p : ptrs) pool_free(p); }
     template <typename T>
     T* get(int64_t n) {
         void* p = nullptr;
-        if (cudaMalloc(&p, std::max<int64_t>(n, 1) * sizeof(T)) != cudaSuccess) { cudaGetLastError(); return nullptr; }
+        if (pool_malloc(stream, &p, std::max<int64_t>(n, 1) * sizeof(T)) != cudaSuccess) { cudaGetLastError(); return nullptr; }
         ptrs.push_back(p);
         return static_cast<T*>(p);
     }
@@ -97,9 +98,9 @@ int alloc_csr(fgpu_ctx* ctx, AmgDevCsr& C, int64_t nrows, int64_t ncols, int64_t
     C.nrows = nrows;
     C.ncols = ncols;
     C.nnz = nnz;
-    DEV_TRY(cudaMalloc(&C.ia, (nrows + 1) * sizeof(int64_t)));
-    DEV_TRY(cudaMalloc(&C.ja, std::max<int64_t>(nnz, 1) * sizeof(int32_t)));
-    DEV_TRY(cudaMalloc(&C.a, std::max<int64_t>(nnz, 1) * sizeof(double)));
+    DEV_TRY(pool_malloc(ctx->stream, &C.ia, (nrows + 1) * sizeof(int64_t)));
+    DEV_TRY(pool_malloc(ctx->stream, &C.ja, std::max<int64_t>(nnz, 1) * sizeof(int32_t)));
+    DEV_TRY(pool_malloc(ctx->stream, &C.a, std::max<int64_t>(nnz, 1) * sizeof(double)));
     return FGPU_OK;
 }
 
@@ -788,7 +789,7 @@ int launch_spgemm(fgpu_ctx* ctx, SpgemmArgs g, int bin) {
 int spgemm_dev(fgpu_ctx* ctx, const AmgDevCsr& A, const AmgDevCsr& B, AmgDevCsr& C, int* d_status, bool* overflow) {
     *overflow = false;
     const int64_t n = A.nrows;
-    Work w;
+    Work w(ctx);
     unsigned long long* stats = w.get<unsigned long long>(2);
     uint32_t* cnt = w.get<uint32_t>(n + 1);
     uint32_t* off32 = w.get<uint32_t>(n + 1);
@@ -856,8 +857,8 @@ int spgemm_dev(fgpu_ctx* ctx, const AmgDevCsr& A, const AmgDevCsr& B, AmgDevCsr&
 
 int seg_sort(fgpu_ctx* ctx, int64_t n, const uint32_t* off32, const int64_t* off64, int32_t* key, double* val, int* d_status) {
     unsigned long long* dmax = nullptr;
-    DEV_TRY(cudaMalloc(&dmax, sizeof(unsigned long long)));
-    struct Free { unsigned long long* p; ~Free() { cudaFree(p); } } fr{dmax};
+    DEV_TRY(pool_malloc(ctx->stream, &dmax, sizeof(unsigned long long)));
+    struct Free { unsigned long long* p; ~Free() { pool_free(p); } } fr{dmax};
     DEV_TRY(cudaMemsetAsync(dmax, 0, sizeof(unsigned long long), ctx->stream));
     max_row_kernel<<<grid_rows(n, 256), 256, 0, ctx->stream>>>(n, off32, off64, dmax);
     unsigned long long hmax = 0;
@@ -881,7 +882,7 @@ int seg_sort(fgpu_ctx* ctx, int64_t n, const uint32_t* off32, const int64_t* off
 // T = M^T of an n x m device CSR (rows of T sorted by column of M)
 int transpose_dev(fgpu_ctx* ctx, const AmgDevCsr& M, AmgDevCsr& T, int* d_status) {
     const int64_t m = M.ncols;
-    Work w;
+    Work w(ctx);
     uint32_t* tcnt = w.get<uint32_t>(m + 1);
     uint32_t* toff = w.get<uint32_t>(m + 1);
     uint32_t* cur = w.get<uint32_t>(m + 1);
@@ -977,7 +978,7 @@ int level_dev(fgpu_ctx* ctx, AmgDevLevel& L, const AmgHostCfg& cfg, const AmgNns
     const AmgDevCsr& A = L.A;
     const int64_t n = A.nrows;
     const int64_t nch = (n + kLanczosChunk - 1) / kLanczosChunk;
-    Work w;
+    Work w(ctx);
     double* d = w.get<double>(n);
     uint32_t* cnt = w.get<uint32_t>(n + 1);
     uint32_t* tp = w.get<uint32_t>(n + 1);
@@ -1000,7 +1001,10 @@ int level_dev(fgpu_ctx* ctx, AmgDevLevel& L, const AmgHostCfg& cfg, const AmgNns
         cudaEvent_t& ev;
         ~LanczosGuard() {
             if (t.joinable()) t.join();
-            if (job.st) cudaStreamDestroy(job.st);
+            if (job.st) {
+                cudaStreamSynchronize(job.st);     // the job's arrays go back to the pool of another stream
+                cudaStreamDestroy(job.st);
+            }
             if (ev) cudaEventDestroy(ev);
         }
     } lanczos_guard{lanczos, lz, d_ready};
@@ -1271,10 +1275,10 @@ int amg_build_device(fgpu_ctx* ctx, const fgpu_matrix* Am, const AmgHostCfg& cfg
     H.levels.clear();
     H.tail = AmgHierarchy();
     int* d_status = nullptr;
-    DEV_TRY(cudaMalloc(&d_status, sizeof(int)));
+    DEV_TRY(pool_malloc(ctx->stream, &d_status, sizeof(int)));
     struct StatusFree {
         int* p;
-        ~StatusFree() { cudaFree(p); }
+        ~StatusFree() { pool_free(p); }
     } status_free{d_status};
     DEV_TRY(cudaMemsetAsync(d_status, 0, sizeof(int), ctx->stream));
     H.levels.emplace_back();
@@ -1381,9 +1385,9 @@ extern "C" int fgpu_space_rigid_body_modes(const fgpu_space* V, fgpu_vector* con
         for (int d = 0; d < 3; ++d) c[d] += M->h_xyz[v * 3 + d];
     for (int d = 0; d < 3; ++d) c[d] /= (double)std::max<int64_t>(M->nv, 1);
     double *dlam = nullptr, *xn = nullptr;
-    DEV_TRY(cudaMalloc(&dlam, lam.size() * sizeof(double)));
-    struct Free { double*& a; double*& b; ~Free() { cudaFree(a); cudaFree(b); } } fr{dlam, xn};
-    DEV_TRY(cudaMalloc(&xn, std::max<int64_t>(nn, 1) * 3 * sizeof(double)));
+    DEV_TRY(pool_malloc(ctx->stream, &dlam, lam.size() * sizeof(double)));
+    struct Free { double*& a; double*& b; ~Free() { pool_free(a); pool_free(b); } } fr{dlam, xn};
+    DEV_TRY(pool_malloc(ctx->stream, &xn, std::max<int64_t>(nn, 1) * 3 * sizeof(double)));
     DEV_TRY(cudaMemcpyAsync(dlam, lam.data(), lam.size() * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
     node_coords_kernel<<<grid_rows(nn, 256), 256, 0, ctx->stream>>>(nn, V->n, V->d_inc_ptr, V->d_inc, M->d_tets, M->d_xyz, dlam, xn);
     rbm_kernel<<<grid_rows(nn, 256), 256, 0, ctx->stream>>>(nn, xn, c[0], c[1], c[2], out[0]->d, out[1]->d, out[2]->d, out[3]->d,

@@ -37,7 +37,7 @@ int set_err(fgpu_ctx* ctx, int code, const std::string& msg) {
 template <typename T>
 int dev_alloc(fgpu_ctx* ctx, T** p, size_t count) {
     if (count == 0) count = 1;
-    cudaError_t e = cudaMalloc((void**)p, count * sizeof(T));
+    cudaError_t e = dev_malloc((void**)p, count * sizeof(T));
     if (e != cudaSuccess) {
         *p = nullptr;
         return set_err(ctx, FGPU_ERR_ALLOC, std::string("cudaMalloc: ") + cudaGetErrorString(e));
@@ -48,10 +48,10 @@ int dev_alloc(fgpu_ctx* ctx, T** p, size_t count) {
 // Resolve pending profiling events (after a stream sync) and check the status word.
 int finish(fgpu_ctx* ctx, bool sync = true) {
     if (!sync || ctx->capturing) return FGPU_OK;   // captured calls: the status is checked at graph launch
-    int hst = 0;
-    cudaError_t e = cudaMemcpyAsync(&hst, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
+    cudaError_t e = cudaMemcpyAsync(ctx->h_status, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) return set_err(ctx, FGPU_ERR_CUDA, std::string("stream: ") + cudaGetErrorString(e));
+    const int hst = *ctx->h_status;
     for (auto& ev : ctx->pending) {
         float ms = 0;
         cudaEventElapsedTime(&ms, ev.start, ev.stop);
@@ -167,7 +167,8 @@ int fgpu_create(const fgpu_config* cfg, fgpu_ctx** out) {
         e = cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking);
         ctx->own_stream = true;
     }
-    if (e == cudaSuccess) e = cudaMalloc(&ctx->d_status, sizeof(int));
+    if (e == cudaSuccess) e = dev_malloc(&ctx->d_status, sizeof(int));
+    if (e == cudaSuccess) e = cudaMallocHost(&ctx->h_status, sizeof(int));
     if (e == cudaSuccess) e = cudaMemset(ctx->d_status, 0, sizeof(int));
     if (e != cudaSuccess) {
         delete ctx;
@@ -190,6 +191,8 @@ int fgpu_destroy(fgpu_ctx* ctx) {
     for (int i = 0; i < 5; ++i)
         if (ctx->copy_events[i]) cudaEventDestroy(ctx->copy_events[i]);
     cudaFree(ctx->d_status);
+    cudaFreeHost(ctx->h_status);
+    pool_release(ctx->stream);
     if (ctx->own_stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
     return FGPU_OK;
@@ -853,11 +856,14 @@ int fgpu_assemble_vector(fgpu_ctx* ctx, const fgpu_space* V, const fgpu_rhs_desc
     DevTables* tab = get_dev_tables(V->order, qdeg, err);
     if (!tab) return set_err(ctx, FGPU_ERR_INVALID, err);
     double* work = nullptr;
-    int rc = dev_alloc(ctx, &work, (size_t)V->mesh->nt * V->n * V->ncomp);
-    if (rc) return rc;
-    rc = launch_rhs(ctx, V, tab, rhs->kind, rhs->c, out->d, accumulate, work);
+    const cudaError_t e = pool_malloc(ctx->stream, &work, (size_t)V->mesh->nt * V->n * V->ncomp * sizeof(double));
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return set_err(ctx, FGPU_ERR_ALLOC, std::string("assemble_vector: ") + cudaGetErrorString(e));
+    }
+    int rc = launch_rhs(ctx, V, tab, rhs->kind, rhs->c, out->d, accumulate, work);
     int rc2 = finish(ctx);
-    cudaFree(work);
+    pool_free(work);
     return rc ? rc : rc2;
 }
 
@@ -877,15 +883,18 @@ int fgpu_dirichlet(fgpu_ctx* ctx, fgpu_matrix* A, fgpu_vector* rhs, int64_t ndof
     }
     uint8_t* dm = nullptr;
     double* dg = nullptr;
-    int rc = dev_alloc(ctx, &dm, A->nrows);
-    if (!rc && values) rc = dev_alloc(ctx, &dg, A->nrows);
-    if (rc) { cudaFree(dm); return rc; }
+    cudaError_t e = pool_malloc(ctx->stream, &dm, A->nrows);
+    if (e == cudaSuccess && values) e = pool_malloc(ctx->stream, &dg, A->nrows * sizeof(double));
+    if (e != cudaSuccess) {
+        pool_free(dm);
+        return set_err(ctx, FGPU_ERR_ALLOC, std::string("dirichlet: ") + cudaGetErrorString(e));
+    }
     cudaMemcpyAsync(dm, mask.data(), A->nrows, cudaMemcpyHostToDevice, ctx->stream);
     if (values) cudaMemcpyAsync(dg, g.data(), A->nrows * sizeof(double), cudaMemcpyHostToDevice, ctx->stream);
-    rc = launch_dirichlet(ctx, A, rhs ? rhs->d : nullptr, dm, dg, mode, diag);
-    int rc2 = finish(ctx);
-    cudaFree(dm);
-    cudaFree(dg);
+    const int rc = launch_dirichlet(ctx, A, rhs ? rhs->d : nullptr, dm, dg, mode, diag);
+    const int rc2 = finish(ctx);
+    pool_free(dm);
+    pool_free(dg);
     return rc ? rc : rc2;
 }
 

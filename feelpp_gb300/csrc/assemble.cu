@@ -42,7 +42,7 @@ static std::map<std::tuple<int, int, int>, DevTables*> g_tabs;
 
 template <typename T>
 static cudaError_t upload(const std::vector<T>& h, T** d) {
-    cudaError_t e = cudaMalloc((void**)d, h.size() * sizeof(T));
+    cudaError_t e = dev_malloc((void**)d, h.size() * sizeof(T));
     if (e != cudaSuccess) return e;
     return cudaMemcpy(*d, h.data(), h.size() * sizeof(T), cudaMemcpyHostToDevice);
 }
@@ -916,7 +916,7 @@ int launch_build_positions(fgpu_ctx* ctx, fgpu_space* V) {
     const int64_t total = V->mesh->nt * (int64_t)V->n * V->n;
     // 64 bytes of padding: the streamed assembly copies the table in aligned 4-byte words that
     // may run up to 12 bytes past an element's last row
-    cudaError_t e = cudaMalloc(&V->d_pos, total + 64);
+    cudaError_t e = dev_malloc(&V->d_pos, total + 64);
     if (e != cudaSuccess) { ctx->err = "position table allocation failed"; V->d_pos = nullptr; return FGPU_ERR_ALLOC; }
     int64_t blocks = std::min<int64_t>((total + 255) / 256, 152 * 64);
     PendingEvent ev;
@@ -1222,8 +1222,8 @@ static int batch_tables(fgpu_ctx* ctx, float** h, float** l) {
     auto it = g_btabs.find(ctx->device);
     if (it != g_btabs.end()) { *h = it->second.first; *l = it->second.second; return FGPU_OK; }
     float *dh = nullptr, *dl = nullptr;
-    FGPU_CUDA_CHECK(ctx, cudaMalloc(&dh, kBatchTabFloats * sizeof(float)));
-    FGPU_CUDA_CHECK(ctx, cudaMalloc(&dl, kBatchTabFloats * sizeof(float)));
+    FGPU_CUDA_CHECK(ctx, dev_malloc(&dh, kBatchTabFloats * sizeof(float)));
+    FGPU_CUDA_CHECK(ctx, dev_malloc(&dl, kBatchTabFloats * sizeof(float)));
     for (int order = 1; order <= 3; ++order) {
         std::string err;
         DevTables* t = get_dev_tables(order, 2 * order, err);
@@ -1660,7 +1660,7 @@ static int run_two_phase(fgpu_ctx* ctx, fgpu_matrix* A, const DevTables* tab, co
         cudaFree(A->d_kbuf);
         A->d_kbuf = nullptr;
         A->kbuf_bytes = 0;
-        if (cudaMalloc(&A->d_kbuf, need) != cudaSuccess) { cudaGetLastError(); ctx->err = "two-phase assembly: element buffer allocation failed"; return FGPU_ERR_ALLOC; }
+        if (dev_malloc(&A->d_kbuf, need) != cudaSuccess) { cudaGetLastError(); ctx->err = "two-phase assembly: element buffer allocation failed"; return FGPU_ERR_ALLOC; }
         A->kbuf_bytes = need;
     }
     int sms = 0;
@@ -1713,7 +1713,7 @@ int ensure_two_phase(fgpu_ctx* ctx, fgpu_matrix* A, size_t need) {
         cudaFree(A->d_kbuf);
         A->d_kbuf = nullptr;
         A->kbuf_bytes = 0;
-        if (cudaMalloc(&A->d_kbuf, need) != cudaSuccess) { cudaGetLastError(); ctx->err = "two-phase assembly: element buffer allocation failed"; return FGPU_ERR_ALLOC; }
+        if (dev_malloc(&A->d_kbuf, need) != cudaSuccess) { cudaGetLastError(); ctx->err = "two-phase assembly: element buffer allocation failed"; return FGPU_ERR_ALLOC; }
         A->kbuf_bytes = need;
     }
     return FGPU_OK;
@@ -1939,7 +1939,7 @@ static int run_el_two_phase(fgpu_ctx* ctx, fgpu_matrix* A, const DevTables* tab,
         cudaFree(A->d_kbuf);
         A->d_kbuf = nullptr;
         A->kbuf_bytes = 0;
-        if (cudaMalloc(&A->d_kbuf, need) != cudaSuccess) { cudaGetLastError(); ctx->err = "two-phase assembly: element buffer allocation failed"; return FGPU_ERR_ALLOC; }
+        if (dev_malloc(&A->d_kbuf, need) != cudaSuccess) { cudaGetLastError(); ctx->err = "two-phase assembly: element buffer allocation failed"; return FGPU_ERR_ALLOC; }
         A->kbuf_bytes = need;
     }
     int sms = 0;
@@ -2067,7 +2067,7 @@ int launch_norms_sine(fgpu_ctx* ctx, const fgpu_space* V, const DevTables* tab, 
     const int threads = 256;
     const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((M->nt + threads - 1) / threads, 152 * 8));
     double* partial = nullptr;
-    FGPU_CUDA_CHECK(ctx, cudaMalloc(&partial, 2 * blocks * sizeof(double)));
+    FGPU_CUDA_CHECK(ctx, dev_malloc(&partial, 2 * blocks * sizeof(double)));
     switch (V->n) {
         case 4: norms_sine_kernel<4><<<blocks, threads, 0, ctx->stream>>>(M->nt, M->d_xyz, M->d_tets, V->d_l2n, d_u, tab->Q, tab->d_qx, tab->d_qw, tab->d_phi, tab->d_dphi, partial); break;
         case 10: norms_sine_kernel<10><<<blocks, threads, 0, ctx->stream>>>(M->nt, M->d_xyz, M->d_tets, V->d_l2n, d_u, tab->Q, tab->d_qx, tab->d_qw, tab->d_phi, tab->d_dphi, partial); break;

@@ -54,10 +54,10 @@ int batch_err(fgpu_ctx* ctx, int code, const char* msg) {
 
 int batch_finish(fgpu_ctx* ctx) {
     if (ctx->capturing) return FGPU_OK;
-    int hst = 0;
-    cudaError_t e = cudaMemcpyAsync(&hst, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
+    cudaError_t e = cudaMemcpyAsync(ctx->h_status, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) { ctx->err = std::string("batch: ") + cudaGetErrorString(e); return FGPU_ERR_CUDA; }
+    const int hst = *ctx->h_status;
     if (hst) {
         cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream);
         cudaStreamSynchronize(ctx->stream);
@@ -161,7 +161,7 @@ int fgpu_batch_create(fgpu_ctx* ctx, int nprob, fgpu_matrix* const* mats, const 
             fgpu_matrix* Am = mats[k];
             Am->d_coef = nullptr;
             Am->coef_cap = 0;
-            if (cudaMalloc(&Am->d_coef, (size_t)V->mesh->nt * 8 * sizeof(double)) != cudaSuccess)
+            if (dev_malloc(&Am->d_coef, (size_t)V->mesh->nt * 8 * sizeof(double)) != cudaSuccess)
                 return batch_err(ctx, FGPU_ERR_ALLOC, "batch_create: record allocation failed");
             Am->coef_cap = V->mesh->nt * 8;
         }
@@ -219,7 +219,7 @@ int fgpu_batch_create(fgpu_ctx* ctx, int nprob, fgpu_matrix* const* mats, const 
             cudaFree(A->d_kbuf);
             A->d_kbuf = nullptr;
             A->kbuf_bytes = 0;
-            if (cudaMalloc(&A->d_kbuf, kb) != cudaSuccess) { cudaGetLastError(); two_phase = false; break; }
+            if (dev_malloc(&A->d_kbuf, kb) != cudaSuccess) { cudaGetLastError(); two_phase = false; break; }
             A->kbuf_bytes = kb;
         }
         probs[k].nnz = A->pattern->nnz;
@@ -241,13 +241,13 @@ int fgpu_batch_create(fgpu_ctx* ctx, int nprob, fgpu_matrix* const* mats, const 
     b->closed_groups = closed_off[nprob];
     b->p3_groups = p3_off[nprob];
     b->mats.assign(mats, mats + nprob);
-    cudaError_t e = cudaMalloc(&b->d_probs, nprob * sizeof(BatchProblem));
-    if (e == cudaSuccess) e = cudaMalloc(&b->d_row_off, (nprob + 1) * sizeof(int64_t));
-    if (e == cudaSuccess) e = cudaMalloc(&b->d_elem_off, (nprob + 1) * sizeof(int64_t));
-    if (e == cudaSuccess) e = cudaMalloc(&b->d_closed_off, (nprob + 1) * sizeof(int64_t));
-    if (e == cudaSuccess) e = cudaMalloc(&b->d_p3_off, (nprob + 1) * sizeof(int64_t));
-    if (e == cudaSuccess) e = cudaMalloc(&b->d_counter, sizeof(unsigned long long));
-    if (e == cudaSuccess) e = cudaMalloc(&b->d_slice_off, (nprob + 1) * sizeof(int64_t));
+    cudaError_t e = dev_malloc(&b->d_probs, nprob * sizeof(BatchProblem));
+    if (e == cudaSuccess) e = dev_malloc(&b->d_row_off, (nprob + 1) * sizeof(int64_t));
+    if (e == cudaSuccess) e = dev_malloc(&b->d_elem_off, (nprob + 1) * sizeof(int64_t));
+    if (e == cudaSuccess) e = dev_malloc(&b->d_closed_off, (nprob + 1) * sizeof(int64_t));
+    if (e == cudaSuccess) e = dev_malloc(&b->d_p3_off, (nprob + 1) * sizeof(int64_t));
+    if (e == cudaSuccess) e = dev_malloc(&b->d_counter, sizeof(unsigned long long));
+    if (e == cudaSuccess) e = dev_malloc(&b->d_slice_off, (nprob + 1) * sizeof(int64_t));
     if (e == cudaSuccess) e = cudaMemcpy(b->d_slice_off, slice_off.data(), (nprob + 1) * sizeof(int64_t), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(b->d_probs, probs.data(), nprob * sizeof(BatchProblem), cudaMemcpyHostToDevice);
     if (e == cudaSuccess) e = cudaMemcpy(b->d_row_off, row_off.data(), (nprob + 1) * sizeof(int64_t), cudaMemcpyHostToDevice);

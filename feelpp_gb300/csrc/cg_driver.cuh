@@ -191,9 +191,9 @@ static int cg_run(fgpu_ctx* ctx, int64_t n, const CgOperator<PL>& A, const typen
     auto cleanup = [&]() {
         if (exec) cudaGraphExecDestroy(exec);
         if (graph) cudaGraphDestroy(graph);
-        cudaFree(r); cudaFree(z); cudaFree(p); cudaFree(q); cudaFree(d); cudaFree(w); cudaFree(dinv0); cudaFree(xe);
-        cudaFree(partial); cudaFree(pq_partial); cudaFree(sc);
-        if (hsc) cudaFreeHost(hsc);
+        pool_free(r); pool_free(z); pool_free(p); pool_free(q); pool_free(d); pool_free(w); pool_free(dinv0); pool_free(xe);
+        pool_free(partial); pool_free(pq_partial); pool_free(sc);
+        if (hsc) pinned_free(hsc);
     };
 #define CK(call)                                                             \
     do {                                                                     \
@@ -204,14 +204,14 @@ static int cg_run(fgpu_ctx* ctx, int64_t n, const CgOperator<PL>& A, const typen
             return FGPU_ERR_CUDA;                                            \
         }                                                                    \
     } while (0)
-    CK(cudaMalloc(&r, n * sizeof(S)));
-    CK(cudaMalloc(&z, n * sizeof(S)));
-    CK(cudaMalloc(&p, n * sizeof(S)));
-    CK(cudaMalloc(&q, n * sizeof(S)));
-    CK(cudaMalloc(&partial, 3 * nbp * sizeof(D)));
-    CK(cudaMalloc(&pq_partial, nbp * sizeof(D)));
-    CK(cudaMalloc(&sc, sizeof(CGScalars<PL>)));
-    CK(cudaMallocHost(&hsc, sizeof(CGScalars<PL>)));
+    CK(pool_malloc(s, &r, n * sizeof(S)));
+    CK(pool_malloc(s, &z, n * sizeof(S)));
+    CK(pool_malloc(s, &p, n * sizeof(S)));
+    CK(pool_malloc(s, &q, n * sizeof(S)));
+    CK(pool_malloc(s, &partial, 3 * nbp * sizeof(D)));
+    CK(pool_malloc(s, &pq_partial, nbp * sizeof(D)));
+    CK(pool_malloc(s, &sc, sizeof(CGScalars<PL>)));
+    CK(pinned_malloc(&hsc, sizeof(CGScalars<PL>)));
     auto poll = [&]() -> cudaError_t {
         cudaError_t e = cudaMemcpyAsync(hsc, sc, sizeof(CGScalars<PL>), cudaMemcpyDeviceToHost, s);
         if (e == cudaSuccess) e = cudaStreamSynchronize(s);
@@ -220,10 +220,10 @@ static int cg_run(fgpu_ctx* ctx, int64_t n, const CgOperator<PL>& A, const typen
     std::vector<D> c1, c2;
     const S* dz = dinv;                   // diagonal the update kernels apply (D^-1, or D^-1 / theta)
     if (cheb) {
-        CK(cudaMalloc(&d, n * sizeof(S)));
-        CK(cudaMalloc(&w, n * sizeof(S)));
-        CK(cudaMalloc(&dinv0, n * sizeof(S)));
-        CK(cudaMalloc(&xe, n * sizeof(S)));
+        CK(pool_malloc(s, &d, n * sizeof(S)));
+        CK(pool_malloc(s, &w, n * sizeof(S)));
+        CK(pool_malloc(s, &dinv0, n * sizeof(S)));
+        CK(pool_malloc(s, &xe, n * sizeof(S)));
         // lmax(D^-1 A): Lanczos tridiagonal from the coefficients of a short
         // Jacobi-CG run on b from x = 0 (in scratch vectors)
         CK(cudaMemsetAsync(xe, 0, n * sizeof(S), s));

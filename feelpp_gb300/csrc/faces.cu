@@ -84,7 +84,7 @@ FaceTablesDev* get_face_tables(fgpu_ctx* ctx, int order) {
         for (int i : d) on[(size_t)f * T.n + i] = 1;
     }
     auto up = [](void** dst, const void* src, size_t bytes) {
-        cudaError_t e = cudaMalloc(dst, bytes);
+        cudaError_t e = dev_malloc(dst, bytes);
         if (e == cudaSuccess) e = cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice);
         return e;
     };
@@ -243,7 +243,7 @@ int get_face_set(fgpu_ctx* ctx, fgpu_space* V, int range, double xmax, int whole
     const int nc = boundary_faces_coloured(M->nt, M->h_tets.data(), M->h_xyz.data(), xmax_on, xmax, whole, faces, fs.colour_ptr);
     if (nc < 0) { ctx->err = "face integrals: more than 64 colours"; return FGPU_ERR_INVALID; }
     if (!faces.empty()) {
-        FGPU_CUDA_CHECK(ctx, cudaMalloc(&fs.d_faces, faces.size() * sizeof(int32_t)));
+        FGPU_CUDA_CHECK(ctx, dev_malloc(&fs.d_faces, faces.size() * sizeof(int32_t)));
         FGPU_CUDA_CHECK(ctx, cudaMemcpy(fs.d_faces, faces.data(), faces.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
     }
     V->face_sets.push_back(fs);
@@ -256,7 +256,7 @@ int face_geometry(fgpu_ctx* ctx, const fgpu_space* V, const fgpu_space::FaceSet&
     *d_geo = nullptr;
     if (nf == 0) return FGPU_OK;
     if (ctx->capturing) { ctx->err = "face integrals: not capturable"; return FGPU_ERR_INVALID; }
-    FGPU_CUDA_CHECK(ctx, cudaMalloc(d_geo, nf * 5 * sizeof(double)));
+    FGPU_CUDA_CHECK(ctx, dev_malloc(d_geo, nf * 5 * sizeof(double)));
     const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((nf + 255) / 256, 152 * 8));
     face_geom_kernel<<<blocks, 256, 0, ctx->stream>>>(nf, fs.d_faces, V->mesh->d_xyz, V->mesh->d_tets, *d_geo);
     ctx->launches++;

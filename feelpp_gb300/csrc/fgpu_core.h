@@ -222,6 +222,7 @@ struct fgpu_ctx {
     std::vector<PendingEvent> pending;
     std::vector<cudaEvent_t> event_pool;
     int* d_status = nullptr;       // device status word written by kernels (bit flags)
+    int* h_status = nullptr;       // page-locked copy of it
     int64_t launches = 0;          // kernels launched by this context
     int host_threads = 1;
     int host_setup = 0;            // 1: dof tables and patterns built on the host (default: device)
@@ -492,6 +493,20 @@ int solve_pcg(fgpu_ctx* ctx, const fgpu_matrix* A, const double* d_b, double* d_
               fgpu_solve_stats* st, fgpu_amg* amg = nullptr);
 int solve_pcg_mixed(fgpu_ctx* ctx, const fgpu_matrix* A64, const fgpu_matrix* A32, const double* d_b, double* d_x,
                     const fgpu_solver_cfg* cfg, fgpu_solve_stats* st);
+// device scratch kept between calls, and allocations that give it back before they fail (pool.cpp)
+cudaError_t dev_malloc_bytes(void** p, size_t bytes);
+cudaError_t pool_malloc_bytes(cudaStream_t stream, void** p, size_t bytes);
+cudaError_t pool_free(void* p);      // also takes blocks of dev_malloc
+void pool_release(cudaStream_t stream);
+cudaError_t pinned_malloc_bytes(void** p, size_t bytes);
+void pinned_free(void* p);
+template <typename T>
+cudaError_t dev_malloc(T** p, size_t bytes) { return dev_malloc_bytes((void**)p, bytes); }
+template <typename T>
+cudaError_t pool_malloc(cudaStream_t stream, T** p, size_t bytes) { return pool_malloc_bytes(stream, (void**)p, bytes); }
+template <typename T>
+cudaError_t pinned_malloc(T** p, size_t bytes) { return pinned_malloc_bytes((void**)p, bytes); }
+
 // launch-shape autotuner store (tune.cpp)
 void tune_load_cache_file(const std::string& path);
 bool tune_lookup(const std::string& file, const std::string& key, std::vector<int>& vals);

@@ -525,7 +525,7 @@ int launch_build_gather_map(fgpu_ctx* ctx, fgpu_space* V) {
                  s_first = ((size_t)entries * 2 + 15) & ~(size_t)15;
     char* scratch = nullptr;
     GatherPlan G{};
-    cudaError_t e = cudaMalloc(&scratch, s_tot + s_sum + s_bin + s_step + 16 + s_first + tri.size() * 2);
+    cudaError_t e = dev_malloc(&scratch, s_tot + s_sum + s_bin + s_step + 16 + s_first + tri.size() * 2);
     unsigned long long* d_total = reinterpret_cast<unsigned long long*>(scratch);
     unsigned long long* sums = d_total + 2;
     uint32_t *cnt = reinterpret_cast<uint32_t*>(scratch + s_tot + s_sum), *slice0 = cnt + nbins, *steps = slice0 + nbins;
@@ -545,7 +545,7 @@ int launch_build_gather_map(fgpu_ctx* ctx, fgpu_space* V) {
         e = cudaGetLastError();
     }
     const size_t slots = (size_t)max_slices * 32;
-    if (e == cudaSuccess) e = cudaMalloc(&G.pos0, (2 * slots + max_slices + 1) * sizeof(uint32_t));
+    if (e == cudaSuccess) e = dev_malloc(&G.pos0, (2 * slots + max_slices + 1) * sizeof(uint32_t));
     G.pos1 = G.pos0 + slots;
     G.soff = G.pos1 + slots;
     if (e == cudaSuccess) e = cudaMemsetAsync(G.pos0, 0xFF, 2 * slots * sizeof(uint32_t), ctx->stream);
@@ -564,7 +564,7 @@ int launch_build_gather_map(fgpu_ctx* ctx, fgpu_space* V) {
         ctx->err = "gather map: more than 2^32 padded contributions";
         rc = FGPU_ERR_INVALID;
     }
-    if (e == cudaSuccess && rc == FGPU_OK) e = cudaMalloc(&G.sidx, words * sizeof(uint32_t));
+    if (e == cudaSuccess && rc == FGPU_OK) e = dev_malloc(&G.sidx, words * sizeof(uint32_t));
     if (e == cudaSuccess && rc == FGPU_OK) e = cudaMemsetAsync(G.sidx, 0xFF, words * sizeof(uint32_t), ctx->stream);
     if (e == cudaSuccess && rc == FGPU_OK) {
         launch_walk<1>(ctx, walkers, in, first, slice0, G.soff, G.pos0, G.pos1, G.sidx);

@@ -131,7 +131,7 @@ struct GmWork {
     double *V = nullptr, *w = nullptr, *z = nullptr, *dinv = nullptr, *partial = nullptr, *small = nullptr;
     float *f_in = nullptr;
     ~GmWork() {
-        cudaFree(V); cudaFree(w); cudaFree(z); cudaFree(dinv); cudaFree(partial); cudaFree(small); cudaFree(f_in);
+        pool_free(V); pool_free(w); pool_free(z); pool_free(dinv); pool_free(partial); pool_free(small); pool_free(f_in);
     }
 };
 
@@ -172,13 +172,13 @@ int solve_gmres(fgpu_ctx* ctx, const fgpu_matrix* A, fgpu_amg* amg, const double
     const int vb = (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 152 * 8));
     GmWork W;
     const int64_t ldv = (n + 31) / 32 * 32;
-    cudaError_t e = cudaMalloc(&W.V, (size_t)(m + 1) * ldv * sizeof(double));
-    if (e == cudaSuccess) e = cudaMalloc(&W.w, n * sizeof(double));
-    if (e == cudaSuccess) e = cudaMalloc(&W.z, n * sizeof(double));
-    if (e == cudaSuccess) e = cudaMalloc(&W.partial, (size_t)(m + 1) * kGmBlocks * sizeof(double));
-    if (e == cudaSuccess) e = cudaMalloc(&W.small, (size_t)(2 * m + 8) * sizeof(double));
-    if (e == cudaSuccess && pc == FGPU_PC_JACOBI) e = cudaMalloc(&W.dinv, n * sizeof(double));
-    if (e == cudaSuccess && pc == FGPU_PC_GAMG) e = cudaMalloc(&W.f_in, n * sizeof(float));
+    cudaError_t e = pool_malloc(ctx->stream, &W.V, (size_t)(m + 1) * ldv * sizeof(double));
+    if (e == cudaSuccess) e = pool_malloc(ctx->stream, &W.w, n * sizeof(double));
+    if (e == cudaSuccess) e = pool_malloc(ctx->stream, &W.z, n * sizeof(double));
+    if (e == cudaSuccess) e = pool_malloc(ctx->stream, &W.partial, (size_t)(m + 1) * kGmBlocks * sizeof(double));
+    if (e == cudaSuccess) e = pool_malloc(ctx->stream, &W.small, (size_t)(2 * m + 8) * sizeof(double));
+    if (e == cudaSuccess && pc == FGPU_PC_JACOBI) e = pool_malloc(ctx->stream, &W.dinv, n * sizeof(double));
+    if (e == cudaSuccess && pc == FGPU_PC_GAMG) e = pool_malloc(ctx->stream, &W.f_in, n * sizeof(float));
     if (e != cudaSuccess) { cudaGetLastError(); ctx->err = "gmres: allocation failed"; return FGPU_ERR_ALLOC; }
     double* h1 = W.small;                 // m + 1: first CGS pass
     double* h2 = W.small + (m + 1);       // m + 1: second pass; h2[m + 1] .. holds w.w (see below)

@@ -71,7 +71,7 @@ std::map<std::tuple<int, int, int>, HoTables*> g_ho_tabs;
 
 template <typename T>
 cudaError_t up(T** dst, const std::vector<T>& v) {
-    cudaError_t e = cudaMalloc(dst, std::max<size_t>(v.size(), 1) * sizeof(T));
+    cudaError_t e = dev_malloc(dst, std::max<size_t>(v.size(), 1) * sizeof(T));
     if (e == cudaSuccess && !v.empty()) e = cudaMemcpy(*dst, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice);
     return e;
 }
@@ -1013,7 +1013,7 @@ int launch_rhs_hex(fgpu_ctx* ctx, const fgpu_space* V, const fgpu_rhs_desc* rhs,
     HoTables* T = get_ho_tables(ctx, V->order, qdeg, true);
     if (!T) return FGPU_ERR_INVALID;
     double* work = nullptr;
-    FGPU_CUDA_CHECK(ctx, cudaMalloc(&work, std::max<int64_t>(M->nt * V->n, 1) * sizeof(double)));
+    FGPU_CUDA_CHECK(ctx, dev_malloc(&work, std::max<int64_t>(M->nt * V->n, 1) * sizeof(double)));
     const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((M->nt + 127) / 128, 152 * 32));
     PendingEvent ev;
     prof_begin(ctx, "rhs_element_hex", ev);
@@ -1089,7 +1089,7 @@ int launch_rhs_ho(fgpu_ctx* ctx, const fgpu_space* V, const fgpu_rhs_desc* rhs, 
     HoTables* T = get_ho_tables(ctx, V->order, qdeg);
     if (!T) return FGPU_ERR_INVALID;
     double* work = nullptr;
-    FGPU_CUDA_CHECK(ctx, cudaMalloc(&work, std::max<int64_t>(M->nt * V->n, 1) * sizeof(double)));
+    FGPU_CUDA_CHECK(ctx, dev_malloc(&work, std::max<int64_t>(M->nt * V->n, 1) * sizeof(double)));
     const int blocks = (int)std::max<int64_t>(1, std::min<int64_t>((M->nt + 127) / 128, 152 * 32));
     PendingEvent ev;
     prof_begin(ctx, "rhs_element_ho", ev);
@@ -1124,7 +1124,7 @@ extern "C" int fgpu_mesh_set_ho_nodes(fgpu_mesh* M, const double* ho) {
         return FGPU_OK;
     }
     const size_t bytes = (size_t)M->nt * 18 * sizeof(double);
-    if (!M->d_ho) FGPU_CUDA_CHECK(ctx, cudaMalloc(&M->d_ho, std::max<size_t>(bytes, 8)));
+    if (!M->d_ho) FGPU_CUDA_CHECK(ctx, dev_malloc(&M->d_ho, std::max<size_t>(bytes, 8)));
     FGPU_CUDA_CHECK(ctx, cudaMemcpyAsync(M->d_ho, ho, bytes, cudaMemcpyHostToDevice, ctx->stream));
     FGPU_CUDA_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
     return FGPU_OK;

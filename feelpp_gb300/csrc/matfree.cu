@@ -484,9 +484,9 @@ int operator_diagonal(fgpu_ctx* ctx, fgpu_operator* op) {
     const int n = V->n;
     const bool f32 = op->precision == FGPU_F32;
     const size_t es = f32 ? sizeof(float) : sizeof(double);
-    if (!op->d_diag) FGPU_CUDA_CHECK(ctx, cudaMalloc(&op->d_diag, op->nnodes * es));
+    if (!op->d_diag) FGPU_CUDA_CHECK(ctx, dev_malloc(&op->d_diag, op->nnodes * es));
     void* ones = nullptr;
-    FGPU_CUDA_CHECK(ctx, cudaMalloc(&ones, op->nnodes * es));
+    FGPU_CUDA_CHECK(ctx, dev_malloc(&ones, op->nnodes * es));
     // Dirichlet rows: diag 1 (x = 1 passes through the mask branch)
     std::vector<char> h(op->nnodes * es);
     if (f32) { float* p = (float*)h.data(); for (int64_t i = 0; i < op->nnodes; ++i) p[i] = 1.0f; }
@@ -730,7 +730,7 @@ static int mf_pcg_core(fgpu_ctx* ctx, fgpu_operator* op, const typename PL::S* b
     const int64_t n = op->nnodes;
     const int vb = vec_blocks(n);
     S* dinv = nullptr;
-    if (cudaMalloc(&dinv, n * sizeof(S)) != cudaSuccess) { ctx->err = "matrix-free CG: allocation failed"; return FGPU_ERR_ALLOC; }
+    if (pool_malloc(ctx->stream, &dinv, n * sizeof(S)) != cudaSuccess) { ctx->err = "matrix-free CG: allocation failed"; return FGPU_ERR_ALLOC; }
     dinv_from_diag_kernel<PL><<<vb, 256, 0, ctx->stream>>>(n, (const S*)op->d_diag, dinv, pc != FGPU_PC_NONE);
     ctx->launches++;
     CgOperator<PL> A;
@@ -750,7 +750,7 @@ static int mf_pcg_core(fgpu_ctx* ctx, fgpu_operator* op, const typename PL::S* b
     PcHook<PL> hook;
     if (pmg) hook = pmg_pc_hook<PL>(pmg);
     const int rc = cg_run<PL>(ctx, n, A, dinv, b, x, o, res, refresh, pmg ? &hook : nullptr);
-    cudaFree(dinv);
+    pool_free(dinv);
     return rc;
 }
 
@@ -758,12 +758,12 @@ static double host_norm(fgpu_ctx* ctx, int64_t n, const double* d) {
     const int vb = vec_blocks(n);
     double* partial = nullptr;
     std::vector<double> h(vb, 0.0);
-    if (cudaMalloc(&partial, vb * sizeof(double)) != cudaSuccess) return NAN;
+    if (pool_malloc(ctx->stream, &partial, vb * sizeof(double)) != cudaSuccess) return NAN;
     norm2_partial_kernel<<<vb, 256, 0, ctx->stream>>>(n, d, partial);
     ctx->launches++;
     cudaMemcpyAsync(h.data(), partial, vb * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream);
     cudaStreamSynchronize(ctx->stream);
-    cudaFree(partial);
+    pool_free(partial);
     double s = 0;
     for (double v : h) s += v;
     return std::sqrt(s);
@@ -811,10 +811,10 @@ int solve_cg_operator(fgpu_ctx* ctx, fgpu_operator* op, fgpu_operator* op32, con
     int rc = FGPU_OK, fail = 0, fallback = 0, fallback_its = 0;
     double rn = 0, bn = host_norm(ctx, n, d_b);
     double *r = nullptr, *q = nullptr, *xc = nullptr, *r2b = nullptr;
-    if (cudaMalloc(&r, n * sizeof(double)) != cudaSuccess || cudaMalloc(&q, n * sizeof(double)) != cudaSuccess ||
-        cudaMalloc(&xc, n * sizeof(double)) != cudaSuccess || cudaMalloc(&r2b, n * sizeof(double)) != cudaSuccess) {
+    if (pool_malloc(ctx->stream, &r, n * sizeof(double)) != cudaSuccess || pool_malloc(ctx->stream, &q, n * sizeof(double)) != cudaSuccess ||
+        pool_malloc(ctx->stream, &xc, n * sizeof(double)) != cudaSuccess || pool_malloc(ctx->stream, &r2b, n * sizeof(double)) != cudaSuccess) {
         cudaGetLastError();
-        cudaFree(r); cudaFree(q); cudaFree(xc);
+        pool_free(r); pool_free(q); pool_free(xc);
         ctx->err = "matrix-free solve: allocation failed";
         return FGPU_ERR_ALLOC;
     }
@@ -828,7 +828,7 @@ int solve_cg_operator(fgpu_ctx* ctx, fgpu_operator* op, fgpu_operator* op32, con
     } else {
         if (!op32 || op32->precision != FGPU_F32 || op32->space != op->space) { ctx->err = "mixed matrix-free solve needs a binary32 inner operator on the same space"; rc = FGPU_ERR_INVALID; }
         float *r32 = nullptr, *d32 = nullptr;
-        if (rc == FGPU_OK && (cudaMalloc(&r32, n * sizeof(float)) != cudaSuccess || cudaMalloc(&d32, n * sizeof(float)) != cudaSuccess)) {
+        if (rc == FGPU_OK && (pool_malloc(ctx->stream, &r32, n * sizeof(float)) != cudaSuccess || pool_malloc(ctx->stream, &d32, n * sizeof(float)) != cudaSuccess)) {
             cudaGetLastError();
             ctx->err = "mixed matrix-free solve: allocation failed";
             rc = FGPU_ERR_ALLOC;
@@ -898,17 +898,17 @@ int solve_cg_operator(fgpu_ctx* ctx, fgpu_operator* op, fgpu_operator* op32, con
                 }
             }
         }
-        cudaFree(r32);
-        cudaFree(d32);
+        pool_free(r32);
+        pool_free(d32);
     }
     if (rc == FGPU_OK && !cfg->mixed) {
         rc = mf_residual64(ctx, op, d_b, d_x, r, q, &rn);
         if (rc == FGPU_OK && fail == 0 && rn > cfg->rtol * bn) fail = 2;
     }
-    cudaFree(r);
-    cudaFree(q);
-    cudaFree(xc);
-    cudaFree(r2b);
+    pool_free(r);
+    pool_free(q);
+    pool_free(xc);
+    pool_free(r2b);
     cudaEventRecord(e1, ctx->stream);
     cudaEventSynchronize(e1);
     float ms = 0;
@@ -964,16 +964,16 @@ extern "C" int fgpu_operator_create(fgpu_ctx* ctx, fgpu_space* V, const fgpu_for
         return code;
     };
     if (f->kappa_elem) {
-        if (cudaMalloc(&dk, op->nt * sizeof(double)) != cudaSuccess) return fail(FGPU_ERR_ALLOC, "operator: allocation failed");
+        if (dev_malloc(&dk, op->nt * sizeof(double)) != cudaSuccess) return fail(FGPU_ERR_ALLOC, "operator: allocation failed");
         cudaMemcpyAsync(dk, f->kappa_elem, op->nt * sizeof(double), cudaMemcpyHostToDevice, ctx->stream);
     }
     const size_t es = precision == FGPU_F32 ? sizeof(float) : sizeof(double);
-    if (cudaMalloc(&op->d_rec, op->nt * 4 * sizeof(float4)) != cudaSuccess ||
-        cudaMalloc(&op->d_ye, op->nt * V->n * es) != cudaSuccess)
+    if (dev_malloc(&op->d_rec, op->nt * 4 * sizeof(float4)) != cudaSuccess ||
+        dev_malloc(&op->d_ye, op->nt * V->n * es) != cudaSuccess)
         return fail(FGPU_ERR_ALLOC, "operator: allocation failed");
     int rc = launch_geometry_df(ctx, V->mesh, dk, f->kappa, f->mass, op->d_rec);
     if (!rc && precision == FGPU_F64) {
-        if (cudaMalloc(&op->d_coef, op->nt * 8 * sizeof(double)) != cudaSuccess) return fail(FGPU_ERR_ALLOC, "operator: allocation failed");
+        if (dev_malloc(&op->d_coef, op->nt * 8 * sizeof(double)) != cudaSuccess) return fail(FGPU_ERR_ALLOC, "operator: allocation failed");
         rc = launch_geometry(ctx, V->mesh, FGPU_FORM_LAPLACE_MASS, dk, f->kappa, f->mass, 0, 0, op->d_coef);
     }
     if (!rc) rc = operator_diagonal(ctx, op);
@@ -993,8 +993,8 @@ extern "C" int fgpu_operator_set_dirichlet(fgpu_operator* op, int64_t ndofs, con
         if (dofs[k] < 0 || dofs[k] >= op->nnodes) { ctx->err = "dirichlet dof out of range"; return FGPU_ERR_OUT_OF_RANGE; }
         m[dofs[k]] = 1;
     }
-    if (!op->d_mask) FGPU_CUDA_CHECK(ctx, cudaMalloc(&op->d_mask, op->nnodes));
-    if (op->precision == FGPU_F32 && !op->d_xm) FGPU_CUDA_CHECK(ctx, cudaMalloc(&op->d_xm, op->nnodes * sizeof(float)));
+    if (!op->d_mask) FGPU_CUDA_CHECK(ctx, dev_malloc(&op->d_mask, op->nnodes));
+    if (op->precision == FGPU_F32 && !op->d_xm) FGPU_CUDA_CHECK(ctx, dev_malloc(&op->d_xm, op->nnodes * sizeof(float)));
     FGPU_CUDA_CHECK(ctx, cudaMemcpyAsync(op->d_mask, m.data(), op->nnodes, cudaMemcpyHostToDevice, ctx->stream));
     int rc = operator_diagonal(ctx, op);
     if (rc) return rc;
@@ -1007,8 +1007,8 @@ extern "C" int fgpu_operator_apply(fgpu_ctx* ctx, fgpu_operator* op, const fgpu_
     int rc;
     if (op->precision == FGPU_F32) {
         // the binary32 copies stay with the operator (no allocation per apply)
-        if (!op->d_xf && (cudaMalloc(&op->d_xf, op->nnodes * 4) != cudaSuccess ||
-                          cudaMalloc(&op->d_yf, op->nnodes * 4) != cudaSuccess)) {
+        if (!op->d_xf && (dev_malloc(&op->d_xf, op->nnodes * 4) != cudaSuccess ||
+                          dev_malloc(&op->d_yf, op->nnodes * 4) != cudaSuccess)) {
             cudaFree(op->d_xf);
             op->d_xf = nullptr;
             ctx->err = "apply: allocation failed";
@@ -1058,11 +1058,11 @@ extern "C" int fgpu_operator_set_algo(fgpu_operator* op, int algo) {
         std::vector<int32_t> perm;
         const int nc = colour_elements(M->nv, M->nt, M->h_tets.data(), perm, M->colour_ptr);
         if (nc < 0) { ctx->err = "colour scatter: more than 64 colours"; return FGPU_ERR_INVALID; }
-        FGPU_CUDA_CHECK(ctx, cudaMalloc(&M->d_colour_perm, perm.size() * sizeof(int32_t)));
+        FGPU_CUDA_CHECK(ctx, dev_malloc(&M->d_colour_perm, perm.size() * sizeof(int32_t)));
         FGPU_CUDA_CHECK(ctx, cudaMemcpy(M->d_colour_perm, perm.data(), perm.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
         M->ncolours = nc;
     }
-    if (!op->d_xs) FGPU_CUDA_CHECK(ctx, cudaMalloc(&op->d_xs, op->nnodes * sizeof(float)));
+    if (!op->d_xs) FGPU_CUDA_CHECK(ctx, dev_malloc(&op->d_xs, op->nnodes * sizeof(float)));
     op->algo = FGPU_ALGO_COLOUR;
     return FGPU_OK;
 }

@@ -401,8 +401,8 @@ extern "C" int fgpu_tc_selftest(fgpu_ctx* ctx, const float* hA, const float* hB,
     constexpr int KPAD = 24, NMMA = 144;
     float *A = nullptr, *B = nullptr, *D = nullptr;
     auto done = [&](int rc) { cudaFree(A); cudaFree(B); cudaFree(D); return rc; };
-    if (cudaMalloc(&A, kTcTile * KPAD * 4) != cudaSuccess || cudaMalloc(&B, NMMA * KPAD * 4) != cudaSuccess ||
-        cudaMalloc(&D, kTcTile * NMMA * 4) != cudaSuccess)
+    if (dev_malloc(&A, kTcTile * KPAD * 4) != cudaSuccess || dev_malloc(&B, NMMA * KPAD * 4) != cudaSuccess ||
+        dev_malloc(&D, kTcTile * NMMA * 4) != cudaSuccess)
         return done(FGPU_ERR_ALLOC);
     cudaMemcpy(A, hA, kTcTile * KPAD * 4, cudaMemcpyHostToDevice);
     cudaMemcpy(B, hB, NMMA * KPAD * 4, cudaMemcpyHostToDevice);

@@ -420,13 +420,13 @@ int lanczos_lmax(fgpu_pmg* P, int m, double* out) {
     float *s = nullptr, *v = nullptr, *vold = nullptr, *t = nullptr, *u = nullptr;
     double* part = nullptr;
     std::vector<double> h(152 * 8);
-    cudaError_t e = cudaMalloc(&s, n * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&v, n * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&vold, n * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&t, n * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&u, n * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&part, h.size() * sizeof(double));
-    if (e != cudaSuccess) { cudaGetLastError(); ctx->err = "pmg: allocation failed"; cudaFree(s); cudaFree(v); cudaFree(vold); cudaFree(t); cudaFree(u); cudaFree(part); return FGPU_ERR_ALLOC; }
+    cudaError_t e = pool_malloc(ctx->stream, &s, n * 4);
+    if (e == cudaSuccess) e = pool_malloc(ctx->stream, &v, n * 4);
+    if (e == cudaSuccess) e = pool_malloc(ctx->stream, &vold, n * 4);
+    if (e == cudaSuccess) e = pool_malloc(ctx->stream, &t, n * 4);
+    if (e == cudaSuccess) e = pool_malloc(ctx->stream, &u, n * 4);
+    if (e == cudaSuccess) e = pool_malloc(ctx->stream, &part, h.size() * sizeof(double));
+    if (e != cudaSuccess) { cudaGetLastError(); ctx->err = "pmg: allocation failed"; pool_free(s); pool_free(v); pool_free(vold); pool_free(t); pool_free(u); pool_free(part); return FGPU_ERR_ALLOC; }
     // s = D^-1/2 (from dinv), v0 pseudo-random (hash of the index), normalised
     lanczos_init_kernel<<<vb_of(n), 256, 0, ctx->stream>>>(n, P->dinv, s, t);
     const double nv = std::sqrt(dot(ctx, n, t, t, part, h));
@@ -449,7 +449,7 @@ int lanczos_lmax(fgpu_pmg* P, int m, double* out) {
         bprev = b;
     }
     cudaError_t e2 = cudaStreamSynchronize(ctx->stream);
-    cudaFree(s); cudaFree(v); cudaFree(vold); cudaFree(t); cudaFree(u); cudaFree(part);
+    pool_free(s); pool_free(v); pool_free(vold); pool_free(t); pool_free(u); pool_free(part);
     if (e2 != cudaSuccess) { ctx->err = cudaGetErrorString(e2); return FGPU_ERR_CUDA; }
     std::vector<double> off(be.begin(), be.end());
     *out = tridiag_max_eig(al, off);
@@ -457,16 +457,17 @@ int lanczos_lmax(fgpu_pmg* P, int m, double* out) {
 }
 
 template <typename T>
-cudaError_t upv(T** dst, const std::vector<T>& v) {
-    cudaError_t e = cudaMalloc(dst, std::max<size_t>(v.size(), 1) * sizeof(T));
-    if (e == cudaSuccess && !v.empty()) e = cudaMemcpy(*dst, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice);
+cudaError_t upv(cudaStream_t stream, T** dst, const std::vector<T>& v) {
+    cudaError_t e = pool_malloc(stream, dst, std::max<size_t>(v.size(), 1) * sizeof(T));
+    if (e == cudaSuccess && !v.empty()) e = cudaMemcpyAsync(*dst, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice, stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(stream);
     return e;
 }
 
 void pmg_free(fgpu_pmg* P) {
-    cudaFree(P->i_col); cudaFree(P->i_val); cudaFree(P->r_ia); cudaFree(P->r_ja); cudaFree(P->r_a);
-    cudaFree(P->dinv); cudaFree(P->rf); cudaFree(P->x); cudaFree(P->w); cudaFree(P->q); cudaFree(P->d0); cudaFree(P->d1);
-    cudaFree(P->e); cudaFree(P->rc);
+    pool_free(P->i_col); pool_free(P->i_val); pool_free(P->r_ia); pool_free(P->r_ja); pool_free(P->r_a);
+    pool_free(P->dinv); pool_free(P->rf); pool_free(P->x); pool_free(P->w); pool_free(P->q); pool_free(P->d0); pool_free(P->d1);
+    pool_free(P->e); pool_free(P->rc);
 }
 
 }  // namespace
@@ -511,17 +512,17 @@ extern "C" int fgpu_pmg_create(fgpu_ctx* ctx, fgpu_operator* op32, const fgpu_ma
     float* d_lam = nullptr;
     uint8_t* d_mc = nullptr;
     uint32_t* cnt = nullptr;
-    cudaError_t e = upv(&d_lam, lam);
-    if (e == cudaSuccess) e = cudaMalloc(&d_mc, std::max<int64_t>(P->nc, 1));
+    cudaError_t e = upv(ctx->stream, &d_lam, lam);
+    if (e == cudaSuccess) e = pool_malloc(ctx->stream, &d_mc, std::max<int64_t>(P->nc, 1));
     if (e == cudaSuccess) e = cudaMemsetAsync(d_mc, 0, std::max<int64_t>(P->nc, 1), ctx->stream);
-    if (e == cudaSuccess) e = cudaMalloc(&P->i_col, std::max<int64_t>(P->nf, 1) * 4 * sizeof(int32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&P->i_val, std::max<int64_t>(P->nf, 1) * 4 * sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc(&cnt, (P->nc + 1) * sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&P->r_ia, (P->nc + 1) * sizeof(uint32_t));
+    if (e == cudaSuccess) e = pool_malloc(ctx->stream, &P->i_col, std::max<int64_t>(P->nf, 1) * 4 * sizeof(int32_t));
+    if (e == cudaSuccess) e = pool_malloc(ctx->stream, &P->i_val, std::max<int64_t>(P->nf, 1) * 4 * sizeof(float));
+    if (e == cudaSuccess) e = pool_malloc(ctx->stream, &cnt, (P->nc + 1) * sizeof(uint32_t));
+    if (e == cudaSuccess) e = pool_malloc(ctx->stream, &P->r_ia, (P->nc + 1) * sizeof(uint32_t));
     if (e == cudaSuccess) e = cudaMemsetAsync(cnt, 0, (P->nc + 1) * sizeof(uint32_t), ctx->stream);
     if (e != cudaSuccess) {
         cudaGetLastError();
-        cudaFree(d_lam); cudaFree(d_mc); cudaFree(cnt);
+        pool_free(d_lam); pool_free(d_mc); pool_free(cnt);
         ctx->err = "pmg: allocation failed";
         pmg_free(P); delete P;
         return FGPU_ERR_ALLOC;
@@ -538,8 +539,8 @@ extern "C" int fgpu_pmg_create(fgpu_ctx* ctx, fgpu_operator* op32, const fgpu_ma
     uint64_t nnzr = 0;
     int rc = scan_u32(ctx, cnt, P->r_ia, P->nc, &nnzr);
     if (rc == FGPU_OK) {
-        e = cudaMalloc(&P->r_ja, std::max<uint64_t>(nnzr, 1) * sizeof(int32_t));
-        if (e == cudaSuccess) e = cudaMalloc(&P->r_a, std::max<uint64_t>(nnzr, 1) * sizeof(float));
+        e = pool_malloc(ctx->stream, &P->r_ja, std::max<uint64_t>(nnzr, 1) * sizeof(int32_t));
+        if (e == cudaSuccess) e = pool_malloc(ctx->stream, &P->r_a, std::max<uint64_t>(nnzr, 1) * sizeof(float));
         if (e == cudaSuccess) e = cudaMemcpyAsync(cnt, P->r_ia, P->nc * sizeof(uint32_t), cudaMemcpyDeviceToDevice, ctx->stream);
         if (e == cudaSuccess) {
             pmg_rfill_kernel<<<gf, 256, 0, ctx->stream>>>(P->nf, P->i_col, P->i_val, cnt, P->r_ja, P->r_a);
@@ -554,13 +555,13 @@ extern "C" int fgpu_pmg_create(fgpu_ctx* ctx, fgpu_operator* op32, const fgpu_ma
         }
         if (e != cudaSuccess) { cudaGetLastError(); ctx->err = std::string("pmg: ") + cudaGetErrorString(e); rc = FGPU_ERR_CUDA; }
     }
-    cudaFree(d_lam); cudaFree(d_mc); cudaFree(cnt);
+    pool_free(d_lam); pool_free(d_mc); pool_free(cnt);
     if (rc) { pmg_free(P); delete P; return rc; }
     P->rG = lanes(P->nc, (int64_t)nnzr);
     float** vecs[8] = {&P->rf, &P->x, &P->w, &P->q, &P->d0, &P->d1, &P->e, &P->dinv};
     for (float** p : vecs)
-        if (e == cudaSuccess) e = cudaMalloc(p, std::max<int64_t>(P->nf, 1) * sizeof(float));
-    if (e == cudaSuccess) e = cudaMalloc(&P->rc, std::max<int64_t>(P->nc, 1) * sizeof(float));
+        if (e == cudaSuccess) e = pool_malloc(ctx->stream, p, std::max<int64_t>(P->nf, 1) * sizeof(float));
+    if (e == cudaSuccess) e = pool_malloc(ctx->stream, &P->rc, std::max<int64_t>(P->nc, 1) * sizeof(float));
     if (e != cudaSuccess) { cudaGetLastError(); ctx->err = "pmg: allocation failed"; pmg_free(P); delete P; return FGPU_ERR_ALLOC; }
     // D^-1 of the binary32 operator (Dirichlet rows: 1)
     const float* diag = operator_diag_f32(ctx, op32);

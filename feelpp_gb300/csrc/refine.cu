@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(256) sumsq_kernel(int64_t n, const double* __r
 
 struct RefineWork {
     double *r = nullptr, *d = nullptr, *lo = nullptr, *part = nullptr;
-    ~RefineWork() { cudaFree(r); cudaFree(d); cudaFree(lo); cudaFree(part); }
+    ~RefineWork() { pool_free(r); pool_free(d); pool_free(lo); pool_free(part); }
 };
 
 int norm2(fgpu_ctx* ctx, int64_t n, const double* v, double* part, double* out) {
@@ -122,9 +122,9 @@ int solve_refine_dd(fgpu_ctx* ctx, const fgpu_matrix* A, const fgpu_matrix* A32,
     if (A->precision != FGPU_F64) { ctx->err = "refine_dd: FP64 matrices"; return FGPU_ERR_INVALID; }
     const int64_t n = A->nrows;
     RefineWork W;
-    if (cudaMalloc(&W.r, n * sizeof(double)) != cudaSuccess || cudaMalloc(&W.d, n * sizeof(double)) != cudaSuccess ||
-        (!xl_out && cudaMalloc(&W.lo, n * sizeof(double)) != cudaSuccess) ||
-        cudaMalloc(&W.part, kNormBlocks * sizeof(double)) != cudaSuccess) {
+    if (pool_malloc(ctx->stream, &W.r, n * sizeof(double)) != cudaSuccess || pool_malloc(ctx->stream, &W.d, n * sizeof(double)) != cudaSuccess ||
+        (!xl_out && pool_malloc(ctx->stream, &W.lo, n * sizeof(double)) != cudaSuccess) ||
+        pool_malloc(ctx->stream, &W.part, kNormBlocks * sizeof(double)) != cudaSuccess) {
         cudaGetLastError();
         ctx->err = "refine_dd: allocation failed";
         return FGPU_ERR_ALLOC;

@@ -88,7 +88,7 @@ static inline void scan_u32_launch(fgpu_ctx* ctx, const uint32_t* in, uint32_t* 
 static int scan_u32(fgpu_ctx* ctx, const uint32_t* in, uint32_t* out, int64_t n, uint64_t* total) {
     const int64_t nchunks = scan_chunks(n);
     unsigned long long* sums = nullptr;
-    if (cudaMalloc(&sums, (nchunks + 1) * sizeof(unsigned long long)) != cudaSuccess) {
+    if (pool_malloc(ctx->stream, &sums, (nchunks + 1) * sizeof(unsigned long long)) != cudaSuccess) {
         cudaGetLastError();
         ctx->err = "scan: allocation failed";
         return FGPU_ERR_ALLOC;
@@ -97,7 +97,7 @@ static int scan_u32(fgpu_ctx* ctx, const uint32_t* in, uint32_t* out, int64_t n,
     unsigned long long t = 0;
     cudaMemcpyAsync(&t, sums + nchunks, sizeof(t), cudaMemcpyDeviceToHost, ctx->stream);
     const cudaError_t e = cudaStreamSynchronize(ctx->stream);
-    cudaFree(sums);
+    pool_free(sums);
     if (e != cudaSuccess) { ctx->err = std::string("scan: ") + cudaGetErrorString(e); return FGPU_ERR_CUDA; }
     if (t > 0xFFFFFFFFull) { ctx->err = "scan: total exceeds 32 bits"; return FGPU_ERR_INVALID; }
     if (total) *total = t;

@@ -181,9 +181,9 @@ int build_sell(fgpu_ctx* ctx, const fgpu_matrix* A, std::shared_ptr<SellLayout>&
     L->nrows = A->nrows;
     L->nslices = (A->nrows + kSellC - 1) / kSellC;
     const int64_t nwin = (A->nrows + kSellSigma - 1) / kSellSigma;
-    FGPU_CUDA_CHECK(ctx, cudaMalloc(&L->d_perm, A->nrows * sizeof(int32_t)));
-    FGPU_CUDA_CHECK(ctx, cudaMalloc(&L->d_slice_len, L->nslices * sizeof(int32_t)));
-    FGPU_CUDA_CHECK(ctx, cudaMalloc(&L->d_slice_ptr, (L->nslices + 1) * sizeof(int64_t)));
+    FGPU_CUDA_CHECK(ctx, pool_malloc(ctx->stream, &L->d_perm, A->nrows * sizeof(int32_t)));
+    FGPU_CUDA_CHECK(ctx, pool_malloc(ctx->stream, &L->d_slice_len, L->nslices * sizeof(int32_t)));
+    FGPU_CUDA_CHECK(ctx, pool_malloc(ctx->stream, &L->d_slice_ptr, (L->nslices + 1) * sizeof(int64_t)));
     sell_sort_kernel<<<(int)nwin, kSellSigma, 0, ctx->stream>>>(A->nrows, A->d_ia, L->d_perm, L->d_slice_len);
     ctx->launches++;
     std::vector<int32_t> hlen(L->nslices);
@@ -193,8 +193,8 @@ int build_sell(fgpu_ctx* ctx, const fgpu_matrix* A, std::shared_ptr<SellLayout>&
     for (int64_t s = 0; s < L->nslices; ++s) hptr[s + 1] = hptr[s] + (int64_t)hlen[s] * kSellC;
     L->nstored = hptr[L->nslices];
     FGPU_CUDA_CHECK(ctx, cudaMemcpyAsync(L->d_slice_ptr, hptr.data(), hptr.size() * sizeof(int64_t), cudaMemcpyHostToDevice, ctx->stream));
-    FGPU_CUDA_CHECK(ctx, cudaMalloc(&L->d_col, L->nstored * sizeof(int32_t)));
-    FGPU_CUDA_CHECK(ctx, cudaMalloc(&L->d_src, L->nstored * sizeof(int32_t)));
+    FGPU_CUDA_CHECK(ctx, pool_malloc(ctx->stream, &L->d_col, L->nstored * sizeof(int32_t)));
+    FGPU_CUDA_CHECK(ctx, pool_malloc(ctx->stream, &L->d_src, L->nstored * sizeof(int32_t)));
     const int64_t tot = L->nslices * kSellC;
     sell_fill_kernel<<<(int)std::max<int64_t>(1, std::min<int64_t>((tot + 255) / 256, 152 * 32)), 256, 0, ctx->stream>>>(
         A->nrows, A->d_ia, A->d_ja, L->d_perm, L->d_slice_ptr, L->d_slice_len, L->d_col, L->d_src);
@@ -282,7 +282,7 @@ struct SpmvPlan {
     int G = 4;                         // 0: SELL
     const SellLayout* sell = nullptr;
     typename PL::V* sval = nullptr;    // SELL values (owned)
-    ~SpmvPlan() { cudaFree(sval); }
+    ~SpmvPlan() { pool_free(sval); }
     void launch(cudaStream_t s, const fgpu_matrix* A, const typename PL::V* val, const typename PL::S* x, typename PL::S* y,
                 int mode, const typename PL::S* b, const typename PL::S* wdot, typename PL::D* partial,
                 const CGScalars<PL>* sc) const {
@@ -318,7 +318,7 @@ static int plan_spmv(fgpu_ctx* ctx, const fgpu_matrix* A, const typename PL::V* 
             int rc = build_sell(ctx, A, A->sell);
             if (rc != FGPU_OK) A->sell.reset();
         }
-        if (A->sell && cudaMalloc(&plan.sval, A->sell->nstored * sizeof(typename PL::V)) == cudaSuccess) {
+        if (A->sell && pool_malloc(ctx->stream, &plan.sval, A->sell->nstored * sizeof(typename PL::V)) == cudaSuccess) {
             const int64_t ns = A->sell->nstored;
             sell_values_kernel<PL><<<(int)std::max<int64_t>(1, std::min<int64_t>((ns + 255) / 256, 152 * 32)), 256, 0, ctx->stream>>>(
                 ns, A->sell->d_src, val, plan.sval);
@@ -368,7 +368,7 @@ static int plan_spmv(fgpu_ctx* ctx, const fgpu_matrix* A, const typename PL::V* 
     if (choice == 0 && !have_sell) choice = spmv_group(A);
     plan.G = choice;
     if (choice != 0 && plan.sval) {
-        cudaFree(plan.sval);
+        pool_free(plan.sval);
         plan.sval = nullptr;
     }
     return FGPU_OK;
@@ -386,8 +386,8 @@ static int pcg_core(fgpu_ctx* ctx, const fgpu_matrix* A, const typename PL::V* v
     const int64_t n = A->nrows;
     const int vb = vec_blocks(n);
     S *dinv = nullptr, *tmp = nullptr;
-    if (cudaMalloc(&dinv, n * sizeof(S)) != cudaSuccess || cudaMalloc(&tmp, n * sizeof(S)) != cudaSuccess) {
-        cudaFree(dinv);
+    if (pool_malloc(ctx->stream, &dinv, n * sizeof(S)) != cudaSuccess || pool_malloc(ctx->stream, &tmp, n * sizeof(S)) != cudaSuccess) {
+        pool_free(dinv);
         ctx->err = "CG: allocation failed";
         return FGPU_ERR_ALLOC;
     }
@@ -395,7 +395,7 @@ static int pcg_core(fgpu_ctx* ctx, const fgpu_matrix* A, const typename PL::V* v
     ctx->launches++;
     SpmvPlan<PL> plan;
     plan_spmv<PL>(ctx, A, val, dinv, tmp, plan);
-    cudaFree(tmp);
+    pool_free(tmp);
     CgOperator<PL> op;
     op.apply = [&plan, A, val, ctx](const S* xx, S* yy, typename PL::D* partial, const CGScalars<PL>* sc) {
         plan.launch(ctx->stream, A, val, xx, yy, 0, nullptr, partial ? xx : nullptr, partial, sc);
@@ -406,7 +406,7 @@ static int pcg_core(fgpu_ctx* ctx, const fgpu_matrix* A, const typename PL::V* v
     PcHook<PL> hook;
     if (amg) hook = amg_pc_hook<PL>(amg);
     const int rc = cg_run<PL>(ctx, n, op, dinv, b, x, o, res, refresh, amg ? &hook : nullptr);
-    cudaFree(dinv);
+    pool_free(dinv);
     return rc;
 }
 
@@ -430,10 +430,10 @@ struct Scratch64 {
     double* r = nullptr;
     double* partial = nullptr;
     double* hpart = nullptr;
-    ~Scratch64() { cudaFree(r); cudaFree(partial); cudaFreeHost(hpart); }
-    bool alloc(int64_t n) {
-        return cudaMalloc(&r, n * sizeof(double)) == cudaSuccess && cudaMalloc(&partial, kVecBlocks * sizeof(double)) == cudaSuccess &&
-               cudaMallocHost(&hpart, kVecBlocks * sizeof(double)) == cudaSuccess;
+    ~Scratch64() { pool_free(r); pool_free(partial); pinned_free(hpart); }
+    bool alloc(fgpu_ctx* ctx, int64_t n) {
+        return pool_malloc(ctx->stream, &r, n * sizeof(double)) == cudaSuccess && pool_malloc(ctx->stream, &partial, kVecBlocks * sizeof(double)) == cudaSuccess &&
+               pinned_malloc(&hpart, kVecBlocks * sizeof(double)) == cudaSuccess;
     }
 };
 
@@ -454,7 +454,7 @@ int solve_pcg(fgpu_ctx* ctx, const fgpu_matrix* A, const double* d_b, double* d_
     // true residual b - A x is computed; if it misses rtol (the recurrence drifts
     // on stiff systems) it replaces r and the iteration goes on from p = z.
     Scratch64 R;
-    if (!R.alloc(n)) { ctx->err = "solve: allocation failed"; return FGPU_ERR_ALLOC; }
+    if (!R.alloc(ctx, n)) { ctx->err = "solve: allocation failed"; return FGPU_ERR_ALLOC; }
     double bn0 = 0;
     {
         const int vb = vec_blocks(n);
@@ -479,7 +479,7 @@ int solve_pcg(fgpu_ctx* ctx, const fgpu_matrix* A, const double* d_b, double* d_
     RefreshFn<PolF64> refresh64 = [&](double* xd, double* rd, bool* conv) -> int { return check_true(xd, rd, conv); };
     double* xtmp = nullptr;
     RefreshFn<PolDF64> refresh_df = [&](float2* xd, float2* rd, bool* conv) -> int {
-        if (!xtmp && cudaMalloc(&xtmp, n * sizeof(double)) != cudaSuccess) { cudaGetLastError(); ctx->err = "solve: allocation failed"; return FGPU_ERR_ALLOC; }
+        if (!xtmp && pool_malloc(ctx->stream, &xtmp, n * sizeof(double)) != cudaSuccess) { cudaGetLastError(); ctx->err = "solve: allocation failed"; return FGPU_ERR_ALLOC; }
         df2d_kernel<<<vec_blocks(n), 256, 0, ctx->stream>>>(n, xd, xtmp);
         const int r2 = check_true(xtmp, R.r, conv);
         if (r2) return r2;
@@ -489,8 +489,8 @@ int solve_pcg(fgpu_ctx* ctx, const fgpu_matrix* A, const double* d_b, double* d_
     };
     if (cfg->arith == FGPU_ARITH_DF64) {
         float2 *val = nullptr, *b = nullptr, *x = nullptr;
-        if (cudaMalloc(&val, A->nnz * sizeof(float2)) != cudaSuccess || cudaMalloc(&b, n * sizeof(float2)) != cudaSuccess ||
-            cudaMalloc(&x, n * sizeof(float2)) != cudaSuccess) {
+        if (pool_malloc(ctx->stream, &val, A->nnz * sizeof(float2)) != cudaSuccess || pool_malloc(ctx->stream, &b, n * sizeof(float2)) != cudaSuccess ||
+            pool_malloc(ctx->stream, &x, n * sizeof(float2)) != cudaSuccess) {
             rc = FGPU_ERR_ALLOC;
             ctx->err = "df64 solve: allocation failed";
         } else {
@@ -505,11 +505,11 @@ int solve_pcg(fgpu_ctx* ctx, const fgpu_matrix* A, const double* d_b, double* d_
                 ctx->launches++;
             }
         }
-        cudaFree(val); cudaFree(b); cudaFree(x);
+        pool_free(val); pool_free(b); pool_free(x);
     } else {
         rc = pcg_core<PolF64>(ctx, A, (const double*)A->d_val, d_b, d_x, opt, cfg->pc, &res, &refresh64, amg);
     }
-    cudaFree(xtmp);
+    pool_free(xtmp);
     if (rc == FGPU_OK)    // final residual recomputed in binary64 from the matrix
         rc = f64_residual(ctx, A, d_b, d_x, R.r, R.partial, R.hpart, &rn);
     cudaEventRecord(e1, ctx->stream);
@@ -558,8 +558,8 @@ int solve_pcg_mixed(fgpu_ctx* ctx, const fgpu_matrix* A64, const fgpu_matrix* A3
         Scratch64 S;
         float *r32 = nullptr, *x32 = nullptr;
         double *xc = nullptr, *rc64 = nullptr;
-        if (!S.alloc(n) || cudaMalloc(&r32, n * sizeof(float)) != cudaSuccess || cudaMalloc(&x32, n * sizeof(float)) != cudaSuccess ||
-            cudaMalloc(&xc, n * sizeof(double)) != cudaSuccess || cudaMalloc(&rc64, n * sizeof(double)) != cudaSuccess) {
+        if (!S.alloc(ctx, n) || pool_malloc(ctx->stream, &r32, n * sizeof(float)) != cudaSuccess || pool_malloc(ctx->stream, &x32, n * sizeof(float)) != cudaSuccess ||
+            pool_malloc(ctx->stream, &xc, n * sizeof(double)) != cudaSuccess || pool_malloc(ctx->stream, &rc64, n * sizeof(double)) != cudaSuccess) {
             cudaGetLastError();
             ctx->err = "mixed solve: allocation failed";
             rc = FGPU_ERR_ALLOC;
@@ -638,10 +638,10 @@ int solve_pcg_mixed(fgpu_ctx* ctx, const fgpu_matrix* A64, const fgpu_matrix* A3
             }
             cudaStreamSynchronize(ctx->stream);
         }
-        cudaFree(r32);
-        cudaFree(x32);
-        cudaFree(xc);
-        cudaFree(rc64);
+        pool_free(r32);
+        pool_free(x32);
+        pool_free(xc);
+        pool_free(rc64);
     }
     cudaEventRecord(e1, ctx->stream);
     cudaEventSynchronize(e1);
@@ -667,9 +667,9 @@ int solve_pcg_mixed(fgpu_ctx* ctx, const fgpu_matrix* A64, const fgpu_matrix* A3
 }  // namespace fgpu
 
 SellLayout::~SellLayout() {
-    cudaFree(d_perm);
-    cudaFree(d_slice_ptr);
-    cudaFree(d_slice_len);
-    cudaFree(d_col);
-    cudaFree(d_src);
+    fgpu::pool_free(d_perm);
+    fgpu::pool_free(d_slice_ptr);
+    fgpu::pool_free(d_slice_len);
+    fgpu::pool_free(d_col);
+    fgpu::pool_free(d_src);
 }

@@ -454,9 +454,9 @@ static int build_stream_plan(fgpu_ctx* ctx, fgpu_space* V, int cap, int ctas, St
     const int64_t ne = (nt + kEC - 1) / kEC;
     int32_t *d_last = nullptr, *d_gseq = nullptr, *d_gmax = nullptr;
     auto cleanup = [&] { cudaFree(d_last); cudaFree(d_gseq); cudaFree(d_gmax); };
-    cudaError_t e = cudaMalloc(&d_last, nrows * sizeof(int32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&d_gseq, nrows * sizeof(int32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&d_gmax, ne * sizeof(int32_t));
+    cudaError_t e = dev_malloc(&d_last, nrows * sizeof(int32_t));
+    if (e == cudaSuccess) e = dev_malloc(&d_gseq, nrows * sizeof(int32_t));
+    if (e == cudaSuccess) e = dev_malloc(&d_gmax, ne * sizeof(int32_t));
     if (e != cudaSuccess) { cudaGetLastError(); cleanup(); ctx->err = "streamed assembly: plan allocation failed"; return FGPU_ERR_ALLOC; }
     row_last_elem_kernel<<<152 * 8, 256, 0, ctx->stream>>>(nrows, V->d_inc_ptr, V->d_inc, d_last);
     std::vector<int32_t> last(nrows);
@@ -554,13 +554,13 @@ static int build_stream_plan(fgpu_ctx* ctx, fgpu_space* V, int cap, int ctas, St
     }
     plan->ntickets = (int64_t)tickets.size();
     plan->ctl_bytes = (4 + ne + ng) * sizeof(uint32_t);
-    e = cudaMalloc(&plan->d_ticket, tickets.size() * sizeof(int32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&plan->d_e_need_g, ne * sizeof(int32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&plan->d_g_need_e, ng * sizeof(int32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&plan->d_g_rows, ng * sizeof(int32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&plan->d_g_cnt, ng * sizeof(int32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&plan->d_g_order, nrows);
-    if (e == cudaSuccess) e = cudaMalloc(&plan->d_ctl, plan->ctl_bytes);
+    e = dev_malloc(&plan->d_ticket, tickets.size() * sizeof(int32_t));
+    if (e == cudaSuccess) e = dev_malloc(&plan->d_e_need_g, ne * sizeof(int32_t));
+    if (e == cudaSuccess) e = dev_malloc(&plan->d_g_need_e, ng * sizeof(int32_t));
+    if (e == cudaSuccess) e = dev_malloc(&plan->d_g_rows, ng * sizeof(int32_t));
+    if (e == cudaSuccess) e = dev_malloc(&plan->d_g_cnt, ng * sizeof(int32_t));
+    if (e == cudaSuccess) e = dev_malloc(&plan->d_g_order, nrows);
+    if (e == cudaSuccess) e = dev_malloc(&plan->d_ctl, plan->ctl_bytes);
     if (e != cudaSuccess) { cudaGetLastError(); ctx->err = "streamed assembly: plan allocation failed"; return FGPU_ERR_ALLOC; }
     e = cudaMemcpyAsync(plan->d_ticket, tickets.data(), tickets.size() * sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(plan->d_e_need_g, e_need_g.data(), ne * sizeof(int32_t), cudaMemcpyHostToDevice, ctx->stream);
@@ -604,7 +604,7 @@ static int run_streamed(fgpu_ctx* ctx, fgpu_matrix* A, const DevTables* tab, con
         cudaFree(A->d_kbuf);
         A->d_kbuf = nullptr;
         A->kbuf_bytes = 0;
-        if (cudaMalloc(&A->d_kbuf, need) != cudaSuccess) { cudaGetLastError(); ctx->err = "streamed assembly: element ring allocation failed"; return FGPU_ERR_ALLOC; }
+        if (dev_malloc(&A->d_kbuf, need) != cudaSuccess) { cudaGetLastError(); ctx->err = "streamed assembly: element ring allocation failed"; return FGPU_ERR_ALLOC; }
         A->kbuf_bytes = need;
     }
     const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>(ctas, plan.ntickets));

@@ -301,15 +301,15 @@ int build_space_device(fgpu_ctx* ctx, fgpu_space* V) {
         cudaFree(kv); cudaFree(ke); cudaFree(kf); cudaFree(occ_e); cudaFree(occ_f); cudaFree(w); cudaFree(off);
         cudaFree(etab); cudaFree(ftab); cudaFree(cnt);
     };
-    cudaError_t e = cudaMalloc(&kv, nv * sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&ke, (size_t)ecap * sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&kf, (size_t)fcap * sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&etab, (size_t)ecap * sizeof(unsigned long long));
-    if (e == cudaSuccess) e = cudaMalloc(&ftab, (size_t)fcap * sizeof(unsigned long long));
-    if (e == cudaSuccess) e = cudaMalloc(&occ_e, (size_t)(ndpe ? nt * 6 : 1) * sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&occ_f, (size_t)(ndpf ? nt * 4 : 1) * sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&w, (size_t)nt * 14 * sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&off, ((size_t)nt * 14 + 1) * sizeof(uint32_t));
+    cudaError_t e = dev_malloc(&kv, nv * sizeof(uint32_t));
+    if (e == cudaSuccess) e = dev_malloc(&ke, (size_t)ecap * sizeof(uint32_t));
+    if (e == cudaSuccess) e = dev_malloc(&kf, (size_t)fcap * sizeof(uint32_t));
+    if (e == cudaSuccess) e = dev_malloc(&etab, (size_t)ecap * sizeof(unsigned long long));
+    if (e == cudaSuccess) e = dev_malloc(&ftab, (size_t)fcap * sizeof(unsigned long long));
+    if (e == cudaSuccess) e = dev_malloc(&occ_e, (size_t)(ndpe ? nt * 6 : 1) * sizeof(uint32_t));
+    if (e == cudaSuccess) e = dev_malloc(&occ_f, (size_t)(ndpf ? nt * 4 : 1) * sizeof(uint32_t));
+    if (e == cudaSuccess) e = dev_malloc(&w, (size_t)nt * 14 * sizeof(uint32_t));
+    if (e == cudaSuccess) e = dev_malloc(&off, ((size_t)nt * 14 + 1) * sizeof(uint32_t));
     if (e != cudaSuccess) { cudaGetLastError(); cleanup(); ctx->err = "device dof table: allocation failed"; return FGPU_ERR_ALLOC; }
     cudaStream_t s = ctx->stream;
     cudaMemsetAsync(kv, 0xFF, nv * sizeof(uint32_t), s);
@@ -333,10 +333,10 @@ int build_space_device(fgpu_ctx* ctx, fgpu_space* V) {
     if (hst & kStatusTableFull) { cudaMemset(ctx->d_status, 0, sizeof(int)); cleanup(); ctx->err = "device dof table: hash table full"; return FGPU_ERR_INVALID; }
     if (ndof_nodes >= ((uint64_t)1 << 31)) { cleanup(); ctx->err = "too many dofs for 32-bit indices"; return FGPU_ERR_INVALID; }
     const int64_t N = (int64_t)ndof_nodes;
-    e = cudaMalloc(&V->d_l2n, (size_t)nt * n * sizeof(int32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&V->d_inc_ptr, (size_t)(N + 1) * sizeof(int64_t));
-    if (e == cudaSuccess) e = cudaMalloc(&V->d_inc, (size_t)nt * n * sizeof(int32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&cnt, (size_t)(N + 1) * sizeof(uint32_t));
+    e = dev_malloc(&V->d_l2n, (size_t)nt * n * sizeof(int32_t));
+    if (e == cudaSuccess) e = dev_malloc(&V->d_inc_ptr, (size_t)(N + 1) * sizeof(int64_t));
+    if (e == cudaSuccess) e = dev_malloc(&V->d_inc, (size_t)nt * n * sizeof(int32_t));
+    if (e == cudaSuccess) e = dev_malloc(&cnt, (size_t)(N + 1) * sizeof(uint32_t));
     if (e != cudaSuccess) { cudaGetLastError(); cleanup(); ctx->err = "device dof table: allocation failed"; return FGPU_ERR_ALLOC; }
     l2n_kernel<<<eb, 256, 0, s>>>(nt, M->d_tets, n, ndpe, ndpf, kv, ke, kf, occ_e, occ_f, off, V->d_l2n);
     ctx->launches++;
@@ -348,7 +348,7 @@ int build_space_device(fgpu_ctx* ctx, fgpu_space* V) {
         cudaStreamSynchronize(s);         // l2n_kernel has read the entity offsets
         cudaFree(off);
         off = nullptr;
-        if (cudaMalloc(&off, (size_t)(N + 1) * sizeof(uint32_t)) != cudaSuccess) {
+        if (dev_malloc(&off, (size_t)(N + 1) * sizeof(uint32_t)) != cudaSuccess) {
             cudaGetLastError(); cleanup(); ctx->err = "device dof table: allocation failed"; return FGPU_ERR_ALLOC;
         }
         cptr = off;
@@ -465,11 +465,11 @@ int boundary_nodes_device(fgpu_ctx* ctx, const fgpu_space* V, int xmax_on, doubl
     int* dfl = nullptr;
     uint8_t* mark = nullptr;
     auto cleanup = [&]() { cudaFree(ftab); cudaFree(occ); cudaFree(cnt); cudaFree(dfl); cudaFree(mark); };
-    cudaError_t e = cudaMalloc(&ftab, (size_t)cap * sizeof(unsigned long long));
-    if (e == cudaSuccess) e = cudaMalloc(&cnt, (size_t)cap * sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&occ, (size_t)nt * 4 * sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&dfl, fl.size() * sizeof(int));
-    if (e == cudaSuccess) e = cudaMalloc(&mark, std::max<int64_t>(nnodes, 1));
+    cudaError_t e = dev_malloc(&ftab, (size_t)cap * sizeof(unsigned long long));
+    if (e == cudaSuccess) e = dev_malloc(&cnt, (size_t)cap * sizeof(uint32_t));
+    if (e == cudaSuccess) e = dev_malloc(&occ, (size_t)nt * 4 * sizeof(uint32_t));
+    if (e == cudaSuccess) e = dev_malloc(&dfl, fl.size() * sizeof(int));
+    if (e == cudaSuccess) e = dev_malloc(&mark, std::max<int64_t>(nnodes, 1));
     if (e == cudaSuccess) e = cudaMemsetAsync(ftab, 0xFF, (size_t)cap * sizeof(unsigned long long), ctx->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(cnt, 0, (size_t)cap * sizeof(uint32_t), ctx->stream);
     if (e == cudaSuccess) e = cudaMemsetAsync(mark, 0, std::max<int64_t>(nnodes, 1), ctx->stream);
@@ -510,10 +510,10 @@ int build_pattern_device(fgpu_ctx* ctx, fgpu_space* V, DevPattern& P, std::vecto
     const int wpb = std::max(1, std::min(8, (int)(32768 / (S * 4))));
     uint32_t *cnt = nullptr, *ptr32 = nullptr;
     int* dmax = nullptr;
-    cudaError_t e = cudaMalloc(&cnt, (size_t)(N + 1) * sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&ptr32, (size_t)(N + 1) * sizeof(uint32_t));
-    if (e == cudaSuccess) e = cudaMalloc(&dmax, sizeof(int));
-    if (e == cudaSuccess) e = cudaMalloc(&P.d_ia, (size_t)(N + 1) * sizeof(int64_t));
+    cudaError_t e = dev_malloc(&cnt, (size_t)(N + 1) * sizeof(uint32_t));
+    if (e == cudaSuccess) e = dev_malloc(&ptr32, (size_t)(N + 1) * sizeof(uint32_t));
+    if (e == cudaSuccess) e = dev_malloc(&dmax, sizeof(int));
+    if (e == cudaSuccess) e = dev_malloc(&P.d_ia, (size_t)(N + 1) * sizeof(int64_t));
     auto cleanup = [&]() { cudaFree(cnt); cudaFree(ptr32); cudaFree(dmax); };
     if (e != cudaSuccess) { cudaGetLastError(); cleanup(); ctx->err = "device pattern: allocation failed"; return FGPU_ERR_ALLOC; }
     cudaStream_t s = ctx->stream;
@@ -528,7 +528,7 @@ int build_pattern_device(fgpu_ctx* ctx, fgpu_space* V, DevPattern& P, std::vecto
     int rc = scan_u32(ctx, cnt, ptr32, N, &nnz);
     if (rc) { cleanup(); return rc; }
     u32_to_i64_kernel<<<sms * 8, 256, 0, s>>>(N + 1, ptr32, P.d_ia);
-    e = cudaMalloc(&P.d_ja, (size_t)std::max<uint64_t>(nnz, 1) * sizeof(int32_t));
+    e = dev_malloc(&P.d_ja, (size_t)std::max<uint64_t>(nnz, 1) * sizeof(int32_t));
     if (e != cudaSuccess) { cudaGetLastError(); cleanup(); ctx->err = "device pattern: allocation failed"; return FGPU_ERR_ALLOC; }
     pattern_rows_kernel<<<sms * 8, wpb * 32, smem, s>>>(N, n, V->d_inc_ptr, V->d_inc, V->d_l2n, S, 1, nullptr, P.d_ia, P.d_ja, dmax,
                                                        ctx->d_status);
