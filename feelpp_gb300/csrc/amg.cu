@@ -29,6 +29,7 @@
 #include <string>
 #include <vector>
 
+#include "ld_stream.cuh"
 #include "cg_driver.cuh"
 
 struct fgpu_amg {
@@ -135,30 +136,53 @@ struct AmgSell {
     const float* val = nullptr;
 };
 
-// row i (in sorted order) of a SELL sweep: the entries of its slice column, four loads issued together
-// (memory-level parallelism), summed in entry order, then the epilogue on the original row
+// Row i (in sorted order) of a SELL sweep: the entries of its slice column eight at a time, the next eight
+// columns and values loaded before this batch's gathers of x, summed in entry order, then the epilogue on
+// the original row. The kernel waits on memory: 45 warps of an SM have to keep some 45 KB in flight, and
+// x has to stay in L1 beside the columns and values streaming through. P2 48^3 (206 MB): 52.9 us with four
+// entries and no load ahead, 48.9 with four loaded ahead, 43.0 with those past L1, 41.2 with eight (47.0
+// through L1).
 template <int MODE>
 __device__ __forceinline__ void sell_row(const AmgSweep& s, const AmgSell& m, int64_t i) {
+    constexpr int U = 8;
     const int64_t sl = i >> 5;
     const int L = __ldg(m.len + sl);
     const int64_t base = __ldg(m.ptr + sl) + (i & 31);
+    const int32_t row = i < s.n ? __ldg(m.perm + i) : -1;
     float acc = 0.0f;
+    int32_t c[U];
+    float v[U];
+    if (L >= U) {
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            c[u] = ld_stream(m.col + base + u * 32);
+            v[u] = ld_stream(m.val + base + u * 32);
+        }
+    }
     int k = 0;
-    for (; k + 4 <= L; k += 4) {
-        const int64_t j = base + (int64_t)k * 32;
-        const int32_t c0 = __ldg(m.col + j), c1 = __ldg(m.col + j + 32), c2 = __ldg(m.col + j + 64), c3 = __ldg(m.col + j + 96);
-        const float v0 = __ldg(m.val + j), v1 = __ldg(m.val + j + 32), v2 = __ldg(m.val + j + 64), v3 = __ldg(m.val + j + 96);
-        const float x0 = __ldg(s.x + c0), x1 = __ldg(s.x + c1), x2 = __ldg(s.x + c2), x3 = __ldg(s.x + c3);
-        acc = fmaf(v0, x0, acc);
-        acc = fmaf(v1, x1, acc);
-        acc = fmaf(v2, x2, acc);
-        acc = fmaf(v3, x3, acc);
+    for (; k + U <= L; k += U) {
+        float x[U], vc[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            x[u] = __ldg(s.x + c[u]);
+            vc[u] = v[u];
+        }
+        if (k + 2 * U <= L) {
+            const int64_t j = base + (int64_t)(k + U) * 32;
+#pragma unroll
+            for (int u = 0; u < U; ++u) {
+                c[u] = ld_stream(m.col + j + u * 32);
+                v[u] = ld_stream(m.val + j + u * 32);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) acc = fmaf(vc[u], x[u], acc);
     }
     for (; k < L; ++k) {
         const int64_t j = base + (int64_t)k * 32;
-        acc = fmaf(__ldg(m.val + j), __ldg(s.x + __ldg(m.col + j)), acc);
+        acc = fmaf(ld_stream(m.val + j), __ldg(s.x + ld_stream(m.col + j)), acc);
     }
-    if (i < s.n) amg_epilogue<MODE>(s, __ldg(m.perm + i), acc);
+    if (row >= 0) amg_epilogue<MODE>(s, row, acc);
 }
 
 // one sweep of a level operator in SELL form: thread per (sorted) row, then the epilogue on the
