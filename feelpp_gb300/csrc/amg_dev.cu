@@ -15,13 +15,11 @@
 //     by the host's Sturm bisection;
 //   * P0(i, agg(i)) = 1/sqrt(|agg|), A P0, and P = P0 - omega D^-1 (A P0) merged row by row;
 //   * R = P^T by counting, a scan, a fill and a per-row sort;
-//   * sparse products A P0, A P and R (A P): one warp per row of the left factor. The row's products
-//     are enumerated in (left column, right column) order 32 at a time; lanes holding the same output
-//     column form a group whose lowest lane inserts the column into a shared-memory hash table and adds
-//     the group's products to its running sum one by one in lane order, so every output entry is the
-//     host's sequential sum. Rows with more distinct columns than the small table holds are listed and
-//     redone with a larger table; the row is then sorted by column in shared memory (bitonic sort of
-//     the table's slot list) and written out.
+//   * sparse products A P0, A P and R (A P): a group of lanes per row of the left factor takes its entries
+//     in order, the lanes beside one another on the distinct columns of the entry's right row, so that
+//     every output entry is the host's sequential sum; columns in a shared-memory hash table per row,
+//     sorted and written at the end. Rows with more distinct columns than the table holds are listed and
+//     redone with a larger one. A P0 of a constant near null space has one thread per row.
 // Levels of at most 2048 rows, and any level with a row beyond the kernels' staging capacity, go to
 // the host set-up for the rest of the hierarchy (the results are the same either way).
 #include <algorithm>
@@ -60,8 +58,10 @@ constexpr int64_t kHandoffRows = 2048;       // levels this small continue on th
                                               // level 1 built on the host took 21 ms of a 50 ms set-up, 1 ms on the device)
 constexpr int kSortMax = 16384;              // longest row sorted by seg_sort_kernel
 constexpr int kNumBins = 4;
-constexpr int kBins[kNumBins] = {256, 1024, 2048, 8192};  // hash table sizes (at most half full)
+constexpr int kBins[kNumBins] = {256, 1024, 2048, 8192};  // hash table sizes of whole warps (at most half full)
 constexpr int kBinLog[kNumBins] = {8, 10, 11, 13};
+constexpr int64_t kPadBytes = (int64_t)2 << 30;   // largest padded form of a product
+constexpr int64_t kGroupRows = 4096;          // products with fewer rows take a warp per row
 
 int grid_rows(int64_t n, int per_block, int cap = 152 * 16) {
     return (int)std::max<int64_t>(1, std::min<int64_t>((n + per_block - 1) / per_block, cap));
@@ -344,26 +344,6 @@ __global__ void u32_to_i64_kernel(int64_t n1, const uint32_t* __restrict__ a, in
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n1; i += (int64_t)gridDim.x * blockDim.x) b[i] = a[i];
 }
 
-// longest row and largest product count of a sparse product's rows (left factor A, right factor B)
-__global__ void row_stats_kernel(int64_t n, const int64_t* __restrict__ ia, const int32_t* __restrict__ ja, const int64_t* __restrict__ ib,
-                                 unsigned long long* __restrict__ out) {
-    unsigned long long mlen = 0, mprod = 0;
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        unsigned long long pr = 0;
-        for (int64_t p = ia[i]; p < ia[i + 1]; ++p) pr += (unsigned long long)(ib[ja[p] + 1] - ib[ja[p]]);
-        mlen = max(mlen, (unsigned long long)(ia[i + 1] - ia[i]));
-        mprod = max(mprod, pr);
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        mlen = max(mlen, __shfl_xor_sync(0xffffffffu, mlen, o));
-        mprod = max(mprod, __shfl_xor_sync(0xffffffffu, mprod, o));
-    }
-    if ((threadIdx.x & 31) == 0) {
-        atomicMax(out, mlen);
-        atomicMax(out + 1, mprod);
-    }
-}
-
 // node of each dof (near null space levels: nodes are consecutive dof ranges)
 __global__ void node_of_kernel(int64_t nn, const int64_t* __restrict__ node_ptr, int32_t* __restrict__ node_of) {
     for (int64_t I = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; I < nn; I += (int64_t)gridDim.x * blockDim.x)
@@ -592,10 +572,20 @@ __global__ void agg_scale_kernel(int64_t nagg, const unsigned int* __restrict__ 
         s0[c] = __ddiv_rn(1.0, __dsqrt_rn((double)sz[c]));
 }
 
-// Sparse product C = A B, one warp per row of A (see the file comment). Count pass (oj == nullptr):
-// cnt[i] = distinct columns of row i, or row i appended to `ovf` when it holds more than tsize / 2
-// (status overflow when ovf is null). Fill pass: rows whose count exceeds tsize / 2 are left to a
-// larger table; the others are written sorted at off[i].
+// Sparse product C = A B, G lanes per row of A. The lanes take one entry of A's row after another and
+// beside it G products with the entry's row of B, whose columns are distinct: no two lanes of a step meet
+// in an output entry, and every output entry is its products' sum in the order of A's row, the host's.
+// Each group has a hash table of T slots in shared memory (slot h of group g at h * (32 / G) + g). kCount:
+// cnt[i] = distinct columns of row i, or row i appended to `ovf` when it holds more than `cap` (status
+// overflow when ovf is null). kFill: rows whose count exceeds the cap are left to a larger table; the others
+// are written sorted at off[i]. kPadded: both at once, the row written sorted at i * cap, from where
+// pad_copy_kernel takes it to its place once the counts are summed. The groups of a warp run in step (each on its own entry),
+// a step's columns and values loaded during the step before it, the entries of A's row two groups ahead.
+// Bound: the FP64 pipe (a warp's product and sum occupy it 32 cycles) and instruction issue, each busy two
+// thirds of the time. P2 48^3, A P (25.8 M entries x 4): 1150 us to count and 2910 to fill -> 1710 padded
+// and 70 to copy; R (A P): 461 + 728 -> 603 + 7, against one warp per row that numbered 32 products at a
+// time by a search over the row's prefix sums and grouped equal columns by __match_any_sync. Four lanes a row
+// give 1600 on A P and lose a third on the next level; two 1600-2300, one 2700-5100.
 struct SpgemmArgs {
     int64_t nrows = 0;
     const int32_t* rows = nullptr;   // row list (null: rows 0..nrows-1)
@@ -605,7 +595,7 @@ struct SpgemmArgs {
     const int64_t* ib = nullptr;
     const int32_t* jb = nullptr;
     const double* b = nullptr;
-    int tsize = 256;                 // hash slots per warp (power of two, >= 64)
+    int tsize = 256;                 // hash slots per row (power of two, >= 64)
     int tshift = 24;                 // 32 - log2(tsize)
     int warps = 8;                   // warps per block
     int wbytes = 0;                  // shared memory per warp
@@ -618,124 +608,159 @@ struct SpgemmArgs {
     int* status = nullptr;
 };
 
-int spgemm_warp_bytes(int tsize) {
-    const int b = tsize * 8 + 32 * 8 + tsize * 4 + (tsize / 2) * 4;
-    return (b + 15) & ~15;
+__host__ __device__ constexpr int spgemm_cap(int tsize, int group) { return group <= 8 ? tsize - tsize / 4 : tsize / 2; }
+int spgemm_warp_bytes(int tsize, int group, bool fill) {
+    return tsize * (32 / group) * ((fill ? 8 : 0) + 4 + 2);
 }
 
+enum { kCount, kFill, kPadded };
+constexpr int kRankMax = 128;        // rows up to this long are sorted by counting smaller columns
+
+template <int G, int MODE>
 __global__ void __launch_bounds__(256) spgemm_kernel(SpgemmArgs g) {
     extern __shared__ __align__(16) unsigned char sg_smem[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    constexpr int NG = 32 / G;
+    constexpr bool FILL = MODE != kCount;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = lane & (G - 1), grp = lane / G;
+    const unsigned gmask = G == 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u) << (grp * G);
+    const int T = g.tsize, cap = spgemm_cap(T, G);
     unsigned char* base = sg_smem + (size_t)warp * g.wbytes;
-    double* hv = reinterpret_cast<double*>(base);                               // tsize values
-    double* stage = hv + g.tsize;                                               // 32 products
-    int32_t* hk = reinterpret_cast<int32_t*>(stage + 32);                       // tsize keys (-1: empty)
-    int32_t* list = hk + g.tsize;                                               // tsize / 2 used slots
-    const int T = g.tsize, half = g.tsize / 2;
-    const bool fill = g.oj != nullptr;
-    for (int k = lane; k < T; k += 32) hk[k] = -1;
+    double* hv = reinterpret_cast<double*>(base) + grp;                                        // values
+    int32_t* hk = reinterpret_cast<int32_t*>(base + (FILL ? (size_t)T * NG * 8 : 0)) + grp;    // keys (-1: empty)
+    uint16_t* list = reinterpret_cast<uint16_t*>(hk - grp + T * NG) + grp;                     // used slots
+    for (int k = sub; k < T; k += G) hk[k * NG] = -1;
     __syncwarp();
-    for (int64_t r = (int64_t)blockIdx.x * g.warps + warp; r < g.nrows; r += (int64_t)gridDim.x * g.warps) {
-        const int64_t i = g.rows ? (int64_t)g.rows[r] : r;
-        if (fill && g.off[i + 1] - g.off[i] > half) continue;        // a larger table's row
-        const int64_t a0 = g.ia[i];
-        const int na = (int)(g.ia[i + 1] - a0);
+    const int64_t step = (int64_t)gridDim.x * g.warps * NG;
+    for (int64_t r0 = ((int64_t)blockIdx.x * g.warps + warp) * NG; r0 < g.nrows; r0 += step) {
+        const int64_t r = r0 + grp;
+        bool act = r < g.nrows;
+        int64_t i = 0, ob = 0;
+        uint32_t a0 = 0;
+        int na = 0;
+        if (act) {
+            i = g.rows ? (int64_t)g.rows[r] : r;
+            if (MODE == kFill) {
+                ob = g.off[i];
+                act = g.off[i + 1] - ob <= cap;                     // else a larger table's row
+            }
+            if (MODE == kPadded) ob = i * cap;
+            a0 = (uint32_t)g.ia[i];                                  // all factors have fewer than 2^32 entries
+            na = act ? (int)((uint32_t)g.ia[i + 1] - a0) : 0;
+        }
+        const bool mine = act;
         int nuniq = 0;
         bool over = false;
-        // the row of A in chunks of 32 entries (one per lane: its B row's start, length and the A value);
-        // the chunk's products in (A column, B column) order, 32 at a time
-        for (int c0 = 0; c0 < na && !over; c0 += 32) {
-            const int cn = min(32, na - c0);
-            int len = 0;
-            int64_t bstart = 0;
-            double av = 0.0;
-            if (lane < cn) {
-                const int32_t c = g.ja[a0 + c0 + lane];
-                bstart = g.ib[c];
-                len = (int)(g.ib[c + 1] - bstart);
-                if (fill) av = g.a[a0 + c0 + lane];
+        // the group's place: entry e of the row, product q of the entry; lane `sub` holds the entries
+        // congruent to it of the current G
+        int e = -1, q = 0, len = 0;
+        uint32_t bstart = 0, cb = 0;
+        int clen = 0;
+        double av = 0.0, ca = 0.0;
+        int32_t ncol = -1;
+        double nb_ = 0.0, na_ = 0.0;
+        // entries t .. t + G - 1 (their columns loaded before), and the columns of the G after them
+        uint32_t pb = 0, pe = 0;
+        int32_t pc = 0;
+        double pa = 0.0;
+        auto ahead = [&](int t) {
+            if (t + sub < na) {
+                pb = (uint32_t)g.ib[pc];
+                pe = (uint32_t)g.ib[pc + 1];
+                if (FILL) pa = g.a[a0 + t + sub];
             }
-            int x = len;
-            for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, x, o);
-                if (lane >= o) x += y;
+            if (t + G + sub < na) pc = g.ja[a0 + t + G + sub];
+        };
+        if (sub < na) pc = g.ja[a0 + sub];
+        ahead(0);
+        auto advance = [&]() {                                       // the next step's column and value
+            const bool next = e < na && q + G >= len;
+            if (next) {
+                ++e;
+                q = 0;
+            } else {
+                q += G;
             }
-            const int excl = x - len;
-            const int ctot = __shfl_sync(0xffffffffu, x, 31);
-            for (int s0 = 0; s0 < ctot; s0 += 32) {
-                const int pidx = s0 + lane;
-                const bool act = pidx < ctot;
-                // the chunk entry of product pidx: the last lane e < cn with excl_e <= pidx (fixed 5 steps)
-                int lo = 0;
-                for (int step = 16; step > 0; step >>= 1) {
-                    const int cand = lo + step;
-                    const int ec = __shfl_sync(0xffffffffu, excl, cand & 31);
-                    if (cand < cn && ec <= pidx) lo = cand;
-                }
-                const int e_excl = __shfl_sync(0xffffffffu, excl, lo);
-                const int64_t e_start = __shfl_sync(0xffffffffu, bstart, lo);
-                const double e_a = __shfl_sync(0xffffffffu, av, lo);
-                int32_t col = -1;
-                double val = 0.0;
-                if (act) {
-                    const int64_t q = e_start + (pidx - e_excl);
-                    col = g.jb[q];
-                    if (fill) val = __dmul_rn(e_a, g.b[q]);
-                }
-                const unsigned grp = __match_any_sync(0xffffffffu, col);
-                const bool leader = act && lane == __ffs(grp) - 1;
-                int slot = -1;
-                bool newkey = false;
-                if (leader) {
-                    uint32_t h = ((uint32_t)col * 2654435761u) >> g.tshift;
-                    for (int probe = 0; probe < T; ++probe) {
-                        const int32_t old = atomicCAS(hk + h, -1, col);
-                        if (old == -1) { newkey = true; slot = (int)h; break; }
-                        if (old == col) { slot = (int)h; break; }
-                        h = (h + 1) & (uint32_t)(T - 1);
-                    }
-                    if (slot < 0) over = true;
-                }
-                const unsigned nb = __ballot_sync(0xffffffffu, newkey);
-                if (newkey) {
-                    const int pos = nuniq + __popc(nb & ((1u << lane) - 1u));
-                    if (pos < half) list[pos] = slot;
-                }
-                nuniq += __popc(nb);
-                if (fill) {
-                    stage[lane] = val;
-                    __syncwarp();
-                    if (leader && slot >= 0) {
-                        double v = newkey ? 0.0 : hv[slot];
-                        for (unsigned m = grp; m; m &= m - 1u) v = __dadd_rn(v, stage[__ffs(m) - 1]);
-                        hv[slot] = v;
-                    }
-                }
-                __syncwarp();
-                if (__any_sync(0xffffffffu, over) || nuniq > half) { over = true; break; }
+            if (next && e < na && (e & (G - 1)) == 0) {              // the next G entries; those after them on their way
+                cb = pb;
+                clen = (int)(pe - pb);
+                ca = pa;
+                ahead(e + G);
             }
+            const int src = (e & (G - 1)) + grp * G;
+            const uint32_t sb = __shfl_sync(0xffffffffu, cb, src);
+            const int sl = __shfl_sync(0xffffffffu, clen, src);
+            if (FILL) av = __shfl_sync(0xffffffffu, ca, src);
+            if (next) {
+                bstart = sb;
+                len = sl;
+            }
+            ncol = -1;
+            if (e < na && q + sub < len) {
+                ncol = g.jb[bstart + q + sub];
+                if (FILL) {
+                    nb_ = g.b[bstart + q + sub];
+                    na_ = av;
+                }
+            }
+        };
+        advance();
+        while (__any_sync(0xffffffffu, e < na)) {
+            const int32_t col = ncol;
+            const double va = na_, vb = nb_;
+            advance();
+            int slot = -1;
+            bool newkey = false;
+            if (col >= 0) {
+                uint32_t h = ((uint32_t)col * 2654435761u) >> g.tshift;
+                for (int probe = 0; probe < T; ++probe) {
+                    int32_t old = hk[h * NG];
+                    if (old == -1) old = atomicCAS(hk + h * NG, -1, col);
+                    if (old == -1) { newkey = true; slot = (int)h; break; }
+                    if (old == col) { slot = (int)h; break; }
+                    h = (h + 1) & (uint32_t)(T - 1);
+                }
+            }
+            const unsigned nb = __ballot_sync(0xffffffffu, newkey) & gmask;
+            if (newkey) {
+                const int pos = nuniq + __popc(nb & ((1u << lane) - 1u));
+                if (pos < cap) list[pos * NG] = (uint16_t)slot;
+            }
+            nuniq += __popc(nb);
+            if (FILL && slot >= 0) hv[slot * NG] = __dadd_rn(newkey ? 0.0 : hv[slot * NG], __dmul_rn(va, vb));
+            if (nuniq > cap && !over) {                             // the row ends here: at most cap + G slots used
+                over = true;
+                na = e = 0;
+                ncol = -1;
+            }
+            __syncwarp();
         }
         if (over) {
-            for (int k = lane; k < T; k += 32) hk[k] = -1;
-            __syncwarp();
-            if (lane == 0) {
-                if (!fill && g.ovf) {
-                    g.ovf[atomicAdd(g.novf, 1u)] = (int32_t)i;
-                    g.cnt[i] = 0;
-                } else {
-                    atomicOr(g.status, kStOverflow);
-                    if (!fill) g.cnt[i] = 0;
-                }
+            for (int k = sub; k < T; k += G) hk[k * NG] = -1;
+            if (sub == 0) {
+                if (MODE != kFill && g.ovf) g.ovf[atomicAdd(g.novf, 1u)] = (int32_t)i;
+                else atomicOr(g.status, kStOverflow);
+                if (MODE != kFill) g.cnt[i] = 0;
             }
-            continue;
+            nuniq = 0;
+        } else if (MODE != kFill && mine && sub == 0) {
+            g.cnt[i] = (uint32_t)nuniq;
         }
-        if (!fill) {
-            if (lane == 0) g.cnt[i] = (uint32_t)nuniq;
-        } else {
-            // sort the used slots by key (padding slots -1 sort last), then write the row
+        if (FILL && nuniq <= kRankMax) {
+            // place of a column: the number of smaller ones in the row
+            for (int k = sub; k < nuniq; k += G) {
+                const int s = list[k * NG];
+                const int32_t key = hk[s * NG];
+                int rank = 0;
+                for (int m = 0; m < nuniq; ++m) rank += hk[list[m * NG] * NG] < key;
+                g.oj[ob + rank] = key;
+                g.oa[ob + rank] = hv[s * NG];
+            }
+        } else if (FILL && G == 32) {
+            // bitonic sort of the used slots by key (padding last), then the row
             int P = 1;
             while (P < nuniq) P <<= 1;
-            for (int k = nuniq + lane; k < P; k += 32) list[k] = -1;
+            constexpr uint16_t kPad = 0xffff;
+            for (int k = nuniq + lane; k < P; k += 32) list[k] = kPad;
             __syncwarp();
             for (int size = 2; size <= P; size <<= 1)
                 for (int stride = size >> 1; stride > 0; stride >>= 1) {
@@ -743,8 +768,8 @@ __global__ void __launch_bounds__(256) spgemm_kernel(SpgemmArgs g) {
                         const int l = k ^ stride;
                         if (l > k) {
                             const bool up = (k & size) == 0;
-                            const int32_t sa = list[k], sb = list[l];
-                            const int32_t ka = sa < 0 ? INT32_MAX : hk[sa], kb = sb < 0 ? INT32_MAX : hk[sb];
+                            const uint16_t sa = list[k], sb = list[l];
+                            const int32_t ka = sa == kPad ? INT32_MAX : hk[sa], kb = sb == kPad ? INT32_MAX : hk[sb];
                             if ((ka > kb) == up) {
                                 list[k] = sb;
                                 list[l] = sa;
@@ -753,16 +778,103 @@ __global__ void __launch_bounds__(256) spgemm_kernel(SpgemmArgs g) {
                     }
                     __syncwarp();
                 }
-            const int64_t ob = g.off[i];
             for (int k = lane; k < nuniq; k += 32) {
-                const int32_t s = list[k];
+                const int s = list[k];
                 g.oj[ob + k] = hk[s];
                 g.oa[ob + k] = hv[s];
             }
         }
         __syncwarp();
-        for (int k = lane; k < nuniq; k += 32) hk[list[k]] = -1;
+        for (int k = sub; k < nuniq; k += G) hk[list[k * NG] * NG] = -1;
         __syncwarp();
+    }
+}
+
+// A P0 for the tentative prolongator of the constant vector (row j of P0: s0[agg_j] at column agg_j, or
+// empty): one thread per row with a table of its own, T columns in first-met order, searched from the last
+// hit on; the row's products summed in its order. Modes as above; rows
+// with more than T columns go to the general product. P2 48^3: 793 us to count and 1740 to fill -> 433
+// padded and 50 to copy (FP64 pipe half busy, table latency).
+constexpr int kAp0T = 16;
+template <int MODE>
+__global__ void __launch_bounds__(128) ap0_kernel(SpgemmArgs g, const int32_t* __restrict__ agg, const double* __restrict__ s0) {
+    constexpr bool FILL = MODE != kCount;
+    __shared__ int32_t tk[kAp0T][128];
+    __shared__ double tv[FILL ? kAp0T : 1][128];
+    const int t = threadIdx.x;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + t; i < g.nrows; i += (int64_t)gridDim.x * blockDim.x) {
+        int64_t ob = 0;
+        if (MODE == kFill) {
+            ob = g.off[i];
+            if (g.off[i + 1] - ob > kAp0T) continue;
+        }
+        if (MODE == kPadded) ob = i * kAp0T;
+        const int64_t pe = g.ia[i + 1];
+        int n = 0, last = 0;
+        bool over = false;
+        for (int64_t p = g.ia[i]; p < pe && !over; p += 4) {
+            int32_t c[4];
+            double v[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                c[u] = p + u < pe ? g.ja[p + u] : -1;
+                if (FILL) v[u] = p + u < pe ? g.a[p + u] : 0.0;
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) c[u] = c[u] >= 0 ? agg[c[u]] : -1;
+            if (FILL) {
+                double w[4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u) w[u] = c[u] >= 0 ? s0[c[u]] : 0.0;
+#pragma unroll
+                for (int u = 0; u < 4; ++u) v[u] = __dmul_rn(v[u], w[u]);
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                if (c[u] < 0) continue;
+                if (n == 0 || tk[last][t] != c[u]) {
+                    int k = 0;
+                    while (k < n && tk[k][t] != c[u]) ++k;
+                    if (k == n) {
+                        if (n == kAp0T) { over = true; break; }
+                        tk[n][t] = c[u];
+                        if (FILL) tv[n][t] = 0.0;
+                        ++n;
+                    }
+                    last = k;
+                }
+                if (FILL) tv[last][t] = __dadd_rn(tv[last][t], v[u]);
+            }
+        }
+        if (MODE != kFill) {
+            if (over) g.ovf[atomicAdd(g.novf, 1u)] = (int32_t)i;
+            g.cnt[i] = over ? 0u : (uint32_t)n;
+        }
+        if (FILL && !over) {
+            for (int k = 0; k < n; ++k) {
+                const int32_t key = tk[k][t];
+                int rank = 0;
+                for (int m = 0; m < n; ++m) rank += tk[m][t] < key;
+                g.oj[ob + rank] = key;
+                g.oa[ob + rank] = tv[k][t];
+            }
+        }
+    }
+}
+
+// rows written padded (row i at i * pad) to their places; longer rows are written there by their own pass
+__global__ void __launch_bounds__(256) pad_copy_kernel(int64_t n, int pad, const int64_t* __restrict__ off,
+                                                       const int32_t* __restrict__ pj, const double* __restrict__ pa,
+                                                       int32_t* __restrict__ oj, double* __restrict__ oa) {
+    const int sub = threadIdx.x & 7;
+    for (int64_t i = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 3; i < n; i += ((int64_t)gridDim.x * blockDim.x) >> 3) {
+        const int64_t o = off[i];
+        const int len = (int)(off[i + 1] - o);
+        if (len > pad) continue;
+        for (int k = sub; k < len; k += 8) {
+            oj[o + k] = pj[i * pad + k];
+            oa[o + k] = pa[i * pad + k];
+        }
     }
 }
 
@@ -770,63 +882,114 @@ __global__ void __launch_bounds__(256) spgemm_kernel(SpgemmArgs g) {
 // host drivers
 // ---------------------------------------------------------------------------------------------------
 
-int launch_spgemm(fgpu_ctx* ctx, SpgemmArgs g, int bin) {
-    g.tsize = kBins[bin];
-    g.tshift = 32 - kBinLog[bin];
-    g.wbytes = spgemm_warp_bytes(g.tsize);
-    g.warps = std::max(1, std::min(8, (110 * 1024) / g.wbytes));
+struct SpgemmTable { int group, tsize, log2; };
+
+template <int G, int MODE>
+int launch_spgemm_g(fgpu_ctx* ctx, SpgemmArgs g, const SpgemmTable& t) {
+    g.tsize = t.tsize;
+    g.tshift = 32 - t.log2;
+    g.wbytes = spgemm_warp_bytes(t.tsize, G, MODE != kCount);
+    const int rows = 32 / G;
+    // few rows: one warp a block, so that they spread over the SMs
+    const int spread = (int)std::max<int64_t>(1, g.nrows / (152 * rows));
+    g.warps = std::max(1, std::min({8, spread, (110 * 1024) / g.wbytes}));
     const int smem = g.warps * g.wbytes;
-    DEV_TRY(cudaFuncSetAttribute(spgemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    auto kernel = spgemm_kernel<G, MODE>;
+    DEV_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     const int per_sm = std::max(1, std::min(2048 / (32 * g.warps), (228 * 1024) / (smem + 1024)));
-    const int blocks = grid_rows(g.nrows, g.warps, 152 * per_sm);
-    spgemm_kernel<<<blocks, 32 * g.warps, smem, ctx->stream>>>(g);
+    const int blocks = grid_rows(g.nrows, g.warps * rows, 152 * per_sm);
+    kernel<<<blocks, 32 * g.warps, smem, ctx->stream>>>(g);
     ctx->launches++;
     DEV_TRY(cudaGetLastError());
     return FGPU_OK;
 }
+template <int MODE>
+int launch_spgemm(fgpu_ctx* ctx, const SpgemmArgs& g, const SpgemmTable& t) {
+    if (t.group == 8) return launch_spgemm_g<8, MODE>(ctx, g, t);
+    if (t.group == 16) return launch_spgemm_g<16, MODE>(ctx, g, t);
+    return launch_spgemm_g<32, MODE>(ctx, g, t);
+}
 
-// C = A B (rows sorted by column). *overflow: a row with more distinct columns than the largest table.
-int spgemm_dev(fgpu_ctx* ctx, const AmgDevCsr& A, const AmgDevCsr& B, AmgDevCsr& C, int* d_status, bool* overflow) {
+// C = A B (rows sorted by column). agg, s0: B is the tentative prolongator of the constant vector.
+// *overflow: a row with more distinct columns than the largest table.
+// Table and lanes per row: the first pass takes 8 lanes up to a mean of 8 entries in B's rows, else 16 (a
+// step of 16 lanes on rows of 13 entries does as much as two of 8), with 256 slots where a row has many
+// products and 64 else; a level of few rows takes whole warps, its time one row's chain of steps. Rows that
+// do not fit go on to whole warps with the next larger table.
+int spgemm_dev(fgpu_ctx* ctx, const AmgDevCsr& A, const AmgDevCsr& B, AmgDevCsr& C, int* d_status, bool* overflow,
+               const int32_t* agg = nullptr, const double* s0 = nullptr) {
     *overflow = false;
     const int64_t n = A.nrows;
+    SpgemmTable first = {32, 256, 8};
+    const double ma = (double)A.nnz / std::max<int64_t>(A.nrows, 1), mb = (double)B.nnz / std::max<int64_t>(B.nrows, 1);
+    if (n >= kGroupRows && mb <= 24.0) {
+        first.group = mb <= 8.0 ? 8 : 16;
+        if (ma * mb <= 512.0) first = {first.group, 64, 6};
+    }
+    SpgemmTable tables[1 + kNumBins];
+    int nt = 0;
+    tables[nt++] = first;
+    for (int k = 0; k < kNumBins; ++k)
+        if (kBins[k] > first.tsize) tables[nt++] = {32, kBins[k], kBinLog[k]};
+    if (agg) {                                   // then the first table is ap0_kernel's own
+        tables[0] = {1, kAp0T, 0};
+        nt = 1;
+        for (int k = 0; k < kNumBins; ++k) tables[nt++] = {32, kBins[k], kBinLog[k]};
+    }
     Work w(ctx);
-    unsigned long long* stats = w.get<unsigned long long>(2);
     uint32_t* cnt = w.get<uint32_t>(n + 1);
     uint32_t* off32 = w.get<uint32_t>(n + 1);
-    int32_t* ovf[kNumBins] = {nullptr, w.get<int32_t>(n), w.get<int32_t>(n), w.get<int32_t>(n)};
-    uint32_t* novf = w.get<uint32_t>(kNumBins);
-    DEV_ALLOC(stats && cnt && off32 && ovf[1] && ovf[2] && ovf[3] && novf);
-    DEV_TRY(cudaMemsetAsync(stats, 0, 2 * sizeof(unsigned long long), ctx->stream));
-    DEV_TRY(cudaMemsetAsync(novf, 0, kNumBins * sizeof(uint32_t), ctx->stream));
-    row_stats_kernel<<<grid_rows(n, 256), 256, 0, ctx->stream>>>(n, A.ia, A.ja, B.ia, stats);
-    ctx->launches++;
-    unsigned long long hs[2] = {0, 0};
-    DEV_TRY(cudaMemcpyAsync(hs, stats, sizeof(hs), cudaMemcpyDeviceToHost, ctx->stream));
-    DEV_TRY(cudaStreamSynchronize(ctx->stream));
-    if (hs[1] > 0x7fffffffull) { *overflow = true; return FGPU_OK; }
+    uint32_t* novf = w.get<uint32_t>(1 + kNumBins);
+    int32_t* ovf[1 + kNumBins] = {nullptr};
+    DEV_ALLOC(cnt && off32 && novf);
+    DEV_TRY(cudaMemsetAsync(novf, 0, (1 + kNumBins) * sizeof(uint32_t), ctx->stream));
     SpgemmArgs g;
     g.ia = A.ia; g.ja = A.ja; g.a = A.a;
     g.ib = B.ia; g.jb = B.ja; g.b = B.a;
     g.status = d_status;
-    // count: all rows with the smallest table, the rows it cannot hold with the next ones in turn
-    int64_t rows_in[kNumBins] = {n, 0, 0, 0};
-    {
-        for (int bin = 0; bin < kNumBins; ++bin) {
-            if (bin > 0 && rows_in[bin] == 0) break;
-            SpgemmArgs c = g;
-            c.nrows = rows_in[bin];
-            c.rows = ovf[bin];
-            c.cnt = cnt;
-            c.ovf = bin + 1 < kNumBins ? ovf[bin + 1] : nullptr;
-            c.novf = bin + 1 < kNumBins ? novf + bin + 1 : nullptr;
-            int rc = launch_spgemm(ctx, c, bin);
-            if (rc) return rc;
-            if (bin + 1 < kNumBins) {
-                uint32_t hn = 0;
-                DEV_TRY(cudaMemcpyAsync(&hn, novf + bin + 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
-                DEV_TRY(cudaStreamSynchronize(ctx->stream));
-                rows_in[bin + 1] = hn;
-            }
+    auto launch = [&](SpgemmArgs& x, int k, int mode) -> int {
+        if (!agg || k > 0)
+            return mode == kCount ? launch_spgemm<kCount>(ctx, x, tables[k])
+                                  : mode == kFill ? launch_spgemm<kFill>(ctx, x, tables[k]) : launch_spgemm<kPadded>(ctx, x, tables[k]);
+        const int blocks = grid_rows(n, 128);
+        if (mode == kCount) ap0_kernel<kCount><<<blocks, 128, 0, ctx->stream>>>(x, agg, s0);
+        else if (mode == kFill) ap0_kernel<kFill><<<blocks, 128, 0, ctx->stream>>>(x, agg, s0);
+        else ap0_kernel<kPadded><<<blocks, 128, 0, ctx->stream>>>(x, agg, s0);
+        ctx->launches++;
+        DEV_TRY(cudaGetLastError());
+        return FGPU_OK;
+    };
+    // the first table's rows in one pass where their padded form stays small (2 GB, 3.7 M rows, and four
+    // entries to one of A), which saves the count pass (P2 48^3: 1.8 of 20 ms of set-up)
+    const int pad = agg ? kAp0T : spgemm_cap(first.tsize, first.group);
+    int32_t* pj = nullptr;
+    double* pa = nullptr;
+    if (n * pad * 12 <= kPadBytes && n * pad <= 4 * A.nnz) {
+        pj = w.get<int32_t>(n * pad);
+        pa = pj ? w.get<double>(n * pad) : nullptr;
+        if (!pa) pj = nullptr;                   // no room: counted first
+    }
+    // count: all rows with the first table, the rows it cannot hold with the next ones in turn
+    int64_t rows_in[1 + kNumBins] = {n};
+    for (int k = 0; k < nt && rows_in[k] > 0; ++k) {
+        SpgemmArgs c = g;
+        c.nrows = rows_in[k];
+        c.rows = ovf[k];
+        c.cnt = cnt;
+        if (k + 1 < nt) {
+            DEV_ALLOC(ovf[k + 1] = w.get<int32_t>(rows_in[k]));
+            c.ovf = ovf[k + 1];
+            c.novf = novf + k + 1;
+        }
+        const bool padded = k == 0 && pj;
+        if (padded) { c.oj = pj; c.oa = pa; }
+        int rc = launch(c, k, padded ? kPadded : kCount);
+        if (rc) return rc;
+        if (k + 1 < nt) {
+            uint32_t hn = 0;
+            DEV_TRY(cudaMemcpyAsync(&hn, novf + k + 1, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
+            DEV_TRY(cudaStreamSynchronize(ctx->stream));
+            rows_in[k + 1] = hn;
         }
     }
     int st = 0;
@@ -841,12 +1004,15 @@ int spgemm_dev(fgpu_ctx* ctx, const AmgDevCsr& A, const AmgDevCsr& B, AmgDevCsr&
     u32_to_i64_kernel<<<grid_rows(n + 1, 256), 256, 0, ctx->stream>>>(n + 1, off32, C.ia);
     ctx->launches++;
     g.off = C.ia; g.oj = C.ja; g.oa = C.a;
-    for (int bin = 0; bin < kNumBins; ++bin) {
-        if (rows_in[bin] == 0) continue;
+    if (pj) {
+        pad_copy_kernel<<<grid_rows(n, 32), 256, 0, ctx->stream>>>(n, pad, C.ia, pj, pa, C.ja, C.a);
+        ctx->launches++;
+    }
+    for (int k = pj ? 1 : 0; k < nt && rows_in[k] > 0; ++k) {
         SpgemmArgs f = g;
-        f.nrows = rows_in[bin];
-        f.rows = ovf[bin];
-        rc = launch_spgemm(ctx, f, bin);
+        f.nrows = rows_in[k];
+        f.rows = ovf[k];
+        rc = launch(f, k, kFill);
         if (rc) return rc;
     }
     rc = read_status(ctx, d_status, &st);
@@ -1151,6 +1317,7 @@ int level_dev(fgpu_ctx* ctx, AmgDevLevel& L, const AmgHostCfg& cfg, const AmgNns
     tphase = clock::now();
     if (nagg == 0 || nagg >= ng) { *handoff = true; tm.handoff = 3; return FGPU_OK; }
     AmgDevCsr P0;
+    double* ds0 = nullptr;
     int64_t ncoarse = nagg;
     if (nns) {
         // tentative prolongator from the near null space (host QR per aggregate, the host set-up's code)
@@ -1176,7 +1343,7 @@ int level_dev(fgpu_ctx* ctx, AmgDevLevel& L, const AmgHostCfg& cfg, const AmgNns
     // tentative prolongator (1/sqrt(|agg|), the host's 1.0 / std::sqrt of the exact size) and A P0
     const int32_t* dagg = dagg_node;
     unsigned int* dsz = w.get<unsigned int>(nagg);
-    double* ds0 = w.get<double>(nagg);
+    ds0 = w.get<double>(nagg);
     DEV_ALLOC(dsz && ds0);
     DEV_TRY(cudaMemsetAsync(dsz, 0, nagg * sizeof(unsigned int), ctx->stream));
     agg_size_kernel<<<grid_rows(n, 256), 256, 0, ctx->stream>>>(n, dagg, dsz);
@@ -1209,7 +1376,7 @@ int level_dev(fgpu_ctx* ctx, AmgDevLevel& L, const AmgHostCfg& cfg, const AmgNns
         if (rc) return rc;
     } else {
         AmgDevCsr AP0;
-        rc = spgemm_dev(ctx, A, P0, AP0, d_status, &ovf);
+        rc = spgemm_dev(ctx, A, P0, AP0, d_status, &ovf, nns ? nullptr : dagg_node, ds0);
         if (rc) return rc;
         if (ovf) { *handoff = true; tm.handoff = 4; return FGPU_OK; }
         rc = join_lanczos();

@@ -1,5 +1,5 @@
-// Read-only loads that leave no line in L1: for arrays that a kernel reads once (matrix columns and values,
-// gather indices), so that L1 keeps what it reads again (the gathered vector or buffer).
+// Read-only loads that leave no line in L1: for arrays that a kernel reads once (matrix columns and values),
+// so that L1 keeps what it reads again (the gathered vector).
 #pragma once
 #include <cstdint>
 
