@@ -9,10 +9,10 @@
 //     sorted lists merged per row (the symmetrised graph);
 //   * aggregation: the host set-up's rounds of a distance-2 independent set (roots), then roots'
 //     neighbours, then the rest by their first aggregated neighbour, each step a kernel over the nodes;
-//   * lambda_max(D^-1 A): 12 Lanczos steps on D^-1/2 A D^-1/2 from the host set-up's start vector, the
-//     products one thread per row in column order, the dot products as sequential sums over chunks of
-//     1024 rows combined in chunk order (the host's partition), the tridiagonal's largest eigenvalue
-//     by the host's Sturm bisection;
+//   * lambda_max(D^-1 A): 12 Lanczos steps on D^-1/2 A D^-1/2 from the host set-up's start vector, rows and
+//     dot products summed in a fixed partition that both set-ups share (four partial sums per row, 128 per
+//     chunk of 1024 rows, 128 over the chunks), the scalars on the device until the end, the tridiagonal's
+//     largest eigenvalue by the host's Sturm bisection;
 //   * P0(i, agg(i)) = 1/sqrt(|agg|), A P0, and P = P0 - omega D^-1 (A P0) merged row by row;
 //   * R = P^T by counting, a scan, a fill and a per-row sort;
 //   * sparse products A P0, A P and R (A P): a group of lanes per row of the left factor takes its entries
@@ -32,6 +32,7 @@
 #include <vector>
 
 #include "fgpu_core.h"
+#include "ld_stream.cuh"
 #include "scan.cuh"
 
 namespace fgpu {
@@ -249,53 +250,127 @@ __global__ void merge_kernel(int64_t n, const uint32_t* __restrict__ pa, const i
     }
 }
 
-// Lanczos: w_i = s_i sum_p (a_p s_j) v_j, the row summed in column order (one thread per row)
-__global__ void lanczos_spmv_kernel(int64_t n, const int64_t* __restrict__ ia, const int32_t* __restrict__ ja, const double* __restrict__ a,
-                                    const double* __restrict__ s, const double* __restrict__ v, double* __restrict__ w) {
+// Lanczos steps. The scalars stay on the device: al[k], be[k], the number of steps done and the stop flag
+// of a breakdown, after which the kernels do nothing.
+struct LanczosScalars {
+    double al[kLanczosSteps], be[kLanczosSteps];
+    int steps, stop;
+    unsigned int ticket;
+};
+// v = x / |x| (the start vector), vold = 0, s = 1/sqrt(d), u = s v
+__global__ void lanczos_start_kernel(int64_t n, const double* __restrict__ d, double norm, double* __restrict__ s, double* __restrict__ v,
+                                     double* __restrict__ vold, double* __restrict__ u) {
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const double si = d[i] > 0.0 ? __ddiv_rn(1.0, __dsqrt_rn(d[i])) : 0.0, vi = __ddiv_rn(v[i], norm);
+        s[i] = si;
+        v[i] = vi;
+        vold[i] = 0.0;
+        u[i] = __dmul_rn(si, vi);
+    }
+}
+// w_i = s_i sum_p a_p u_j, four lanes per row: lane l sums the entries congruent to l mod 4, then
+// (0 + 2) + (1 + 3). Bound: the FP64 pipe, which an instruction occupies for the whole warp: rows in the
+// order of their lengths (windows of 256, like the smoother's layout) keep the warp's eight rows alike,
+// and u = s v is formed once, not in each entry. P2 48^3 (25.8 M entries of rows of 24 to 65): a thread
+// per row 378 us, four lanes in row order 345 (half the lanes idle), by length 188.
+__global__ void __launch_bounds__(256) lanczos_spmv_kernel(int64_t n, const int64_t* __restrict__ ia, const int32_t* __restrict__ ja,
+                                                           const double* __restrict__ a, const int32_t* __restrict__ perm,
+                                                           const double* __restrict__ s, const double* __restrict__ u,
+                                                           double* __restrict__ w, const LanczosScalars* __restrict__ sc) {
+    if (sc->stop) return;
+    const int sub = threadIdx.x & 3;
+    const int64_t step = ((int64_t)gridDim.x * blockDim.x) >> 2;
+    for (int64_t r = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 2; __any_sync(0xffffffffu, r < n); r += step) {
         double acc = 0.0;
-        for (int64_t p = ia[i]; p < ia[i + 1]; ++p) {
-            const int32_t j = ja[p];
-            acc = __dadd_rn(acc, __dmul_rn(__dmul_rn(a[p], s[j]), v[j]));
+        int32_t i = 0;
+        if (r < n) {
+            i = perm[r];
+            const int64_t e = ia[i + 1];
+            int64_t p = ia[i] + sub;
+            for (; p + 4 < e; p += 8) {
+                const int32_t j0 = ld_stream(ja + p), j1 = ld_stream(ja + p + 4);
+                const double a0 = ld_stream(a + p), a1 = ld_stream(a + p + 4);
+                const double u0 = u[j0], u1 = u[j1];
+                acc = __dadd_rn(acc, __dmul_rn(a0, u0));
+                acc = __dadd_rn(acc, __dmul_rn(a1, u1));
+            }
+            if (p < e) acc = __dadd_rn(acc, __dmul_rn(ld_stream(a + p), u[ld_stream(ja + p)]));
         }
-        w[i] = __dmul_rn(s[i], acc);
+        acc = __dadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, 2));
+        acc = __dadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, 1));
+        if (r < n && sub == 0) w[i] = __dmul_rn(s[i], acc);
     }
 }
-// partial[c] = sum over the rows of chunk c of x_i y_i, in row order: one block per chunk; the block
-// forms a tile's products in shared memory, one thread adds them in order
-constexpr int kDotTile = 1024;
-__global__ void __launch_bounds__(128) chunk_dot_kernel(int64_t n, const double* __restrict__ x, const double* __restrict__ y,
-                                                        double* __restrict__ partial) {
-    __shared__ double buf[kDotTile];
-    const int64_t c = blockIdx.x;
-    const int64_t r0 = c * kLanczosChunk, r1 = min(n, r0 + kLanczosChunk);
+// the sum of 128 partial sums, one per thread, in the host set-up's order
+__device__ double lanczos_tree(double t, double* sw) {
+    for (int o = 16; o > 0; o >>= 1) t = __dadd_rn(t, __shfl_xor_sync(0xffffffffu, t, o));
+    if ((threadIdx.x & 31) == 0) sw[threadIdx.x >> 5] = t;
+    __syncthreads();
+    t = __dadd_rn(__dadd_rn(sw[0], sw[1]), __dadd_rn(sw[2], sw[3]));
+    __syncthreads();
+    return t;
+}
+// UPDATE: w -= al_k v + be_(k-1) vold, then w.w and be_k; else w.v and al_k. A block per chunk of 1024 rows,
+// thread t the rows congruent to t mod 128; the last block to finish adds the chunks' sums in the same way.
+// (One thread adding a chunk's products in row order took 62 us of a dot product at 0.9 M rows, and the
+// scalar went through the host; now 12 to 16, 20 with the update. P2 48^3: the estimate's chain 9.2 -> 3.1 ms.)
+template <bool UPDATE>
+__global__ void __launch_bounds__(128) lanczos_dot_kernel(int64_t n, int k, const double* __restrict__ v, const double* __restrict__ vold,
+                                                          double* __restrict__ w, double* __restrict__ partial, LanczosScalars* sc) {
+    __shared__ double sw[4];
+    __shared__ bool last;
+    if (sc->stop) return;
+    const double al = UPDATE ? sc->al[k] : 0.0, be = UPDATE && k > 0 ? sc->be[k - 1] : 0.0;
+    const int64_t r0 = blockIdx.x * kLanczosChunk, r1 = min(n, r0 + kLanczosChunk);
     double t = 0.0;
-    for (int64_t b = r0; b < r1; b += kDotTile) {
-        const int m = (int)min((int64_t)kDotTile, r1 - b);
-        for (int k = threadIdx.x; k < m; k += blockDim.x) buf[k] = __dmul_rn(x[b + k], y[b + k]);
-        __syncthreads();
-        if (threadIdx.x == 0)
-            for (int k = 0; k < m; ++k) t = __dadd_rn(t, buf[k]);
-        __syncthreads();
+#pragma unroll
+    for (int q = 0; q < (int)(kLanczosChunk / 128); ++q) {
+        const int64_t i = r0 + q * 128 + threadIdx.x;
+        if (i < r1) {
+            double x = w[i];
+            const double vi = v[i];
+            if (UPDATE) {
+                x = __dsub_rn(x, __dadd_rn(__dmul_rn(al, vi), __dmul_rn(be, vold[i])));
+                w[i] = x;
+            }
+            t = __dadd_rn(t, __dmul_rn(x, UPDATE ? x : vi));
+        }
     }
-    if (threadIdx.x == 0) partial[c] = t;
+    t = lanczos_tree(t, sw);
+    if (threadIdx.x == 0) {
+        partial[blockIdx.x] = t;
+        __threadfence();
+        last = atomicAdd(&sc->ticket, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    t = 0.0;
+    for (int c = threadIdx.x; c < (int)gridDim.x; c += 128) t = __dadd_rn(t, __ldcg(partial + c));
+    t = lanczos_tree(t, sw);
+    if (threadIdx.x == 0) {
+        sc->ticket = 0;
+        if (UPDATE) {
+            const double b = __dsqrt_rn(t);
+            sc->be[k] = b;
+            sc->steps = k + 1;
+            if (b < 1e-14 * fabs(al)) sc->stop = 1;
+        } else {
+            sc->al[k] = t;
+        }
+    }
 }
-// w_i -= a v_i + b vold_i
-__global__ void lanczos_update_kernel(int64_t n, double a, double b, const double* __restrict__ v, const double* __restrict__ vold,
-                                      double* __restrict__ w) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        w[i] = __dsub_rn(w[i], __dadd_rn(__dmul_rn(a, v[i]), __dmul_rn(b, vold[i])));
-}
-// vold = v; v = w / b
-__global__ void lanczos_next_kernel(int64_t n, double b, const double* __restrict__ w, double* __restrict__ v, double* __restrict__ vold) {
+// vold = v; v = w / be_k; u = s v
+__global__ void lanczos_next_kernel(int64_t n, int k, const double* __restrict__ s, const double* __restrict__ w, double* __restrict__ v,
+                                    double* __restrict__ vold, double* __restrict__ u, const LanczosScalars* __restrict__ sc) {
+    if (sc->stop) return;
+    const double b = sc->be[k];
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
         vold[i] = v[i];
-        v[i] = __ddiv_rn(w[i], b);
+        const double x = __ddiv_rn(w[i], b);
+        v[i] = x;
+        u[i] = __dmul_rn(s[i], x);
     }
-}
-__global__ void inv_sqrt_kernel(int64_t n, const double* __restrict__ d, double* __restrict__ s) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        s[i] = d[i] > 0.0 ? __ddiv_rn(1.0, __dsqrt_rn(d[i])) : 0.0;
 }
 
 // tentative prolongator rows: one entry (agg_i, s0[agg_i]) where agg_i >= 0
@@ -1078,7 +1153,9 @@ struct LanczosJob {
     const int32_t* ja = nullptr;
     const double* a = nullptr;
     const double* d = nullptr;
-    double *s = nullptr, *v = nullptr, *vold = nullptr, *wv = nullptr, *part = nullptr;
+    double *s = nullptr, *v = nullptr, *vold = nullptr, *wv = nullptr, *u = nullptr, *part = nullptr;
+    LanczosScalars* sc = nullptr;
+    int32_t *perm = nullptr, *slice_len = nullptr;
     cudaStream_t st = nullptr;
     double lmax = 0;
     int launches = 0;
@@ -1091,43 +1168,34 @@ struct LanczosJob {
     int device = 0;
     void run() {
         if (!ok(cudaSetDevice(device))) return;
-        std::vector<double> hv0;
-        amg_lanczos_start(n, hv0);
-        const int64_t nch = (n + kLanczosChunk - 1) / kLanczosChunk;
-        if (!ok(cudaMemcpyAsync(v, hv0.data(), n * sizeof(double), cudaMemcpyHostToDevice, st))) return;
-        if (!ok(cudaMemsetAsync(vold, 0, n * sizeof(double), st))) return;
-        inv_sqrt_kernel<<<grid_rows(n, 256), 256, 0, st>>>(n, d, s);
-        ++launches;
-        std::vector<double> al, be, hp(nch);
-        double bprev = 0.0;
-        auto dot = [&](const double* x, const double* y, double* out) {
-            chunk_dot_kernel<<<(int)nch, 128, 0, st>>>(n, x, y, part);
-            ++launches;
-            if (!ok(cudaMemcpyAsync(hp.data(), part, nch * sizeof(double), cudaMemcpyDeviceToHost, st)) || !ok(cudaStreamSynchronize(st)))
-                return false;
-            double t = 0.0;
-            for (int64_t c = 0; c < nch; ++c) t += hp[c];
-            *out = t;
-            return true;
-        };
-        for (int k = 0; k < kLanczosSteps; ++k) {
-            lanczos_spmv_kernel<<<grid_rows(n, 256), 256, 0, st>>>(n, ia, ja, a, s, v, wv);
-            ++launches;
-            double al_k = 0.0, b2 = 0.0;
-            if (!dot(wv, v, &al_k)) return;
-            lanczos_update_kernel<<<grid_rows(n, 256), 256, 0, st>>>(n, al_k, bprev, v, vold, wv);
-            ++launches;
-            if (!dot(wv, wv, &b2)) return;
-            const double b = std::sqrt(b2);
-            al.push_back(al_k);
-            if (b < 1e-14 * std::fabs(al_k) || k + 1 == kLanczosSteps) break;
-            be.push_back(b);
-            lanczos_next_kernel<<<grid_rows(n, 256), 256, 0, st>>>(n, b, wv, v, vold);
-            ++launches;
-            bprev = b;
+        sell_order_launch(st, n, ia, perm, slice_len);
+        // the start vector (a serial recurrence) in pieces, each copied while the next is formed
+        std::vector<double> hv0(n);
+        AmgLanczosStart start;
+        for (int64_t b = 0; b < n; b += 65536) {
+            const int64_t m = std::min<int64_t>(65536, n - b);
+            start.fill(hv0.data() + b, m);
+            if (!ok(cudaMemcpyAsync(v + b, hv0.data() + b, m * sizeof(double), cudaMemcpyHostToDevice, st))) return;
         }
-        ok(cudaGetLastError());
-        lmax = amg_tridiag_lmax(al, be);
+        const int nch = (int)((n + kLanczosChunk - 1) / kLanczosChunk);
+        const int g = grid_rows(n, 256);
+        if (!ok(cudaMemsetAsync(sc, 0, sizeof(LanczosScalars), st))) return;
+        lanczos_start_kernel<<<g, 256, 0, st>>>(n, d, start.norm(), s, v, vold, u);
+        launches += 2;
+        for (int k = 0; k < kLanczosSteps; ++k) {
+            lanczos_spmv_kernel<<<grid_rows(n, 64), 256, 0, st>>>(n, ia, ja, a, perm, s, u, wv, sc);
+            lanczos_dot_kernel<false><<<nch, 128, 0, st>>>(n, k, v, vold, wv, part, sc);
+            lanczos_dot_kernel<true><<<nch, 128, 0, st>>>(n, k, v, vold, wv, part, sc);
+            launches += 3;
+            if (k + 1 < kLanczosSteps) {
+                lanczos_next_kernel<<<g, 256, 0, st>>>(n, k, s, wv, v, vold, u, sc);
+                ++launches;
+            }
+        }
+        LanczosScalars h;
+        if (!ok(cudaGetLastError()) || !ok(cudaMemcpyAsync(&h, sc, sizeof(h), cudaMemcpyDeviceToHost, st)) || !ok(cudaStreamSynchronize(st)))
+            return;
+        lmax = amg_tridiag_lmax(std::vector<double>(h.al, h.al + h.steps), std::vector<double>(h.be, h.be + h.steps - 1));
     }
 };
 
@@ -1154,8 +1222,12 @@ int level_dev(fgpu_ctx* ctx, AmgDevLevel& L, const AmgHostCfg& cfg, const AmgNns
     lz.v = w.get<double>(n);
     lz.vold = w.get<double>(n);
     lz.wv = w.get<double>(n);
+    lz.u = w.get<double>(n);
     lz.part = w.get<double>(nch);
-    DEV_ALLOC(d && cnt && tp && lz.s && lz.v && lz.vold && lz.wv && lz.part);
+    lz.sc = w.get<LanczosScalars>(1);
+    lz.perm = w.get<int32_t>(n);
+    lz.slice_len = w.get<int32_t>((n + 31) / 32);
+    DEV_ALLOC(d && cnt && tp && lz.s && lz.v && lz.vold && lz.wv && lz.u && lz.part && lz.sc && lz.perm && lz.slice_len);
     diag_kernel<<<grid_rows(n, 256), 256, 0, ctx->stream>>>(n, A.ia, A.ja, A.a, d, d_status);
     ctx->launches++;
     // the Lanczos thread and stream: started once the diagonal is formed, joined before any return

@@ -136,44 +136,65 @@ std::vector<double> diagonal(const HostCsr& A) {
     return d;
 }
 
+// the sum of 128 partial sums: halves of each 32 added, then the four sums in pairs (t is overwritten)
+double tree128(double* t) {
+    for (int w = 0; w < 4; ++w)
+        for (int o = 16; o > 0; o >>= 1)
+            for (int l = 0; l < o; ++l) t[w * 32 + l] += t[w * 32 + l + o];
+    return (t[0] + t[32]) + (t[64] + t[96]);
+}
+
 // lmax(D^-1 A) of a symmetric positive definite A: Lanczos on D^-1/2 A D^-1/2
 // (m steps from a fixed pseudo-random start), largest Ritz value by bisection
 double lmax_estimate(const HostCsr& A, const std::vector<double>& d, int m, int nthreads) {
     const int64_t n = A.nrows;
     if (n == 0) return 1.0;
-    std::vector<double> s(n), v, vold(n, 0.0), w(n);
+    std::vector<double> s(n), v(n), vold(n, 0.0), w(n), u(n);
     for (int64_t i = 0; i < n; ++i) s[i] = d[i] > 0 ? 1.0 / std::sqrt(d[i]) : 0.0;
-    amg_lanczos_start(n, v);
+    AmgLanczosStart start;
+    start.fill(v.data(), n);
+    const double norm = start.norm();
+    for (int64_t i = 0; i < n; ++i) {
+        v[i] /= norm;
+        u[i] = s[i] * v[i];
+    }
     std::vector<double> al, be;
     double bprev = 0;
     const int T = (int)std::max<int64_t>(1, std::min<int64_t>(nthreads, (n + 4095) / 4096));
     constexpr int64_t kChunk = 1024;
     const int64_t nch = (n + kChunk - 1) / kChunk;
     std::vector<double> pa(nch), pb(nch);
+    // 128 partial sums over i mod 128, added in a fixed tree (the device set-up's order)
+    auto total = [&](const std::vector<double>& p) {
+        double t[128] = {0.0};
+        for (int64_t c = 0; c < nch; ++c) t[c & 127] += p[c];
+        return tree128(t);
+    };
     for (int k = 0; k < m; ++k) {
         parallel_chunks(T, n, kChunk, [&](int64_t c, int64_t r0, int64_t r1) {
-            double sa = 0;
+            double t[128] = {0.0};
             for (int64_t i = r0; i < r1; ++i) {
-                double acc = 0;
-                for (int64_t p = A.ia[i]; p < A.ia[i + 1]; ++p) acc += A.a[p] * s[A.ja[p]] * v[A.ja[p]];
-                w[i] = s[i] * acc;
-                sa += w[i] * v[i];
+                double acc[4] = {0.0, 0.0, 0.0, 0.0};
+                const int64_t e = A.ia[i + 1];
+                int64_t p = A.ia[i];
+                for (; p + 4 <= e; p += 4)
+                    for (int q = 0; q < 4; ++q) acc[q] += A.a[p + q] * u[A.ja[p + q]];
+                for (int q = 0; p < e; ++p, ++q) acc[q] += A.a[p] * u[A.ja[p]];
+                w[i] = s[i] * ((acc[0] + acc[2]) + (acc[1] + acc[3]));
+                t[(i - r0) & 127] += w[i] * v[i];
             }
-            pa[c] = sa;
+            pa[c] = tree128(t);
         });
-        double a = 0;
-        for (int64_t c = 0; c < nch; ++c) a += pa[c];
+        const double a = total(pa);
         parallel_chunks(T, n, kChunk, [&](int64_t c, int64_t r0, int64_t r1) {
-            double sb = 0;
+            double t[128] = {0.0};
             for (int64_t i = r0; i < r1; ++i) {
                 w[i] -= a * v[i] + bprev * vold[i];
-                sb += w[i] * w[i];
+                t[(i - r0) & 127] += w[i] * w[i];
             }
-            pb[c] = sb;
+            pb[c] = tree128(t);
         });
-        double b = 0;
-        for (int64_t c = 0; c < nch; ++c) b += pb[c];
-        b = std::sqrt(b);
+        const double b = std::sqrt(total(pb));
         al.push_back(a);
         if (b < 1e-14 * std::fabs(a) || k + 1 == m) break;
         be.push_back(b);
@@ -181,6 +202,7 @@ double lmax_estimate(const HostCsr& A, const std::vector<double>& d, int m, int 
             for (int64_t i = r0; i < r1; ++i) {
                 vold[i] = v[i];
                 v[i] = w[i] / b;
+                u[i] = s[i] * v[i];
             }
         });
         bprev = b;
@@ -435,19 +457,15 @@ bool spd_inverse(int64_t n, std::vector<double>& M, int nthreads) {
 
 }  // namespace
 
-// fixed pseudo-random start of the Lanczos estimate, normalised
-void amg_lanczos_start(int64_t n, std::vector<double>& v) {
-    v.assign(n, 0.0);
-    uint64_t h = 0x9E3779B97F4A7C15ull;
-    double nv = 0;
+// fixed pseudo-random start of the Lanczos estimate: the next n numbers
+void AmgLanczosStart::fill(double* v, int64_t n) {
     for (int64_t i = 0; i < n; ++i) {
         h ^= h >> 33; h *= 0xff51afd7ed558ccdull; h ^= h >> 33;
         v[i] = (double)(h >> 11) * (1.0 / 9007199254740992.0) - 0.5;
-        nv += v[i] * v[i];
+        sum += v[i] * v[i];
     }
-    nv = std::sqrt(nv);
-    for (auto& x : v) x /= nv;
 }
+double AmgLanczosStart::norm() const { return std::sqrt(sum); }
 
 // largest eigenvalue of the symmetric tridiagonal (al, be) by Sturm bisection
 double amg_tridiag_lmax(const std::vector<double>& al, const std::vector<double>& be) {

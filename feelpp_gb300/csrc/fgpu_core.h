@@ -147,7 +147,12 @@ __host__ __device__ inline uint64_t amg_mis_key(int64_t i) {
     z ^= z >> 31;
     return ((z >> 32) << 32) | (uint64_t)(uint32_t)i;
 }
-void amg_lanczos_start(int64_t n, std::vector<double>& v);
+struct AmgLanczosStart {                      // the Lanczos start vector in pieces, to be divided by norm()
+    uint64_t h = 0x9E3779B97F4A7C15ull;
+    double sum = 0.0;
+    void fill(double* v, int64_t n);
+    double norm() const;
+};
 double amg_tridiag_lmax(const std::vector<double>& al, const std::vector<double>& be);
 
 // The hierarchy built on the device (amg_dev.cu): device CSR levels down to the first level handed to
@@ -426,6 +431,8 @@ int amg_vcycle_f32(fgpu_amg* M, const float* r, const int* stop, const float** x
 int64_t amg_rows(const fgpu_amg* M);
 const fgpu_ctx* amg_context(const fgpu_amg* M);
 int build_sell(fgpu_ctx* ctx, const fgpu_matrix* A, std::shared_ptr<SellLayout>& out);
+// rows ordered by length within windows of 256 (perm: n; slice_len: the longest of each 32, ceil(n / 32))
+void sell_order_launch(cudaStream_t st, int64_t nrows, const int64_t* ia, int32_t* perm, int32_t* slice_len);
 int solve_gmres(fgpu_ctx* ctx, const fgpu_matrix* A, fgpu_amg* amg, const double* b, double* x, const fgpu_solver_cfg* cfg,
                 int restart, fgpu_solve_stats* st);
 int ensure_two_phase(fgpu_ctx* ctx, fgpu_matrix* A, size_t need);

@@ -176,16 +176,19 @@ __global__ void sell_fill_kernel(int64_t nrows, const int64_t* __restrict__ ia, 
     }
 }
 
+void sell_order_launch(cudaStream_t st, int64_t nrows, const int64_t* ia, int32_t* perm, int32_t* slice_len) {
+    sell_sort_kernel<<<(int)((nrows + kSellSigma - 1) / kSellSigma), kSellSigma, 0, st>>>(nrows, ia, perm, slice_len);
+}
+
 int build_sell(fgpu_ctx* ctx, const fgpu_matrix* A, std::shared_ptr<SellLayout>& out) {
     if (A->nnz >= ((int64_t)1 << 31)) { ctx->err = "SELL layout: more than 2^31 entries"; return FGPU_ERR_INVALID; }
     auto L = std::make_shared<SellLayout>();
     L->nrows = A->nrows;
     L->nslices = (A->nrows + kSellC - 1) / kSellC;
-    const int64_t nwin = (A->nrows + kSellSigma - 1) / kSellSigma;
     FGPU_CUDA_CHECK(ctx, pool_malloc(ctx->stream, &L->d_perm, A->nrows * sizeof(int32_t)));
     FGPU_CUDA_CHECK(ctx, pool_malloc(ctx->stream, &L->d_slice_len, L->nslices * sizeof(int32_t)));
     FGPU_CUDA_CHECK(ctx, pool_malloc(ctx->stream, &L->d_slice_ptr, (L->nslices + 1) * sizeof(int64_t)));
-    sell_sort_kernel<<<(int)nwin, kSellSigma, 0, ctx->stream>>>(A->nrows, A->d_ia, L->d_perm, L->d_slice_len);
+    sell_order_launch(ctx->stream, A->nrows, A->d_ia, L->d_perm, L->d_slice_len);
     ctx->launches++;
     std::vector<int32_t> hlen(L->nslices);
     FGPU_CUDA_CHECK(ctx, cudaMemcpyAsync(hlen.data(), L->d_slice_len, L->nslices * sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
