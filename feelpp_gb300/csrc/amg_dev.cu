@@ -276,21 +276,10 @@ __global__ void __launch_bounds__(256) symmetric_kernel(int64_t n, const uint32_
 // Lanczos steps. The scalars stay on the device: al[k], be[k], the number of steps done and the stop flag
 // of a breakdown, after which the kernels do nothing.
 struct LanczosScalars {
-    double al[kLanczosSteps], be[kLanczosSteps];
+    double al[kLanczosSteps], be[kLanczosSteps], norm;
     int steps, stop;
     unsigned int ticket;
 };
-// v = x / |x| (the start vector), vold = 0, s = 1/sqrt(d), u = s v
-__global__ void lanczos_start_kernel(int64_t n, const double* __restrict__ d, double norm, double* __restrict__ s, double* __restrict__ v,
-                                     double* __restrict__ vold, double* __restrict__ u) {
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-        const double si = d[i] > 0.0 ? __ddiv_rn(1.0, __dsqrt_rn(d[i])) : 0.0, vi = __ddiv_rn(v[i], norm);
-        s[i] = si;
-        v[i] = vi;
-        vold[i] = 0.0;
-        u[i] = __dmul_rn(si, vi);
-    }
-}
 // w_i = s_i sum_p a_p u_j, four lanes per row: lane l sums the entries congruent to l mod 4, then
 // (0 + 2) + (1 + 3). Bound: the FP64 pipe, which an instruction occupies for the whole warp: rows in the
 // order of their lengths (windows of 256, like the smoother's layout) keep the warp's eight rows alike,
@@ -333,10 +322,59 @@ __device__ double lanczos_tree(double t, double* sw) {
     __syncthreads();
     return t;
 }
+// the sum over the blocks of a grid of the sums over their threads; true on the thread that has it in sw[0]
+__device__ bool lanczos_sum(double t, double* partial, LanczosScalars* sc, double* sw, bool* last) {
+    t = lanczos_tree(t, sw);
+    if (threadIdx.x == 0) {
+        partial[blockIdx.x] = t;
+        __threadfence();
+        *last = atomicAdd(&sc->ticket, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!*last) return false;
+    __threadfence();
+    t = 0.0;
+    for (int c = threadIdx.x; c < (int)gridDim.x; c += 128) t = __dadd_rn(t, __ldcg(partial + c));
+    t = lanczos_tree(t, sw);
+    if (threadIdx.x != 0) return false;
+    sc->ticket = 0;
+    sw[0] = t;
+    return true;
+}
+// the start vector x (amg_lanczos_entry) and |x|: its recurrence applies X (h ^= h >> 33, its own inverse),
+// a product with C and X in turn, so that the i-th state is X(C^i X(h_0)) and every entry can be formed by
+// itself (on the host, as the one serial chain, it took 3 of the estimate's 6 ms at 0.9 M rows)
+__global__ void __launch_bounds__(128) lanczos_random_kernel(int64_t n, double* __restrict__ v, double* __restrict__ partial,
+                                                             LanczosScalars* sc) {
+    __shared__ double sw[4];
+    __shared__ bool last;
+    const int64_t r0 = blockIdx.x * kLanczosChunk, r1 = min(n, r0 + kLanczosChunk);
+    uint64_t p = amg_lanczos_power((uint64_t)(r0 + threadIdx.x + 1));
+    const uint64_t p128 = amg_lanczos_power(128);
+    double t = 0.0;
+    for (int64_t i = r0 + threadIdx.x; i < r1; i += 128, p *= p128) {
+        const double x = amg_lanczos_entry(p);
+        v[i] = x;
+        t = __dadd_rn(t, __dmul_rn(x, x));
+    }
+    if (lanczos_sum(t, partial, sc, sw, &last)) sc->norm = __dsqrt_rn(sw[0]);
+}
+// v = x / |x| (the start vector), vold = 0, s = 1/sqrt(d), u = s v
+__global__ void lanczos_start_kernel(int64_t n, const double* __restrict__ d, double* __restrict__ s, double* __restrict__ v,
+                                     double* __restrict__ vold, double* __restrict__ u, const LanczosScalars* __restrict__ sc) {
+    const double norm = sc->norm;
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const double si = d[i] > 0.0 ? __ddiv_rn(1.0, __dsqrt_rn(d[i])) : 0.0, vi = __ddiv_rn(v[i], norm);
+        s[i] = si;
+        v[i] = vi;
+        vold[i] = 0.0;
+        u[i] = __dmul_rn(si, vi);
+    }
+}
 // UPDATE: w -= al_k v + be_(k-1) vold, then w.w and be_k; else w.v and al_k. A block per chunk of 1024 rows,
 // thread t the rows congruent to t mod 128; the last block to finish adds the chunks' sums in the same way.
 // (One thread adding a chunk's products in row order took 62 us of a dot product at 0.9 M rows, and the
-// scalar went through the host; now 12 to 16, 20 with the update. P2 48^3: the estimate's chain 9.2 -> 3.1 ms.)
+// scalar went through the host; now 12 to 16, 20 with the update. P2 48^3: the estimate's steps 9.2 -> 3.1 ms.)
 template <bool UPDATE>
 __global__ void __launch_bounds__(128) lanczos_dot_kernel(int64_t n, int k, const double* __restrict__ v, const double* __restrict__ vold,
                                                           double* __restrict__ w, double* __restrict__ partial, LanczosScalars* sc) {
@@ -359,20 +397,8 @@ __global__ void __launch_bounds__(128) lanczos_dot_kernel(int64_t n, int k, cons
             t = __dadd_rn(t, __dmul_rn(x, UPDATE ? x : vi));
         }
     }
-    t = lanczos_tree(t, sw);
-    if (threadIdx.x == 0) {
-        partial[blockIdx.x] = t;
-        __threadfence();
-        last = atomicAdd(&sc->ticket, 1u) == gridDim.x - 1;
-    }
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
-    t = 0.0;
-    for (int c = threadIdx.x; c < (int)gridDim.x; c += 128) t = __dadd_rn(t, __ldcg(partial + c));
-    t = lanczos_tree(t, sw);
-    if (threadIdx.x == 0) {
-        sc->ticket = 0;
+    if (lanczos_sum(t, partial, sc, sw, &last)) {
+        t = sw[0];
         if (UPDATE) {
             const double b = __dsqrt_rn(t);
             sc->be[k] = b;
@@ -1193,19 +1219,12 @@ struct LanczosJob {
     void run() {
         if (!ok(cudaSetDevice(device))) return;
         sell_order_launch(st, n, ia, perm, slice_len);
-        // the start vector (a serial recurrence) in pieces, each copied while the next is formed
-        std::vector<double> hv0(n);
-        AmgLanczosStart start;
-        for (int64_t b = 0; b < n; b += 65536) {
-            const int64_t m = std::min<int64_t>(65536, n - b);
-            start.fill(hv0.data() + b, m);
-            if (!ok(cudaMemcpyAsync(v + b, hv0.data() + b, m * sizeof(double), cudaMemcpyHostToDevice, st))) return;
-        }
         const int nch = (int)((n + kLanczosChunk - 1) / kLanczosChunk);
         const int g = grid_rows(n, 256);
         if (!ok(cudaMemsetAsync(sc, 0, sizeof(LanczosScalars), st))) return;
-        lanczos_start_kernel<<<g, 256, 0, st>>>(n, d, start.norm(), s, v, vold, u);
-        launches += 2;
+        lanczos_random_kernel<<<nch, 128, 0, st>>>(n, v, part, sc);
+        lanczos_start_kernel<<<g, 256, 0, st>>>(n, d, s, v, vold, u, sc);
+        launches += 3;
         for (int k = 0; k < kLanczosSteps; ++k) {
             lanczos_spmv_kernel<<<grid_rows(n, 64), 256, 0, st>>>(n, ia, ja, a, perm, s, u, wv, sc);
             lanczos_dot_kernel<false><<<nch, 128, 0, st>>>(n, k, v, vold, wv, part, sc);

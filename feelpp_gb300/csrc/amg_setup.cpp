@@ -151,13 +151,6 @@ double lmax_estimate(const HostCsr& A, const std::vector<double>& d, int m, int 
     if (n == 0) return 1.0;
     std::vector<double> s(n), v(n), vold(n, 0.0), w(n), u(n);
     for (int64_t i = 0; i < n; ++i) s[i] = d[i] > 0 ? 1.0 / std::sqrt(d[i]) : 0.0;
-    AmgLanczosStart start;
-    start.fill(v.data(), n);
-    const double norm = start.norm();
-    for (int64_t i = 0; i < n; ++i) {
-        v[i] /= norm;
-        u[i] = s[i] * v[i];
-    }
     std::vector<double> al, be;
     double bprev = 0;
     const int T = (int)std::max<int64_t>(1, std::min<int64_t>(nthreads, (n + 4095) / 4096));
@@ -170,6 +163,23 @@ double lmax_estimate(const HostCsr& A, const std::vector<double>& d, int m, int 
         for (int64_t c = 0; c < nch; ++c) t[c & 127] += p[c];
         return tree128(t);
     };
+    // fixed pseudo-random start, normalised
+    parallel_chunks(T, n, kChunk, [&](int64_t c, int64_t r0, int64_t r1) {
+        double t[128] = {0.0};
+        uint64_t p = amg_lanczos_power((uint64_t)r0 + 1);
+        for (int64_t i = r0; i < r1; ++i, p *= kLanczosMul) {
+            v[i] = amg_lanczos_entry(p);
+            t[(i - r0) & 127] += v[i] * v[i];
+        }
+        pa[c] = tree128(t);
+    });
+    const double norm = std::sqrt(total(pa));
+    parallel_rows(T, n, [&](int, int64_t r0, int64_t r1) {
+        for (int64_t i = r0; i < r1; ++i) {
+            v[i] /= norm;
+            u[i] = s[i] * v[i];
+        }
+    });
     for (int k = 0; k < m; ++k) {
         parallel_chunks(T, n, kChunk, [&](int64_t c, int64_t r0, int64_t r1) {
             double t[128] = {0.0};
@@ -456,16 +466,6 @@ bool spd_inverse(int64_t n, std::vector<double>& M, int nthreads) {
 }
 
 }  // namespace
-
-// fixed pseudo-random start of the Lanczos estimate: the next n numbers
-void AmgLanczosStart::fill(double* v, int64_t n) {
-    for (int64_t i = 0; i < n; ++i) {
-        h ^= h >> 33; h *= 0xff51afd7ed558ccdull; h ^= h >> 33;
-        v[i] = (double)(h >> 11) * (1.0 / 9007199254740992.0) - 0.5;
-        sum += v[i] * v[i];
-    }
-}
-double AmgLanczosStart::norm() const { return std::sqrt(sum); }
 
 // largest eigenvalue of the symmetric tridiagonal (al, be) by Sturm bisection
 double amg_tridiag_lmax(const std::vector<double>& al, const std::vector<double>& be) {

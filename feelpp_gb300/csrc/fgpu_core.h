@@ -147,12 +147,20 @@ __host__ __device__ inline uint64_t amg_mis_key(int64_t i) {
     z ^= z >> 31;
     return ((z >> 32) << 32) | (uint64_t)(uint32_t)i;
 }
-struct AmgLanczosStart {                      // the Lanczos start vector in pieces, to be divided by norm()
+// entry i of the Lanczos start vector, before it is normalised: from the power C^(i + 1) of the multiplier
+constexpr uint64_t kLanczosMul = 0xff51afd7ed558ccdull;
+__host__ __device__ inline uint64_t amg_lanczos_power(uint64_t e) {
+    uint64_t r = 1;
+    for (uint64_t b = kLanczosMul; e; e >>= 1, b *= b)
+        if (e & 1) r *= b;
+    return r;
+}
+__host__ __device__ inline double amg_lanczos_entry(uint64_t power) {
     uint64_t h = 0x9E3779B97F4A7C15ull;
-    double sum = 0.0;
-    void fill(double* v, int64_t n);
-    double norm() const;
-};
+    h = (h ^ (h >> 33)) * power;
+    h ^= h >> 33;
+    return (double)(h >> 11) * (1.0 / 9007199254740992.0) - 0.5;
+}
 double amg_tridiag_lmax(const std::vector<double>& al, const std::vector<double>& be);
 
 // The hierarchy built on the device (amg_dev.cu): device CSR levels down to the first level handed to
