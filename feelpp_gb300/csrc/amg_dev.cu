@@ -20,7 +20,7 @@
 //     every output entry is the host's sequential sum; columns in a shared-memory hash table per row,
 //     sorted and written at the end. Rows with more distinct columns than the table holds are listed and
 //     redone with a larger one. A P0 of a constant near null space has one thread per row.
-// Levels of at most 2048 rows, and any level with a row beyond the kernels' staging capacity, go to
+// Levels of at most 512 rows, and any level with a row beyond the kernels' staging capacity, go to
 // the host set-up for the rest of the hierarchy (the results are the same either way).
 #include <algorithm>
 #include <atomic>
@@ -55,8 +55,9 @@ constexpr int kStOverflow = 1;               // a row beyond a kernel's staging 
 constexpr int kStDiag = 2;                   // a non-positive diagonal entry
 constexpr int64_t kLanczosChunk = 1024;      // rows per partial sum (the host set-up's partition)
 constexpr int kLanczosSteps = 12;
-constexpr int64_t kHandoffRows = 2048;       // levels this small continue on the host (P2 48^3: an 11 K-row
-                                              // level 1 built on the host took 21 ms of a 50 ms set-up, 1 ms on the device)
+// Levels this small continue on the host: below it only the coarsest levels are left, whose time is the
+// launches (a level takes about 60). P2 24^3, level 1 of 1455 rows: 3.9 ms on the host, 1.2 on the device.
+constexpr int64_t kHandoffRows = 512;
 constexpr int kSortMax = 16384;              // longest row sorted by seg_sort_kernel
 constexpr int kNumBins = 4;
 constexpr int kBins[kNumBins] = {256, 1024, 2048, 8192};  // hash table sizes of whole warps (at most half full)

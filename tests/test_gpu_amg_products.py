@@ -11,6 +11,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("order,box,cfg", [
+    (1, (220, 1, 1), {}),                       # 884 rows: the smallest levels set up on the device
     (1, (700, 1, 1), {}),                       # 2804 rows: whole warps from the start
     (1, (3000, 1, 1), {}),                      # ten entries a row: counted first, then filled
     (2, (15, 13, 14), {}),                      # padded rows, eight lanes, odd sizes
