@@ -8,8 +8,9 @@
 //   K_e(i, j) = sum_q dphi_i(q)^T G_q dphi_j(q) + m_q phi_i(q) phi_j(q),
 //   G_q = w_q |det K_q| kappa B_q^T B_q,  m_q = w_q |det K_q| mass,
 // where dphi are reference gradients, in double-float on the FP32 pipes for FP64 matrices (binary64 runs
-// at 1/71 of the binary32 rate here). P1 and P2 tetrahedra: one lane per element (ho_lane_kernel). P3
-// tetrahedra and hexahedra (and binary32 without the tensor cores): one warp per element
+// at 1/71 of the binary32 rate here). P1 and P2 tetrahedra: one lane per element (ho_lane_kernel). Q2
+// hexahedra: sum factorisation (hex_q2.cuh). P3 tetrahedra and Q1 hexahedra (and binary32 without the tensor
+// cores): one warp per element, or four elements per warp
 // (ho_element_kernel): the lanes first take one quadrature point each and form G_q, m_q in shared memory;
 // then for every q they form W_q = G_q dphi_j(q) for one local dof each, and each lane adds
 // dphi_i . W_j + m_q phi_i phi_j into the upper-triangle entries it owns. The element matrices go to the
@@ -29,6 +30,7 @@
 #include "closed.cuh"
 #include "entries.h"
 #include "fgpu_core.h"
+#include "hex_q2.cuh"
 #include "tc_ptx.cuh"
 
 namespace fgpu {
@@ -62,6 +64,7 @@ struct HoTables {
     uint8_t* d_ti = nullptr;   // ntri: row of each upper-triangle entry (entry_order)
     uint8_t* d_tj = nullptr;   // ntri: column
     float2* d_lane = nullptr;  // per point: tables of ho_lane_kernel (P1, P2 tetrahedra)
+    uint16_t* d_place = nullptr;   // Q2 hexahedra: 27 x 27 place in entry_order of a pair of tensor indices
     float* d_tcB = nullptr;    // tensor-core B operand: per chunk of points, per accumulator, tf32 hi / lo
     std::vector<double> dphi, phi;   // Q n 3, Q n (host copies for building d_tcB)
 };
@@ -166,6 +169,19 @@ HoTables* get_ho_tables(fgpu_ctx* ctx, int order, int qdeg, bool hex = false) {
     if (e == cudaSuccess) e = up(&T->d_ti, ti);
     if (e == cudaSuccess) e = up(&T->d_tj, tj);
     if (e == cudaSuccess && !hex && order <= 2) e = up(&T->d_lane, lane_tables(order, R));
+    if (e == cudaSuccess && hex && order == 2) {
+        int tensor[27];
+        for (int i = 0; i < 27; ++i) {
+            tensor[i] = 0;
+            for (int c = 0; c < 3; ++c) tensor[i] = 3 * tensor[i] + 1 + (int)std::lround(R.nodes[3 * i + c]);
+        }
+        std::vector<uint16_t> place(27 * 27);
+        for (int t = 0; t < T->ntri; ++t) {
+            const int a = tensor[ti[t]], b = tensor[tj[t]];
+            place[27 * a + b] = place[27 * b + a] = (uint16_t)t;
+        }
+        e = up(&T->d_place, place);
+    }
     if (e != cudaSuccess) {
         cudaGetLastError();
         ctx->err = std::string("curved-element tables: ") + cudaGetErrorString(e);
@@ -944,6 +960,17 @@ int ho_qdeg_ok(fgpu_ctx* ctx, int order, int qdeg) {
     return FGPU_OK;
 }
 
+template <int M>
+int launch_hex_q2(fgpu_ctx* ctx, fgpu_matrix* A, const HoTables* T, const double* d_kappa, const fgpu_form_desc* f) {
+    const fgpu_mesh* mesh = A->space->mesh;
+    constexpr int smem = hex_q2_smem<M>();
+    FGPU_CUDA_CHECK(ctx, cudaFuncSetAttribute(hex_q2_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    hex_q2_kernel<M><<<(int)std::max<int64_t>(1, (mesh->nt + kHexBlock - 1) / kHexBlock), 128, smem, ctx->stream>>>(
+        mesh->nt, mesh->d_xyz, mesh->d_tets, T->d_qwh, T->d_qwl, T->d_place, d_kappa, f->kappa, f->mass, f->kappa_scale,
+        (float2*)A->d_kbuf, ctx->d_status);
+    return FGPU_OK;
+}
+
 int hex_qdeg_ok(fgpu_ctx* ctx, int order, int qdeg) {
     const int lim = order == 1 ? 6 : 4;   // 4^3 / 3^3 Gauss points
     if (qdeg > lim) {
@@ -990,7 +1017,12 @@ int launch_assemble_hex(fgpu_ctx* ctx, fgpu_matrix* A, const fgpu_form_desc* f, 
     } else if (V->n == 8) {
         if (f32) HEX_LAUNCH(kHoF32, 8, 32, blocks); else HEX_LAUNCH(kHoDF64, 8, 32, blocks);
     } else {
-        if (f32) HEX_LAUNCH(kHoF32, 27, 32, blocks); else HEX_LAUNCH(kHoDF64, 27, 32, blocks);
+        if (f32) {
+            HEX_LAUNCH(kHoF32, 27, 32, blocks);
+        } else {
+            rc = T->Q == 27 ? launch_hex_q2<3>(ctx, A, T, d_kappa, f) : launch_hex_q2<2>(ctx, A, T, d_kappa, f);
+            if (rc) return rc;
+        }
     }
 #undef HEX_LAUNCH
     prof_end(ctx, ev);
