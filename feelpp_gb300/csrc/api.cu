@@ -672,10 +672,8 @@ static int assemble_impl(fgpu_ctx* ctx, fgpu_matrix* A, const fgpu_form_desc* f,
     }
     if (f->kappa_scale) return set_err(ctx, FGPU_ERR_INVALID, "kappa_scale: Laplace/mass forms on the default path only");
     if (f->kind == FGPU_FORM_ELASTICITY && algo == FGPU_ALGO_TWO_PHASE) {
-        // df64 (FP64 matrices) or binary32 element blocks, then the gather map
-        rc = launch_geometry_el_df(ctx, V->mesh, f->lambda, f->mu, reinterpret_cast<float4*>(A->d_coef));
-        if (rc) return rc;
-        rc = launch_assemble_elasticity_two_phase(ctx, A, tab, reinterpret_cast<const float4*>(A->d_coef), accumulate);
+        // df64 (FP64 matrices) or binary32 blocks, summed per node pair
+        rc = launch_assemble_elasticity_two_phase(ctx, A, tab, f->lambda, f->mu, reinterpret_cast<float4*>(A->d_coef), accumulate);
         if (rc) return rc;
         return finish(ctx);
     }

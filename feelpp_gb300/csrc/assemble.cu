@@ -76,6 +76,30 @@ static bool closed_form_holds(const RefTables& R) {
     return off <= 1e-14 * top * n;
 }
 
+// The same for the gradient tensors S_ab alone (P1 and P2, a rule of degree 2p - 2 or more): the sums that
+// gather_elasticity_fused_kernel forms.
+static bool closed_gradients_hold(const RefTables& R) {
+    const int n = R.n;
+    if (n != 4 && n != 10) return false;
+    double top = 0.0, off = 0.0;
+    for (int a = 0; a < 3; ++a)
+        for (int b = 0; b < 3; ++b)
+            for (int i = 0; i < n; ++i)
+                for (int j = 0; j < n; ++j) {
+                    double v = 0.0;
+                    for (int k = 0; k < (n == 4 ? 1 : bary_comps(i)); ++k)
+                        for (int m = 0; m < (n == 4 ? 1 : bary_comps(j)); ++m) {
+                            const int c = n == 4 ? i : bary_comp(i, k), d = n == 4 ? j : bary_comp(j, m);
+                            const double da = c == 0 ? -0.5 : c == a + 1 ? 0.5 : 0.0, db = d == 0 ? -0.5 : d == b + 1 ? 0.5 : 0.0;
+                            v += (n == 4 ? 4.0 / 3.0 : p2_stiff_coef(i, k, j, m) * 4.0 / 15.0) * da * db;
+                        }
+                    const double t = R.S[((size_t)(3 * a + b) * n + i) * n + j];
+                    top = std::max(top, std::fabs(t));
+                    off = std::max(off, std::fabs(t - v));
+                }
+    return off <= 1e-14 * top * n;
+}
+
 DevTables* get_dev_tables(int order, int qdeg, std::string& err) {
     int dev = 0;
     cudaGetDevice(&dev);
@@ -120,6 +144,7 @@ DevTables* get_dev_tables(int order, int qdeg, std::string& err) {
         }
     }
     D->closed = closed_form_holds(R);
+    D->closed_el = closed_gradients_hold(R);
     cudaError_t e = cudaSuccess;
     if (e == cudaSuccess) e = upload(T7bh, &D->d_T7bh);
     if (e == cudaSuccess) e = upload(T7bl, &D->d_T7bl);
@@ -1762,6 +1787,8 @@ int launch_assemble_two_phase(fgpu_ctx* ctx, fgpu_matrix* A, const DevTables* ta
 // Y = B X B^T (B = K^-T), the 3x3 block of K_e at rows (c, i), columns (d, j) is
 //   lambda J Y_cd + mu J Y_dc + delta_cd mu J tr(Y).
 // Records: 24 floats per element: hi parts of (B_00..B_22, lambda J, mu J, 0), then lo parts.
+// With exact gradient tensors the blocks are formed inside the gather (gather.cu,
+// gather_elasticity_fused_kernel). Else (a rule below degree 2p - 2):
 // Phase 1 stores the blocks of the pairs i <= j (n(n+1)/2 x 9 values per element);
 // phase 2 (gather.cu), one lane per node pair, sums the 9 entries over the
 // contributions of the gather map in element order (a contribution with li > lj
@@ -1809,7 +1836,7 @@ __global__ void geometry_el_df_kernel(int64_t nt, const double* __restrict__ xyz
     }
 }
 
-int launch_geometry_el_df(fgpu_ctx* ctx, const fgpu_mesh* mesh, double lam, double mu, float4* d_rec) {
+static int launch_geometry_el_df(fgpu_ctx* ctx, const fgpu_mesh* mesh, double lam, double mu, float4* d_rec) {
     const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((mesh->nt + 255) / 256, 152 * 16));
     PendingEvent ev;
     prof_begin(ctx, "geometry", ev);
@@ -1924,7 +1951,7 @@ __global__ void __launch_bounds__(128) element_el_kernel(int64_t nt, const float
 }
 
 template <int MODE, int N>
-static int run_el_two_phase(fgpu_ctx* ctx, fgpu_matrix* A, const DevTables* tab, const float4* rec, int accumulate) {
+static int run_el_two_phase(fgpu_ctx* ctx, fgpu_matrix* A, const DevTables* tab, double lam, double mu, float4* rec, int accumulate) {
     fgpu_space* V = A->space;
     const int64_t nt = V->mesh->nt;
     constexpr int NTRI = N * (N + 1) / 2;
@@ -1933,6 +1960,13 @@ static int run_el_two_phase(fgpu_ctx* ctx, fgpu_matrix* A, const DevTables* tab,
         int rc = launch_build_gather_map(ctx, V);
         if (rc) return rc;
     }
+    if (tab->closed_el) {                        // blocks formed from the barycentric gradients inside the gather
+        if (ctx->capturing && !A->assembled_fused) { ctx->err = "two-phase assembly: assemble once before capturing"; return FGPU_ERR_INVALID; }
+        A->assembled_fused = true;
+        return launch_gather_elasticity_fused(ctx, A, lam, mu, rec, accumulate);
+    }
+    int rc = launch_geometry_el_df(ctx, V->mesh, lam, mu, rec);
+    if (rc) return rc;
     const size_t need = (size_t)nt * NTRI * 9 * (MODE == kModeDF64 ? 8 : 4);
     if (A->kbuf_bytes < need) {
         if (ctx->capturing) { ctx->err = "two-phase assembly: assemble once before capturing (element buffer)"; return FGPU_ERR_INVALID; }
@@ -1955,14 +1989,14 @@ static int run_el_two_phase(fgpu_ctx* ctx, fgpu_matrix* A, const DevTables* tab,
     return launch_gather_elasticity(ctx, A, accumulate);
 }
 
-int launch_assemble_elasticity_two_phase(fgpu_ctx* ctx, fgpu_matrix* A, const DevTables* tab, const float4* rec, int accumulate) {
+int launch_assemble_elasticity_two_phase(fgpu_ctx* ctx, fgpu_matrix* A, const DevTables* tab, double lam, double mu, float4* rec, int accumulate) {
     const int order = A->space->order;
     const bool f32 = A->precision == FGPU_F32;
     if (A->ncomp != 3) { ctx->err = "elasticity needs a 3-component space"; return FGPU_ERR_INVALID; }
-    if (order == 1) return f32 ? run_el_two_phase<kModeF32, 4>(ctx, A, tab, rec, accumulate)
-                               : run_el_two_phase<kModeDF64, 4>(ctx, A, tab, rec, accumulate);
-    if (order == 2) return f32 ? run_el_two_phase<kModeF32, 10>(ctx, A, tab, rec, accumulate)
-                               : run_el_two_phase<kModeDF64, 10>(ctx, A, tab, rec, accumulate);
+    if (order == 1) return f32 ? run_el_two_phase<kModeF32, 4>(ctx, A, tab, lam, mu, rec, accumulate)
+                               : run_el_two_phase<kModeDF64, 4>(ctx, A, tab, lam, mu, rec, accumulate);
+    if (order == 2) return f32 ? run_el_two_phase<kModeF32, 10>(ctx, A, tab, lam, mu, rec, accumulate)
+                               : run_el_two_phase<kModeDF64, 10>(ctx, A, tab, lam, mu, rec, accumulate);
     ctx->err = "elasticity supports P1 and P2";
     return FGPU_ERR_INVALID;
 }

@@ -17,6 +17,7 @@
 //   df_add (sloppy)       |err| <= 2u^2 (|x| + |y|)
 //   df_mul                |err| <= 4u^2 |x y|
 //   df_recip              |err| <= 2^-46 |1/x|  (one Newton step from the rounded binary32 reciprocal)
+//   df_rsqrt              |err| <= 2^-47 x^(-1/2)
 //   d2df                  |err| <= 2^-48 |x|   for 2^-100 <= |x| <= 2^127 (both halves normal)
 //   df2d                  |err| <= 2^-53 |hi + lo|
 #pragma once
@@ -148,6 +149,23 @@ FGPU_HD df df_recip(df x) {
     df e = df_sub(df{1.0f, 0.0f}, xr);
     df t = df_mul(df{r, 0.0f}, e);
     return df_add(df{r, 0.0f}, t);
+}
+// x^(-1/2), x > 0: r (1 + e / 2 + 3 e^2 / 8) from the binary32 value r, with e = 1 - x r^2 (at most some 2^-22)
+// summed from exact products: x r^2 is near 1, so 1 minus its high part is exact.
+FGPU_HD df df_rsqrt(df x) {
+#if defined(__CUDA_ARCH__)
+    float r = __frsqrt_rn(x.hi);
+#else
+    float r = 1.0f / std::sqrt(x.hi);
+#endif
+    const float p = f_mul(r, r), q = f_fma(r, r, -p);        // r^2 = p + q
+    const float a = f_mul(x.hi, p), b = f_fma(x.hi, p, -a);  // x.hi p = a + b
+    const df u = two_sum(f_sub(1.0f, a), -b);
+    const df v = two_sum(u.hi, -f_fma(x.hi, q, f_mul(x.lo, p)));
+    const float th = f_mul(0.5f, v.hi), tl = f_fma(f_mul(0.375f, v.hi), v.hi, f_mul(0.5f, f_add(u.lo, v.lo)));
+    const float m = f_mul(r, th);
+    const df y = quick_two_sum(r, m);
+    return quick_two_sum(y.hi, f_add(y.lo, f_fma(r, tl, f_fma(r, th, -m))));
 }
 
 // double -> df64 with integer operations only. Zero, subnormal doubles and

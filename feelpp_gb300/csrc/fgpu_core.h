@@ -345,6 +345,7 @@ struct fgpu_matrix {
     double* d_kappa_stage = nullptr; // staging copy of a host per-element kappa (T doubles)
     void* d_kbuf = nullptr;          // two-phase assembly: element matrices (upper triangles)
     size_t kbuf_bytes = 0;
+    bool assembled_fused = false;    // elasticity: assembled once without an element buffer
     mutable std::shared_ptr<SellLayout> sell; // solver layout, built on first solve
 };
 
@@ -383,6 +384,7 @@ struct DevTables {                     // device copies of the reference tables
     float* d_T7tl = nullptr;
     uint16_t* d_tri = nullptr;         // n x n: (i, j) -> upper-triangle index of (min, max)
     bool closed = false;               // closed.cuh's closed form equals these tensors
+    bool closed_el = false;            // the gradient tensors S are the exact integrals (P1, P2)
     float* d_T7bh = nullptr;           // the split in the two-phase element buffer's order (entry_order)
     float* d_T7bl = nullptr;
     float* d_Sbh = nullptr;            // elasticity tensors S_ab in that order, df64 split: 9 x n(n+1)/2
@@ -420,8 +422,8 @@ int launch_assemble_two_phase(fgpu_ctx* ctx, fgpu_matrix* A, const DevTables* ta
 constexpr int kStreamedUnsupported = -1;   // launch_assemble_streamed: use the two-phase path
 int launch_assemble_streamed(fgpu_ctx* ctx, fgpu_matrix* A, const DevTables* tab, const double* d_kappa, double kappa,
                              double mass, const double* kscale, int accumulate, double* hout);
-int launch_geometry_el_df(fgpu_ctx* ctx, const fgpu_mesh* mesh, double lam, double mu, float4* d_rec);
-int launch_assemble_elasticity_two_phase(fgpu_ctx* ctx, fgpu_matrix* A, const DevTables* tab, const float4* rec, int accumulate);
+int launch_assemble_elasticity_two_phase(fgpu_ctx* ctx, fgpu_matrix* A, const DevTables* tab, double lam, double mu, float4* rec, int accumulate);
+int launch_gather_elasticity_fused(fgpu_ctx* ctx, const fgpu_matrix* A, double lam, double mu, float4* rec, int accumulate);
 int launch_build_gather_map(fgpu_ctx* ctx, fgpu_space* V);
 bool gather_plan_ready(const fgpu_space* V);
 void gather_plan_free(fgpu_space* V);

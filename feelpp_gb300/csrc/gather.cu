@@ -34,6 +34,7 @@
 #include "fgpu_core.h"
 #include "scan.cuh"
 #include "asm_device.cuh"
+#include "closed.cuh"
 
 namespace fgpu {
 
@@ -138,6 +139,31 @@ __global__ void __launch_bounds__(256) batch_gather_slices_kernel(int nprob, con
     gather_slice<MODE, PIPE ? 8 : 4, PIPE>(P.plan, s - slice_off[lo], P.kbuf, P.val, accumulate);
 }
 
+// a pair's block at its position k0 of the scalar pattern and its transpose at k1 (x: the values, acc: the same
+// as double-float)
+template <int MODE, class T>
+__device__ __forceinline__ void elasticity_store(T* __restrict__ val, const int64_t* __restrict__ sia, const int32_t* __restrict__ ja,
+                                                 uint32_t k0, uint32_t k1, const T (&x)[9], const df (&acc)[9], int accumulate) {
+    auto put = [&](uint32_t k, int32_t row, bool tr) {
+        const int64_t s0 = sia[row];
+        const int64_t len = sia[row + 1] - s0;
+        T* const out = val + 9 * s0 + 3 * ((int64_t)k - s0);
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                T* const o = out + c * 3 * len + d;
+                const int q = tr ? d * 3 + c : c * 3 + d;
+                if (!accumulate) *o = x[q];
+                else if constexpr (MODE == kModeDF64) *o = df2d(df_add(d2df(*o), acc[q]));
+                else *o = f_add(*o, x[q]);
+            }
+    };
+    const int32_t j = __ldg(ja + k0), i = k1 == kNoIndex ? j : __ldg(ja + k1);
+    put(k0, i, false);
+    if (k1 != kNoIndex) put(k1, j, true);
+}
+
 // Vector elasticity: one lane per pair of nodes i <= j, its 3x3 block (row 3i+c, columns 3j+d) summed
 // over the contributions in element order (bit 31 of an index: stored as (j, i), read transposed) and
 // stored with its transpose at (j, i). sia, ja: the scalar pattern.
@@ -194,24 +220,222 @@ __global__ void __launch_bounds__(128) gather_elasticity_slices_kernel(GatherPla
         if constexpr (MODE == kModeDF64) x[k] = df2d(acc[k]);
         else x[k] = acc[k].hi;
     }
-    auto put = [&](uint32_t k, int32_t row, bool tr) {
-        const int64_t s0 = sia[row];
-        const int64_t len = sia[row + 1] - s0;
-        T* const out = val + 9 * s0 + 3 * ((int64_t)k - s0);
+    elasticity_store<MODE>(val, sia, ja, k0, k1, x, acc, accumulate);
+}
+
+// ---- vector elasticity without an element buffer ----
+// With exact quadrature the tensor of a pair of functions is Y = sum n_kl u_k u_l^T over their barycentric
+// derivatives (one for a vertex function, two for an edge function; p2_stiff_coef), u_a = (|T| / 5)^(1/2)
+// grad l_a (P1: |T|^(1/2), n = 1), and lambda and mu enter after the sum over the elements:
+// block = lambda Y + mu Y^T + mu tr(Y) 1.
+
+// u_0 .. u_3 of each element: double-float, (hi, lo) of three coordinates and two words of padding each, so
+// that a vector is one 32-byte sector (binary32: 16 bytes)
+template <int MODE, int N>
+__global__ void elasticity_vectors_kernel(int64_t nt, const double* __restrict__ xyz, const int32_t* __restrict__ tets,
+                                          float4* __restrict__ rec, int* __restrict__ status) {
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nt; e += (int64_t)gridDim.x * blockDim.x) {
+        const int4 t = *reinterpret_cast<const int4*>(tets + 4 * e);
+        const double* X0 = xyz + 3 * (int64_t)t.x;
+        const double* Xv[3] = {xyz + 3 * (int64_t)t.y, xyz + 3 * (int64_t)t.z, xyz + 3 * (int64_t)t.w};
+        // cofactors and determinant in binary64 (30 operations): the vectors' error enters every entry
+        double K[9];
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+#pragma unroll
+            for (int r = 0; r < 3; ++r) K[r * 3 + c] = Xv[c][r] - X0[r];
+        const double C[9] = {K[4] * K[8] - K[5] * K[7], K[5] * K[6] - K[3] * K[8], K[3] * K[7] - K[4] * K[6],
+                             K[2] * K[7] - K[1] * K[8], K[0] * K[8] - K[2] * K[6], K[1] * K[6] - K[0] * K[7],
+                             K[1] * K[5] - K[2] * K[4], K[2] * K[3] - K[0] * K[5], K[0] * K[4] - K[1] * K[3]};
+        const df J = d2df(0.125 * fabs(fma(K[0], C[0], fma(K[1], C[1], K[2] * C[2]))));
+        if (!(J.hi > 0.0f) || !isfinite(J.hi)) atomicOr(status, kStatusBadElement);
+        // grad l_a = C_a / (8 J), |T| = 4 J / 3: u = C_a / 4 (15 J)^(-1/2), P1 C_a / 4 (3 J)^(-1/2)
+        const float m = N == 10 ? 15.0f : 3.0f;
+        const df s = df_scale(df_rsqrt(df_mul(J, df{m, 0.0f})), 0.25f);
+        df u[4][3];
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+#pragma unroll
+            for (int a = 1; a < 4; ++a) u[a][r] = df_mul(d2df(C[3 * r + a - 1]), s);
+            const df v = two_sum(u[1][r].hi, u[2][r].hi), w = two_sum(v.hi, u[3][r].hi);
+            u[0][r] = df_neg(two_sum(w.hi, f_add(f_add(v.lo, w.lo), f_add(f_add(u[1][r].lo, u[2][r].lo), u[3][r].lo))));
+        }
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            if (MODE == kModeDF64) {
+                rec[8 * e + 2 * a] = make_float4(u[a][0].hi, u[a][0].lo, u[a][1].hi, u[a][1].lo);
+                rec[8 * e + 2 * a + 1] = make_float4(u[a][2].hi, u[a][2].lo, 0.0f, 0.0f);
+            } else {
+                rec[4 * e + a] = make_float4(u[a][0].hi, u[a][1].hi, u[a][2].hi, 0.0f);
+            }
+        }
+    }
+}
+
+// per entry of entry_order: the factors n_00, n_01, n_10, n_11 and its vectors (two bits each: a_0, a_1, b_0, b_1)
+template <int N>
+struct PairTable {
+    float4 terms[N * (N + 1) / 2];
+    uint32_t which[N * (N + 1) / 2];
+};
+template <int N>
+constexpr PairTable<N> make_pair_table() {
+    PairTable<N> P{};
+    const EntryOrder O = make_entry_order(4, N == 10 ? 2 : 1, N);
+    for (int t = 0; t < N * (N + 1) / 2; ++t) {
+        const int i = O.a[t], j = O.b[t], ni = N == 10 ? bary_comps(i) : 1, nj = N == 10 ? bary_comps(j) : 1;
+        for (int k = 0; k < 2; ++k) {
+            P.which[t] |= (uint32_t)(N == 10 ? bary_comp(i, k < ni ? k : 0) : i) << (2 * k);
+            P.which[t] |= (uint32_t)(N == 10 ? bary_comp(j, k < nj ? k : 0) : j) << (4 + 2 * k);
+        }
+        auto n = [&](int k, int l) { return k >= ni || l >= nj ? 0.0f : N == 10 ? (float)p2_stiff_coef(i, k, j, l) : 1.0f; };
+        P.terms[t].x = n(0, 0);
+        P.terms[t].y = n(0, 1);
+        P.terms[t].z = n(1, 0);
+        P.terms[t].w = n(1, 1);
+    }
+    return P;
+}
+__device__ const PairTable<4> kPairs1 = make_pair_table<4>();
+__device__ const PairTable<10> kPairs2 = make_pair_table<10>();
+template <int N>
+__device__ __forceinline__ const PairTable<N>& pair_table() {
+    if constexpr (N == 10) return kPairs2;
+    else return kPairs1;
+}
+
+// One lane per pair of nodes i <= j (the slices of the scalar plan): Y summed over the pair's elements in
+// element order, each from the element's vectors, then lambda and mu; stored with its transpose at (j, i).
+// The 3x3 blocks of the element matrices (3 960 bytes per P2 element, 718 MB at 36x28x30) are never stored:
+// 128 bytes of vectors are, which stay in L2, and a slice's lanes mostly share their elements, so that a
+// step's loads are few sectors.
+// Bound: FP32 issue half the time (18 compensated products and six two-term sums per contribution and lane,
+// then the moduli and 18 stores per pair), the rest latency: pairs have three contributions on average. 64
+// registers and two warps a block: 337 us, without the bound (72 registers) 372, two contributions in flight
+// (96 registers) 405; fewer, longer-lived blocks 390-550 (neighbouring slices no longer run together). P2
+// 36x28x30 in double-float: geometry 25, element blocks 413, gather 378 us -> vectors 15 and here 337; a pass
+// 821 -> 372 us, P1 45^3 1070 -> 164 us, binary32 P2 20^3 193 -> 89 us. Error against
+// binary64 5.7e-15 -> 5.1e-15.
+template <int MODE, int N, int B>
+__global__ void __launch_bounds__(64, 16) gather_elasticity_fused_kernel(GatherPlan G, const int64_t* __restrict__ sia,
+                                                                      const int32_t* __restrict__ ja, const float4* __restrict__ rec,
+                                                                      double lam, double mu, void* __restrict__ valv, int accumulate) {
+    constexpr int NTRI = N * (N + 1) / 2;
+    const PairTable<N>& pairs = pair_table<N>();
+    const int lane = threadIdx.x & 31;
+    const int64_t s = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (s >= G.nslices) return;
+    const uint32_t r0 = __ldg(G.soff + s), r1 = __ldg(G.soff + s + 1);
+    const uint32_t k0 = __ldg(G.pos0 + s * 32 + lane), k1 = __ldg(G.pos1 + s * 32 + lane);
+    float ys[9], ye[9];
+#pragma unroll
+    for (int k = 0; k < 9; ++k) ys[k] = ye[k] = 0.0f;
+    constexpr int NV = N == 10 ? 2 : 1, W = MODE == kModeDF64 ? 2 : 1;       // vectors per function; float4 per vector
+    uint32_t ix[B];
+#pragma unroll
+    for (int u = 0; u < B; ++u) ix[u] = r0 + u < r1 ? __ldg(G.sidx + (size_t)(r0 + u) * 32 + lane) : kNoIndex;
+    for (uint32_t r = r0; r < r1; r += B) {
+        float4 va[B][NV * W], vb[B][NV * W];
+        float4 pt[B];
+        uint32_t cur[B];
+#pragma unroll
+        for (int u = 0; u < B; ++u) {
+            cur[u] = ix[u];
+            const uint32_t idx = cur[u] == kNoIndex ? 0u : cur[u] & 0x7FFFFFFFu, e = idx / NTRI, t = idx - e * NTRI;
+            uint32_t w = __ldg(&pairs.which[t]);
+            pt[u] = __ldg(&pairs.terms[t]);
+            if (cur[u] & 0x80000000u) {                              // stored as (j, i)
+                w = (w >> 4 | w << 4) & 255u;
+                const float x = pt[u].y;
+                pt[u].y = pt[u].z;
+                pt[u].z = x;
+            }
+            const float4* base = rec + (size_t)e * (4 * W);
+#pragma unroll
+            for (int q = 0; q < NV; ++q)
+#pragma unroll
+                for (int x = 0; x < W; ++x) {
+                    va[u][q * W + x] = __ldg(base + (w >> (2 * q) & 3u) * W + x);
+                    vb[u][q * W + x] = __ldg(base + (w >> (4 + 2 * q) & 3u) * W + x);
+                }
+        }
+#pragma unroll
+        for (int u = 0; u < B; ++u) ix[u] = r + B + u < r1 ? __ldg(G.sidx + (size_t)(r + B + u) * 32 + lane) : kNoIndex;
+#pragma unroll
+        for (int u = 0; u < B; ++u) {
+            if (cur[u] == kNoIndex) continue;
+#pragma unroll
+            for (int q = 0; q < NV; ++q) {
+                if constexpr (MODE == kModeDF64) {
+                    auto vec = [](const float4* v, int c) {
+                        return c == 0 ? df{v[0].x, v[0].y} : c == 1 ? df{v[0].z, v[0].w} : df{v[1].x, v[1].y};
+                    };
+                    df h[3];
+#pragma unroll
+                    for (int c = 0; c < 3; ++c) {
+                        if constexpr (N == 4) {
+                            h[c] = vec(vb[u], c);
+                        } else {
+                            // n_q0 b_0 + n_q1 b_1, the factors small integers
+                            const df b0 = vec(vb[u], c), b1 = vec(vb[u] + W, c);
+                            const float n0 = q == 0 ? pt[u].x : pt[u].z, n1 = q == 0 ? pt[u].y : pt[u].w;
+                            const float p0 = f_mul(n0, b0.hi), p1 = f_mul(n1, b1.hi);
+                            float e = f_fma(n0, b0.lo, f_fma(n0, b0.hi, -p0));
+                            e = f_fma(n1, b1.lo, f_add(e, f_fma(n1, b1.hi, -p1)));
+                            const df x = two_sum(p0, p1);
+                            h[c] = quick_two_sum(x.hi, f_add(x.lo, e));
+                        }
+                    }
+#pragma unroll
+                    for (int c = 0; c < 3; ++c)
+#pragma unroll
+                        for (int d = 0; d < 3; ++d) df_dot_term(vec(va[u] + q * W, c), h[d], ys[3 * c + d], ye[3 * c + d]);
+                } else {
+                    auto vec = [](const float4& v, int c) { return c == 0 ? v.x : c == 1 ? v.y : v.z; };
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) {
+                        const float h = N == 4 ? vec(vb[u][0], d)
+                                               : fmaf(q == 0 ? pt[u].x : pt[u].z, vec(vb[u][0], d), (q == 0 ? pt[u].y : pt[u].w) * vec(vb[u][NV - 1], d));
+#pragma unroll
+                        for (int c = 0; c < 3; ++c) ys[3 * c + d] = fmaf(vec(va[u][q], c), h, ys[3 * c + d]);
+                    }
+                }
+            }
+        }
+    }
+    if (k0 == kNoIndex) return;
+    typedef typename std::conditional<MODE == kModeDF64, double, float>::type T;
+    T* const val = reinterpret_cast<T*>(valv);
+    df acc[9];
+    T x[9];
+    if constexpr (MODE == kModeDF64) {
+        const df l = d2df(lam), m = d2df(mu);
+        df y[9];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) y[k] = two_sum(ys[k], ye[k]);
+        const df mtr = df_mul(m, df_add(df_add(y[0], y[4]), y[8]));
 #pragma unroll
         for (int c = 0; c < 3; ++c)
 #pragma unroll
             for (int d = 0; d < 3; ++d) {
-                T* const o = out + c * 3 * len + d;
-                const int q = tr ? d * 3 + c : c * 3 + d;
-                if (!accumulate) *o = x[q];
-                else if constexpr (MODE == kModeDF64) *o = df2d(df_add(d2df(*o), acc[q]));
-                else *o = f_add(*o, x[q]);
+                df v = df_add(df_mul(l, y[c * 3 + d]), df_mul(m, y[d * 3 + c]));
+                if (c == d) v = df_add(v, mtr);
+                acc[c * 3 + d] = v;
+                x[c * 3 + d] = df2d(v);
             }
-    };
-    const int32_t j = __ldg(ja + k0), i = k1 == kNoIndex ? j : __ldg(ja + k1);
-    put(k0, i, false);
-    if (k1 != kNoIndex) put(k1, j, true);
+    } else {
+        const float l = (float)lam, m = (float)mu, tr = ys[0] + ys[4] + ys[8];
+#pragma unroll
+        for (int c = 0; c < 3; ++c)
+#pragma unroll
+            for (int d = 0; d < 3; ++d) {
+                float v = fmaf(l, ys[c * 3 + d], m * ys[d * 3 + c]);
+                if (c == d) v = fmaf(m, tr, v);
+                x[c * 3 + d] = v;
+                acc[c * 3 + d] = df{v, 0.0f};
+            }
+    }
+    elasticity_store<MODE>(val, sia, ja, k0, k1, x, acc, accumulate);
 }
 
 // the values of the matrix to a mapped page-locked host buffer
@@ -618,6 +842,32 @@ int launch_gather_elasticity(fgpu_ctx* ctx, const fgpu_matrix* A, int accumulate
     } else {
         if (A->precision == FGPU_F32) EL_GATHER(kModeF32, 2); else EL_GATHER(kModeDF64, 2);
     }
+#undef EL_GATHER
+    prof_end(ctx, ev);
+    FGPU_CUDA_CHECK(ctx, cudaGetLastError());
+    return FGPU_OK;
+}
+
+// rec: 128 bytes per element
+int launch_gather_elasticity_fused(fgpu_ctx* ctx, const fgpu_matrix* A, double lam, double mu, float4* rec, int accumulate) {
+    const GatherPlan& G = A->space->plan;
+    const DevPattern& P = *A->pattern;
+    const fgpu_mesh* M = A->space->mesh;
+    const bool f32 = A->precision == FGPU_F32, p2 = A->space->order == 2;
+    PendingEvent ev;
+    prof_begin(ctx, "geometry", ev);
+    const int gb = (int)std::max<int64_t>(1, std::min<int64_t>((M->nt + 127) / 128, 152 * 16));
+#define EL_VECTORS(MODE, N) elasticity_vectors_kernel<MODE, N><<<gb, 128, 0, ctx->stream>>>(M->nt, M->d_xyz, M->d_tets, rec, ctx->d_status)
+    if (p2) { if (f32) EL_VECTORS(kModeF32, 10); else EL_VECTORS(kModeDF64, 10); }
+    else { if (f32) EL_VECTORS(kModeF32, 4); else EL_VECTORS(kModeDF64, 4); }
+#undef EL_VECTORS
+    prof_end(ctx, ev);
+    FGPU_CUDA_CHECK(ctx, cudaGetLastError());
+    const int blocks = (int)std::max<int64_t>(1, (G.nslices + 1) / 2);
+    prof_begin(ctx, "assemble_gather_elasticity", ev);
+#define EL_GATHER(MODE, N, B) gather_elasticity_fused_kernel<MODE, N, B><<<blocks, 64, 0, ctx->stream>>>(G, P.d_ia, P.d_ja, rec, lam, mu, A->d_val, accumulate)
+    if (p2) { if (f32) EL_GATHER(kModeF32, 10, 2); else EL_GATHER(kModeDF64, 10, 1); }
+    else { if (f32) EL_GATHER(kModeF32, 4, 4); else EL_GATHER(kModeDF64, 4, 2); }
 #undef EL_GATHER
     prof_end(ctx, ev);
     FGPU_CUDA_CHECK(ctx, cudaGetLastError());
