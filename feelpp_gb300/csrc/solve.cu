@@ -30,6 +30,7 @@
 #include <tuple>
 #include <vector>
 
+#include "block_order.cuh"
 #include "ld_stream.cuh"
 #include "cg_driver.cuh"
 #include "df64.h"
@@ -54,7 +55,6 @@ static void launch_spmv_t(cudaStream_t s, const fgpu_matrix* A, const typename P
                           typename PL::S* y, int mode, const typename PL::S* b, const typename PL::S* wdot,
                           typename PL::D* partial, const CGScalars<PL>* sc, int blocks) {
     switch (G) {
-        case 2: spmv_kernel<PL, 2><<<blocks, 256, 0, s>>>(A->nrows, A->d_ia, A->d_ja, val, x, y, mode, b, wdot, partial, sc); break;
         case 4: spmv_kernel<PL, 4><<<blocks, 256, 0, s>>>(A->nrows, A->d_ia, A->d_ja, val, x, y, mode, b, wdot, partial, sc); break;
         case 8: spmv_kernel<PL, 8><<<blocks, 256, 0, s>>>(A->nrows, A->d_ia, A->d_ja, val, x, y, mode, b, wdot, partial, sc); break;
         case 16: spmv_kernel<PL, 16><<<blocks, 256, 0, s>>>(A->nrows, A->d_ia, A->d_ja, val, x, y, mode, b, wdot, partial, sc); break;
@@ -75,20 +75,47 @@ static int spmv_blocks(const fgpu_matrix* A, int G) {
     return (int)std::max<int64_t>(1, std::min<int64_t>(need, 152 * 16));
 }
 
-// without per-block partial sums the grid does not change the result: one block per 256 / G rows
-// (P2 64^3 y = A x: 0.40 against 0.43 ms with the capped grid; 8 lanes per row took 0.48 ms, and each
-// lane's entries in explicit batches of 8 with their loads issued together 0.53 ms: 64 registers)
-static int spmv_blocks_uncapped(const fgpu_matrix* A, int G) {
-    return (int)std::max<int64_t>(1, (A->nrows + (256 / G) - 1) / (256 / G));
+// y = A x (or b - A x) for rows of up to 40 entries on average: two lanes per row as spmv_kernel sums it (lane l
+// the entries congruent to l mod 2, then one addition), four entries' loads together, a block's 128 rows in
+// the order of their lengths, and the sums stored in row order. Bound: FP64 pipe and memory. An FP64
+// instruction occupies the pipe for the whole warp, so that rows of 24 and of 65 entries in one warp cost the
+// longer one's time; two lanes read half a sector, whose other half L1 keeps for the next load (past L1: 137
+// us). P2 48^3 (25.8 M entries): in row order with one entry at a time 156 us, here 112.
+__global__ void __launch_bounds__(256) spmv_mult_kernel(int64_t nrows, const int64_t* __restrict__ ia, const int32_t* __restrict__ ja,
+                                                        const double* __restrict__ val, const double* __restrict__ x,
+                                                        double* __restrict__ y, const double* __restrict__ b) {
+    __shared__ BlockOrder<128> order;
+    __shared__ int64_t first[129];
+    __shared__ double out[128];
+    const int t = threadIdx.x;
+    const int64_t r0 = (int64_t)blockIdx.x * 128;
+    if (t < 129) first[t] = ia[r0 + t < nrows ? r0 + t : nrows];
+    __syncthreads();
+    block_order(order, t < 128 ? (int)min((first[t + 1] - first[t]) >> 1, (int64_t)31) : 0);
+    const int k = order.row[t >> 1];
+    const int64_t pe = first[k + 1];
+    double s = 0.0;
+    constexpr int U = 4;
+    for (int64_t p = first[k] + (t & 1); p < pe; p += 2 * U) {
+        int32_t c[U];
+        double v[U], w[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) {
+            const bool in = p + 2 * u < pe;
+            c[u] = in ? __ldg(ja + p + 2 * u) : 0;
+            v[u] = in ? __ldg(val + p + 2 * u) : 0.0;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) w[u] = x[c[u]];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+            if (p + 2 * u < pe) s = fma(v[u], w[u], s);
+    }
+    s += __shfl_xor_sync(0xffffffffu, s, 1);
+    if (!(t & 1)) out[k] = s;
+    __syncthreads();
+    if (t < 128 && r0 + t < nrows) y[r0 + t] = b ? b[r0 + t] - out[t] : out[t];
 }
-
-// lanes per row of y = A x: two for rows of up to 40 entries (one FP64 shuffle-add per lane; P2 64^3:
-// 0.36 against 0.40 ms with four), else as in the solver
-static int mult_group(const fgpu_matrix* A) {
-    const double avg = A->nrows ? (double)A->nnz / (double)A->nrows : 1.0;
-    return avg <= 40 ? 2 : spmv_group(A);
-}
-
 
 int launch_spmv(fgpu_ctx* ctx, const fgpu_matrix* A, const double* x, double* y, double alpha_b, const double* b) {
     (void)alpha_b;
@@ -96,11 +123,17 @@ int launch_spmv(fgpu_ctx* ctx, const fgpu_matrix* A, const double* x, double* y,
         ctx->err = "y = A x with binary64 vectors needs an FP64 matrix";
         return FGPU_ERR_INVALID;
     }
-    const int G = mult_group(A);
     PendingEvent ev;
     prof_begin(ctx, "spmv", ev);
-    launch_spmv_t<PolF64>(ctx->stream, A, (const double*)A->d_val, G, x, y, b ? 1 : 0, b, nullptr, nullptr, nullptr,
-                          spmv_blocks_uncapped(A, G));
+    if (A->nnz <= 40 * A->nrows) {
+        spmv_mult_kernel<<<(int)std::max<int64_t>(1, (A->nrows + 127) / 128), 256, 0, ctx->stream>>>(
+            A->nrows, A->d_ia, A->d_ja, (const double*)A->d_val, x, y, b);
+    } else {
+        // without per-block partial sums the grid does not change the result: one block per 256 / G rows
+        const int G = spmv_group(A);
+        launch_spmv_t<PolF64>(ctx->stream, A, (const double*)A->d_val, G, x, y, b ? 1 : 0, b, nullptr, nullptr, nullptr,
+                              (int)std::max<int64_t>(1, (A->nrows + (256 / G) - 1) / (256 / G)));
+    }
     prof_end(ctx, ev);
     FGPU_CUDA_CHECK(ctx, cudaGetLastError());
     return FGPU_OK;
