@@ -301,13 +301,13 @@ __global__ void __launch_bounds__(256) lanczos_spmv_kernel(int64_t n, const int6
             const int64_t e = ia[i + 1];
             int64_t p = ia[i] + sub;
             for (; p + 4 < e; p += 8) {
-                const int32_t j0 = ld_stream(ja + p), j1 = ld_stream(ja + p + 4);
+                const int32_t j0 = __ldg(ja + p), j1 = __ldg(ja + p + 4);
                 const double a0 = ld_stream(a + p), a1 = ld_stream(a + p + 4);
                 const double u0 = u[j0], u1 = u[j1];
                 acc = __dadd_rn(acc, __dmul_rn(a0, u0));
                 acc = __dadd_rn(acc, __dmul_rn(a1, u1));
             }
-            if (p < e) acc = __dadd_rn(acc, __dmul_rn(ld_stream(a + p), u[ld_stream(ja + p)]));
+            if (p < e) acc = __dadd_rn(acc, __dmul_rn(ld_stream(a + p), u[__ldg(ja + p)]));
         }
         acc = __dadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, 2));
         acc = __dadd_rn(acc, __shfl_xor_sync(0xffffffffu, acc, 1));
