@@ -269,37 +269,51 @@ __global__ void __launch_bounds__(256) sell_spmv_kernel(int64_t nrows, int64_t n
         const int L = slice_len[s];
         const int64_t base = slice_ptr[s] + (i - s * kSellC);
         typename PL::D accd = PL::dzero();     // row sums in the dot-product type (see spmv_kernel)
-        // four entries at a time, the next columns and values loaded past L1 before this batch's gathers
-        // of x; summed in entry order. FP64, P2 48^3 (310 MB): 104 -> 97 us
-        constexpr int U = 4;
-        int32_t c[U];
-        typename PL::V v[U];
-        if (L >= U) {
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                c[u] = ld_stream(col + base + u * kSellC);
-                v[u] = ld_stream(val + base + u * kSellC);
-            }
-        }
+        // four entries' loads together, summed in entry order. FP64 values: the next columns and values are loaded
+        // past L1 before this batch's gathers of x (P2 48^3, 310 MB: 123 us -> 94; P2 34x30x33, in L2: 41 -> 35);
+        // with the other formats that costs more than it gives (binary32 in L2: 19 us -> 29).
         int k = 0;
-        for (; k + U <= L; k += U) {
-            typename PL::S xs[U];
-            typename PL::V vc[U];
-#pragma unroll
-            for (int u = 0; u < U; ++u) {
-                xs[u] = x[c[u]];
-                vc[u] = v[u];
-            }
-            if (k + 2 * U <= L) {
-                const int64_t j = base + (int64_t)(k + U) * kSellC;
+        if constexpr (std::is_same<typename PL::V, double>::value) {
+            constexpr int U = 4;
+            int32_t c[U];
+            typename PL::V v[U];
+            if (L >= U) {
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
-                    c[u] = ld_stream(col + j + u * kSellC);
-                    v[u] = ld_stream(val + j + u * kSellC);
+                    c[u] = ld_stream(col + base + u * kSellC);
+                    v[u] = ld_stream(val + base + u * kSellC);
                 }
             }
+            for (; k + U <= L; k += U) {
+                typename PL::S xs[U];
+                typename PL::V vc[U];
 #pragma unroll
-            for (int u = 0; u < U; ++u) accd = PL::dmadd(accd, PL::ldv(vc[u]), PL::ld(xs[u]));
+                for (int u = 0; u < U; ++u) {
+                    xs[u] = x[c[u]];
+                    vc[u] = v[u];
+                }
+                if (k + 2 * U <= L) {
+                    const int64_t j = base + (int64_t)(k + U) * kSellC;
+#pragma unroll
+                    for (int u = 0; u < U; ++u) {
+                        c[u] = ld_stream(col + j + u * kSellC);
+                        v[u] = ld_stream(val + j + u * kSellC);
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < U; ++u) accd = PL::dmadd(accd, PL::ldv(vc[u]), PL::ld(xs[u]));
+            }
+        } else {
+            for (; k + 4 <= L; k += 4) {
+                const int64_t j = base + (int64_t)k * kSellC;
+                const int32_t c0 = col[j], c1 = col[j + kSellC], c2 = col[j + 2 * kSellC], c3 = col[j + 3 * kSellC];
+                const typename PL::V v0 = val[j], v1 = val[j + kSellC], v2 = val[j + 2 * kSellC], v3 = val[j + 3 * kSellC];
+                const typename PL::S x0 = x[c0], x1 = x[c1], x2 = x[c2], x3 = x[c3];
+                accd = PL::dmadd(accd, PL::ldv(v0), PL::ld(x0));
+                accd = PL::dmadd(accd, PL::ldv(v1), PL::ld(x1));
+                accd = PL::dmadd(accd, PL::ldv(v2), PL::ld(x2));
+                accd = PL::dmadd(accd, PL::ldv(v3), PL::ld(x3));
+            }
         }
         for (; k < L; ++k) {
             const int64_t j = base + (int64_t)k * kSellC;
