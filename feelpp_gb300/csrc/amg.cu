@@ -46,6 +46,7 @@ struct fgpu_amg {
         int32_t* s_perm = nullptr;
         int32_t* s_col = nullptr;
         float* s_val = nullptr;
+        int64_t s_bytes = 0;             // columns and values
         int64_t* p_ia = nullptr;     // P_l: n x n_{l+1}
         int32_t* p_ja = nullptr;
         float* p_a = nullptr;
@@ -139,10 +140,17 @@ struct AmgSell {
 // Row i (in sorted order) of a SELL sweep: the entries of its slice column eight at a time, the next eight
 // columns and values loaded before this batch's gathers of x, summed in entry order, then the epilogue on
 // the original row. The kernel waits on memory: 45 warps of an SM have to keep some 45 KB in flight, and
-// x has to stay in L1 beside the columns and values streaming through. P2 48^3 (206 MB): 52.9 us with four
-// entries and no load ahead, 48.9 with four loaded ahead, 43.0 with those past L1, 41.2 with eight (47.0
-// through L1).
-template <int MODE>
+// x has to stay in L1 beside the columns and values streaming through. STREAM: those are loaded past L1, for
+// levels that do not stay in L2 between sweeps. Four entries and no load ahead / eight ahead through L1 /
+// past L1: P2 48^3 (206 MB) 52.7 / 47.2 / 41.5 us, P3 22x20x21 (100 MB) 45.2 / 33.2 / 31.2, P2 34x30x33 (64 MB)
+// 14.7 / 12.9 / 16.4.
+template <bool STREAM>
+__device__ __forceinline__ int32_t sell_col(const int32_t* p) { return STREAM ? ld_stream(p) : __ldg(p); }
+template <bool STREAM>
+__device__ __forceinline__ float sell_val(const float* p) { return STREAM ? ld_stream(p) : __ldg(p); }
+constexpr int64_t kSellStreamBytes = (int64_t)80 << 20;
+
+template <int MODE, bool STREAM>
 __device__ __forceinline__ void sell_row(const AmgSweep& s, const AmgSell& m, int64_t i) {
     constexpr int U = 8;
     const int64_t sl = i >> 5;
@@ -155,8 +163,8 @@ __device__ __forceinline__ void sell_row(const AmgSweep& s, const AmgSell& m, in
     if (L >= U) {
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            c[u] = ld_stream(m.col + base + u * 32);
-            v[u] = ld_stream(m.val + base + u * 32);
+            c[u] = sell_col<STREAM>(m.col + base + u * 32);
+            v[u] = sell_val<STREAM>(m.val + base + u * 32);
         }
     }
     int k = 0;
@@ -171,8 +179,8 @@ __device__ __forceinline__ void sell_row(const AmgSweep& s, const AmgSell& m, in
             const int64_t j = base + (int64_t)(k + U) * 32;
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                c[u] = ld_stream(m.col + j + u * 32);
-                v[u] = ld_stream(m.val + j + u * 32);
+                c[u] = sell_col<STREAM>(m.col + j + u * 32);
+                v[u] = sell_val<STREAM>(m.val + j + u * 32);
             }
         }
 #pragma unroll
@@ -180,19 +188,19 @@ __device__ __forceinline__ void sell_row(const AmgSweep& s, const AmgSell& m, in
     }
     for (; k < L; ++k) {
         const int64_t j = base + (int64_t)k * 32;
-        acc = fmaf(ld_stream(m.val + j), __ldg(s.x + ld_stream(m.col + j)), acc);
+        acc = fmaf(sell_val<STREAM>(m.val + j), __ldg(s.x + sell_col<STREAM>(m.col + j)), acc);
     }
     if (row >= 0) amg_epilogue<MODE>(s, row, acc);
 }
 
 // one sweep of a level operator in SELL form: thread per (sorted) row, then the epilogue on the
 // original row; every lane of a warp belongs to one slice, so the entry loop is warp-uniform
-template <int MODE>
+template <int MODE, bool STREAM>
 __global__ void __launch_bounds__(128) amg_sell_kernel(AmgSweep s, AmgSell m, const int* __restrict__ stop) {
     if (stop && *stop) return;
     const int64_t total = m.nslices * 32;
     for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x)
-        sell_row<MODE>(s, m, i);
+        sell_row<MODE, STREAM>(s, m, i);
 }
 
 // the same sweep for levels with few rows: a block of W warps per slice, warp w summing the entries
@@ -350,7 +358,8 @@ void sell_sweep(cudaStream_t st, const fgpu_amg::Level& V, const AmgSweep& s, co
     // with 256 and 1.29 / 6.68 ms with 64; persistent warps taking four slices at a time from an atomic
     // counter: 1.35 / 6.93 ms
     const int g = (int)std::max<int64_t>(1, (V.nslices * 32 + 127) / 128);
-    amg_sell_kernel<MODE><<<g, 128, 0, st>>>(s, m, stop);
+    if (V.s_bytes > kSellStreamBytes) amg_sell_kernel<MODE, true><<<g, 128, 0, st>>>(s, m, stop);
+    else amg_sell_kernel<MODE, false><<<g, 128, 0, st>>>(s, m, stop);
 }
 
 int vblocks(int64_t n) { return (int)std::max<int64_t>(1, std::min<int64_t>((n + 255) / 256, 152 * 8)); }
@@ -571,6 +580,7 @@ cudaError_t upload_sell(cudaStream_t stream, fgpu_amg::Level& V, const HostCsr& 
     if (e == cudaSuccess) e = upload(stream, &V.s_len, len.data(), len.size());
     if (e == cudaSuccess) e = upload(stream, &V.s_perm, perm.data(), perm.size());
     if (e == cudaSuccess) e = upload(stream, &V.s_col, col.data(), col.size());
+    V.s_bytes = (int64_t)val.size() * 8;
     if (e == cudaSuccess) e = upload(stream, &V.s_val, val.data(), val.size());
     return e;
 }
@@ -606,6 +616,7 @@ int upload_level0_device(fgpu_ctx* ctx, const fgpu_matrix* A, fgpu_amg::Level& V
     V.s_len = L->d_slice_len; L->d_slice_len = nullptr;
     V.s_perm = L->d_perm; L->d_perm = nullptr;
     V.s_col = L->d_col; L->d_col = nullptr;
+    V.s_bytes = L->nstored * 8;
     FGPU_CUDA_CHECK(ctx, pool_malloc(ctx->stream, &V.s_val, std::max<int64_t>(L->nstored, 1) * sizeof(float)));
     FGPU_CUDA_CHECK(ctx, pool_malloc(ctx->stream, &V.dinv, std::max<int64_t>(V.n, 1) * sizeof(float)));
     const int g = (int)std::max<int64_t>(1, std::min<int64_t>((L->nstored + 255) / 256, 152 * 32));
