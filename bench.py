@@ -538,9 +538,9 @@ def run_gb300(args, rank, world, local):
     dom = max(kern_ms, key=kern_ms.get)
     per_launch_ms = kern_ms[dom]
     achieved = b_asm / (per_launch_ms / 1e3) / 1e9
-    # bytes the two-phase design itself moves in its gather (gptr, gidx, the buffered element
-    # entries, the CSR values): explains the gap between the two fractions
-    design_bytes = (nnz + 1) * 4 + T * n_loc * n_loc * 4 + T * ntri * 8 + nnz * 8
+    # bytes the two-phase design itself moves in its gather (two positions per sum, an index per buffered
+    # entry, the buffered entries, the CSR values): explains the gap between the two fractions
+    design_bytes = (nnz + N) // 2 * 8 + T * ntri * 4 + T * ntri * 8 + nnz * 8
     tr = load_traffic()
     traffic = None
     if tr and tr.get("order") == args.order and tr.get("algo") == "two_phase":
@@ -548,7 +548,8 @@ def run_gb300(args, rank, world, local):
     step_ms = ms_max / args.steps
     roofline = {"bound": "hbm", "achieved": achieved, "peak": hbm_peak, "unit": "GB/s",
                 "frac": achieved / hbm_peak, "traffic": traffic, "peak_source": peak_kind,
-                "kernel": "%s (two-phase)" % {"assemble_gather": "gather_map_kernel", "assemble_elements": "element_tri_kernel",
+                "kernel": "%s (two-phase)" % {"assemble_gather": "gather_slices_kernel",
+                                              "assemble_elements": "element_closed_kernel" if args.order < 3 else "element_tri_kernel",
                                               "geometry": "geometry_df_kernel"}[dom],
                 "kernel_ms": per_launch_ms, "algorithmic_bytes": b_asm,
                 "algorithmic_bytes_def": "B_asm = nnz*(8+4) + (N+1)*4 + V*24 + T*(4 n_loc + 8)",
