@@ -637,7 +637,7 @@ def run_gb300(args, rank, world, local):
     t_e2e = e2e_by_mode["auto"]
     e2e = {"value": nnz * args.steps * world / t_e2e / 1e6, "unit": UNIT,
            "h2d_bytes_per_step": int(xyz.nbytes + kappa.nbytes), "d2h_bytes_per_step": int(nnz * 8),
-           "host_transfer": "direct stores from the gather kernel into the page-locked buffer",
+           "host_transfer": "copy-engine ranges of complete rows beside the gather, into the page-locked buffer",
            "value_copy_engines": nnz * args.steps * world / e2e_by_mode["copy"] / 1e6}
 
     # ---- CG time-to-1e-10 on the same system (homogeneous Dirichlet) ----

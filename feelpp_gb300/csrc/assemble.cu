@@ -1715,7 +1715,7 @@ static int run_two_phase(fgpu_ctx* ctx, fgpu_matrix* A, const DevTables* tab, co
         prof_end(ctx, ev);
         FGPU_CUDA_CHECK(ctx, cudaGetLastError());
     }
-    if (host) return launch_gather_phase_to_host(ctx, A, host, 4);
+    if (host) return launch_gather_phase_to_host(ctx, A, host);
     PendingEvent ev;
     prof_begin(ctx, "assemble_gather", ev);
     launch_gather_map(ctx, A, shape, accumulate);

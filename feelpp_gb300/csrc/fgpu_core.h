@@ -20,6 +20,7 @@ struct GatherPlan {                  // two-phase gather map of a space, in slic
     uint32_t* pos1 = nullptr;        // position of the transpose, 0xFFFFFFFF on the diagonal
     uint32_t* soff = nullptr;        // slices + 1: first row of a slice in sidx
     uint32_t* sidx = nullptr;        // rows of 32 element-buffer indices, one row per step of a slice
+    int64_t part_end[4] = {-1, -1, -1, -1};   // CSR entries [0, part_end[c]) are complete after quarter c of the slices
 };
 void stream_plan_free(StreamPlan* p);
 
@@ -448,7 +449,7 @@ int solve_gmres(fgpu_ctx* ctx, const fgpu_matrix* A, fgpu_amg* amg, const double
 int ensure_two_phase(fgpu_ctx* ctx, fgpu_matrix* A, size_t need);
 int launch_assemble_two_phase_host(fgpu_ctx* ctx, fgpu_matrix* A, const DevTables* tab, const float4* rec, const GeoIn* geo,
                                    double* host);
-int launch_gather_phase_to_host(fgpu_ctx* ctx, fgpu_matrix* A, double* host, int nchunks);
+int launch_gather_phase_to_host(fgpu_ctx* ctx, fgpu_matrix* A, double* host);
 int launch_gather_phase(fgpu_ctx* ctx, fgpu_matrix* A, int accumulate);
 int launch_rhs_gather(fgpu_ctx* ctx, const fgpu_space* V, const double* d_work, double* d_out, int accumulate);
 int launch_assemble_ho(fgpu_ctx* ctx, fgpu_matrix* A, const fgpu_form_desc* f, const double* d_kappa, int accumulate);

@@ -25,6 +25,7 @@
 // (no symmetry) with the sums staged in shared memory and stored in CSR order, 0.244 ms at P2 48^3
 // (62 M load sectors: 8-byte values in scattered 32-byte sectors).
 #include <algorithm>
+#include <climits>
 #include <string>
 #include <type_traits>
 #include <vector>
@@ -443,6 +444,18 @@ __global__ void __launch_bounds__(256) values_to_host_kernel(int64_t nnz, const 
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < nnz; k += (int64_t)gridDim.x * blockDim.x) hout[k] = val[k];
 }
 
+// lowest[c]: the lowest row that quarter c of the slices writes to (the row of a position is the column of its
+// transpose's)
+__global__ void __launch_bounds__(256) part_rows_kernel(GatherPlan G, const int32_t* __restrict__ ja, int* __restrict__ lowest) {
+    const int64_t q = (G.nslices + 3) / 4, n = G.nslices * 32;
+    for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x) {
+        const uint32_t k0 = G.pos0[k], k1 = G.pos1[k];
+        int r = k0 == kNoIndex ? INT_MAX : k1 == kNoIndex ? ja[k0] : min(ja[k0], ja[k1]);
+        r = __reduce_min_sync(0xffffffffu, r);
+        if ((threadIdx.x & 31) == 0 && r != INT_MAX) atomicMin(lowest + (k >> 5) / q, r);
+    }
+}
+
 // ---- the plan (once per space) ----
 
 // The space's tables that the plan is built from; tri: pair (a, b) of local dofs -> buffer entry.
@@ -691,8 +704,7 @@ void launch_walk(fgpu_ctx* ctx, int blocks, const PlanIn& in, uint16_t* first, c
 }
 
 template <int MODE, bool PIPE>
-void launch_slices(fgpu_ctx* ctx, const fgpu_matrix* A, int threads, int bpsm, int batch, int accumulate) {
-    const GatherPlan& G = A->space->plan;
+void launch_slices(fgpu_ctx* ctx, const fgpu_matrix* A, const GatherPlan& G, int threads, int bpsm, int batch, int accumulate) {
     const int64_t need = (G.nslices + threads / 32 - 1) / (threads / 32);
     const int blocks = (int)std::max<int64_t>(1, bpsm > 0 ? std::min<int64_t>(need, (int64_t)sm_count(ctx) * bpsm) : need);
     switch (batch) {
@@ -811,11 +823,11 @@ int launch_build_gather_map(fgpu_ctx* ctx, fgpu_space* V) {
 
 void launch_gather_slices(fgpu_ctx* ctx, const fgpu_matrix* A, int threads, int bpsm, int batch, int pipe, int accumulate) {
     if (A->precision == FGPU_F32) {
-        if (pipe) launch_slices<kModeF32, true>(ctx, A, threads, bpsm, batch, accumulate);
-        else launch_slices<kModeF32, false>(ctx, A, threads, bpsm, batch, accumulate);
+        if (pipe) launch_slices<kModeF32, true>(ctx, A, A->space->plan, threads, bpsm, batch, accumulate);
+        else launch_slices<kModeF32, false>(ctx, A, A->space->plan, threads, bpsm, batch, accumulate);
     } else {
-        if (pipe) launch_slices<kModeDF64, true>(ctx, A, threads, bpsm, batch, accumulate);
-        else launch_slices<kModeDF64, false>(ctx, A, threads, bpsm, batch, accumulate);
+        if (pipe) launch_slices<kModeDF64, true>(ctx, A, A->space->plan, threads, bpsm, batch, accumulate);
+        else launch_slices<kModeDF64, false>(ctx, A, A->space->plan, threads, bpsm, batch, accumulate);
     }
 }
 
@@ -875,11 +887,41 @@ int launch_gather_elasticity_fused(fgpu_ctx* ctx, const fgpu_matrix* A, double l
     return FGPU_OK;
 }
 
-// Phase 2, then the values to the host: by kernel stores where the buffer is page-locked and mapped
-// (CSR order, at the host link's rate), else in nchunks ranges on as many copy streams. FP64 matrices.
-int launch_gather_phase_to_host(fgpu_ctx* ctx, fgpu_matrix* A, double* host, int nchunks) {
+// part_end of the space's plan, once
+int plan_parts(fgpu_ctx* ctx, fgpu_space* V) {
+    GatherPlan& G = V->plan;
+    if (G.part_end[3] >= 0) return FGPU_OK;
+    const DevPattern& P = *V->pattern;
+    int* lowest = nullptr;
+    FGPU_CUDA_CHECK(ctx, pool_malloc(ctx->stream, &lowest, 4 * sizeof(int)));
+    struct Free { int* p; ~Free() { pool_free(p); } } fr{lowest};
+    int h[4];
+    FGPU_CUDA_CHECK(ctx, cudaMemsetAsync(lowest, 0x7F, sizeof(h), ctx->stream));
+    const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((G.nslices * 32 + 255) / 256, (int64_t)sm_count(ctx) * 16));
+    part_rows_kernel<<<(int)blocks, 256, 0, ctx->stream>>>(G, P.d_ja, lowest);
+    ctx->launches++;
+    FGPU_CUDA_CHECK(ctx, cudaGetLastError());
+    FGPU_CUDA_CHECK(ctx, cudaMemcpyAsync(h, lowest, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
+    FGPU_CUDA_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
+    int64_t low = P.nrows;                       // the lowest row of the quarters after c
+    int64_t end[4];
+    end[3] = P.nnz;
+    for (int c = 2; c >= 0; --c) {
+        low = std::min<int64_t>(low, h[c + 1]);
+        FGPU_CUDA_CHECK(ctx, cudaMemcpyAsync(&end[c], P.d_ia + low, sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
+    }
+    FGPU_CUDA_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
+    for (int c = 0; c < 4; ++c) G.part_end[c] = end[c];
+    return FGPU_OK;
+}
+
+// Phase 2, then the values to the host. FP64 matrices. A gather that fits the device at once is followed by one
+// transfer: kernel stores where the buffer is page-locked and mapped, else the copy engine. Else the slices
+// run in quarters, and the rows that no later quarter writes to leave by the copy engine meanwhile: with dofs
+// numbered along the elements that is all but the last plane's. P2 64^3 (487 MB, 2.55 ms on the link) through
+// fgpu_assemble_matrix_host: 3.24 ms without the overlap, 2.99 with it; kernel stores beside the gather 3.8.
+int launch_gather_phase_to_host(fgpu_ctx* ctx, fgpu_matrix* A, double* host) {
     const int64_t nnz = A->pattern->nnz;
-    nchunks = std::max(1, std::min(nchunks, 4));
     if (!ctx->copy_streams[0]) {
         for (int i = 0; i < 4; ++i) FGPU_CUDA_CHECK(ctx, cudaStreamCreateWithFlags(&ctx->copy_streams[i], cudaStreamNonBlocking));
         for (int i = 0; i < 5; ++i) FGPU_CUDA_CHECK(ctx, cudaEventCreateWithFlags(&ctx->copy_events[i], cudaEventDisableTiming));
@@ -896,27 +938,52 @@ int launch_gather_phase_to_host(fgpu_ctx* ctx, fgpu_matrix* A, double* host, int
             return FGPU_ERR_INVALID;
         }
     }
-    int rc = launch_gather_phase(ctx, A, 0);
-    if (rc) return rc;
-    if (hdev) {
-        const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((nnz + 255) / 256, (int64_t)sm_count(ctx) * 32));
-        values_to_host_kernel<<<(int)blocks, 256, 0, ctx->stream>>>(nnz, (const double*)A->d_val, hdev);
-        ctx->launches++;
-        FGPU_CUDA_CHECK(ctx, cudaGetLastError());
-        FGPU_CUDA_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
-        return FGPU_OK;
+    fgpu_space* V = A->space;
+    const GatherPlan& G = V->plan;
+    int rc = FGPU_OK;
+    const bool whole = one_wave(ctx, G.nslices);
+    if (!whole && (rc = plan_parts(ctx, V))) return rc;
+    const int64_t q = (G.nslices + 3) / 4;
+    PendingEvent ev;
+    prof_begin(ctx, "assemble_gather", ev);
+    int64_t done = 0;
+    cudaError_t e = cudaSuccess;
+    for (int c = whole ? 3 : 0; c < 4; ++c) {
+        if (whole) {
+            launch_gather_slices(ctx, A, 256, 0, 8, 1, 0);
+        } else {
+            GatherPlan part = G;
+            part.nslices = std::max<int64_t>(0, std::min(G.nslices, (c + 1) * q) - c * q);
+            part.soff += c * q;
+            part.pos0 += c * q * 32;
+            part.pos1 += c * q * 32;
+            if (part.nslices > 0) launch_slices<kModeDF64, false>(ctx, A, part, 256, 0, 4, 0);
+        }
+        if (c > 0 && !whole) ctx->launches++;
+        if (e == cudaSuccess) e = cudaGetLastError();
+        if (e == cudaSuccess) e = cudaEventRecord(ctx->copy_events[c], ctx->stream);
+        const int64_t end = c == 3 ? nnz : G.part_end[c];
+        if (end <= done) continue;
+        const cudaStream_t cs = ctx->copy_streams[c];
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(cs, ctx->copy_events[c], 0);
+        if (e != cudaSuccess) break;
+        if (hdev && whole) {
+            const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((nnz + 255) / 256, (int64_t)sm_count(ctx) * 32));
+            values_to_host_kernel<<<(int)blocks, 256, 0, cs>>>(nnz, (const double*)A->d_val, hdev);
+            ctx->launches++;
+            e = cudaGetLastError();
+        } else {
+            e = cudaMemcpyAsync(host + done, (const double*)A->d_val + done, (end - done) * sizeof(double), cudaMemcpyDeviceToHost, cs);
+        }
+        done = end;
     }
-    const int64_t chunk = ((nnz + nchunks - 1) / nchunks + 255) & ~(int64_t)255;
-    FGPU_CUDA_CHECK(ctx, cudaEventRecord(ctx->copy_events[0], ctx->stream));
-    for (int c = 0; c < nchunks; ++c) {
-        const int64_t k0 = (int64_t)c * chunk;
-        if (k0 >= nnz) break;
-        const int64_t k1 = std::min(nnz, k0 + chunk);
-        FGPU_CUDA_CHECK(ctx, cudaStreamWaitEvent(ctx->copy_streams[c], ctx->copy_events[0], 0));
-        FGPU_CUDA_CHECK(ctx, cudaMemcpyAsync(host + k0, (const double*)A->d_val + k0, (k1 - k0) * sizeof(double),
-                                             cudaMemcpyDeviceToHost, ctx->copy_streams[c]));
+    prof_end(ctx, ev);
+    for (int c = 0; c < 4; ++c) {
+        const cudaError_t es = cudaStreamSynchronize(ctx->copy_streams[c]);
+        if (e == cudaSuccess) e = es;
     }
-    for (int c = 0; c < nchunks; ++c) FGPU_CUDA_CHECK(ctx, cudaStreamSynchronize(ctx->copy_streams[c]));
+    FGPU_CUDA_CHECK(ctx, e);
+    FGPU_CUDA_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
     return FGPU_OK;
 }
 
