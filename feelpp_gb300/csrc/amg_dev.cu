@@ -734,13 +734,18 @@ struct SpgemmArgs {
     int* status = nullptr;
 };
 
-__host__ __device__ constexpr int spgemm_cap(int tsize, int group) { return group <= 8 ? tsize - tsize / 4 : tsize / 2; }
+constexpr int kRankMax = 128;        // rows up to this long are sorted by counting smaller columns
+// The longest row that a table keeps; longer ones are listed for the next. Only a whole warp can sort more than
+// kRankMax columns (the bitonic sort).
+__host__ __device__ constexpr int spgemm_cap(int tsize, int group) {
+    const int c = group <= 8 ? tsize - tsize / 4 : tsize / 2;
+    return group == 32 || c <= kRankMax ? c : kRankMax;
+}
 int spgemm_warp_bytes(int tsize, int group, bool fill) {
     return tsize * (32 / group) * ((fill ? 8 : 0) + 4 + 2);
 }
 
 enum { kCount, kFill, kPadded };
-constexpr int kRankMax = 128;        // rows up to this long are sorted by counting smaller columns
 
 template <int G, int MODE>
 __global__ void __launch_bounds__(256) spgemm_kernel(SpgemmArgs g) {
@@ -749,6 +754,7 @@ __global__ void __launch_bounds__(256) spgemm_kernel(SpgemmArgs g) {
     constexpr bool FILL = MODE != kCount;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = lane & (G - 1), grp = lane / G;
     const unsigned gmask = G == 32 ? 0xffffffffu : ((1u << (G & 31)) - 1u) << (grp * G);
+    static_assert(G == 32 || spgemm_cap(kBins[kNumBins - 1], G) <= kRankMax, "a row that is counted has to be written");
     const int T = g.tsize, cap = spgemm_cap(T, G);
     unsigned char* base = sg_smem + (size_t)warp * g.wbytes;
     double* hv = reinterpret_cast<double*>(base) + grp;                                        // values
@@ -881,7 +887,7 @@ __global__ void __launch_bounds__(256) spgemm_kernel(SpgemmArgs g) {
                 g.oj[ob + rank] = key;
                 g.oa[ob + rank] = hv[s * NG];
             }
-        } else if (FILL && G == 32) {
+        } else if (FILL && G == 32) {        // (narrower groups keep no row above kRankMax)
             // bitonic sort of the used slots by key (padding last), then the row
             int P = 1;
             while (P < nuniq) P <<= 1;
