@@ -2,11 +2,13 @@
 //
 // A solve or an AMG set-up allocates and frees a few hundred work arrays; cudaMalloc and cudaFree take tens
 // of microseconds each (14 of the 52 ms of an AMG set-up and solve at P2 48^3), and cudaFree waits for the
-// device. Freed blocks are kept per stream instead and handed out again in stream order: a block freed while
-// its kernels are still queued on its stream is only reused by later work on the same stream. (Work on
-// another stream has to be joined before the block is freed.)
+// device. Freed blocks are kept per device and stream instead and handed out again in stream order: a block
+// freed while its kernels are still queued on its stream is only reused by later work on the same stream. (Work
+// on another stream has to be joined before the block is freed.) The handle alone does not name a stream:
+// cudaStreamLegacy is one handle for a stream of every device (the key holds the device), and cudaStreamPerThread
+// one for a stream of every thread (its blocks are not kept: any thread may free them).
 //
-// Bounded: at most a sixteenth of the device's memory is kept, the rest goes back to the driver at once; a
+// Bounded: at most a sixteenth of a device's memory is kept, the rest goes back to the driver at once; a
 // context gives its stream's blocks back when it is destroyed; and an allocation that fails, here or in
 // dev_malloc, is tried again after everything kept has been given back. Page-locked host blocks (a few
 // kilobytes for scalars that are read back) are kept in the same way, at most 1 MB. All functions may be
@@ -15,6 +17,7 @@
 #include <map>
 #include <mutex>
 #include <unordered_map>
+#include <utility>
 #include <vector>
 
 #include "fgpu_core.h"
@@ -23,15 +26,19 @@ namespace fgpu {
 
 namespace {
 
+typedef std::pair<int, cudaStream_t> Key;                                  // device, stream
 struct Block {
-    cudaStream_t stream;
+    Key key;
     size_t bytes;
+};
+struct Device {
+    size_t kept = 0, limit = 0;      // bytes
 };
 
 std::mutex g_mutex;
 std::unordered_map<void*, Block> g_live;                                   // handed out
-std::map<cudaStream_t, std::multimap<size_t, void*>> g_kept;               // free, per stream, by size
-size_t g_kept_bytes = 0, g_limit = 0;
+std::map<Key, std::multimap<size_t, void*>> g_kept;                        // free, by size
+std::map<int, Device> g_device;
 std::multimap<size_t, void*> g_pinned;                                     // free page-locked blocks
 std::unordered_map<void*, size_t> g_pinned_live;
 size_t g_pinned_bytes = 0;
@@ -41,14 +48,22 @@ void give_back(std::vector<void*>& blocks) {
     for (void* p : blocks) cudaFree(p);
 }
 
-// everything kept, out of the lists (the caller frees it without the lock)
-std::vector<void*> take_all() {
+int current_device() {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    return dev;
+}
+
+// everything kept on a device, out of the lists (the caller frees it without the lock)
+std::vector<void*> take_all(int dev) {
     std::vector<void*> out;
     std::lock_guard<std::mutex> lock(g_mutex);
-    for (auto& s : g_kept)
-        for (auto& b : s.second) out.push_back(b.second);
-    g_kept.clear();
-    g_kept_bytes = 0;
+    for (auto s = g_kept.begin(); s != g_kept.end();) {
+        if (s->first.first != dev) { ++s; continue; }
+        for (auto& b : s->second) out.push_back(b.second);
+        s = g_kept.erase(s);
+    }
+    g_device[dev].kept = 0;
     return out;
 }
 
@@ -57,7 +72,7 @@ std::vector<void*> take_all() {
 cudaError_t dev_malloc_bytes(void** p, size_t bytes) {
     cudaError_t e = cudaMalloc(p, bytes);
     if (e != cudaErrorMemoryAllocation) return e;
-    std::vector<void*> kept = take_all();
+    std::vector<void*> kept = take_all(current_device());
     if (kept.empty()) return e;
     cudaGetLastError();
     give_back(kept);
@@ -66,15 +81,17 @@ cudaError_t dev_malloc_bytes(void** p, size_t bytes) {
 
 cudaError_t pool_malloc_bytes(cudaStream_t stream, void** p, size_t bytes) {
     bytes = (std::max<size_t>(bytes, 1) + 511) & ~(size_t)511;
+    if (stream == cudaStreamPerThread) return dev_malloc_bytes(p, bytes);
+    const Key key(current_device(), stream);
     {
         std::lock_guard<std::mutex> lock(g_mutex);
-        auto s = g_kept.find(stream);
+        auto s = g_kept.find(key);
         if (s != g_kept.end()) {
             auto b = s->second.lower_bound(bytes);
             if (b != s->second.end() && b->first <= bytes + bytes / 4 + 4096) {      // little is wasted
                 *p = b->second;
-                g_live[*p] = Block{stream, b->first};
-                g_kept_bytes -= b->first;
+                g_live[*p] = Block{key, b->first};
+                g_device[key.first].kept -= b->first;
                 s->second.erase(b);
                 return cudaSuccess;
             }
@@ -83,7 +100,7 @@ cudaError_t pool_malloc_bytes(cudaStream_t stream, void** p, size_t bytes) {
     const cudaError_t e = dev_malloc_bytes(p, bytes);
     if (e == cudaSuccess) {
         std::lock_guard<std::mutex> lock(g_mutex);
-        g_live[*p] = Block{stream, bytes};
+        g_live[*p] = Block{key, bytes};
     }
     return e;
 }
@@ -94,15 +111,16 @@ cudaError_t pool_free(void* p) {
         std::lock_guard<std::mutex> lock(g_mutex);
         auto b = g_live.find(p);
         if (b != g_live.end()) {
-            if (g_limit == 0) {
-                size_t free_b = 0, total_b = 0;
-                g_limit = cudaMemGetInfo(&free_b, &total_b) == cudaSuccess ? std::max<size_t>(total_b / 16, 1) : 1;
-            }
             const Block blk = b->second;
             g_live.erase(b);
-            if (g_kept_bytes + blk.bytes <= g_limit) {
-                g_kept[blk.stream].emplace(blk.bytes, p);
-                g_kept_bytes += blk.bytes;
+            Device& d = g_device[blk.key.first];
+            if (d.limit == 0) {
+                cudaDeviceProp prop{};
+                d.limit = cudaGetDeviceProperties(&prop, blk.key.first) == cudaSuccess ? std::max<size_t>(prop.totalGlobalMem / 16, 1) : 1;
+            }
+            if (d.kept + blk.bytes <= d.limit) {
+                g_kept[blk.key].emplace(blk.bytes, p);
+                d.kept += blk.bytes;
                 return cudaSuccess;
             }
         }
@@ -115,16 +133,16 @@ void pool_release(cudaStream_t stream) {
     std::vector<void*> out;
     {
         std::lock_guard<std::mutex> lock(g_mutex);
-        auto s = g_kept.find(stream);
-        if (s != g_kept.end()) {
+        for (auto s = g_kept.begin(); s != g_kept.end();) {
+            if (s->first.second != stream) { ++s; continue; }
             for (auto& b : s->second) {
                 out.push_back(b.second);
-                g_kept_bytes -= b.first;
+                g_device[s->first.first].kept -= b.first;
             }
-            g_kept.erase(s);
+            s = g_kept.erase(s);
         }
         for (auto b = g_live.begin(); b != g_live.end();) {
-            if (b->second.stream == stream) b = g_live.erase(b);
+            if (b->second.key.second == stream) b = g_live.erase(b);
             else ++b;
         }
     }
