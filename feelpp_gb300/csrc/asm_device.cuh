@@ -51,6 +51,11 @@ __device__ __forceinline__ df df_dot3(df a0, df b0, df a1, df b1, df a2, df b2) 
     df_dot_term(a2, b2, s, e);
     return two_sum(s, e);
 }
+// DOT: the determinant and the metric as compensated dot products (fewer instructions, for the closed form of
+// closed.cuh, whose few terms keep the whole below the error of the sums over reference tensors); else as
+// renormalised double-float sums: a P3 entry adds 84 products of the record, and with compensated ones its
+// error was 6 % larger (P3 41x37x40 against binary64 1.17e-14 of the largest entry, here 1.11e-14).
+template <bool DOT = false>
 __device__ __forceinline__ void geometry_df_record(const GeoElem& g, const double* __restrict__ kappa, df kc, df mc, df ksc,
                                                    float4* __restrict__ o, int* __restrict__ status) {
     df K[9];
@@ -68,7 +73,11 @@ __device__ __forceinline__ void geometry_df_record(const GeoElem& g, const doubl
     C[6] = df_sub(df_mul(K[1], K[5]), df_mul(K[2], K[4]));
     C[7] = df_sub(df_mul(K[2], K[3]), df_mul(K[0], K[5]));
     C[8] = df_sub(df_mul(K[0], K[4]), df_mul(K[1], K[3]));
-    const df det = df_dot3(K[0], C[0], K[1], C[1], K[2], C[2]);
+    auto dot3 = [](df a0, df b0, df a1, df b1, df a2, df b2) {
+        if constexpr (DOT) return df_dot3(a0, b0, a1, b1, a2, b2);
+        else return df_add(df_add(df_mul(a0, b0), df_mul(a1, b1)), df_mul(a2, b2));
+    };
+    const df det = dot3(K[0], C[0], K[1], C[1], K[2], C[2]);
     const df J = det.hi < 0.0f ? df_neg(det) : det;
     if (!(J.hi > 0.0f) || !isfinite(J.hi)) atomicOr(status, kStatusBadElement);
     const df s = df_mul(df_mul(kappa ? d2df(g.kappa) : kc, ksc), df_recip(J));
@@ -76,7 +85,7 @@ __device__ __forceinline__ void geometry_df_record(const GeoElem& g, const doubl
     df c[8];
 #pragma unroll
     for (int k = 0; k < 6; ++k)
-        c[k] = df_mul(s, df_dot3(C[pa[k]], C[pb[k]], C[3 + pa[k]], C[3 + pb[k]], C[6 + pa[k]], C[6 + pb[k]]));
+        c[k] = df_mul(s, dot3(C[pa[k]], C[pb[k]], C[3 + pa[k]], C[3 + pb[k]], C[6 + pa[k]], C[6 + pb[k]]));
     c[6] = df_mul(mc, J);
     c[7] = J;
     o[0] = make_float4(c[0].hi, c[1].hi, c[2].hi, c[3].hi);
@@ -84,10 +93,11 @@ __device__ __forceinline__ void geometry_df_record(const GeoElem& g, const doubl
     o[2] = make_float4(c[0].lo, c[1].lo, c[2].lo, c[3].lo);
     o[3] = make_float4(c[4].lo, c[5].lo, c[6].lo, c[7].lo);
 }
+template <bool DOT = false>
 __device__ __forceinline__ void geometry_df_record(int64_t e, const double* __restrict__ xyz, const int32_t* __restrict__ tets,
                                                    const double* __restrict__ kappa, df kc, df mc, df ksc,
                                                    float4* __restrict__ o, int* __restrict__ status) {
-    geometry_df_record(geometry_load(e, xyz, tets, kappa), kappa, kc, mc, ksc, o, status);
+    geometry_df_record<DOT>(geometry_load(e, xyz, tets, kappa), kappa, kc, mc, ksc, o, status);
 }
 
 // Element-matrix entry K_e(i, j) = sum_k c_k T_k(i, j) (the 7 reference tensors

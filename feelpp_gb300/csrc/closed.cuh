@@ -157,7 +157,7 @@ __device__ __forceinline__ void closed_group(int64_t e0, int cnt, const GeoElem&
     V* st = reinterpret_cast<V*>(stage);
     V* out = reinterpret_cast<V*>(kbuf) + e0 * NTRI;
     float4 rec[4];
-    if (lane < cnt) geometry_df_record(in, kappa, kc, mc, ksc, rec, status);
+    if (lane < cnt) geometry_df_record<true>(in, kappa, kc, mc, ksc, rec, status);
     closed_stage_free();
     if (lane < cnt) {
         closed_entries<MODE, N>(rec, [&](auto I, V v) { st[lane * NTRI + decltype(I)::value] = v; });

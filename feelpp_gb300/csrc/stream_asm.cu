@@ -261,9 +261,11 @@ __global__ void __launch_bounds__(kThreads, 3) stream_assemble_kernel(StreamArgs
                                     : !ld_acquire(abort);
                 if (lane == 0) s_ok = ok;
             }
-            if (tid < cnt)
-                geometry_df_record(e0 + tid, a.xyz, a.tets, a.kappa, kc, mc, ksc, reinterpret_cast<float4*>(rec + 16 * tid),
-                                   a.status);
+            if (tid < cnt) {
+                float4* const r = reinterpret_cast<float4*>(rec + 16 * tid);
+                if (N <= 10 && a.closed) geometry_df_record<true>(e0 + tid, a.xyz, a.tets, a.kappa, kc, mc, ksc, r, a.status);
+                else geometry_df_record(e0 + tid, a.xyz, a.tets, a.kappa, kc, mc, ksc, r, a.status);
+            }
             __syncthreads();
             if (!s_ok) break;
             const int esub = lane / NTRI < EPW ? lane / NTRI : EPW;
