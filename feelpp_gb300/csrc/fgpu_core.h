@@ -14,13 +14,15 @@
 namespace fgpu {
 
 struct StreamPlan;                   // schedule of the streamed assembly (stream_asm.cu)
+constexpr int kHostParts = 12;
 struct GatherPlan {                  // two-phase gather map of a space, in slices of 32 sums (gather.cu)
     int64_t nslices = 0;
     uint32_t* pos0 = nullptr;        // slices x 32: CSR position of the sum (row <= column), 0xFFFFFFFF: none
     uint32_t* pos1 = nullptr;        // position of the transpose, 0xFFFFFFFF on the diagonal (not set where pos0 is none)
     uint32_t* soff = nullptr;        // slices + 1: first row of a slice in sidx
     uint32_t* sidx = nullptr;        // rows of 32 element-buffer indices, one row per step of a slice
-    int64_t part_end[4] = {-1, -1, -1, -1};   // CSR entries [0, part_end[c]) are complete after quarter c of the slices
+    int parts = 0;                   // transfers of the host assembly (0: not planned yet):
+    int64_t part_end[kHostParts] = {};   // CSR entries [0, part_end[c]) are complete after part c of the slices
 };
 void stream_plan_free(StreamPlan* p);
 

@@ -444,10 +444,10 @@ __global__ void __launch_bounds__(256) values_to_host_kernel(int64_t nnz, const 
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < nnz; k += (int64_t)gridDim.x * blockDim.x) hout[k] = val[k];
 }
 
-// lowest[c]: the lowest row that quarter c of the slices writes to (the row of a position is the column of its
+// lowest[c]: the lowest row that part c of the slices writes to (the row of a position is the column of its
 // transpose's)
-__global__ void __launch_bounds__(256) part_rows_kernel(GatherPlan G, const int32_t* __restrict__ ja, int* __restrict__ lowest) {
-    const int64_t q = (G.nslices + 3) / 4, n = G.nslices * 32;
+__global__ void __launch_bounds__(256) part_rows_kernel(GatherPlan G, int parts, const int32_t* __restrict__ ja, int* __restrict__ lowest) {
+    const int64_t q = (G.nslices + parts - 1) / parts, n = G.nslices * 32;
     for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x) {
         const uint32_t k0 = G.pos0[k], k1 = G.pos1[k];
         int r = k0 == kNoIndex ? INT_MAX : k1 == kNoIndex ? ja[k0] : min(ja[k0], ja[k1]);
@@ -926,103 +926,121 @@ int launch_gather_elasticity_fused(fgpu_ctx* ctx, const fgpu_matrix* A, double l
     return FGPU_OK;
 }
 
-// part_end of the space's plan, once
-int plan_parts(fgpu_ctx* ctx, fgpu_space* V) {
+// part_end of the space's plan, once. The ends are rounded down to whole lines of 512 bytes: a part that starts
+// anywhere makes partial writes of its stores to the host (P2 64^3 by kernel stores: 3.67 against 3.02 ms).
+int plan_parts(fgpu_ctx* ctx, fgpu_space* V, int parts) {
     GatherPlan& G = V->plan;
-    if (G.part_end[3] >= 0) return FGPU_OK;
+    if (G.parts == parts) return FGPU_OK;
     const DevPattern& P = *V->pattern;
     int* lowest = nullptr;
-    FGPU_CUDA_CHECK(ctx, pool_malloc(ctx->stream, &lowest, 4 * sizeof(int)));
+    FGPU_CUDA_CHECK(ctx, pool_malloc(ctx->stream, &lowest, kHostParts * sizeof(int)));
     struct Free { int* p; ~Free() { pool_free(p); } } fr{lowest};
-    int h[4];
+    int h[kHostParts];
     FGPU_CUDA_CHECK(ctx, cudaMemsetAsync(lowest, 0x7F, sizeof(h), ctx->stream));
     const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((G.nslices * 32 + 255) / 256, (int64_t)sm_count(ctx) * 16));
-    part_rows_kernel<<<(int)blocks, 256, 0, ctx->stream>>>(G, P.d_ja, lowest);
+    part_rows_kernel<<<(int)blocks, 256, 0, ctx->stream>>>(G, parts, P.d_ja, lowest);
     ctx->launches++;
     FGPU_CUDA_CHECK(ctx, cudaGetLastError());
     FGPU_CUDA_CHECK(ctx, cudaMemcpyAsync(h, lowest, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
     FGPU_CUDA_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
-    int64_t low = P.nrows;                       // the lowest row of the quarters after c
-    int64_t end[4];
-    end[3] = P.nnz;
-    for (int c = 2; c >= 0; --c) {
+    int64_t low = P.nrows;                       // the lowest row of the parts after c
+    int64_t end[kHostParts];
+    for (int c = parts - 2; c >= 0; --c) {
         low = std::min<int64_t>(low, h[c + 1]);
         FGPU_CUDA_CHECK(ctx, cudaMemcpyAsync(&end[c], P.d_ia + low, sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
     }
     FGPU_CUDA_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
-    for (int c = 0; c < 4; ++c) G.part_end[c] = end[c];
+    for (int c = 0; c + 1 < parts; ++c) G.part_end[c] = end[c] & ~(int64_t)63;
+    G.part_end[parts - 1] = P.nnz;
+    G.parts = parts;
     return FGPU_OK;
 }
 
-// Phase 2, then the values to the host. FP64 matrices. A gather that fits the device at once is followed by one
-// transfer: kernel stores where the buffer is page-locked and mapped, else the copy engine. Else the slices
-// run in quarters, and the rows that no later quarter writes to leave by the copy engine meanwhile: with dofs
-// numbered along the elements that is all but the last plane's. P2 64^3 (487 MB, 2.55 ms on the link) through
-// fgpu_assemble_matrix_host: 3.24 ms without the overlap, 2.99 with it; kernel stores beside the gather 3.8.
+// Phase 2, then the values to the host (FP64 matrices): the slices run in parts, and the rows that no later part
+// writes to leave meanwhile on a copy stream: with dofs numbered along the elements that is all but the last
+// plane's. By the copy engine, or (FGPU_HOST_TRANSFER_DIRECT) by kernel stores into a page-locked, mapped buffer.
+// Parts by the number of values: another part saves some of the gather's time and costs 5 to 10 us. Milliseconds
+// with 1 / 2 / 4 / 8 / 12 parts through fgpu_assemble_matrix_host: P1 20^3 (0.13 M values) 0.037 / 0.046 / 0.065 / -,
+// P2 14^3 (0.66 M) 0.070 / 0.067 / 0.075 / -, P2 20^3 (1.9 M) 0.124 / 0.126 / 0.128 / 0.135, P2 30^3 (6.3 M) 0.370 /
+// 0.353 / 0.344 / 0.347, P2 64^3 (61 M, 2.55 ms on the link) 3.19 / 3.01 / 2.92 / 2.88 / 2.88, P3 40^3 (85 M) 4.32 /
+// 4.09 / 3.96 / 3.90 / 3.89. On four copy streams in turn: P2 30^3 0.354, P2 20^3 0.134.
+// Kernel stores: 32 blocks beside the gather (P2 30^3 0.359, 64 blocks 0.371; P2 64^3 2.94 and 2.92), on four streams
+// in turn (on one, P2 64^3 3.07: a kernel's last stores run under the next one's), in one part up to 4 M values (P2
+// 14^3 0.069, two parts 0.077; P2 30^3 0.367, four 0.359).
+int host_parts(int64_t nnz, bool direct) {
+    return nnz < ((int64_t)1 << (direct ? 22 : 19)) ? 1 : nnz < ((int64_t)1 << 22) ? 2 : nnz < ((int64_t)24 << 20) ? 4 : kHostParts;
+}
+constexpr int64_t kDirectBlocks = 32;
 int launch_gather_phase_to_host(fgpu_ctx* ctx, fgpu_matrix* A, double* host) {
     const int64_t nnz = A->pattern->nnz;
-    if (!ctx->copy_streams[0]) {
-        for (int i = 0; i < 4; ++i) FGPU_CUDA_CHECK(ctx, cudaStreamCreateWithFlags(&ctx->copy_streams[i], cudaStreamNonBlocking));
-        for (int i = 0; i < 5; ++i) FGPU_CUDA_CHECK(ctx, cudaEventCreateWithFlags(&ctx->copy_events[i], cudaEventDisableTiming));
-    }
+    const bool direct = ctx->host_transfer == FGPU_HOST_TRANSFER_DIRECT;
     double* hdev = nullptr;
-    if (ctx->host_transfer != FGPU_HOST_TRANSFER_COPY) {
+    if (direct) {
         cudaPointerAttributes pa{};
         if (cudaPointerGetAttributes(&pa, host) == cudaSuccess && pa.type == cudaMemoryTypeHost && pa.devicePointer)
             hdev = static_cast<double*>(pa.devicePointer);
-        else
+        if (!hdev) {
             cudaGetLastError();
-        if (!hdev && ctx->host_transfer == FGPU_HOST_TRANSFER_DIRECT) {
             ctx->err = "direct host transfer: the host buffer is not page-locked and mapped";
             return FGPU_ERR_INVALID;
         }
     }
     fgpu_space* V = A->space;
+    const int parts = host_parts(nnz, direct);
+    auto transfer = [&](int64_t k0, int64_t k1, cudaStream_t st, int64_t max_blocks) -> cudaError_t {
+        if (!direct)
+            return cudaMemcpyAsync(host + k0, (const double*)A->d_val + k0, (k1 - k0) * sizeof(double), cudaMemcpyDeviceToHost, st);
+        const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((k1 - k0 + 255) / 256, max_blocks));
+        values_to_host_kernel<<<(int)blocks, 256, 0, st>>>(k1 - k0, (const double*)A->d_val + k0, hdev + k0);
+        ctx->launches++;
+        return cudaGetLastError();
+    };
+    if (parts == 1) {                            // (the caller synchronises)
+        const int rc = launch_gather_phase(ctx, A, 0);
+        if (rc) return rc;
+        FGPU_CUDA_CHECK(ctx, transfer(0, nnz, ctx->stream, (int64_t)sm_count(ctx) * 32));
+        return FGPU_OK;
+    }
+    if (!ctx->copy_streams[0]) {
+        for (int i = 0; i < 4; ++i) FGPU_CUDA_CHECK(ctx, cudaStreamCreateWithFlags(&ctx->copy_streams[i], cudaStreamNonBlocking));
+        for (int i = 0; i < 5; ++i) FGPU_CUDA_CHECK(ctx, cudaEventCreateWithFlags(&ctx->copy_events[i], cudaEventDisableTiming));
+    }
+    const int rc = plan_parts(ctx, V, parts);
+    if (rc) return rc;
     const GatherPlan& G = V->plan;
-    int rc = FGPU_OK;
-    const bool whole = one_wave(ctx, G.nslices);
-    if (!whole && (rc = plan_parts(ctx, V))) return rc;
-    const int64_t q = (G.nslices + 3) / 4;
+    const int64_t q = (G.nslices + parts - 1) / parts;
     PendingEvent ev;
     prof_begin(ctx, "assemble_gather", ev);
     int64_t done = 0;
     cudaError_t e = cudaSuccess;
-    for (int c = whole ? 3 : 0; c < 4; ++c) {
-        if (whole) {
-            launch_gather_slices(ctx, A, 256, 0, 8, 1, 0);
-        } else {
-            GatherPlan part = G;
-            part.nslices = std::max<int64_t>(0, std::min(G.nslices, (c + 1) * q) - c * q);
-            part.soff += c * q;
-            part.pos0 += c * q * 32;
-            part.pos1 += c * q * 32;
-            if (part.nslices > 0) launch_slices<kModeDF64, false>(ctx, A, part, 256, 0, 4, 0);
-        }
-        if (c > 0 && !whole) ctx->launches++;
-        if (e == cudaSuccess) e = cudaGetLastError();
-        if (e == cudaSuccess) e = cudaEventRecord(ctx->copy_events[c], ctx->stream);
-        const int64_t end = c == 3 ? nnz : G.part_end[c];
-        if (end <= done) continue;
-        const cudaStream_t cs = ctx->copy_streams[c];
-        if (e == cudaSuccess) e = cudaStreamWaitEvent(cs, ctx->copy_events[c], 0);
-        if (e != cudaSuccess) break;
-        if (hdev && whole) {
-            const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((nnz + 255) / 256, (int64_t)sm_count(ctx) * 32));
-            values_to_host_kernel<<<(int)blocks, 256, 0, cs>>>(nnz, (const double*)A->d_val, hdev);
-            ctx->launches++;
-            e = cudaGetLastError();
-        } else {
-            e = cudaMemcpyAsync(host + done, (const double*)A->d_val + done, (end - done) * sizeof(double), cudaMemcpyDeviceToHost, cs);
-        }
+    for (int c = 0; c < parts && e == cudaSuccess; ++c) {
+        GatherPlan part = G;
+        part.nslices = std::max<int64_t>(0, std::min(G.nslices, (c + 1) * q) - c * q);
+        part.soff += c * q;
+        part.pos0 += c * q * 32;
+        part.pos1 += c * q * 32;
+        if (part.nslices > 0) launch_slices<kModeDF64, false>(ctx, A, part, 256, 0, 4, 0);
+        if (c > 0) ctx->launches++;
+        e = cudaGetLastError();
+        const int64_t end = G.part_end[c];
+        if (end <= done || e != cudaSuccess) continue;
+        const cudaStream_t cs = ctx->copy_streams[direct ? c & 3 : 0];
+        // (the event is recorded again by the next part: a wait takes the record it finds)
+        e = cudaEventRecord(ctx->copy_events[4], ctx->stream);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(cs, ctx->copy_events[4], 0);
+        if (e == cudaSuccess) e = transfer(done, end, cs, kDirectBlocks);
         done = end;
     }
     prof_end(ctx, ev);
-    for (int c = 0; c < 4; ++c) {
-        const cudaError_t es = cudaStreamSynchronize(ctx->copy_streams[c]);
-        if (e == cudaSuccess) e = es;
+    // the context's stream waits for the copy streams: the caller's one wait covers all
+    const int used = direct ? 4 : 1;
+    for (int i = 0; i < used && e == cudaSuccess; ++i) {
+        e = cudaEventRecord(ctx->copy_events[i], ctx->copy_streams[i]);
+        if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->stream, ctx->copy_events[i], 0);
     }
+    if (e != cudaSuccess)
+        for (int i = 0; i < used; ++i) cudaStreamSynchronize(ctx->copy_streams[i]);
     FGPU_CUDA_CHECK(ctx, e);
-    FGPU_CUDA_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
     return FGPU_OK;
 }
 

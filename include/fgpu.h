@@ -65,10 +65,11 @@ extern "C" {
    256 entries, GATHER otherwise. A buffer it cannot allocate is an error (FGPU_ERR_ALLOC). */
 
 /* how fgpu_assemble_matrix_host moves the values to host memory */
-#define FGPU_HOST_TRANSFER_AUTO 0   /* DIRECT when the host buffer is page-locked and mapped, else COPY */
+#define FGPU_HOST_TRANSFER_AUTO 0   /* two-phase assembly: as COPY (the faster at every size measured); streamed: as
+                                       DIRECT when the buffer is page-locked and mapped, else COPY */
 #define FGPU_HOST_TRANSFER_COPY 1   /* copy-engine transfers of ranges of entries, overlapping the gather */
-#define FGPU_HOST_TRANSFER_DIRECT 2 /* page-locked buffers only: kernel stores of small matrices' values, and the
-                                       copy-engine ranges beside the gather of larger ones */
+#define FGPU_HOST_TRANSFER_DIRECT 2 /* a kernel stores each value to host memory, in the same ranges
+                                       (page-locked buffers only; over NVLink-C2C on Grace hosts) */
 
 #define FGPU_RANGE_ELEMENTS 0       /* _range=elements(mesh) */
 #define FGPU_RANGE_BOUNDARY_FACES 1 /* _range=boundaryfaces(mesh): faces of one element */
