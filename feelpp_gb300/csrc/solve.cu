@@ -252,8 +252,13 @@ __global__ void sell_values_kernel(int64_t nstored, const int32_t* __restrict__ 
 }
 
 // y = A x (mode 0) or y = b - A x (mode 1) on the SELL layout, one thread per row,
-// optional per-block partial of dot(w, y)
-template <class PL>
+// optional per-block partial of dot(w, y). AHEAD (FP64 values of matrices that do not stay in L2): the next
+// columns and values are loaded past L1 before this batch's gathers of x. FP64, us without / with, by the bytes of
+// columns and values: P1 64^3 48 MB 13.3 / 15.2, P2 28^3 62 MB 21.4 / 30.6, P3 17^3 79 MB 71.6 / 38.7, P2 32^3
+// 92 MB 35.9 / 33.4, P2 36^3 131 MB 66.9 / 46.1, P2 48^3 310 MB 123 / 94; with the other formats it costs more than
+// it gives (binary32 in L2: 19 us -> 29).
+constexpr int64_t kSellAheadBytes = (int64_t)70 << 20;
+template <class PL, bool AHEAD>
 __global__ void __launch_bounds__(256) sell_spmv_kernel(int64_t nrows, int64_t nslices, const int32_t* __restrict__ perm,
                                                        const int64_t* __restrict__ slice_ptr, const int32_t* __restrict__ slice_len,
                                                        const int32_t* __restrict__ col, const typename PL::V* __restrict__ val,
@@ -269,11 +274,9 @@ __global__ void __launch_bounds__(256) sell_spmv_kernel(int64_t nrows, int64_t n
         const int L = slice_len[s];
         const int64_t base = slice_ptr[s] + (i - s * kSellC);
         typename PL::D accd = PL::dzero();     // row sums in the dot-product type (see spmv_kernel)
-        // four entries' loads together, summed in entry order. FP64 values: the next columns and values are loaded
-        // past L1 before this batch's gathers of x (P2 48^3, 310 MB: 123 us -> 94; P2 34x30x33, in L2: 41 -> 35);
-        // with the other formats that costs more than it gives (binary32 in L2: 19 us -> 29).
+        // four entries' loads together, summed in entry order
         int k = 0;
-        if constexpr (std::is_same<typename PL::V, double>::value) {
+        if constexpr (AHEAD) {
             constexpr int U = 4;
             int32_t c[U];
             typename PL::V v[U];
@@ -360,12 +363,20 @@ struct SpmvPlan {
     void launch(cudaStream_t s, const fgpu_matrix* A, const typename PL::V* val, const typename PL::S* x, typename PL::S* y,
                 int mode, const typename PL::S* b, const typename PL::S* wdot, typename PL::D* partial,
                 const CGScalars<PL>* sc) const {
-        if (G == 0)
-            sell_spmv_kernel<PL><<<sell_blocks(*sell), 256, 0, s>>>(sell->nrows, sell->nslices, sell->d_perm, sell->d_slice_ptr,
-                                                                   sell->d_slice_len, sell->d_col, sval, x, y, mode, b, wdot,
-                                                                   partial, sc);
-        else
+        if (G == 0) {
+            if constexpr (std::is_same<typename PL::V, double>::value) {
+                if (sell->nstored * 12 > kSellAheadBytes) { launch_sell<true>(s, x, y, mode, b, wdot, partial, sc); return; }
+            }
+            launch_sell<false>(s, x, y, mode, b, wdot, partial, sc);
+        } else {
             launch_spmv_t<PL>(s, A, val, G, x, y, mode, b, wdot, partial, sc, spmv_blocks(A, G));
+        }
+    }
+    template <bool AHEAD>
+    void launch_sell(cudaStream_t s, const typename PL::S* x, typename PL::S* y, int mode, const typename PL::S* b,
+                     const typename PL::S* wdot, typename PL::D* partial, const CGScalars<PL>* sc) const {
+        sell_spmv_kernel<PL, AHEAD><<<sell_blocks(*sell), 256, 0, s>>>(sell->nrows, sell->nslices, sell->d_perm, sell->d_slice_ptr,
+                                                                     sell->d_slice_len, sell->d_col, sval, x, y, mode, b, wdot, partial, sc);
     }
     int blocks(const fgpu_matrix* A) const { return G == 0 ? sell_blocks(*sell) : spmv_blocks(A, G); }
 };
