@@ -346,8 +346,8 @@ static int sell_blocks(const SellLayout& L) {
 // SpMV autotuner for the CG: CSR with G lanes per row (G in 4, 8, 16, 32) or
 // the SELL layout, timed with CUDA events on the actual matrix (1 warm-up + 3
 // timed products per candidate) the first time a (device, number format, rows,
-// nonzeros) combination of 2^20 nonzeros or more is solved; the choice is cached
-// (0 = SELL, else G).
+// nonzeros) combination of 2^20 nonzeros or more (any, with a tuning file) is solved;
+// the choice is cached (0 = SELL, else G).
 // ---------------------------------------------------------------------------
 static std::mutex g_tune_mutex;
 static std::map<std::tuple<std::string, int, int, int64_t, int64_t>, int> g_spmv_tune;
@@ -396,13 +396,10 @@ static int plan_spmv(fgpu_ctx* ctx, const fgpu_matrix* A, const typename PL::V* 
     std::vector<int> tv;
     if (choice == -1 && tune_lookup(ctx->tune_file, skey, tv) && tv.size() == 1) choice = tv[0];
     if (choice == -1 && ctx->tune != 0) choice = spmv_group(A);
-    // Small matrices take the row-length rule: their candidates lie within a microsecond of one another (P1
-    // 16^3, 67 K entries: 3.7-4.2 us), so timing them (30 launches and a SELL layout in the first solve)
-    // would only make the summation order, and with it the last bits of the iterates, depend on noise.
-    if (choice == -1 && A->nnz < kSpmvTimedNnz) {
-        choice = spmv_group(A);
-        tune_record(ctx->tune_file, skey, {choice});
-    }
+    // Small matrices take the row-length rule: timing them (30 launches and a SELL layout in the first solve) would
+    // only make the summation order, and with it the last bits of the iterates, depend on noise. But a tuning file
+    // holds measured picks only: where one is named they are timed.
+    if (choice == -1 && A->nnz < kSpmvTimedNnz && ctx->tune_file.empty()) choice = spmv_group(A);
     // SELL layout and values (needed to time it, and to use it)
     bool have_sell = false;
     if (choice == -1 || choice == 0) {
