@@ -354,6 +354,26 @@ static std::map<std::tuple<std::string, int, int, int64_t, int64_t>, int> g_spmv
 
 static constexpr int64_t kSpmvTimedNnz = (int64_t)1 << 20;
 
+// Layout of matrices below kSpmvTimedNnz by their rows and mean row length, not by timing: 30 launches and a SELL
+// layout in the first solve would cost more than the solve, and the summation order, and with it the last bits of
+// the iterates, would depend on noise. As many lanes per row (16, 8, 4) as keep the lanes within 3200 (FP64; else
+// 6000) times the mean length: few long rows are a latency chain, many fill the device with four lanes. Rows of
+// up to 16 take four (a block's partial sum more in the update costs what eight gain), in numbers the SELL layout.
+// Products in us with 4 / 8 / 16 lanes / SELL, FP64: P1 8^3 3.2 /
+// 2.8 / 2.6 / 3.6, P1 16^3 3.8 / 3.7 / 4.4 / 4.6, P1 24^3 4.8 / 6.4 / 9.2 / 5.1, P1 28^3 5.4 / 7.6 / 11.6 / 4.8, P1
+// 40^3 10.7 / 16 / 22 / 5.3, P2 4^3 7.1 / 5.0 / 4.1 / 11.6, P2 8^3 6.7 / 4.8 / 4.7 / 10.7, P2 12^3 8.1 / 7.7 / 10 / 12,
+// P3 3^3 9.4 / 7.7 / 4.8 / 24, P3 6^3 10.2 / 8.2 / 5.8 / 25, P3 9^3 12.2 / 11.9 / 14.7 / 28; binary32 P1 16^3 2.9 / 2.8 /
+// 2.8 / 3.9, P1 34^3 4.1 / 5.3 / 7.4 / 4.1, P1 40^3 5.2 / 7.2 / 9.3 / 4.4, P2 12^3 5.9 / 4.6 / 4.9 / 9.6, P3 9^3 8.8 / 6.4 /
+// 6.7 / 21.
+template <class PL>
+static int spmv_small(const fgpu_matrix* A) {
+    const bool f64 = std::is_same<typename PL::V, double>::value;
+    const double rows = (double)std::max<int64_t>(A->nrows, 1), mean = (double)A->nnz / rows;
+    if (mean <= 16.0) return rows >= (f64 ? 20000.0 : 50000.0) ? 0 : 4;
+    const double lanes = (f64 ? 3200.0 : 6000.0) * mean / rows;
+    return lanes >= 16.0 ? 16 : lanes >= 8.0 ? 8 : 4;
+}
+
 template <class PL>
 struct SpmvPlan {
     int G = 4;                         // 0: SELL
@@ -396,10 +416,8 @@ static int plan_spmv(fgpu_ctx* ctx, const fgpu_matrix* A, const typename PL::V* 
     std::vector<int> tv;
     if (choice == -1 && tune_lookup(ctx->tune_file, skey, tv) && tv.size() == 1) choice = tv[0];
     if (choice == -1 && ctx->tune != 0) choice = spmv_group(A);
-    // Small matrices take the row-length rule: timing them (30 launches and a SELL layout in the first solve) would
-    // only make the summation order, and with it the last bits of the iterates, depend on noise. But a tuning file
-    // holds measured picks only: where one is named they are timed.
-    if (choice == -1 && A->nnz < kSpmvTimedNnz && ctx->tune_file.empty()) choice = spmv_group(A);
+    // a tuning file holds measured picks only: small matrices are timed where one is named, else take the rule
+    if (choice == -1 && A->nnz < kSpmvTimedNnz && ctx->tune_file.empty()) choice = spmv_small<PL>(A);
     // SELL layout and values (needed to time it, and to use it)
     bool have_sell = false;
     if (choice == -1 || choice == 0) {
