@@ -14,15 +14,17 @@
 namespace fgpu {
 
 struct StreamPlan;                   // schedule of the streamed assembly (stream_asm.cu)
-constexpr int kHostParts = 12;
-struct GatherPlan {                  // two-phase gather map of a space, in slices of 32 sums (gather.cu)
+struct GatherPlan {                  // two-phase gather map of a space, in slices of 32 sums (gather.cu); passed to the kernels
     int64_t nslices = 0;
     uint32_t* pos0 = nullptr;        // slices x 32: CSR position of the sum (row <= column), 0xFFFFFFFF: none
     uint32_t* pos1 = nullptr;        // position of the transpose, 0xFFFFFFFF on the diagonal (not set where pos0 is none)
     uint32_t* soff = nullptr;        // slices + 1: first row of a slice in sidx
     uint32_t* sidx = nullptr;        // rows of 32 element-buffer indices, one row per step of a slice
-    int parts = 0;                   // transfers of the host assembly (0: not planned yet):
-    int64_t part_end[kHostParts] = {};   // CSR entries [0, part_end[c]) are complete after part c of the slices
+};
+constexpr int kHostParts = 12;
+struct HostParts {                   // transfers of the host assembly (0: not planned yet)
+    int count = 0;
+    int64_t end[kHostParts] = {};    // CSR entries [0, end[c]) are complete after part c of the slices
 };
 void stream_plan_free(StreamPlan* p);
 
@@ -319,6 +321,7 @@ struct fgpu_space {
     double bnd_xmax = 0;
     uint64_t bnd_coords = 0;
     fgpu::GatherPlan plan;           // two-phase gather map (built on first use)
+    fgpu::HostParts host_parts;
     fgpu::StreamPlan* stream_plan = nullptr;   // streamed assembly: task order and waits (built on first use)
 };
 

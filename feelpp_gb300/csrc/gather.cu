@@ -926,11 +926,12 @@ int launch_gather_elasticity_fused(fgpu_ctx* ctx, const fgpu_matrix* A, double l
     return FGPU_OK;
 }
 
-// part_end of the space's plan, once. The ends are rounded down to whole lines of 512 bytes: a part that starts
+// The host assembly's parts, once per space. The ends are rounded down to whole lines of 512 bytes: a part that starts
 // anywhere makes partial writes of its stores to the host (P2 64^3 by kernel stores: 3.67 against 3.02 ms).
 int plan_parts(fgpu_ctx* ctx, fgpu_space* V, int parts) {
-    GatherPlan& G = V->plan;
-    if (G.parts == parts) return FGPU_OK;
+    const GatherPlan& G = V->plan;
+    HostParts& H = V->host_parts;
+    if (H.count == parts) return FGPU_OK;
     const DevPattern& P = *V->pattern;
     int* lowest = nullptr;
     FGPU_CUDA_CHECK(ctx, pool_malloc(ctx->stream, &lowest, kHostParts * sizeof(int)));
@@ -950,9 +951,9 @@ int plan_parts(fgpu_ctx* ctx, fgpu_space* V, int parts) {
         FGPU_CUDA_CHECK(ctx, cudaMemcpyAsync(&end[c], P.d_ia + low, sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
     }
     FGPU_CUDA_CHECK(ctx, cudaStreamSynchronize(ctx->stream));
-    for (int c = 0; c + 1 < parts; ++c) G.part_end[c] = end[c] & ~(int64_t)63;
-    G.part_end[parts - 1] = P.nnz;
-    G.parts = parts;
+    for (int c = 0; c + 1 < parts; ++c) H.end[c] = end[c] & ~(int64_t)63;
+    H.end[parts - 1] = P.nnz;
+    H.count = parts;
     return FGPU_OK;
 }
 
@@ -1022,7 +1023,7 @@ int launch_gather_phase_to_host(fgpu_ctx* ctx, fgpu_matrix* A, double* host) {
         if (part.nslices > 0) launch_slices<kModeDF64, false>(ctx, A, part, 256, 0, 4, 0);
         if (c > 0) ctx->launches++;
         e = cudaGetLastError();
-        const int64_t end = G.part_end[c];
+        const int64_t end = V->host_parts.end[c];
         if (end <= done || e != cudaSuccess) continue;
         const cudaStream_t cs = ctx->copy_streams[direct ? c & 3 : 0];
         // (the event is recorded again by the next part: a wait takes the record it finds)
