@@ -46,13 +46,17 @@ constexpr uint32_t kNoIndex = 0xFFFFFFFFu;
 // Sum of the lane's contributions in steps r0 .. r1 - 1 of its slice, B steps' loads together; PIPE: the
 // next batch's indices travel with this batch's values. df64: compensated sum in element order, the high
 // parts through TwoSum, their rounding errors and the low parts in one binary32 accumulator, normalised
-// once by the caller (error ~ (count) u^2 |sum|). binary32: a plain sum.
+// once by the caller (error ~ (count) u^2 |sum|). binary32: a plain sum from -0 with -0 for absent terms, which
+// changes no value and no sign; without a test per term the whole batch is loads and additions (P2 48^3 gather 117
+// -> 114 us, P3 28^3 114 -> 105).
 template <int MODE, int B, bool PIPE>
 __device__ __forceinline__ float2 slice_sum(uint32_t r0, uint32_t r1, int lane, const uint32_t* __restrict__ sidx,
                                             const void* __restrict__ kbuf) {
     typedef typename std::conditional<MODE == kModeDF64, float2, float>::type V;
     const V* kb = reinterpret_cast<const V*>(kbuf);
-    float sh = 0.0f, sl = 0.0f;
+    float sh = MODE == kModeDF64 ? 0.0f : -0.0f, sl = 0.0f;
+    V none{};
+    if constexpr (MODE == kModeF32) none = -0.0f;
     uint32_t ix[B];
     if (PIPE) {
 #pragma unroll
@@ -65,69 +69,74 @@ __device__ __forceinline__ float2 slice_sum(uint32_t r0, uint32_t r1, int lane, 
             for (int u = 0; u < B; ++u) ix[u] = r + u < r1 ? __ldg(sidx + (size_t)(r + u) * 32 + lane) : kNoIndex;
         }
 #pragma unroll
-        for (int u = 0; u < B; ++u) v[u] = ix[u] != kNoIndex ? __ldg(kb + ix[u]) : V{};
+        for (int u = 0; u < B; ++u) v[u] = ix[u] != kNoIndex ? __ldg(kb + ix[u]) : none;
         if (PIPE && r + B < r1) {
 #pragma unroll
             for (int u = 0; u < B; ++u) ix[u] = r + B + u < r1 ? __ldg(sidx + (size_t)(r + B + u) * 32 + lane) : kNoIndex;
         }
 #pragma unroll
-        for (int u = 0; u < B; ++u)
-            if (r + u < r1) {
-                if constexpr (MODE == kModeDF64) {
-                    const df t = two_sum(sh, v[u].x);
-                    sh = t.hi;
-                    sl = f_add(sl, f_add(t.lo, v[u].y));
-                } else {
-                    sh = r + u == r0 ? v[u] : f_add(sh, v[u]);
-                }
+        for (int u = 0; u < B; ++u) {
+            if constexpr (MODE == kModeF32) {
+                sh = f_add(sh, v[u]);
+            } else if (r + u < r1) {
+                const df t = two_sum(sh, v[u].x);
+                sh = t.hi;
+                sl = f_add(sl, f_add(t.lo, v[u].y));
             }
+        }
     }
     return make_float2(sh, sl);
 }
 
-template <int MODE>
-__device__ __forceinline__ void store_sum(float2 v, void* __restrict__ valv, uint32_t k0, uint32_t k1, int accumulate) {
-    if (MODE == kModeDF64) {
-        double* val = reinterpret_cast<double*>(valv);
+template <int MODE, bool ACC, class T>
+__device__ __forceinline__ void store_sum(float2 v, T* __restrict__ val, uint32_t k0, uint32_t k1, T o0, T o1) {
+    if constexpr (MODE == kModeDF64) {
         const df s = two_sum(v.x, v.y);
-        if (accumulate) {
-            val[k0] = df2d(df_add(d2df(val[k0]), s));
-            if (k1 != kNoIndex) val[k1] = df2d(df_add(d2df(val[k1]), s));
+        if (ACC) {
+            val[k0] = df2d(df_add(d2df(o0), s));
+            if (k1 != kNoIndex) val[k1] = df2d(df_add(d2df(o1), s));
         } else {
             const double r = df2d(s);
             val[k0] = r;
             if (k1 != kNoIndex) val[k1] = r;
         }
     } else {
-        float* val = reinterpret_cast<float*>(valv);
-        val[k0] = accumulate ? f_add(val[k0], v.x) : v.x;
-        if (k1 != kNoIndex) val[k1] = accumulate ? f_add(val[k1], v.x) : v.x;
+        val[k0] = ACC ? f_add(o0, v.x) : v.x;
+        if (k1 != kNoIndex) val[k1] = ACC ? f_add(o1, v.x) : v.x;
     }
 }
 
-// one slice per warp
-template <int MODE, int B, bool PIPE>
-__device__ __forceinline__ void gather_slice(const GatherPlan& G, int64_t s, const void* __restrict__ kbuf, void* __restrict__ valv,
-                                             int accumulate) {
+// one slice per warp; ACC: added to the values, which are loaded before the sum (a load after it would be one more
+// round trip to memory at the end of the chain)
+template <int MODE, int B, bool PIPE, bool ACC>
+__device__ __forceinline__ void gather_slice(const GatherPlan& G, int64_t s, const void* __restrict__ kbuf, void* __restrict__ valv) {
+    typedef typename std::conditional<MODE == kModeDF64, double, float>::type T;
+    T* const val = reinterpret_cast<T*>(valv);
     const int lane = threadIdx.x & 31;
     const uint32_t r0 = __ldg(G.soff + s), r1 = __ldg(G.soff + s + 1);
     const uint32_t k0 = __ldg(G.pos0 + s * 32 + lane), k1 = __ldg(G.pos1 + s * 32 + lane);
+    T o0 = 0, o1 = 0;
+    if constexpr (ACC) {
+        if (k0 != kNoIndex) {
+            o0 = val[k0];
+            if (k1 != kNoIndex) o1 = val[k1];
+        }
+    }
     const float2 v = slice_sum<MODE, B, PIPE>(r0, r1, lane, G.sidx, kbuf);
-    if (k0 != kNoIndex) store_sum<MODE>(v, valv, k0, k1, accumulate);
+    if (k0 != kNoIndex) store_sum<MODE, ACC>(v, val, k0, k1, o0, o1);
 }
 
-template <int MODE, int B, bool PIPE>
-__global__ void __launch_bounds__(256) gather_slices_kernel(GatherPlan G, const void* __restrict__ kbuf, void* __restrict__ valv,
-                                                            int accumulate) {
+template <int MODE, int B, bool PIPE, bool ACC>
+__global__ void __launch_bounds__(256) gather_slices_kernel(GatherPlan G, const void* __restrict__ kbuf, void* __restrict__ valv) {
     const int64_t nw = (int64_t)gridDim.x * (blockDim.x >> 5);
     for (int64_t s = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); s < G.nslices; s += nw)
-        gather_slice<MODE, B, PIPE>(G, s, kbuf, valv, accumulate);
+        gather_slice<MODE, B, PIPE, ACC>(G, s, kbuf, valv);
 }
 
 // the slices of all problems of a batch (slice_off: prefix sums of their slice counts)
-template <int MODE, bool PIPE>
+template <int MODE, bool PIPE, bool ACC>
 __global__ void __launch_bounds__(256) batch_gather_slices_kernel(int nprob, const BatchProblem* __restrict__ probs,
-                                                                  const int64_t* __restrict__ slice_off, int64_t total, int accumulate) {
+                                                                  const int64_t* __restrict__ slice_off, int64_t total) {
     const int64_t s = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (s >= total) return;
     int lo = 0, hi = nprob - 1;
@@ -137,27 +146,33 @@ __global__ void __launch_bounds__(256) batch_gather_slices_kernel(int nprob, con
         else hi = mid - 1;
     }
     const BatchProblem& P = probs[lo];
-    gather_slice<MODE, PIPE ? 8 : 4, PIPE>(P.plan, s - slice_off[lo], P.kbuf, P.val, accumulate);
+    gather_slice<MODE, PIPE ? 8 : 4, PIPE, ACC>(P.plan, s - slice_off[lo], P.kbuf, P.val);
 }
 
 // a pair's block at its position k0 of the scalar pattern and its transpose at k1 (x: the values, acc: the same
-// as double-float)
-template <int MODE, class T>
+// as double-float). ACC: added to the nine values of a block, loaded together (a load, a sum and a store in turn
+// are nine round trips to memory one after another).
+template <int MODE, bool ACC, class T>
 __device__ __forceinline__ void elasticity_store(T* __restrict__ val, const int64_t* __restrict__ sia, const int32_t* __restrict__ ja,
-                                                 uint32_t k0, uint32_t k1, const T (&x)[9], const df (&acc)[9], int accumulate) {
+                                                 uint32_t k0, uint32_t k1, const T (&x)[9], const df (&acc)[9]) {
     auto put = [&](uint32_t k, int32_t row, bool tr) {
         const int64_t s0 = sia[row];
         const int64_t len = sia[row + 1] - s0;
         T* const out = val + 9 * s0 + 3 * ((int64_t)k - s0);
+        T old[9];
+        if (ACC) {
+#pragma unroll
+            for (int q = 0; q < 9; ++q) old[q] = out[(q / 3) * 3 * len + q % 3];
+        }
 #pragma unroll
         for (int c = 0; c < 3; ++c)
 #pragma unroll
             for (int d = 0; d < 3; ++d) {
                 T* const o = out + c * 3 * len + d;
                 const int q = tr ? d * 3 + c : c * 3 + d;
-                if (!accumulate) *o = x[q];
-                else if constexpr (MODE == kModeDF64) *o = df2d(df_add(d2df(*o), acc[q]));
-                else *o = f_add(*o, x[q]);
+                if constexpr (!ACC) *o = x[q];
+                else if constexpr (MODE == kModeDF64) *o = df2d(df_add(d2df(old[c * 3 + d]), acc[q]));
+                else *o = f_add(old[c * 3 + d], x[q]);
             }
     };
     const int32_t j = __ldg(ja + k0), i = k1 == kNoIndex ? j : __ldg(ja + k1);
@@ -168,10 +183,10 @@ __device__ __forceinline__ void elasticity_store(T* __restrict__ val, const int6
 // Vector elasticity: one lane per pair of nodes i <= j, its 3x3 block (row 3i+c, columns 3j+d) summed
 // over the contributions in element order (bit 31 of an index: stored as (j, i), read transposed) and
 // stored with its transpose at (j, i). sia, ja: the scalar pattern.
-template <int MODE, int B>
+template <int MODE, int B, bool ACC>
 __global__ void __launch_bounds__(128) gather_elasticity_slices_kernel(GatherPlan G, const int64_t* __restrict__ sia,
                                                                        const int32_t* __restrict__ ja, const void* __restrict__ kbuf,
-                                                                       void* __restrict__ valv, int accumulate) {
+                                                                       void* __restrict__ valv) {
     typedef typename std::conditional<MODE == kModeDF64, float2, float>::type V;
     const int lane = threadIdx.x & 31;
     const int64_t s = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -221,7 +236,7 @@ __global__ void __launch_bounds__(128) gather_elasticity_slices_kernel(GatherPla
         if constexpr (MODE == kModeDF64) x[k] = df2d(acc[k]);
         else x[k] = acc[k].hi;
     }
-    elasticity_store<MODE>(val, sia, ja, k0, k1, x, acc, accumulate);
+    elasticity_store<MODE, ACC>(val, sia, ja, k0, k1, x, acc);
 }
 
 // ---- vector elasticity without an element buffer ----
@@ -317,10 +332,10 @@ __device__ __forceinline__ const PairTable<N>& pair_table() {
 // 36x28x30 in double-float: geometry 25, element blocks 413, gather 378 us -> vectors 15 and here 337; a pass
 // 821 -> 372 us, P1 45^3 1070 -> 164 us, binary32 P2 20^3 193 -> 89 us. Error against
 // binary64 5.7e-15 -> 5.1e-15.
-template <int MODE, int N, int B>
+template <int MODE, int N, int B, bool ACC>
 __global__ void __launch_bounds__(64, 16) gather_elasticity_fused_kernel(GatherPlan G, const int64_t* __restrict__ sia,
                                                                       const int32_t* __restrict__ ja, const float4* __restrict__ rec,
-                                                                      double lam, double mu, void* __restrict__ valv, int accumulate) {
+                                                                      double lam, double mu, void* __restrict__ valv) {
     constexpr int NTRI = N * (N + 1) / 2;
     const PairTable<N>& pairs = pair_table<N>();
     const int lane = threadIdx.x & 31;
@@ -436,7 +451,7 @@ __global__ void __launch_bounds__(64, 16) gather_elasticity_fused_kernel(GatherP
                 acc[c * 3 + d] = df{v, 0.0f};
             }
     }
-    elasticity_store<MODE>(val, sia, ja, k0, k1, x, acc, accumulate);
+    elasticity_store<MODE, ACC>(val, sia, ja, k0, k1, x, acc);
 }
 
 // the values of the matrix to a mapped page-locked host buffer
@@ -743,14 +758,14 @@ void launch_walk(fgpu_ctx* ctx, int blocks, const PlanIn& in, uint16_t* first, c
     plan_walk_kernel<FILL, 2><<<blocks, 256, 0, ctx->stream>>>(in, first, slice0, soff, pos0, pos1, sidx, ctx->d_status);
 }
 
-template <int MODE, bool PIPE>
-void launch_slices(fgpu_ctx* ctx, const fgpu_matrix* A, const GatherPlan& G, int threads, int bpsm, int batch, int accumulate) {
+template <int MODE, bool PIPE, bool ACC>
+void launch_slices(fgpu_ctx* ctx, const fgpu_matrix* A, const GatherPlan& G, int threads, int bpsm, int batch) {
     const int64_t need = (G.nslices + threads / 32 - 1) / (threads / 32);
     const int blocks = (int)std::max<int64_t>(1, bpsm > 0 ? std::min<int64_t>(need, (int64_t)sm_count(ctx) * bpsm) : need);
     switch (batch) {
-        case 2: gather_slices_kernel<MODE, 2, PIPE><<<blocks, threads, 0, ctx->stream>>>(G, A->d_kbuf, A->d_val, accumulate); break;
-        case 8: gather_slices_kernel<MODE, 8, PIPE><<<blocks, threads, 0, ctx->stream>>>(G, A->d_kbuf, A->d_val, accumulate); break;
-        default: gather_slices_kernel<MODE, 4, PIPE><<<blocks, threads, 0, ctx->stream>>>(G, A->d_kbuf, A->d_val, accumulate); break;
+        case 2: gather_slices_kernel<MODE, 2, PIPE, ACC><<<blocks, threads, 0, ctx->stream>>>(G, A->d_kbuf, A->d_val); break;
+        case 8: gather_slices_kernel<MODE, 8, PIPE, ACC><<<blocks, threads, 0, ctx->stream>>>(G, A->d_kbuf, A->d_val); break;
+        default: gather_slices_kernel<MODE, 4, PIPE, ACC><<<blocks, threads, 0, ctx->stream>>>(G, A->d_kbuf, A->d_val); break;
     }
 }
 
@@ -861,13 +876,24 @@ int launch_build_gather_map(fgpu_ctx* ctx, fgpu_space* V) {
 }
 
 void launch_gather_slices(fgpu_ctx* ctx, const fgpu_matrix* A, int threads, int bpsm, int batch, int pipe, int accumulate) {
-    if (A->precision == FGPU_F32) {
-        if (pipe) launch_slices<kModeF32, true>(ctx, A, A->space->plan, threads, bpsm, batch, accumulate);
-        else launch_slices<kModeF32, false>(ctx, A, A->space->plan, threads, bpsm, batch, accumulate);
-    } else {
-        if (pipe) launch_slices<kModeDF64, true>(ctx, A, A->space->plan, threads, bpsm, batch, accumulate);
-        else launch_slices<kModeDF64, false>(ctx, A, A->space->plan, threads, bpsm, batch, accumulate);
+    const GatherPlan& G = A->space->plan;
+    if (accumulate) {                // (the shapes are timed on plain assemblies)
+        pipe = one_wave(ctx, G.nslices);
+        threads = 256;
+        bpsm = 0;
+        batch = pipe ? 8 : 4;
     }
+#define SLICES(MODE, PIPE)                                                             \
+    do {                                                                               \
+        if (accumulate) launch_slices<MODE, PIPE, true>(ctx, A, G, threads, bpsm, batch);  \
+        else launch_slices<MODE, PIPE, false>(ctx, A, G, threads, bpsm, batch);            \
+    } while (0)
+    if (A->precision == FGPU_F32) {
+        if (pipe) SLICES(kModeF32, true); else SLICES(kModeF32, false);
+    } else {
+        if (pipe) SLICES(kModeDF64, true); else SLICES(kModeDF64, false);
+    }
+#undef SLICES
 }
 
 int launch_gather_phase(fgpu_ctx* ctx, fgpu_matrix* A, int accumulate) {
@@ -888,7 +914,11 @@ int launch_gather_elasticity(fgpu_ctx* ctx, const fgpu_matrix* A, int accumulate
     prof_begin(ctx, "assemble_gather_elasticity", ev);
     // two blocks in flight per lane (P2 36x28x30: 0.378 ms, 0.635 one at a time); six where every slice is
     // resident and the longest chain, a vertex's 24 blocks, is what counts (P1 8^3: 48 against 56 us a pass)
-#define EL_GATHER(MODE, B) gather_elasticity_slices_kernel<MODE, B><<<blocks, 128, 0, ctx->stream>>>(G, P.d_ia, P.d_ja, A->d_kbuf, A->d_val, accumulate)
+#define EL_GATHER(MODE, B)                                                                                                 \
+    do {                                                                                                                   \
+        if (accumulate) gather_elasticity_slices_kernel<MODE, B, true><<<blocks, 128, 0, ctx->stream>>>(G, P.d_ia, P.d_ja, A->d_kbuf, A->d_val);  \
+        else gather_elasticity_slices_kernel<MODE, B, false><<<blocks, 128, 0, ctx->stream>>>(G, P.d_ia, P.d_ja, A->d_kbuf, A->d_val);            \
+    } while (0)
     if (one_wave(ctx, G.nslices)) {
         if (A->precision == FGPU_F32) EL_GATHER(kModeF32, 6); else EL_GATHER(kModeDF64, 6);
     } else {
@@ -917,7 +947,11 @@ int launch_gather_elasticity_fused(fgpu_ctx* ctx, const fgpu_matrix* A, double l
     FGPU_CUDA_CHECK(ctx, cudaGetLastError());
     const int blocks = (int)std::max<int64_t>(1, (G.nslices + 1) / 2);
     prof_begin(ctx, "assemble_gather_elasticity", ev);
-#define EL_GATHER(MODE, N, B) gather_elasticity_fused_kernel<MODE, N, B><<<blocks, 64, 0, ctx->stream>>>(G, P.d_ia, P.d_ja, rec, lam, mu, A->d_val, accumulate)
+#define EL_GATHER(MODE, N, B)                                                                                              \
+    do {                                                                                                                   \
+        if (accumulate) gather_elasticity_fused_kernel<MODE, N, B, true><<<blocks, 64, 0, ctx->stream>>>(G, P.d_ia, P.d_ja, rec, lam, mu, A->d_val);  \
+        else gather_elasticity_fused_kernel<MODE, N, B, false><<<blocks, 64, 0, ctx->stream>>>(G, P.d_ia, P.d_ja, rec, lam, mu, A->d_val);            \
+    } while (0)
     if (p2) { if (f32) EL_GATHER(kModeF32, 10, 2); else EL_GATHER(kModeDF64, 10, 1); }
     else { if (f32) EL_GATHER(kModeF32, 4, 4); else EL_GATHER(kModeDF64, 4, 2); }
 #undef EL_GATHER
@@ -1020,7 +1054,7 @@ int launch_gather_phase_to_host(fgpu_ctx* ctx, fgpu_matrix* A, double* host) {
         part.soff += c * q;
         part.pos0 += c * q * 32;
         part.pos1 += c * q * 32;
-        if (part.nslices > 0) launch_slices<kModeDF64, false>(ctx, A, part, 256, 0, 4, 0);
+        if (part.nslices > 0) launch_slices<kModeDF64, false, false>(ctx, A, part, 256, 0, 4);
         if (c > 0) ctx->launches++;
         e = cudaGetLastError();
         const int64_t end = V->host_parts.end[c];
@@ -1050,7 +1084,11 @@ int launch_batch_gather_slices(fgpu_ctx* ctx, int nprob, const BatchProblem* d_p
     const int blocks = (int)std::max<int64_t>(1, (total_slices + threads / 32 - 1) / (threads / 32));
     PendingEvent ev;
     prof_begin(ctx, "batch_gather", ev);
-#define BATCH_GATHER(MODE, PIPE) batch_gather_slices_kernel<MODE, PIPE><<<blocks, threads, 0, ctx->stream>>>(nprob, d_probs, d_slice_off, total_slices, accumulate)
+#define BATCH_GATHER(MODE, PIPE)                                                                                          \
+    do {                                                                                                                  \
+        if (accumulate) batch_gather_slices_kernel<MODE, PIPE, true><<<blocks, threads, 0, ctx->stream>>>(nprob, d_probs, d_slice_off, total_slices);  \
+        else batch_gather_slices_kernel<MODE, PIPE, false><<<blocks, threads, 0, ctx->stream>>>(nprob, d_probs, d_slice_off, total_slices);            \
+    } while (0)
     if (one_wave(ctx, total_slices)) {
         if (f32) BATCH_GATHER(kModeF32, true); else BATCH_GATHER(kModeDF64, true);
     } else {
