@@ -587,8 +587,8 @@ int fgpu_matrix_destroy(fgpu_matrix* A) {
 // has a position table (pattern rows of at most 256 entries), the fused gather
 // otherwise. A buffer the chosen path cannot allocate is an error. (The
 // streamed assembly gives the two-phase bits with a third of the memory
-// traffic, but measured slower at P2/P3 64^3: 2.10 against 1.14 ms, 11.7
-// against 4.3 ms; it is latency- and issue-bound, so it is not the default.)
+// traffic, but measured slower at P2 64^3: 1.38 against 0.59 ms (P3 28^3 0.95
+// against 0.30); it is latency- and issue-bound, so it is not the default.)
 // ---------------------------------------------------------------------------
 static int auto_assembly_algo(const fgpu_matrix* A, int kind) {
     (void)kind;

@@ -118,21 +118,13 @@ DevTables* get_dev_tables(int order, int qdeg, std::string& err) {
         T7l[k] = (float)(R.T7[k] - (double)T7h[k]);
     }
     const int n = R.n, ntri = n * (n + 1) / 2;
-    std::vector<float> T7th((size_t)7 * ntri), T7tl((size_t)7 * ntri);
-    std::vector<uint16_t> tri((size_t)n * n);
-    for (int i = 0, t = 0; i < n; ++i)
-        for (int j = i; j < n; ++j, ++t) {
-            tri[(size_t)i * n + j] = tri[(size_t)j * n + i] = (uint16_t)t;
-            for (int k = 0; k < 7; ++k) {
-                T7th[(size_t)k * ntri + t] = T7h[((size_t)k * n + i) * n + j];
-                T7tl[(size_t)k * ntri + t] = T7l[((size_t)k * n + i) * n + j];
-            }
-        }
     // the two-phase element buffer's order
     const std::vector<uint16_t> pairs = entry_order(4, order, n);
     std::vector<float> T7bh((size_t)7 * ntri), T7bl((size_t)7 * ntri), Sbh((size_t)9 * ntri), Sbl((size_t)9 * ntri);
+    std::vector<uint16_t> tri((size_t)n * n);
     for (int t = 0; t < ntri; ++t) {
         const size_t ij = (size_t)(pairs[t] >> 8) * n + (pairs[t] & 255);
+        tri[ij] = tri[(size_t)(pairs[t] & 255) * n + (pairs[t] >> 8)] = (uint16_t)t;
         for (int k = 0; k < 7; ++k) {
             T7bh[(size_t)k * ntri + t] = T7h[(size_t)k * n * n + ij];
             T7bl[(size_t)k * ntri + t] = T7l[(size_t)k * n * n + ij];
@@ -150,8 +142,6 @@ DevTables* get_dev_tables(int order, int qdeg, std::string& err) {
     if (e == cudaSuccess) e = upload(T7bl, &D->d_T7bl);
     if (e == cudaSuccess) e = upload(Sbh, &D->d_Sbh);
     if (e == cudaSuccess) e = upload(Sbl, &D->d_Sbl);
-    if (e == cudaSuccess) e = upload(T7th, &D->d_T7th);
-    if (e == cudaSuccess) e = upload(T7tl, &D->d_T7tl);
     if (e == cudaSuccess) e = upload(tri, &D->d_tri);
     if (e == cudaSuccess) e = upload(T7h, &D->d_T7h);
     if (e == cudaSuccess) e = upload(T7l, &D->d_T7l);

@@ -386,9 +386,7 @@ struct DevTables {                     // device copies of the reference tables
     float* d_Sf = nullptr;
     float* d_T7h = nullptr;            // df64 split of T7: hi = fl32(T), lo = fl32(T - hi)
     float* d_T7l = nullptr;
-    float* d_T7th = nullptr;           // the same split in upper-triangle order: 7 x n(n+1)/2
-    float* d_T7tl = nullptr;
-    uint16_t* d_tri = nullptr;         // n x n: (i, j) -> upper-triangle index of (min, max)
+    uint16_t* d_tri = nullptr;         // n x n: (i, j) -> place of (min, max) in entry_order
     bool closed = false;               // closed.cuh's closed form equals these tensors
     bool closed_el = false;            // the gradient tensors S are the exact integrals (P1, P2)
     float* d_T7bh = nullptr;           // the split in the two-phase element buffer's order (entry_order)

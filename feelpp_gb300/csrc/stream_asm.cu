@@ -189,9 +189,8 @@ struct StreamSmem {
     static constexpr size_t tab_bytes = (size_t)((14 * NTRI + 3) & ~3) * 4;
     static constexpr size_t tri_bytes = (size_t)((N * N + 7) & ~7) * 2;
     __host__ __device__ static size_t acc_bytes(int maxrow) { return ((size_t)kWarps * RPW * maxrow * VB + 15) & ~(size_t)15; }
-    static constexpr size_t region_bytes() {
-        return (size_t)kEC * 64 > (size_t)CAP * PER_INC ? (size_t)kEC * 64 : (size_t)CAP * PER_INC;
-    }
+    static constexpr size_t task_bytes = (size_t)kEC * 64 + (N == 10 ? kEC * 11 * VB : N == 4 ? kEC * 10 * VB : 0);   // records, closed form's stage
+    static constexpr size_t region_bytes() { return task_bytes > (size_t)CAP * PER_INC ? task_bytes : (size_t)CAP * PER_INC; }
     static size_t bytes(int maxrow) { return tab_bytes + tri_bytes + acc_bytes(maxrow) + region_bytes(); }
 };
 
@@ -272,13 +271,24 @@ __global__ void __launch_bounds__(kThreads, 3) stream_assemble_kernel(StreamArgs
             const int t0 = EPW > 1 ? lane - esub * NTRI : lane;
             const int64_t slot0 = e0 & a.ring_mask;
             if constexpr (N <= 10) {
-                if (a.closed && tid < cnt) {
-                    // the two-phase kernel's closed form (same bits), one lane per element
-                    closed_entries<MODE, N>(reinterpret_cast<const float4*>(rec + 16 * tid), [&](auto I, VT v) {
-                        constexpr EntryOrder O = make_entry_order(4, N == 10 ? 2 : 1, N);
-                        constexpr int i = O.a[decltype(I)::value], j = O.b[decltype(I)::value], tt = i * N - i * (i - 1) / 2 + j - i;
-                        st_keep(reinterpret_cast<VT*>(a.ring) + (slot0 + tid) * NTRI + tt, v, keep);
-                    });
+                if (a.closed) {
+                    // the two-phase kernel's closed form (same bits), one lane per element; a warp's values leave through
+                    // shared memory, CH entries of each element at a time: the ring takes runs of CH values instead of
+                    // single ones N (N + 1) / 2 apart (P2 28^3 binary32 174 -> 124 us, FP64 210 -> 165)
+                    constexpr int CH = N == 10 ? 11 : 10;
+                    VT* const st = reinterpret_cast<VT*>(region + (size_t)kEC * 64) + warp * 32 * CH;
+                    VT* const out = reinterpret_cast<VT*>(a.ring) + (slot0 + warp * 32) * NTRI;
+                    const int live = min(32, cnt - warp * 32);
+                    if (live > 0)
+                        closed_entries<MODE, N>(reinterpret_cast<const float4*>(rec + 16 * min(tid, cnt - 1)), [&](auto I, VT v) {
+                            constexpr int t = decltype(I)::value, c = t % CH;
+                            st[lane * CH + c] = v;
+                            if constexpr (c == CH - 1) {
+                                __syncwarp();
+                                for (int k = lane; k < live * CH; k += 32) st_keep(out + (k / CH) * NTRI + (t - c) + k % CH, st[k], keep);
+                                __syncwarp();
+                            }
+                        });
                 }
             }
             if (!a.closed)
@@ -624,8 +634,8 @@ static int run_streamed(fgpu_ctx* ctx, fgpu_matrix* A, const DevTables* tab, con
     args.inc_ptr = V->d_inc_ptr;
     args.inc = V->d_inc;
     args.pos = V->d_pos;
-    args.Th = tab->d_T7th;                  // binary32 matrices use the high parts (fl32 of the tensors)
-    args.Tl = tab->d_T7tl;
+    args.Th = tab->d_T7bh;                  // binary32 matrices use the high parts (fl32 of the tensors)
+    args.Tl = tab->d_T7bl;
     args.tri = tab->d_tri;
     args.closed = tab->closed;
     args.ring = A->d_kbuf;
