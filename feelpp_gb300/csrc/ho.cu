@@ -241,12 +241,12 @@ constexpr int bary_product(int i, int k, int j, int m) {
 //    columns, c_0 = -(c_1 + c_2 + c_3)), a vertex function has one derivative and an edge function two, so
 //    the 55 stiffness entries take 129 products per point (3 x 3 reference gradients: 220, and 90 for W).
 //  * An entry is a compensated dot product over the points (df_dot_term): 110 registers of accumulators,
-//    so eight warps per SM, whose independent chains keep the pipes busy. The four warps of a block take
-//    every fourth point of the same 32 elements and add their sums in warp order at the end: a block per
+//    so eight warps per SM, whose independent chains keep the pipes busy. The W warps of a block take
+//    every W-th point of the same 32 elements and add their sums in warp order at the end: a block per
 //    SM slot lasts a quarter as long as a warp per 32 elements would and the last wave costs little
 //    (P2 32^3: 5.05 waves took the time of 6).
-template <int N>
-__global__ void __launch_bounds__(128, 2) ho_lane_kernel(int64_t nt, const double* __restrict__ xyz, const int32_t* __restrict__ tets,
+template <int N, int W>
+__global__ void __launch_bounds__(32 * W, 8 / W) ho_lane_kernel(int64_t nt, const double* __restrict__ xyz, const int32_t* __restrict__ tets,
                                                          const double* __restrict__ ho, int Q, const float2* __restrict__ tabg,
                                                          const double* __restrict__ d_kappa, double kappa, double mass,
                                                          const double* __restrict__ kscale, float2* __restrict__ kbuf,
@@ -256,7 +256,7 @@ __global__ void __launch_bounds__(128, 2) ho_lane_kernel(int64_t nt, const doubl
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float2* tab = smem;                            // Q x S
     float2* geo = smem + Q * S + lane;             // 27 values per element, 32 apart: A_c[r], h_cd[r]
-    for (int k = threadIdx.x; k < Q * S; k += 128) tab[k] = tabg[k];
+    for (int k = threadIdx.x; k < Q * S; k += 32 * W) tab[k] = tabg[k];
     const int64_t e0 = (int64_t)blockIdx.x * 32;
     const bool live = e0 + lane < nt;
     const int64_t e = live ? e0 + lane : nt - 1;   // lanes past the end repeat the last element and store nothing
@@ -289,7 +289,7 @@ __global__ void __launch_bounds__(128, 2) ho_lane_kernel(int64_t nt, const doubl
     for (int t = 0; t < NTRI; ++t) s[t] = er[t] = 0.0f;
     bool bad = false;
 #pragma unroll 1
-    for (int q = warp; q < Q; q += 4) {
+    for (int q = warp; q < Q; q += W) {
         const float2* P = tab + q * S;
         df g[10], m;
         {
@@ -359,30 +359,39 @@ __global__ void __launch_bounds__(128, 2) ho_lane_kernel(int64_t nt, const doubl
         });
     }
     if (bad && live) atomicOr(status, kStatusBadElement);
-    // the four warps' sums, in warp order (over the tables and the geometry)
+    // the warps' sums, in warp order (over the tables and the geometry)
     __syncthreads();
 #pragma unroll
     for (int t = 0; t < NTRI; ++t) smem[(warp * NTRI + t) * 33 + lane] = dfpack(quick_two_sum(s[t], er[t]));
     __syncthreads();
     const int cnt = (int)(nt - e0 < 32 ? nt - e0 : 32) * NTRI;
-    for (int k = threadIdx.x; k < cnt; k += 128) {
+    for (int k = threadIdx.x; k < cnt; k += 32 * W) {
         const int el = k / NTRI, t = k - el * NTRI;
         df v = dfun(smem[t * 33 + el]);
 #pragma unroll
-        for (int w = 1; w < 4; ++w) v = df_add(v, dfun(smem[(w * NTRI + t) * 33 + el]));
+        for (int w = 1; w < W; ++w) v = df_add(v, dfun(smem[(w * NTRI + t) * 33 + el]));
         kbuf[e0 * NTRI + k] = dfpack(v);
     }
 }
 
-template <int N>
+template <int N, int W>
 int launch_ho_lane(fgpu_ctx* ctx, fgpu_matrix* A, const HoTables* T, const double* d_kappa, const fgpu_form_desc* f) {
     const fgpu_mesh* M = A->space->mesh;
-    auto kern = ho_lane_kernel<N>;
-    const int smem = std::max(T->Q * lane_stride(N) + 27 * 32, 4 * 33 * (N * (N + 1) / 2)) * (int)sizeof(float2);
+    auto kern = ho_lane_kernel<N, W>;
+    const int smem = std::max(T->Q * lane_stride(N) + 27 * 32, W * 33 * (N * (N + 1) / 2)) * (int)sizeof(float2);
     FGPU_CUDA_CHECK(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    kern<<<(int)((M->nt + 31) / 32), 128, smem, ctx->stream>>>(M->nt, M->d_xyz, M->d_tets, M->d_ho, T->Q, T->d_lane, d_kappa, f->kappa,
-                                                                f->mass, f->kappa_scale, (float2*)A->d_kbuf, ctx->d_status);
+    kern<<<(int)((M->nt + 31) / 32), 32 * W, smem, ctx->stream>>>(M->nt, M->d_xyz, M->d_tets, M->d_ho, T->Q, T->d_lane, d_kappa, f->kappa,
+                                                                   f->mass, f->kappa_scale, (float2*)A->d_kbuf, ctx->d_status);
     return FGPU_OK;
+}
+// Eight warps a block while every block has an SM to itself: the kernel then lasts as long as one warp's points (a P2
+// pass over 162 to 4374 elements: 67 to 74 us with four warps, 50 with eight; 6000 elements, four 75).
+template <int N>
+int launch_ho_lane(fgpu_ctx* ctx, fgpu_matrix* A, const HoTables* T, const double* d_kappa, const fgpu_form_desc* f) {
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+    if ((A->space->mesh->nt + 31) / 32 <= sms) return launch_ho_lane<N, 8>(ctx, A, T, d_kappa, f);
+    return launch_ho_lane<N, 4>(ctx, A, T, d_kappa, f);
 }
 
 // LPG lanes per element (32: one element per warp; 8: four elements per warp, for at most 8 points)
