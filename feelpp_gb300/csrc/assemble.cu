@@ -1950,16 +1950,24 @@ static int run_el_two_phase(fgpu_ctx* ctx, fgpu_matrix* A, const DevTables* tab,
         int rc = launch_build_gather_map(ctx, V);
         if (rc) return rc;
     }
+    const size_t need = (size_t)nt * NTRI * 9 * (MODE == kModeDF64 ? 8 : 4);
+    // (captured once the matrix has been assembled in two phases, by whichever rule)
+    const bool assembled = A->assembled_fused || A->kbuf_bytes >= need;
     if (tab->closed_el) {                        // blocks formed from the barycentric gradients inside the gather
-        if (ctx->capturing && !A->assembled_fused) { ctx->err = "two-phase assembly: assemble once before capturing"; return FGPU_ERR_INVALID; }
+        if (ctx->capturing && !assembled) { ctx->err = "two-phase assembly: assemble once before capturing"; return FGPU_ERR_INVALID; }
         A->assembled_fused = true;
         return launch_gather_elasticity_fused(ctx, A, lam, mu, rec, accumulate);
     }
     int rc = launch_geometry_el_df(ctx, V->mesh, lam, mu, rec);
     if (rc) return rc;
-    const size_t need = (size_t)nt * NTRI * 9 * (MODE == kModeDF64 ? 8 : 4);
     if (A->kbuf_bytes < need) {
-        if (ctx->capturing) { ctx->err = "two-phase assembly: assemble once before capturing (element buffer)"; return FGPU_ERR_INVALID; }
+        // assembled by an exact rule so far: the element buffer is allocated beside the capture
+        struct Relaxed {
+            cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+            Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+            ~Relaxed() { cudaThreadExchangeStreamCaptureMode(&mode); }
+        } relaxed;
+        if (ctx->capturing && !assembled) { ctx->err = "two-phase assembly: assemble once before capturing (element buffer)"; return FGPU_ERR_INVALID; }
         cudaFree(A->d_kbuf);
         A->d_kbuf = nullptr;
         A->kbuf_bytes = 0;
