@@ -81,6 +81,7 @@ SIGNATURES = {
     "fgpu_destroy": (i32, [P]),
     "fgpu_last_error": (C.c_char_p, [P]),
     "fgpu_sync": (i32, [P]),
+    "fgpu_release_scratch": (i32, [P]),
     "fgpu_launch_count": (i64, [P]),
     "fgpu_mesh_upload": (i32, [P, i64, P, i64, P, PP]),
     "fgpu_mesh_upload_hex": (i32, [P, i64, P, i64, P, PP]),

@@ -205,6 +205,13 @@ int fgpu_sync(fgpu_ctx* ctx) {
     return finish(ctx, true);
 }
 
+int fgpu_release_scratch(fgpu_ctx* ctx) {
+    if (!ctx) return FGPU_ERR_INVALID;
+    FGPU_NO_CAPTURE(ctx, "release_scratch");
+    pool_trim(ctx->stream);
+    return FGPU_OK;
+}
+
 int64_t fgpu_launch_count(const fgpu_ctx* ctx) { return ctx ? ctx->launches : 0; }
 
 // ---------------------------------------------------------------------------

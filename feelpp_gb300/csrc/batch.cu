@@ -206,7 +206,7 @@ int fgpu_batch_create(fgpu_ctx* ctx, int nprob, fgpu_matrix* const* mats, const 
         }
         size_t free_b = 0, total_b = 0;
         if (cudaMemGetInfo(&free_b, &total_b) != cudaSuccess) { cudaGetLastError(); two_phase = false; }
-        if (need + need / 10 >= free_b) two_phase = false;
+        if (need + need / 10 >= free_b + pool_kept_bytes()) two_phase = false;
     }
     std::vector<int64_t> slice_off(nprob + 1, 0);
     for (int k = 0; k < nprob && two_phase; ++k) {

@@ -518,6 +518,8 @@ int solve_pcg_mixed(fgpu_ctx* ctx, const fgpu_matrix* A64, const fgpu_matrix* A3
 cudaError_t dev_malloc_bytes(void** p, size_t bytes);
 cudaError_t pool_malloc_bytes(cudaStream_t stream, void** p, size_t bytes);
 cudaError_t pool_free(void* p);      // also takes blocks of dev_malloc
+size_t pool_kept_bytes();
+void pool_trim(cudaStream_t stream);
 void pool_release(cudaStream_t stream);
 cudaError_t pinned_malloc_bytes(void** p, size_t bytes);
 void pinned_free(void* p);

@@ -8,7 +8,8 @@
 // cudaStreamLegacy is one handle for a stream of every device (the key holds the device), and cudaStreamPerThread
 // one for a stream of every thread (its blocks are not kept: any thread may free them).
 //
-// Bounded: at most a sixteenth of a device's memory is kept, the rest goes back to the driver at once; a
+// Bounded: at most a sixty-fourth of a device's memory is kept (4.3 GB; CG + AMG at P2 48^3 keeps 1.3 GB, at P3 40^3
+// 3.4), the rest goes back to the driver at once, and pool_trim gives back what is kept for a stream; a
 // context gives its stream's blocks back when it is destroyed; and an allocation that fails, here or in
 // dev_malloc, is tried again after everything kept has been given back. Page-locked host blocks (a few
 // kilobytes for scalars that are read back) are kept in the same way, at most 1 MB. All functions may be
@@ -116,7 +117,7 @@ cudaError_t pool_free(void* p) {
             Device& d = g_device[blk.key.first];
             if (d.limit == 0) {
                 cudaDeviceProp prop{};
-                d.limit = cudaGetDeviceProperties(&prop, blk.key.first) == cudaSuccess ? std::max<size_t>(prop.totalGlobalMem / 16, 1) : 1;
+                d.limit = cudaGetDeviceProperties(&prop, blk.key.first) == cudaSuccess ? std::max<size_t>(prop.totalGlobalMem / 64, 1) : 1;
             }
             if (d.kept + blk.bytes <= d.limit) {
                 g_kept[blk.key].emplace(blk.bytes, p);
@@ -128,19 +129,38 @@ cudaError_t pool_free(void* p) {
     return cudaFree(p);
 }
 
-// the blocks kept for a stream that goes away; blocks still handed out are freed for good when they come back
+// bytes kept on the current device (dev_malloc can have them)
+size_t pool_kept_bytes() {
+    const int dev = current_device();
+    std::lock_guard<std::mutex> lock(g_mutex);
+    return g_device[dev].kept;
+}
+
+// the blocks kept for a stream, back to the driver
+static void take_stream(cudaStream_t stream, std::vector<void*>& out) {
+    for (auto s = g_kept.begin(); s != g_kept.end();) {
+        if (s->first.second != stream) { ++s; continue; }
+        for (auto& b : s->second) {
+            out.push_back(b.second);
+            g_device[s->first.first].kept -= b.first;
+        }
+        s = g_kept.erase(s);
+    }
+}
+void pool_trim(cudaStream_t stream) {
+    std::vector<void*> out;
+    {
+        std::lock_guard<std::mutex> lock(g_mutex);
+        take_stream(stream, out);
+    }
+    give_back(out);
+}
+// the same for a stream that goes away; blocks still handed out are freed for good when they come back
 void pool_release(cudaStream_t stream) {
     std::vector<void*> out;
     {
         std::lock_guard<std::mutex> lock(g_mutex);
-        for (auto s = g_kept.begin(); s != g_kept.end();) {
-            if (s->first.second != stream) { ++s; continue; }
-            for (auto& b : s->second) {
-                out.push_back(b.second);
-                g_device[s->first.first].kept -= b.first;
-            }
-            s = g_kept.erase(s);
-        }
+        take_stream(stream, out);
         for (auto b = g_live.begin(); b != g_live.end();) {
             if (b->second.key.second == stream) b = g_live.erase(b);
             else ++b;

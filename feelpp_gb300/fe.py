@@ -46,6 +46,10 @@ class Environment:
     def sync(self):
         self.check(self.lib.fgpu_sync(self.h))
 
+    def release_scratch(self):
+        """Give the device scratch that solves and AMG set-ups keep back to the driver."""
+        self.check(self.lib.fgpu_release_scratch(self.h))
+
     def launches(self):
         return int(self.lib.fgpu_launch_count(self.h))
 

@@ -209,6 +209,10 @@ int fgpu_create(const fgpu_config* cfg, fgpu_ctx** out);
 int fgpu_destroy(fgpu_ctx* ctx);
 const char* fgpu_last_error(const fgpu_ctx* ctx);
 int fgpu_sync(fgpu_ctx* ctx);
+/* Solves and AMG set-ups keep their device scratch with the context's stream for the next one (at most a
+   sixty-fourth of the device's memory in all; the library's own allocations take it back when they would fail).
+   This gives it back to the driver, for other allocators of the process. */
+int fgpu_release_scratch(fgpu_ctx* ctx);
 /* number of kernels this context has launched so far */
 int64_t fgpu_launch_count(const fgpu_ctx* ctx);
 

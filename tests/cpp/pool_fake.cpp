@@ -85,11 +85,13 @@ int main() {
     // the bound holds for each device by itself
     std::vector<void*> v;
     for (int dev : {0, 1})
-        for (int k = 0; k < 8; ++k) v.push_back(take(a, 256u << 10, dev));
+        for (int k = 0; k < 8; ++k) v.push_back(take(a, 64u << 10, dev));
     for (void* x : v) fgpu::pool_free(x);
     size_t kept[2] = {0, 0};
     for (auto& x : g_blocks) kept[x.second.first] += x.second.second;
-    CHECK(kept[0] > 0 && kept[0] == kept[1] && kept[0] <= (16u << 20) / 16);
+    CHECK(kept[0] > 0 && kept[0] == kept[1] && kept[0] <= (16u << 20) / 64);
+    t_device = 1;
+    CHECK(fgpu::pool_kept_bytes() == kept[1]);
     // an allocation that would fail gets what is kept on its device, and on no other
     t_device = 0;
     void* big = nullptr;
@@ -101,6 +103,18 @@ int main() {
     fgpu::pool_free(big);
     fgpu::pool_release(a);
     CHECK(g_blocks.empty());
+    // given back on request, blocks handed out stay
+    p = take(a, 4096);
+    q = take(a, 8192);
+    fgpu::pool_free(p);
+    fgpu::pool_trim(b);
+    CHECK(g_blocks.count(p) == 1 && fgpu::pool_kept_bytes() == 4096);
+    fgpu::pool_trim(a);
+    CHECK(g_blocks.count(p) == 0 && g_blocks.count(q) == 1 && fgpu::pool_kept_bytes() == 0);
+    fgpu::pool_free(q);
+    CHECK(take(a, 8192) == q);
+    fgpu::pool_free(q);
+    fgpu::pool_release(a);
     // a block still handed out when its stream goes is freed for good
     p = take(a, 4096);
     fgpu::pool_release(a);
