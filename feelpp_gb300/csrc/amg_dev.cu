@@ -1048,8 +1048,8 @@ int launch_spgemm(fgpu_ctx* ctx, const SpgemmArgs& g, const SpgemmTable& t) {
 // step of 16 lanes on rows of 13 entries does as much as two of 8), with 256 slots where a row has many
 // products and 64 else; a level of few rows takes whole warps, its time one row's chain of steps. Rows that
 // do not fit go on to whole warps with the next larger table.
-int spgemm_dev(fgpu_ctx* ctx, const AmgDevCsr& A, const AmgDevCsr& B, AmgDevCsr& C, int* d_status, bool* overflow,
-               const int32_t* agg = nullptr, const double* s0 = nullptr) {
+int spgemm_once(fgpu_ctx* ctx, const AmgDevCsr& A, const AmgDevCsr& B, AmgDevCsr& C, int* d_status, bool* overflow,
+                const int32_t* agg, const double* s0, bool* padded_form) {
     *overflow = false;
     const int64_t n = A.nrows;
     SpgemmTable first = {32, 256, 8};
@@ -1096,7 +1096,8 @@ int spgemm_dev(fgpu_ctx* ctx, const AmgDevCsr& A, const AmgDevCsr& B, AmgDevCsr&
     const int pad = agg ? kAp0T : spgemm_cap(first.tsize, first.group);
     int32_t* pj = nullptr;
     double* pa = nullptr;
-    if (n * pad * 12 <= kPadBytes && n * pad <= 4 * A.nnz) {
+    *padded_form = *padded_form && n * pad * 12 <= kPadBytes && n * pad <= 4 * A.nnz;
+    if (*padded_form) {
         pj = w.get<int32_t>(n * pad);
         pa = pj ? w.get<double>(n * pad) : nullptr;
         if (!pa) pj = nullptr;                   // no room: counted first
@@ -1151,6 +1152,16 @@ int spgemm_dev(fgpu_ctx* ctx, const AmgDevCsr& A, const AmgDevCsr& B, AmgDevCsr&
     if (rc) return rc;
     *overflow = (st & kStOverflow) != 0;
     return FGPU_OK;
+}
+// Where the padded form leaves no room for the product itself, the rows are counted first.
+int spgemm_dev(fgpu_ctx* ctx, const AmgDevCsr& A, const AmgDevCsr& B, AmgDevCsr& C, int* d_status, bool* overflow,
+               const int32_t* agg = nullptr, const double* s0 = nullptr) {
+    bool padded = true;
+    const int rc = spgemm_once(ctx, A, B, C, d_status, overflow, agg, s0, &padded);
+    if (!padded || (rc != FGPU_ERR_ALLOC && !(rc == FGPU_ERR_CUDA && cudaPeekAtLastError() == cudaErrorMemoryAllocation))) return rc;
+    cudaGetLastError();
+    padded = false;
+    return spgemm_once(ctx, A, B, C, d_status, overflow, agg, s0, &padded);
 }
 
 int seg_sort(fgpu_ctx* ctx, int64_t n, const uint32_t* off32, const int64_t* off64, int32_t* key, double* val, int* d_status) {
