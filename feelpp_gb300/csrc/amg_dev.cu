@@ -1047,7 +1047,10 @@ int launch_spgemm(fgpu_ctx* ctx, const SpgemmArgs& g, const SpgemmTable& t) {
 // Table and lanes per row: the first pass takes 8 lanes up to a mean of 8 entries in B's rows, else 16 (a
 // step of 16 lanes on rows of 13 entries does as much as two of 8), with 256 slots where a row has many
 // products and 64 else; a level of few rows takes whole warps, its time one row's chain of steps. Rows that
-// do not fit go on to whole warps with the next larger table.
+// do not fit go on to whole warps with the next larger table. Neither line is sharp (prolongation and Galerkin
+// products of a set-up, ms): 64 slots up to 512 products a row P2 48^3 5.3, P1 64^3 1.9, rigid body modes P2 16^3
+// 20.4, the same from 200 to 800; never 7.0 / 2.1 / 20.4, up to 2000 5.3 / 2.2 / 22.0. Groups from 4096 rows P2 48^3
+// 5.3, P3 24^3 4.7, from 1024 5.3 / 4.8, 8192 5.3 / 4.7, 16384 5.4 / 4.7, always whole warps 10.4 / 6.6.
 int spgemm_once(fgpu_ctx* ctx, const AmgDevCsr& A, const AmgDevCsr& B, AmgDevCsr& C, int* d_status, bool* overflow,
                 const int32_t* agg, const double* s0, bool* padded_form) {
     *overflow = false;
@@ -1213,8 +1216,8 @@ int transpose_dev(fgpu_ctx* ctx, const AmgDevCsr& M, AmgDevCsr& T, int* d_status
     return FGPU_OK;
 }
 
-// lambda_max(D^-1 A) by Lanczos on its own stream, driven by its own host thread (it runs while the
-// host aggregates); the same arithmetic as the host set-up's estimate
+// lambda_max(D^-1 A) by Lanczos on its own stream, driven by its own host thread (it runs beside the
+// aggregation and the first products); the same arithmetic as the host set-up's estimate
 struct LanczosJob {
     int64_t n = 0;
     const int64_t* ia = nullptr;
@@ -1260,7 +1263,7 @@ struct LanczosJob {
     }
 };
 
-// One level on the device: lambda_max, strength graph, aggregation (host), P, R, A_c = R (A P).
+// One level on the device: lambda_max, strength graph, aggregation, P, R, A_c = R (A P).
 // *handoff: the level goes to the host set-up instead (a row beyond a kernel's capacity, or nothing
 // to coarsen); *last: the coarsening stagnates and A_c is the coarsest operator.
 int level_dev(fgpu_ctx* ctx, AmgDevLevel& L, const AmgHostCfg& cfg, const AmgNns* nns, AmgNns* next, int* d_status, AmgDevCsr& Ac,

@@ -222,7 +222,6 @@ int fgpu_batch_create(fgpu_ctx* ctx, int nprob, fgpu_matrix* const* mats, const 
             if (dev_malloc(&A->d_kbuf, kb) != cudaSuccess) { cudaGetLastError(); two_phase = false; break; }
             A->kbuf_bytes = kb;
         }
-        probs[k].nnz = A->pattern->nnz;
         probs[k].plan = V->plan;
         probs[k].kbuf = A->d_kbuf;
         slice_off[k + 1] = slice_off[k] + V->plan.nslices;

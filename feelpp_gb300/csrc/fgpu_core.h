@@ -484,7 +484,6 @@ struct BatchProblem {
     float4* rec;                     // coefficient records (the matrix's d_coef)
     void* val;                       // matrix values
     // two-phase batches
-    int64_t nnz;                     // CSR entries
     GatherPlan plan;                 // the space's gather map
     void* kbuf;                      // the matrix's element buffer
 };
