@@ -617,8 +617,8 @@ def run_gb300(args, rank, world, local):
 
     def e2e_step():
         # one reference-facing call with host buffers: coordinates and kappa up, values down (page-locked
-        # values buffer: the gather kernel stores each value to device and host memory; "copy": the
-        # gather of each quarter of the entries overlaps the copy-engine transfer of the previous one)
+        # values buffer; the gather runs in parts, and the rows that no later part writes to leave by the
+        # copy engine meanwhile)
         env.check(lib.fgpu_mesh_set_coords(M.h, C.c_void_p(h_xyz.data_ptr())))
         env.check(lib.fgpu_assemble_matrix_host(env.h, a.h, C.byref(desc_h), C.c_void_p(h_vals.data_ptr())))
 

@@ -1358,7 +1358,7 @@ __device__ __forceinline__ void tri_group_entries(void* __restrict__ kbuf, int64
     }
 }
 
-// ---- two-phase batches: the element kernel and the gather-map kernel of the
+// ---- two-phase batches: the element kernels and the sliced gather of the
 // single-problem path over all problems (same per-entry arithmetic and order,
 // so each matrix gets the bits FGPU_ALGO_TWO_PHASE gives it alone) ----
 // the P1 and P2 problems of a batch (grp_off counts their groups only): the single-problem kernel's groups
@@ -1494,13 +1494,13 @@ int launch_batch_gather(fgpu_ctx* ctx, int nprob, const BatchProblem* d_probs, c
 
 // ---------------------------------------------------------------------------
 // Two-phase assembly.
-//   Phase 1 (element_tri_kernel): each element matrix is computed once, as its
+//   Phase 1 (element_closed_kernel, below, or element_tri_kernel): each element matrix is computed once, as its
 //   upper triangle (NTRI = n (n + 1) / 2 entries; the reference tensors are
-//   exactly symmetric), into a device buffer; each warp forms the coefficient
+//   exactly symmetric), into a device buffer; in element_tri_kernel each warp forms the coefficient
 //   records of 32 elements (one per lane, in shared memory), then their
 //   matrices with lanes over entries, contiguous writes.
 //   Phase 2 (gather.cu): one lane per pair of dofs sums its contributions in
-//   element order through a gather map built once per space, which is the
+//   element order by a plan built once per space, which is the
 //   order in which the reference's element loop adds element blocks into the
 //   matrix (bilinearformcontext.hpp:784-847 -> MatSetValues ADD_VALUES).
 //   No float atomics.

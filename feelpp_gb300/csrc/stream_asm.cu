@@ -2,9 +2,9 @@
 //
 // The two-phase assembly (assemble.cu) computes every element matrix once into
 // a T x n(n+1)/2 element buffer in device memory, then sums each CSR entry's
-// contributions in element order through a gather map of T n^2 indices. Both
-// buffers make it move about three times the algorithmic bytes of an assembly
-// (CSR values written once, pattern and element data read once).
+// contributions in element order by the plan of gather.cu. Buffer and plan make
+// it move about twice the algorithmic bytes of an assembly (CSR values written
+// once, pattern and element data read once).
 //
 // This kernel does the same arithmetic in the same order, so its values are
 // bit-identical to the two-phase path, without either buffer:
